@@ -684,7 +684,7 @@ extern "C" ZIM_API zim_status zim_batch_submit(zim_batch* b, const zim_batch_pai
         b->groute[i].on = f.use_sor || f.use_mls || f.use_metric_gaussian;
         if (b->groute[i].on) {
             const zim_rect_state& C = b->calibs[b->pairs[i].calib];
-            lane_scratch = std::max(lane_scratch, zim_grid_scratch_bytes((size_t)C.rect_w * C.rect_h) + 4096);
+            lane_scratch = std::max(lane_scratch, zim_grid_scratch_bytes(C.rect_h, C.rect_w, zim_rays_from(C.Q, C.R1, true, 0, 0).valid != 0) + 4096);
             n_filtered++;
         }
     }

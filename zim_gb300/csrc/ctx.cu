@@ -249,7 +249,7 @@ size_t pair_scratch_bytes(const zim_ctx* ctx, const zim_recon_config* r, int row
     if (need_disp) b += zim_align256(dst * 4);
     b += 2 * (zim_align256(dst * 12) + zim_align256(dst));
     if (r->use_mls) b += zim_align256(dst * 12);
-    if (r->use_sor || r->use_metric_gaussian) b += zim_grid_scratch_bytes(dst);
+    if (r->use_sor || r->use_metric_gaussian) b += zim_grid_scratch_bytes(ctx->rect_h, ctx->rect_w, zim_rays_of(ctx, true, 0, 0).valid != 0);
     if (host) b += 2 * zim_align256((size_t)frames * src * sample_bytes);
     return b + 4096;
 }

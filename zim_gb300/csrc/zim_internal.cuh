@@ -155,6 +155,7 @@ struct zim_rect_state {
 zim_status zim_rect_build(zim_ctx* ctx, const zim_stereo_calib* c, int use_full_left, zim_rect_state& st);
 void zim_rect_free(zim_rect_state& st);
 
-// Scratch bytes needed by the grid filters for n points.
-size_t zim_grid_scratch_bytes(size_t n_points);
+// Scratch bytes needed by the whole-cloud filters (SOR, metric Gaussian) of a
+// rows x cols cloud, with or without pixel rays.
+size_t zim_grid_scratch_bytes(int rows, int cols, bool rays);
 size_t zim_mls_scratch_bytes(size_t n_points);
