@@ -63,3 +63,22 @@ def test_tree_searches_match_brute_force(native, rows, cols, fill, rays):
     tol = 1e-5 + 2 * np.spacing(np.abs(ref).max(axis=1, keepdims=True).astype(np.float32))
     assert (np.abs(got - ref) <= tol)[sure].all()
     assert ctx.check_device() == 0
+
+
+@pytest.mark.parametrize("rows,cols", SIZES[1:])
+@pytest.mark.parametrize("window,sigma,order,radius", [(1, 1.0, 1, 0.0), (5, 1.0, 2, 0.0), (13, 2.0, 0, 0.0),
+                                                       (30, 1.2, 1, 0.0), (30, 6.0, 2, 16.0), (40, 1.5, 2, 4.0)])
+def test_mls_ray_window_equals_full_window(native, rows, cols, window, sigma, order, radius):
+    """The ray bound only leaves out pixels beyond the cut-off, staged in shared
+    memory or read from global memory: the same bits as the full window (the
+    cloud padded by an invalid column has no pixel rays)."""
+    from zim_gb300 import api
+    xyz, mask = _cloud(rows, cols, 0.95, 77 * rows + cols)
+    xp = np.zeros((rows, cols + 1, 3), np.float32)
+    mp = np.zeros((rows, cols + 1), np.uint8)
+    xp[:, :cols], mp[:, :cols] = xyz, mask
+    args = (window, sigma, order, radius, 2)
+    a = api.filter_mls(_context(rows, cols, True), torch.from_numpy(xyz).cuda(), torch.from_numpy(mask).cuda(), *args)
+    b = api.filter_mls(_context(rows, cols, False), torch.from_numpy(xp).cuda(), torch.from_numpy(mp).cuda(), *args)
+    assert torch.equal(a, b[:, :cols].contiguous())
+    assert not torch.equal(a.cpu(), torch.from_numpy(xyz))

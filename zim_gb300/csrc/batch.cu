@@ -386,6 +386,7 @@ zim_status lane_filters(zim_batch* b, int pi, zim_ctx* lctx, cudaStream_t st) {
                                       r.mls_polynomial_order, r.mls_max_radius, r.mls_iterations, ox, g.mls_tmp, rays,
                                       st);
         if (s) return s;
+        zim_scratch_reset(lctx);
         cx = ox;
     }
     if (r.use_metric_gaussian) {

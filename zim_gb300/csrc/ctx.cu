@@ -248,7 +248,7 @@ size_t pair_scratch_bytes(const zim_ctx* ctx, const zim_recon_config* r, int row
     b += zim_align256(dst * 4);
     if (need_disp) b += zim_align256(dst * 4);
     b += 2 * (zim_align256(dst * 12) + zim_align256(dst));
-    if (r->use_mls) b += zim_align256(dst * 12);
+    if (r->use_mls) b += zim_align256(dst * 12) + zim_mls_scratch_bytes(ctx->rect_h, ctx->rect_w);
     if (r->use_sor || r->use_metric_gaussian) b += zim_grid_scratch_bytes(ctx->rect_h, ctx->rect_w, zim_rays_of(ctx, true, 0, 0).valid != 0);
     if (host) b += 2 * zim_align256((size_t)frames * src * sample_bytes);
     return b + 4096;
@@ -372,6 +372,7 @@ static zim_status run_pair(zim_ctx* ctx, const zim_decode_config* d, const zim_r
                            r->mls_max_radius, r->mls_iterations, ox, B.mls_tmp,
                            zim_rays_of(ctx, r->use_rectified_coords != 0, 0, 0), st);
         if (s) return s;
+        ctx->scratch_used = grid_mark;
         cx = ox;
     }
     if (on[ST_MG]) {

@@ -13,7 +13,7 @@
 // query point, which keeps FP32 sums at millimetre scale.
 #include <cmath>
 
-#include "zim_tiles.cuh"
+#include "zim_leaf.cuh"
 
 namespace {
 
@@ -332,8 +332,9 @@ __device__ __forceinline__ void mls_solve_project(const MlsFrame& F, int cur, co
 
 // MLS of one valid point.  visit(fn) calls fn((dx, dy), dz) with the offset from
 // the query point of every valid neighbour of its window (in a fixed order);
-// the distance test against the cut-off is made here.
-template <typename Visit>
+// the distance test against the cut-off is made here.  ORDER2 false: orders 0 and
+// 1 only, without the second sweep's code and registers.
+template <bool ORDER2 = true, typename Visit>
 __device__ __forceinline__ void mls_point(float inv_2s2, int order, float r2c, Visit visit, float& ox, float& oy,
                                           float& oz, bool& moved) {
     moved = false;
@@ -368,10 +369,12 @@ __device__ __forceinline__ void mls_point(float inv_2s2, int order, float r2c, V
     // Polynomial basis in tangent coordinates scaled by 1/h (h = cut-off
     // radius): the fitted surface is the same, the normal equations are O(1).
     const float is = rsqrtf(r2c);
-    if (F.cur == 2) {
-        float A[6][6], bv[6];
-        fit_normal_equations<6>(visit, kw, r2c, is, ws, C, F, A, bv);
-        mls_solve_project<6>(F, 2, A, bv, is, ox, oy, oz);
+    if (ORDER2 && F.cur == 2) {
+        if constexpr (ORDER2) {
+            float A[6][6], bv[6];
+            fit_normal_equations<6>(visit, kw, r2c, is, ws, C, F, A, bv);
+            mls_solve_project<6>(F, 2, A, bv, is, ox, oy, oz);
+        }
     } else {
         float A[3][3], bv[3];
         fit_normal_equations<3>(visit, kw, r2c, is, ws, C, F, A, bv);
@@ -412,116 +415,179 @@ __global__ void __launch_bounds__(MX* MY) mls_kernel(const float* __restrict__ s
 inline size_t mls_smem_bytes(int hw) { return (size_t)(MX + 2 * hw) * (MY + 2 * hw) * sizeof(float4); }
 
 
-// With pixel rays (rays != 0) each row of the window is cut to the disk beyond
-// which the ray bound puts every point outside the cut-off: the pixels left out
-// would fail the distance test, so the neighbours and their order are those
-// of the full window.  The disk is the largest of the warp's (one loop bound).
-// Every neighbour is a staged pixel, so the bound takes the largest distance of
-// a staged point from its own ray (points smoothed across a depth edge lie far
-// off their rays, but only near the edge).
-// HW: the half-window at compile time (0: the hw argument), which makes the
-// tile width and every neighbour offset constants.
+// Without pixel rays: the whole window.  HW: the half-window at compile time (0:
+// the hw argument), which makes the tile width and every neighbour offset
+// constants.
 template <int HW>
 __global__ void __launch_bounds__(MX* MY) mls_smem_kernel(const float* __restrict__ src,
                                                           const uint8_t* __restrict__ mask, int rows, int cols, int hw_arg,
-                                                          float inv_2s2, int order, float r2c, int rays,
-                                                          zt::RayParams rp, float* __restrict__ dst) {
+                                                          float inv_2s2, int order, float r2c, float* __restrict__ dst) {
     extern __shared__ float4 mls_sp[];
-    __shared__ unsigned warp_dev[MX * MY / 32];
     const int hw = HW ? HW : hw_arg;
     const int TW = MX + 2 * hw, TH = MY + 2 * hw;
     const int gx0 = blockIdx.x * MX - hw, gy0 = blockIdx.y * MY - hw;
-    const int tid = threadIdx.y * MX + threadIdx.x;
-    unsigned tdev = 0u;  // largest ray distance of this thread's staged points (float bits, >= 0)
-    for (int t = tid; t < TW * TH; t += MX * MY) {
+    for (int t = threadIdx.y * MX + threadIdx.x; t < TW * TH; t += MX * MY) {
         const int ty = t / TW, tx = t - ty * TW;
         const int gx = gx0 + tx, gy = gy0 + ty;
         float4 v = make_float4(__int_as_float(0x7fc00000), 0.f, 0.f, 0.f);
         if (gx >= 0 && gy >= 0 && gx < cols && gy < rows) {
             const size_t q = (size_t)gy * cols + gx;
-            if (__ldg(mask + q)) {
-                v = make_float4(__ldg(src + 3 * q), __ldg(src + 3 * q + 1), __ldg(src + 3 * q + 2), 1.f);
-                if (rays) {
-                    float ax, ay, az;
-                    zt::ray_dir(rp, gx, gy, ax, ay, az);
-                    const float d = zt::ray_dev(v.x, v.y, v.z, ax, ay, az);
-                    tdev = max(tdev, __float_as_uint(d == d ? d : INFINITY));  // NaN counts as unbounded
-                }
-            }
+            if (__ldg(mask + q)) v = make_float4(__ldg(src + 3 * q), __ldg(src + 3 * q + 1), __ldg(src + 3 * q + 2), 1.f);
         }
         mls_sp[t] = v;
     }
-    tdev = __reduce_max_sync(0xffffffffu, tdev);
-    if ((tid & 31) == 0) warp_dev[tid >> 5] = tdev;
     __syncthreads();
-#pragma unroll
-    for (int j = 0; j < MX * MY / 32; j++) tdev = max(tdev, warp_dev[j]);
     const int x = blockIdx.x * MX + threadIdx.x, y = blockIdx.y * MY + threadIdx.y;
-    const bool inside = x < cols && y < rows;
+    if (x >= cols || y >= rows) return;
     const int cc = (threadIdx.y + hw) * TW + threadIdx.x + hw;
-    const float4 c = mls_sp[cc];
-    float wr2 = INFINITY;  // squared pixel radius of the warp's disk
-    if (rays) {
-        float rs2 = 0.f;
-        if (inside && c.w != 0.f) {
-            float ax, ay, az;
-            zt::ray_dir(rp, x, y, ax, ay, az);
-            const float an = sqrtf(fmaf(ax, ax, fmaf(ay, ay, az * az)));
-            const float qn = sqrtf(fmaf(c.x, c.x, fmaf(c.y, c.y, c.z * c.z)));
-            const float C = qn * rp.f / an;
-            const float sd = sqrtf(r2c) + zt::ray_dev(c.x, c.y, c.z, ax, ay, az) + __uint_as_float(tdev) + 1e-5f * qn;
-            rs2 = INFINITY;
-            if (C > sd) {
-                const float r = sd * an / (C - sd);
-                rs2 = r * r;
-            }
-        }
-        wr2 = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(rs2)));
-    }
-    if (!inside) return;
     const size_t o = (size_t)y * cols + x;
     const float px = src[3 * o], py = src[3 * o + 1], pz = src[3 * o + 2];
     const float2 npxy = make_float2(-px, -py);  // q - p as q + (-p): the same rounding
     float ox = 0.f, oy = 0.f, oz = 0.f;
     bool moved = false;
-    if (c.w != 0.f) {
+    if (mls_sp[cc].w != 0.f) {
         // invalid and off-image neighbours are NaN and fail the distance test
-        if constexpr (HW >= 1 && HW <= 7) {
-            // half-width of window rows +-i, found once for both sweeps
-            // (warp-uniform; 15 = row skipped)
-            unsigned wpack = 0u;
+        auto visit = [&](auto&& fn) {
+#pragma unroll 1
+            for (int i = -hw; i <= hw; i++)
+                for (int j = -hw; j <= hw; j++) {
+                    const float4 q = mls_sp[cc + i * TW + j];
+                    fn(__fadd2_rn(make_float2(q.x, q.y), npxy), q.z - pz);
+                }
+        };
+        mls_point(inv_2s2, order, r2c, visit, ox, oy, oz, moved);
+    }
+    dst[3 * o] = moved ? px + ox : px;
+    dst[3 * o + 1] = moved ? py + oy : py;
+    dst[3 * o + 2] = moved ? pz + oz : pz;
+}
+
+// With pixel rays: what the cut-off needs is usually a few pixels, whatever the
+// window (the reference's default of 61 x 61 pixels with a 1.8 mm cut-off needs
+// 11 x 11 at 0.38 mm a pixel), so the tile stages only that. The ray bound with the largest ray distance of the window's leaves
+// (zim_leaf.cuh) gives each query a pixel radius; once more with the leaves
+// within the tile's largest radius, and the tile and a halo of that radius go to
+// shared memory.  Beyond MLS_LEAF_R pixels the neighbours are read from global
+// memory instead.  The neighbours and their order are those of the full window.
+// The default parameters (three passes) on a 2448 x 2048 cloud: 4975 us with the
+// whole window staged (two CTAs per SM, 22 staged points per query), 1733 us so;
+// a 15 x 15 window (order 2, 2 mm) takes the same time either way.
+constexpr int MLS_LEAF_R = 12;
+template <bool ORDER2>
+__global__ void __launch_bounds__(MX* MY) mls_leaf_kernel(const float* __restrict__ src,
+                                                          const uint8_t* __restrict__ mask, int rows, int cols, int hw,
+                                                          float inv_2s2, int order, float r2c, zt::RayParams rp,
+                                                          zl::Tree t, float* __restrict__ dst) {
+    constexpr int TMAX = MX + 2 * MLS_LEAF_R, WARPS = MX * MY / 32;
+    __shared__ float4 sp[TMAX * TMAX];
+    __shared__ unsigned s_red[2][WARPS];
+    __shared__ signed char s_w[WARPS][MLS_LEAF_R + 1];
+    const unsigned full = 0xffffffffu;
+    const int tid = threadIdx.y * MX + threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const int x0 = blockIdx.x * MX, y0 = blockIdx.y * MY;
+    const int x = x0 + threadIdx.x, y = y0 + threadIdx.y;
+    const bool inside = x < cols && y < rows;
+    const size_t o = inside ? (size_t)y * cols + x : 0;
+    const bool act = inside && __ldg(mask + o) != 0;
+    const float px = __ldg(src + 3 * o), py = __ldg(src + 3 * o + 1), pz = __ldg(src + 3 * o + 2);
+    // largest value over the block (float bits, >= 0); each use has its own slots
+    auto block_max = [&](unsigned v, unsigned* slots) {
+        v = __reduce_max_sync(full, v);
+        if (lane == 0) slots[wid] = v;
+        __syncthreads();
 #pragma unroll
-            for (int ai = 0; ai <= HW; ai++) {
-                const float rem = wr2 - (float)(ai * ai);
-                const unsigned code =
-                    rem < 0.f ? 15u : (rem < (float)(HW * HW) ? (unsigned)(int)sqrtf(rem) : (unsigned)HW);
-                wpack |= code << (4 * ai);
+        for (int j = 0; j < WARPS; j++) v = max(v, slots[j]);
+        return v;
+    };
+    // largest ray distance of the leaves that the tile dilated by R touches
+    auto leaf_dev = [&](int R) {
+        const int lx0 = max(x0 - R, 0) / zl::LEAF, lx1 = min((x0 + MX - 1 + R) / zl::LEAF, t.lw - 1);
+        const int ly0 = max(y0 - R, 0) / zl::LEAF, ly1 = min((y0 + MY - 1 + R) / zl::LEAF, t.lh - 1);
+        const int nx = lx1 - lx0 + 1, n = nx * (ly1 - ly0 + 1);
+        unsigned d = 0u;
+        for (int e = tid; e < n; e += MX * MY)
+            d = max(d, __float_as_uint(__ldg(t.leaf + 2 * ((size_t)(ly0 + e / nx) * t.lw + lx0 + e % nx) + 1).w));
+        return __uint_as_float(block_max(d, s_red[0]));
+    };
+    float ax, ay, az;
+    zt::ray_dir(rp, x, y, ax, ay, az);
+    const float an = sqrtf(fmaf(ax, ax, fmaf(ay, ay, az * az)));
+    const float qn = sqrtf(fmaf(px, px, fmaf(py, py, pz * pz)));
+    const float C = qn * rp.f / an;
+    const float sd0 = sqrtf(r2c) + zt::ray_dev(px, py, pz, ax, ay, az) + 1e-5f * qn;
+    // squared pixel radius beyond which no window point lies within the cut-off
+    auto radius2 = [&](float dev) {
+        if (!act) return 0.f;
+        const float sd = sd0 + dev;
+        if (!(C > sd)) return INFINITY;
+        const float r = sd * an / (C - sd);
+        return r * r;
+    };
+    int R = hw;
+    float rs2 = 0.f;
+    for (int pass = 0; pass < 2; pass++) {
+        rs2 = radius2(leaf_dev(R));
+        const float br2 = __uint_as_float(block_max(__float_as_uint(rs2), s_red[1]));
+        const int Rn = br2 < (float)(hw * hw) ? (int)sqrtf(br2) : hw;
+        if (Rn >= R) break;
+        R = Rn;
+    }
+    const float wr2 = __uint_as_float(__reduce_max_sync(full, __float_as_uint(rs2)));
+    const bool staged = R <= MLS_LEAF_R;  // uniform over the block
+    const int TW = MX + 2 * R;
+    if (staged) {
+        if (lane <= R) {  // half-width of window rows +-lane, -1: row skipped
+            const float rem = wr2 - (float)(lane * lane);
+            s_w[wid][lane] = rem < 0.f ? -1 : (rem < (float)(hw * hw) ? min((int)sqrtf(rem), R) : R);
+        }
+        for (int e = tid; e < TW * (MY + 2 * R); e += MX * MY) {
+            const int ey = e / TW, gx = x0 - R + (e - ey * TW), gy = y0 - R + ey;
+            const float nan = __int_as_float(0x7fc00000);  // invalid and off-image: the distance test fails
+            float4 v = make_float4(nan, nan, nan, 0.f);
+            if (gx >= 0 && gy >= 0 && gx < cols && gy < rows) {
+                const size_t q = (size_t)gy * cols + gx;
+                const float vx = __ldg(src + 3 * q), vy = __ldg(src + 3 * q + 1), vz = __ldg(src + 3 * q + 2);
+                if (__ldg(mask + q)) v = make_float4(vx, vy, vz, 1.f);
             }
+            sp[e] = v;
+        }
+        __syncthreads();
+    }
+    if (!inside) return;
+    float ox = 0.f, oy = 0.f, oz = 0.f;
+    bool moved = false;
+    if (act) {
+        const float2 npxy = make_float2(-px, -py);  // q - p as q + (-p): the same rounding
+        if (staged) {
+            const float4* c = sp + (threadIdx.y + R) * TW + threadIdx.x + R;
             auto visit = [&](auto&& fn) {
 #pragma unroll 1
-                for (int i = -HW; i <= HW; i++) {
-                    const int w = (int)((wpack >> (4 * (i < 0 ? -i : i))) & 15u);
-                    if (w == 15) continue;
+                for (int i = -R; i <= R; i++) {
+                    const int w = s_w[wid][i < 0 ? -i : i];
+                    const float4* row = c + i * TW;
                     for (int j = -w; j <= w; j++) {
-                        const float4 q = mls_sp[cc + i * TW + j];
+                        const float4 q = row[j];
                         fn(__fadd2_rn(make_float2(q.x, q.y), npxy), q.z - pz);
                     }
                 }
             };
-            mls_point(inv_2s2, order, r2c, visit, ox, oy, oz, moved);
+            mls_point<ORDER2>(inv_2s2, order, r2c, visit, ox, oy, oz, moved);
         } else {
             auto visit = [&](auto&& fn) {
-                for (int i = -hw; i <= hw; i++) {
+#pragma unroll 1
+                for (int i = max(-R, -y); i <= min(R, rows - 1 - y); i++) {
                     const float rem = wr2 - (float)(i * i);
                     if (rem < 0.f) continue;
                     const int w = rem < (float)(hw * hw) ? (int)sqrtf(rem) : hw;
-                    for (int j = -w; j <= w; j++) {
-                        const float4 q = mls_sp[cc + i * TW + j];
-                        fn(__fadd2_rn(make_float2(q.x, q.y), npxy), q.z - pz);
+                    for (int j = max(-w, -x); j <= min(w, cols - 1 - x); j++) {
+                        const size_t q = o + (ptrdiff_t)i * cols + j;
+                        if (!__ldg(mask + q)) continue;
+                        fn(__fadd2_rn(make_float2(__ldg(src + 3 * q), __ldg(src + 3 * q + 1)), npxy),
+                           __ldg(src + 3 * q + 2) - pz);
                     }
                 }
             };
-            mls_point(inv_2s2, order, r2c, visit, ox, oy, oz, moved);
+            mls_point<ORDER2>(inv_2s2, order, r2c, visit, ox, oy, oz, moved);
         }
     }
     dst[3 * o] = moved ? px + ox : px;
@@ -531,7 +597,7 @@ __global__ void __launch_bounds__(MX* MY) mls_smem_kernel(const float* __restric
 
 }  // namespace
 
-size_t zim_mls_scratch_bytes(size_t n_points) { return zim_align256(n_points * 12); }
+size_t zim_mls_scratch_bytes(int rows, int cols) { return zim_leaf_bytes(rows, cols); }
 
 zim_status zim_mls_launch(zim_ctx* ctx, const float* xyz, const uint8_t* mask, int rows, int cols, int window,
                           float sigma, int order, float max_radius, int iterations, float* out, float* tmp,
@@ -545,15 +611,25 @@ zim_status zim_mls_launch(zim_ctx* ctx, const float* xyz, const uint8_t* mask, i
     const bool use_smem = smem <= 96 * 1024;
     auto kern = window == 7 ? mls_smem_kernel<7> : mls_smem_kernel<0>;
     if (use_smem) ZIM_CUDA_TRY(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    const int use_rays = use_smem && rays.valid;
     const zt::RayParams rp = zt::ray_params(rays);
+    const bool leaf = rays.valid != 0;
+    zl::Tree t{};
+    if (leaf) {
+        zim_status s = zim_leaf_carve(ctx, rows, cols, t);
+        if (s) return s;
+    }
     // ping-pong so that the last pass lands in `out`
     const float* in = xyz;
     for (int it = 0; it < n_iter; it++) {
         float* dst = ((n_iter - 1 - it) % 2 == 0) ? out : tmp;
         if (dst == in) return zim_fail(ctx, ZIM_ERR_INVALID_ARG, "MLS in-place not supported");
-        if (use_smem)
-            kern<<<grd, blk, smem, st>>>(in, mask, rows, cols, window, inv_2s2, ord, r2c, use_rays, rp, dst);
+        if (leaf) {
+            zim_status s = zim_leaf_build(ctx, in, mask, rows, cols, &rp, t, st);
+            if (s) return s;
+            auto lk = ord == 2 ? mls_leaf_kernel<true> : mls_leaf_kernel<false>;
+            lk<<<grd, blk, 0, st>>>(in, mask, rows, cols, window, inv_2s2, ord, r2c, rp, t, dst);
+        } else if (use_smem)
+            kern<<<grd, blk, smem, st>>>(in, mask, rows, cols, window, inv_2s2, ord, r2c, dst);
         else
             mls_kernel<<<grd, blk, 0, st>>>(in, mask, rows, cols, window, inv_2s2, ord, r2c, dst);
         ctx->launches += 1;
@@ -572,7 +648,7 @@ extern "C" ZIM_API zim_status zim_filter_mls(zim_ctx* ctx, const float* xyz, con
     if (out == xyz) return zim_fail(ctx, ZIM_ERR_INVALID_ARG, "MLS in-place not supported");
     ZIM_CUDA_TRY(ctx, cudaSetDevice(ctx->device));
     float* tmp = nullptr;
-    zim_status s = zim_scratch_reserve(ctx, zim_mls_scratch_bytes((size_t)rows * cols) + 512);
+    zim_status s = zim_scratch_reserve(ctx, zim_mls_scratch_bytes(rows, cols) + zim_align256((size_t)rows * cols * 12) + 512);
     if (s) return s;
     zim_scratch_reset(ctx);
     if (iterations > 1) tmp = (float*)zim_scratch_take(ctx, (size_t)rows * cols * 12);

@@ -357,7 +357,7 @@ extern "C" ZIM_API zim_status zim_reconstruct_roi(zim_ctx* ctx, const zim_recon_
     const int H = L.height, W = L.width;
     const size_t n = (size_t)H * W;
     size_t need = 2 * zim_align256(n * 4) + 3 * (zim_align256(n * 12) + zim_align256(n)) + 512;
-    if (r->use_mls) need += zim_align256(n * 12);
+    if (r->use_mls) need += zim_align256(n * 12) + zim_mls_scratch_bytes(H, W);
     if (r->use_sor || r->use_metric_gaussian) need += zim_grid_scratch_bytes(H, W, zim_rays_of(ctx, true, 0, 0).valid != 0);
     s = zim_scratch_reserve(ctx, need + 4096);
     if (s) return s;
@@ -435,6 +435,7 @@ extern "C" ZIM_API zim_status zim_reconstruct_roi(zim_ctx* ctx, const zim_recon_
                            r->mls_max_radius, r->mls_iterations, xo, mls_tmp,
                            zim_rays_of(ctx, r->use_rectified_coords != 0, L.x, L.y), st);
         if (s) return s;
+        ctx->scratch_used = grid_mark;
         cx = xo;
     }
     if (r->use_metric_gaussian) {

@@ -158,4 +158,5 @@ void zim_rect_free(zim_rect_state& st);
 // Scratch bytes needed by the whole-cloud filters (SOR, metric Gaussian) of a
 // rows x cols cloud, with or without pixel rays.
 size_t zim_grid_scratch_bytes(int rows, int cols, bool rays);
-size_t zim_mls_scratch_bytes(size_t n_points);
+// Scratch bytes that MLS carves per call, beside the caller's ping-pong cloud.
+size_t zim_mls_scratch_bytes(int rows, int cols);
