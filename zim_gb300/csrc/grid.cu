@@ -948,10 +948,11 @@ __global__ void __launch_bounds__(WT_T) sor_window_kernel(const float* __restric
     md_out[i] = fixed_mean(sum, e, k);
 }
 
-constexpr int FW_CAP = 256;  // tree search: list entries per warp (8 per lane)
+constexpr int FW_CAP = 384;  // tree search: list entries per warp (12 per lane)
+constexpr int TS_LEAVES = 4;  // tree search: leaves read together (at most 256 new entries)
 
 // Smallest list value v with at least K entries <= v (entries: lane j holds
-// keys[r] for r < 8, 0xffffffff = empty; keys are non-negative float bits).
+// keys[r], 0xffffffff = empty; keys are non-negative float bits).
 __device__ __forceinline__ unsigned warp_kth_key(const unsigned (&keys)[FW_CAP / 32], int K) {
     unsigned lo = 0u, hi = 0x7f800000u;  // +inf bits
     while (lo < hi) {
@@ -970,30 +971,31 @@ __device__ __forceinline__ unsigned warp_kth_key(const unsigned (&keys)[FW_CAP /
 // distances below its bound in a list; the bound starts at the window pass's
 // (the root of its heap) or, without one, at the farthest corner of the
 // nearest-cornered node and then leaf that holds k + 1 points, and tightens to
-// the (k + 1)-th smallest held whenever the list fills.  Nodes, then their
-// leaves, then the leaves' pixels are read only where the box lies below the
-// bound.  Work is handed out through an atomic counter.
+// the (k + 1)-th smallest held whenever the list fills.  With pixel rays the
+// bound also limits the search to a rectangle of pixels (the window pass's ray
+// bound with the cloud's largest ray distance).  Nodes, then their leaves, then
+// the leaves' pixels are read only where the box lies below the bound.  Work is
+// handed out through an atomic counter.
 //
-// Bound by latency (a few dozen dependent loads per query), so the loads of a
-// step are issued together and eight CTAs per SM run side by side.  It took the
-// place of a counting-sorted coarse grid with a ring search and an occupied-cell
-// search, whose build alone was eleven launches: the SOR stage of a 640 x 480
-// cloud (k = 50) 305 -> 195 us, of a 1280 x 1024 one (k = 20) 385 -> 235 us, of a
-// 2448 x 2048 one (k = 30) 1033 -> 756 us.
+// Bound by the latency of its dependent loads (one box or pixel access takes
+// ~1000 cycles with eight CTAs per SM), so a step reads four leaves' pixels at
+// once and the rectangle leaves mostly one step of nodes.  It took the place of a
+// counting-sorted coarse grid with a ring search and an occupied-cell search,
+// whose build alone was eleven launches.
 __global__ void __launch_bounds__(TS_WARPS * 32) sor_tree_kernel(const float* __restrict__ xyz,
                                                                  const uint8_t* __restrict__ mask, int rows, int cols,
-                                                                 int k, zl::Tree t,
+                                                                 int k, int rays, RayParams rp, zl::Tree t,
                                                                  const unsigned* __restrict__ deferred,
                                                                  float* __restrict__ md_out,
                                                                  const float* __restrict__ bound,
                                                                  uint32_t* __restrict__ err) {
+    constexpr int NEW = TS_LEAVES * zl::LEAF * zl::LEAF;  // entries a step may add
     __shared__ float lst[TS_WARPS][FW_CAP];
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int K1 = k + 1;
     float* lw = lst[w];
     const unsigned nd = t.head->n_deferred;
-    const int nn = t.nw * t.nh;
     for (;;) {
         unsigned item = 0;
         if (lane == 0) item = atomicAdd(&t.head->next, 1u);
@@ -1009,8 +1011,8 @@ __global__ void __launch_bounds__(TS_WARPS * 32) sor_tree_kernel(const float* __
             thr = above(bound[i]);
         } else {
             unsigned long long best = ~0ull;  // (distance bits, node)
-            for (int n0 = lane; n0 < nn; n0 += 32) {
-                const zl::Box b = zl::load_node(t, n0);
+            for (int n0 = lane; n0 < t.nw * t.nh; n0 += 32) {
+                const zl::Box b = zl::load_box(t.node, n0);
                 if (b.n < (unsigned)K1) continue;
                 const float f = zl::far_d2(b, q);
                 if (f < INFINITY) best = min(best, (unsigned long long)__float_as_uint(f) << 32 | (unsigned)n0);
@@ -1021,10 +1023,30 @@ __global__ void __launch_bounds__(TS_WARPS * 32) sor_tree_kernel(const float* __
                 for (int c = lane; c < zl::FAN * zl::FAN; c += 32) {
                     const int l = zl::child_leaf(t, (int)(unsigned)best, c);
                     if (l < 0) continue;
-                    const zl::Box b = zl::load_leaf(t, l);
+                    const zl::Box b = zl::load_box(t.leaf, l);
                     if (b.n >= (unsigned)K1) fb = min(fb, __float_as_uint(zl::far_d2(b, q)));
                 }
                 thr = above(__uint_as_float(__reduce_min_sync(full, fb)));
+            }
+        }
+        // the nodes of the rectangle of pixels that can hold a point below thr
+        int nx0 = 0, ny0 = 0, nx1 = t.nw - 1, ny1 = t.nh - 1;
+        if (rays) {
+            const int qx = (int)(i % (unsigned)cols), qy = (int)(i / (unsigned)cols);
+            float ax, ay, az;
+            ray_dir(rp, qx, qy, ax, ay, az);
+            const float an = sqrtf(fmaf(ax, ax, fmaf(ay, ay, az * az)));
+            const float qn = sqrtf(fmaf(q[0], q[0], fmaf(q[1], q[1], q[2] * q[2])));
+            const float C = qn * rp.f / an;
+            const float sd = sqrtf(thr) + ray_dev(q[0], q[1], q[2], ax, ay, az) + 2e-5f * qn +
+                             __uint_as_float(t.head->ray_dev_bits);
+            if (C > sd) {
+                const float r = fminf(sd * an / (C - sd) * 1.0001f + 1.f, 1e6f);
+                const int ri = (int)r;
+                nx0 = max(qx - ri, 0) / zl::NODE;
+                ny0 = max(qy - ri, 0) / zl::NODE;
+                nx1 = min((qx + ri) / zl::NODE, nx1);
+                ny1 = min((qy + ri) / zl::NODE, ny1);
             }
         }
         int n = 0;
@@ -1052,10 +1074,13 @@ __global__ void __launch_bounds__(TS_WARPS * 32) sor_tree_kernel(const float* __
             thr = __uint_as_float(kk);
             __syncwarp();
         };
-        for (int n0 = 0; n0 < nn; n0 += 32) {
+        const int rw = nx1 - nx0 + 1, rn = rw * (ny1 - ny0 + 1);
+        for (int n0 = 0; n0 < rn; n0 += 32) {
             float nd2 = INFINITY;
-            if (n0 + lane < nn) {
-                const zl::Box b = zl::load_node(t, n0 + lane);
+            int node = 0;
+            if (n0 + lane < rn) {
+                node = (ny0 + (n0 + lane) / rw) * t.nw + nx0 + (n0 + lane) % rw;
+                const zl::Box b = zl::load_box(t.node, node);
                 if (b.n) nd2 = zl::gap_d2(b, q, q);
             }
             unsigned nm = __ballot_sync(full, nd2 < thr);
@@ -1063,46 +1088,50 @@ __global__ void __launch_bounds__(TS_WARPS * 32) sor_tree_kernel(const float* __
                 const int nb = __ffs(nm) - 1;
                 nm &= nm - 1;
                 if (!(__shfl_sync(full, nd2, nb) < thr)) continue;  // the bound may have moved
+                const int nsel = __shfl_sync(full, node, nb);
                 float ld2[2];
                 int ll[2];
 #pragma unroll
                 for (int h = 0; h < 2; h++) {
-                    ll[h] = zl::child_leaf(t, n0 + nb, lane + 32 * h);
+                    ll[h] = zl::child_leaf(t, nsel, lane + 32 * h);
                     ld2[h] = INFINITY;
                     if (ll[h] >= 0) {
-                        const zl::Box b = zl::load_leaf(t, ll[h]);
+                        const zl::Box b = zl::load_box(t.leaf, ll[h]);
                         if (b.n) ld2[h] = zl::gap_d2(b, q, q);
                     }
                 }
 #pragma unroll
                 for (int h = 0; h < 2; h++) {
-                    unsigned lm = __ballot_sync(full, ld2[h] < thr);
-                    while (lm) {
-                        const int lb = __ffs(lm) - 1;
-                        lm &= lm - 1;
-                        if (!(__shfl_sync(full, ld2[h], lb) < thr)) continue;
-                        const int l = __shfl_sync(full, ll[h], lb);
-                        const int px = (l % t.lw) * zl::LEAF + (lane & 7), py = (l / t.lw) * zl::LEAF + (lane >> 3);
-                        float d2[2];
+                    for (unsigned lm = __ballot_sync(full, ld2[h] < thr); lm; lm &= __ballot_sync(full, ld2[h] < thr)) {
+                        float d2[TS_LEAVES][2];
 #pragma unroll
-                        for (int u = 0; u < 2; u++) {
-                            d2[u] = INFINITY;
-                            const int y = py + 4 * u;
-                            if (px < cols && y < rows) {
-                                const size_t j = (size_t)y * cols + px;
-                                const float x = __ldg(xyz + 3 * j), yy = __ldg(xyz + 3 * j + 1), z = __ldg(xyz + 3 * j + 2);
-                                if (__ldg(mask + j)) d2[u] = sqdist(x - q[0], yy - q[1], z - q[2]);
+                        for (int g = 0; g < TS_LEAVES; g++) {
+                            const int lb = __ffs(lm) - 1;  // -1: none left
+                            lm &= lm - 1;
+                            const int l = __shfl_sync(full, ll[h], lb < 0 ? 0 : lb);
+                            const int px = (l % t.lw) * zl::LEAF + (lane & 7), py = (l / t.lw) * zl::LEAF + (lane >> 3);
+#pragma unroll
+                            for (int u = 0; u < 2; u++) {
+                                d2[g][u] = INFINITY;
+                                const int y = py + 4 * u;
+                                if (lb >= 0 && px < cols && y < rows) {
+                                    const size_t j = (size_t)y * cols + px;
+                                    const float a = __ldg(xyz + 3 * j), b = __ldg(xyz + 3 * j + 1), c = __ldg(xyz + 3 * j + 2);
+                                    if (__ldg(mask + j)) d2[g][u] = sqdist(a - q[0], b - q[1], c - q[2]);
+                                }
                             }
                         }
 #pragma unroll
-                        for (int u = 0; u < 2; u++) {
-                            const bool kp = d2[u] < thr;  // false for NaN
-                            const unsigned bb = __ballot_sync(full, kp);
-                            if (kp) lw[n + __popc(bb & ((1u << lane) - 1u))] = d2[u];
-                            n += __popc(bb);
-                        }
-                        if (n > FW_CAP - 64) {
-                            if (K1 <= FW_CAP - 64) tighten();
+                        for (int g = 0; g < TS_LEAVES; g++)
+#pragma unroll
+                            for (int u = 0; u < 2; u++) {
+                                const bool kp = d2[g][u] < thr;  // false for NaN
+                                const unsigned bb = __ballot_sync(full, kp);
+                                if (kp) lw[n + __popc(bb & ((1u << lane) - 1u))] = d2[g][u];
+                                n += __popc(bb);
+                            }
+                        if (n > FW_CAP - NEW) {
+                            if (K1 <= FW_CAP - NEW) tighten();
                             else n = 0;
                         }
                     }
@@ -1110,7 +1139,7 @@ __global__ void __launch_bounds__(TS_WARPS * 32) sor_tree_kernel(const float* __
             }
         }
         __syncwarp();
-        if (n < K1 || K1 > FW_CAP - 64) {  // fewer than k + 1 finite points (or a k beyond the list)
+        if (n < K1 || K1 > FW_CAP - NEW) {  // fewer than k + 1 finite points (or a k beyond the list)
             if (lane == 0) {
                 atomicOr(err, 0x10u);
                 md_out[i] = 0.f;
@@ -1155,9 +1184,23 @@ __device__ __forceinline__ void comp_add(float& sum, float& comp, float x) {
     sum = t;
 }
 
-constexpr int SOR_STAT_BLOCKS = 608;
+constexpr int SOR_STAT_BLOCKS = 152;
+constexpr int SOR_STAT_STEPS = 4;
 
-// Four pixels per thread and step (md 16-byte, mask 4-byte aligned: vec).  The
+// The sums over a warp of a (in even lanes) and b (in odd lanes): six FP64 adds
+// in place of ten (FP64 adds were half of this kernel's time).
+__device__ __forceinline__ double warp_sum2(double a, double b) {
+    const unsigned full = 0xffffffffu;
+    const bool odd = threadIdx.x & 1;
+    const double other = __shfl_xor_sync(full, odd ? a : b, 1);
+    double v = (odd ? b : a) + other;
+#pragma unroll
+    for (int off = 2; off < 32; off <<= 1) v += __shfl_xor_sync(full, v, off);
+    return v;
+}
+
+// One block per SM, four pixels per thread and step and four steps' loads in
+// flight (md 16-byte, mask 4-byte aligned: vec).  The
 // threshold mean + std_mul * stddev; the classifier compares the float mean
 // distances with thr_f, the largest float <= thr, which decides exactly as
 // (double)md > thr.
@@ -1171,34 +1214,57 @@ __global__ void __launch_bounds__(GB) sor_stats_kernel(const uint8_t* __restrict
         comp_add(as, ac, v);
         comp_add(bs, bc, v * v);  // PCL: float square, double sum
     };
-    for (size_t g = (size_t)blockIdx.x * GB + threadIdx.x; 4 * g < n; g += (size_t)gridDim.x * GB) {
-        if (vec && 4 * g + 4 <= n) {
-            const uchar4 m = __ldg(reinterpret_cast<const uchar4*>(mask) + g);
-            const float4 v = __ldg(reinterpret_cast<const float4*>(md) + g);
-            take(m.x, v.x); take(m.y, v.y); take(m.z, v.z); take(m.w, v.w);
-        } else {
-            for (size_t i = 4 * g; i < n && i < 4 * g + 4; i++) take(mask[i], md[i]);
+    const size_t step = (size_t)gridDim.x * GB, full4 = vec ? n / 4 : 0;
+    size_t g = (size_t)blockIdx.x * GB + threadIdx.x;
+    for (; g < full4; g += SOR_STAT_STEPS * step) {
+        uchar4 m[SOR_STAT_STEPS];
+        float4 v[SOR_STAT_STEPS];
+#pragma unroll
+        for (int u = 0; u < SOR_STAT_STEPS; u++) {
+            m[u] = make_uchar4(0, 0, 0, 0);
+            v[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (g + u * step < full4) {
+                m[u] = __ldg(reinterpret_cast<const uchar4*>(mask) + g + u * step);
+                v[u] = __ldg(reinterpret_cast<const float4*>(md) + g + u * step);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < SOR_STAT_STEPS; u++) {
+            take(m[u].x, v[u].x); take(m[u].y, v[u].y); take(m[u].z, v[u].z); take(m[u].w, v[u].w);
         }
     }
-    double a = block_reduce((double)as + (double)ac, Add(), 0.0);
-    double b = block_reduce((double)bs + (double)bc, Add(), 0.0);
+    for (size_t i = 4 * full4 + (size_t)blockIdx.x * GB + threadIdx.x; i < n; i += step) take(mask[i], md[i]);
+    __shared__ double s_sum[GB / 32][2];
     __shared__ bool last;
-    if (threadIdx.x == 0) {
-        part[2 * blockIdx.x] = a;
-        part[2 * blockIdx.x + 1] = b;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    // a in lane 0, b in lane 1
+    auto block_sum2 = [&](double a, double b) {
+        const double v = warp_sum2(a, b);
+        if (lane < 2) s_sum[w][lane] = v;
+        __syncthreads();
+        double r = 0.0;
+        if (threadIdx.x < 2)
+            for (int j = 0; j < GB / 32; j++) r += s_sum[j][threadIdx.x];
+        __syncthreads();
+        return r;
+    };
+    const double mine = block_sum2((double)as + (double)ac, (double)bs + (double)bc);
+    if (threadIdx.x < 2) {
+        part[2 * blockIdx.x + threadIdx.x] = mine;
         __threadfence();
-        last = atomicAdd(&h->done, 1u) == gridDim.x - 1;
     }
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(&h->done, 1u) == gridDim.x - 1;
     __syncthreads();
     if (!last) return;
     __threadfence();
-    a = b = 0.0;
+    double a = 0.0, b = 0.0;
     for (int i = threadIdx.x; i < (int)gridDim.x; i += GB) {
         a += __ldcg(part + 2 * i);
         b += __ldcg(part + 2 * i + 1);
     }
-    a = block_reduce(a, Add(), 0.0);
-    b = block_reduce(b, Add(), 0.0);
+    a = block_sum2(a, b);
+    b = __shfl_down_sync(0xffffffffu, a, 1);
     if (threadIdx.x == 0) {
         GridStats o{};
         const double nv = (double)h->n_valid;
@@ -1337,13 +1403,12 @@ __global__ void __launch_bounds__(WT_T) mg_window_kernel(const float* __restrict
     const float kq = -1.44269504088896341f * inv2s2;
     float sx = 0.f, sy = 0.f, sz = 0.f, sw = 0.f;
     const int R2 = (int)(rs * rs);  // offsets with dx^2 + dy^2 <= R2 (< (WRG + 1)^2)
+    const int R = min((int)rs, WRG);
 #pragma unroll 1
-    for (int dy = -WRG; dy <= WRG; dy++) {
-        const int rem = R2 - dy * dy;
-        if (rem < 0) continue;
-        // exact floor of the root: a root of a non-square below 64 lies at
-        // least 0.06 from an integer, far beyond the float error
-        const int w = min((int)sqrtf((float)rem), WRG);
+    for (int dy = -R; dy <= R; dy++) {
+        // exact floor of the root: a root of a non-square below 64 lies at least
+        // 0.06 from an integer, and the approximate root's error is far smaller
+        const int w = min((int)(root_approx((float)max(R2 - dy * dy, 0)) + 0.03f), WRG);
         const float4* row = W + wc + dy * GW;
 #pragma unroll 2
         for (int dx = -w; dx <= w; dx++) {
@@ -1415,7 +1480,7 @@ __global__ void __launch_bounds__(MT_WARPS * 32) metric_gaussian_tree_kernel(
         for (int n0 = 0; n0 < nn; n0 += 32) {
             bool hit = false;
             if (n0 + lane < nn) {
-                const zl::Box b = zl::load_node(t, n0 + lane);
+                const zl::Box b = zl::load_box(t.node, n0 + lane);
                 hit = b.n && zl::gap_d2(b, lo, hi) <= r2;
             }
             unsigned nm = __ballot_sync(full, hit);
@@ -1427,7 +1492,7 @@ __global__ void __launch_bounds__(MT_WARPS * 32) metric_gaussian_tree_kernel(
                     const int ll = zl::child_leaf(t, nb, lane + 32 * h);
                     bool lhit = false;
                     if (ll >= 0) {
-                        const zl::Box b = zl::load_leaf(t, ll);
+                        const zl::Box b = zl::load_box(t.leaf, ll);
                         lhit = b.n && zl::gap_d2(b, lo, hi) <= r2;
                     }
                     unsigned lm = __ballot_sync(full, lhit);
@@ -1595,8 +1660,8 @@ zim_status zim_sor_launch(zim_ctx* ctx, const float* xyz, const uint8_t* mask, i
                                                         stats, t.head, md, deferred);
     }
     const unsigned sms = (unsigned)(ctx->sm_count > 0 ? ctx->sm_count : 152);
-    sor_tree_kernel<<<8 * sms, TS_WARPS * 32, 0, st>>>(xyz, mask, rows, cols, mean_k, t, deferred, md, bound,
-                                                       ctx->d_error);
+    sor_tree_kernel<<<8 * sms, TS_WARPS * 32, 0, st>>>(xyz, mask, rows, cols, mean_k, rays.valid, rp, t, deferred,
+                                                       md, bound, ctx->d_error);
     const size_t quads = (n + 3) / 4;
     const uintptr_t mal = (uintptr_t)mask | (uintptr_t)mask_out;
     const int vs = ((uintptr_t)md & 15) == 0 && ((uintptr_t)mask & 3) == 0;

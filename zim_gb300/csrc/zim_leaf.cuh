@@ -17,9 +17,8 @@ namespace zl {
 constexpr int LEAF = 8;             // leaf side in pixels
 constexpr int FAN = 8;              // node side in leaves
 constexpr int NODE = LEAF * FAN;    // node side in pixels
-constexpr int NODE_WORDS = 8;
 
-// Counters of one filter run, zeroed with the nodes before the build.
+// Counters of one filter run, zeroed before the build.
 struct Head {
     unsigned n_valid;       // valid points
     unsigned ray_dev_bits;  // largest distance of a point from its pixel ray (float bits)
@@ -29,10 +28,11 @@ struct Head {
     unsigned pad[3];
 };
 
+// Boxes are two float4 each: (lo, finite points as int bits), (hi, largest ray
+// distance); an empty one has lo = +inf, hi = -inf.
 struct Tree {
     Head* head;
-    unsigned* node;  // NODE_WORDS per node: ~key of the minima, key of the maxima (0: empty), finite points
-    float4* leaf;    // two per leaf: (lo, finite points as int bits), (hi, largest ray distance)
+    float4 *node, *leaf;
     int lw, lh, nw, nh;
 };
 
@@ -48,14 +48,9 @@ struct Box {
     unsigned n;
 };
 
-__device__ __forceinline__ Box load_leaf(const Tree& t, int l) {
-    const float4 a = __ldg(t.leaf + 2 * l), b = __ldg(t.leaf + 2 * l + 1);
+__device__ __forceinline__ Box load_box(const float4* boxes, int i) {
+    const float4 a = __ldg(boxes + 2 * (size_t)i), b = __ldg(boxes + 2 * (size_t)i + 1);
     return Box{{a.x, a.y, a.z}, {b.x, b.y, b.z}, __float_as_uint(a.w)};
-}
-__device__ __forceinline__ Box load_node(const Tree& t, int n) {
-    const uint4* p = reinterpret_cast<const uint4*>(t.node) + 2 * n;
-    const uint4 a = __ldg(p), b = __ldg(p + 1);
-    return Box{{keyf(~a.x), keyf(~a.y), keyf(~a.z)}, {keyf(a.w), keyf(b.x), keyf(b.y)}, b.z};
 }
 
 __device__ __forceinline__ float sq3(float dx, float dy, float dz) { return fmaf(dz, dz, fmaf(dy, dy, dx * dx)); }
