@@ -949,10 +949,13 @@ __global__ void __launch_bounds__(WT_T) sor_window_kernel(const float* __restric
 }
 
 constexpr int FW_CAP = 384;  // tree search: list entries per warp (12 per lane)
+constexpr int TS_QUEUE = 256;  // tree search: queued leaves per warp
 constexpr int TS_LEAVES = 4;  // tree search: leaves read together (at most 256 new entries)
 
 // Smallest list value v with at least K entries <= v (entries: lane j holds
-// keys[r], 0xffffffff = empty; keys are non-negative float bits).
+// keys[r], 0xffffffff = empty; keys are non-negative float bits).  Bisection on
+// the bits that stops at the first split with exactly K entries below it: about
+// as many steps as the entries have bits, the full 31 only among ties.
 __device__ __forceinline__ unsigned warp_kth_key(const unsigned (&keys)[FW_CAP / 32], int K) {
     unsigned lo = 0u, hi = 0x7f800000u;  // +inf bits
     while (lo < hi) {
@@ -961,7 +964,13 @@ __device__ __forceinline__ unsigned warp_kth_key(const unsigned (&keys)[FW_CAP /
 #pragma unroll
         for (int r = 0; r < FW_CAP / 32; r++) c += keys[r] <= mid;
         c = __reduce_add_sync(0xffffffffu, c);
-        if (c >= K) hi = mid;
+        if (c == K) {
+            unsigned m = 0u;
+#pragma unroll
+            for (int r = 0; r < FW_CAP / 32; r++) m = max(m, keys[r] <= mid ? keys[r] : 0u);
+            return __reduce_max_sync(0xffffffffu, m);
+        }
+        if (c > K) hi = mid;
         else lo = mid + 1;
     }
     return lo;
@@ -978,8 +987,9 @@ __device__ __forceinline__ unsigned warp_kth_key(const unsigned (&keys)[FW_CAP /
 // handed out through an atomic counter.
 //
 // Bound by the latency of its dependent loads (one box or pixel access takes
-// ~1000 cycles with eight CTAs per SM), so a step reads four leaves' pixels at
-// once and the rectangle leaves mostly one step of nodes.  It took the place of a
+// ~1000 cycles with eight CTAs per SM) and of its own instructions, so the leaves
+// in question are queued first and read four at a time, those within a third of
+// the bound before the others (they tighten it), and no index is divided.  It took the place of a
 // counting-sorted coarse grid with a ring search and an occupied-cell search,
 // whose build alone was eleven launches.
 __global__ void __launch_bounds__(TS_WARPS * 32) sor_tree_kernel(const float* __restrict__ xyz,
@@ -991,6 +1001,8 @@ __global__ void __launch_bounds__(TS_WARPS * 32) sor_tree_kernel(const float* __
                                                                  uint32_t* __restrict__ err) {
     constexpr int NEW = TS_LEAVES * zl::LEAF * zl::LEAF;  // entries a step may add
     __shared__ float lst[TS_WARPS][FW_CAP];
+    __shared__ int2 qpos[TS_WARPS][TS_QUEUE];   // queued leaves: first pixel
+    __shared__ float qd2[TS_WARPS][TS_QUEUE];   // and squared box distance
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int K1 = k + 1;
@@ -1074,13 +1086,63 @@ __global__ void __launch_bounds__(TS_WARPS * 32) sor_tree_kernel(const float* __
             thr = __uint_as_float(kk);
             __syncwarp();
         };
+        // reads the queued leaves with a box distance in [from, to) and below thr
+        int nq = 0;
+        auto scan = [&](float from, float to) {
+            for (int q0 = 0; q0 < nq; q0 += 32) {
+                const float d = q0 + lane < nq ? qd2[w][q0 + lane] : INFINITY;
+                const bool mine = d >= from && d < to;
+                for (unsigned m = __ballot_sync(full, mine && d < thr); m; m &= __ballot_sync(full, d < thr)) {
+                    float d2[TS_LEAVES][2];
+#pragma unroll
+                    for (int g = 0; g < TS_LEAVES; g++) {
+                        const bool any = m != 0u;
+                        const int2 p0 = qpos[w][q0 + (any ? __ffs(m) - 1 : 0)];
+                        m &= m - 1;
+                        const int px = p0.x + (lane & 7), py = p0.y + (lane >> 3);
+                        const bool in0 = any && px < cols && py < rows, in1 = any && px < cols && py + 4 < rows;
+                        const size_t j = in0 ? (size_t)py * cols + px : 0, j1 = in1 ? j + 4 * (size_t)cols : 0;
+                        const float* a = xyz + 3 * j;
+                        const float* b = xyz + 3 * j1;
+                        const float ax = __ldg(a), ay = __ldg(a + 1), az = __ldg(a + 2);
+                        const float bx = __ldg(b), by = __ldg(b + 1), bz = __ldg(b + 2);
+                        const bool v0 = in0 && __ldg(mask + j) != 0, v1 = in1 && __ldg(mask + j1) != 0;
+                        d2[g][0] = v0 ? sqdist(ax - q[0], ay - q[1], az - q[2]) : INFINITY;
+                        d2[g][1] = v1 ? sqdist(bx - q[0], by - q[1], bz - q[2]) : INFINITY;
+                    }
+#pragma unroll
+                    for (int g = 0; g < TS_LEAVES; g++)
+#pragma unroll
+                        for (int u = 0; u < 2; u++) {
+                            const bool kp = d2[g][u] < thr;  // false for NaN
+                            const unsigned bb = __ballot_sync(full, kp);
+                            if (kp) lw[n + __popc(bb & ((1u << lane) - 1u))] = d2[g][u];
+                            n += __popc(bb);
+                        }
+                    if (n > FW_CAP - NEW) {
+                        if (K1 <= FW_CAP - NEW) tighten();
+                        else n = 0;
+                    }
+                }
+            }
+        };
+        auto flush = [&]() {
+            __syncwarp();
+            const float near = thr < INFINITY ? 0.1f * thr : 0.f;
+            scan(0.f, near);
+            if (n >= K1 && n > 2 * K1 && K1 <= FW_CAP - NEW) tighten();
+            scan(near, INFINITY);
+            __syncwarp();
+            nq = 0;
+        };
         const int rw = nx1 - nx0 + 1, rn = rw * (ny1 - ny0 + 1);
         for (int n0 = 0; n0 < rn; n0 += 32) {
             float nd2 = INFINITY;
-            int node = 0;
+            int nx = 0, ny = 0;
             if (n0 + lane < rn) {
-                node = (ny0 + (n0 + lane) / rw) * t.nw + nx0 + (n0 + lane) % rw;
-                const zl::Box b = zl::load_box(t.node, node);
+                ny = ny0 + (n0 + lane) / rw;
+                nx = nx0 + (n0 + lane) % rw;
+                const zl::Box b = zl::load_box(t.node, ny * t.nw + nx);
                 if (b.n) nd2 = zl::gap_d2(b, q, q);
             }
             unsigned nm = __ballot_sync(full, nd2 < thr);
@@ -1088,56 +1150,32 @@ __global__ void __launch_bounds__(TS_WARPS * 32) sor_tree_kernel(const float* __
                 const int nb = __ffs(nm) - 1;
                 nm &= nm - 1;
                 if (!(__shfl_sync(full, nd2, nb) < thr)) continue;  // the bound may have moved
-                const int nsel = __shfl_sync(full, node, nb);
+                const int lx0 = __shfl_sync(full, nx, nb) * zl::FAN, ly0 = __shfl_sync(full, ny, nb) * zl::FAN;
+                const int lx = lx0 + (lane & 7), ly = ly0 + (lane >> 3);
                 float ld2[2];
-                int ll[2];
 #pragma unroll
                 for (int h = 0; h < 2; h++) {
-                    ll[h] = zl::child_leaf(t, nsel, lane + 32 * h);
                     ld2[h] = INFINITY;
-                    if (ll[h] >= 0) {
-                        const zl::Box b = zl::load_box(t.leaf, ll[h]);
+                    if (lx < t.lw && ly + 4 * h < t.lh) {
+                        const zl::Box b = zl::load_box(t.leaf, (ly + 4 * h) * t.lw + lx);
                         if (b.n) ld2[h] = zl::gap_d2(b, q, q);
                     }
                 }
 #pragma unroll
                 for (int h = 0; h < 2; h++) {
-                    for (unsigned lm = __ballot_sync(full, ld2[h] < thr); lm; lm &= __ballot_sync(full, ld2[h] < thr)) {
-                        float d2[TS_LEAVES][2];
-#pragma unroll
-                        for (int g = 0; g < TS_LEAVES; g++) {
-                            const int lb = __ffs(lm) - 1;  // -1: none left
-                            lm &= lm - 1;
-                            const int l = __shfl_sync(full, ll[h], lb < 0 ? 0 : lb);
-                            const int px = (l % t.lw) * zl::LEAF + (lane & 7), py = (l / t.lw) * zl::LEAF + (lane >> 3);
-#pragma unroll
-                            for (int u = 0; u < 2; u++) {
-                                d2[g][u] = INFINITY;
-                                const int y = py + 4 * u;
-                                if (lb >= 0 && px < cols && y < rows) {
-                                    const size_t j = (size_t)y * cols + px;
-                                    const float a = __ldg(xyz + 3 * j), b = __ldg(xyz + 3 * j + 1), c = __ldg(xyz + 3 * j + 2);
-                                    if (__ldg(mask + j)) d2[g][u] = sqdist(a - q[0], b - q[1], c - q[2]);
-                                }
-                            }
-                        }
-#pragma unroll
-                        for (int g = 0; g < TS_LEAVES; g++)
-#pragma unroll
-                            for (int u = 0; u < 2; u++) {
-                                const bool kp = d2[g][u] < thr;  // false for NaN
-                                const unsigned bb = __ballot_sync(full, kp);
-                                if (kp) lw[n + __popc(bb & ((1u << lane) - 1u))] = d2[g][u];
-                                n += __popc(bb);
-                            }
-                        if (n > FW_CAP - NEW) {
-                            if (K1 <= FW_CAP - NEW) tighten();
-                            else n = 0;
-                        }
+                    const bool hit = ld2[h] < thr;
+                    const unsigned bb = __ballot_sync(full, hit);
+                    if (hit) {
+                        const int at = nq + __popc(bb & ((1u << lane) - 1u));
+                        qpos[w][at] = make_int2(lx * zl::LEAF, (ly + 4 * h) * zl::LEAF);
+                        qd2[w][at] = ld2[h];
                     }
+                    nq += __popc(bb);
                 }
+                if (nq > TS_QUEUE - 64) flush();
             }
         }
+        flush();
         __syncwarp();
         if (n < K1 || K1 > FW_CAP - NEW) {  // fewer than k + 1 finite points (or a k beyond the list)
             if (lane == 0) {
@@ -1184,7 +1222,7 @@ __device__ __forceinline__ void comp_add(float& sum, float& comp, float x) {
     sum = t;
 }
 
-constexpr int SOR_STAT_BLOCKS = 152;
+constexpr int SOR_STAT_BLOCKS = 456;
 constexpr int SOR_STAT_STEPS = 4;
 
 // The sums over a warp of a (in even lanes) and b (in odd lanes): six FP64 adds
@@ -1199,7 +1237,7 @@ __device__ __forceinline__ double warp_sum2(double a, double b) {
     return v;
 }
 
-// One block per SM, four pixels per thread and step and four steps' loads in
+// Three blocks per SM, four pixels per thread and step and four steps' loads in
 // flight (md 16-byte, mask 4-byte aligned: vec).  The
 // threshold mean + std_mul * stddev; the classifier compares the float mean
 // distances with thr_f, the largest float <= thr, which decides exactly as
