@@ -7,8 +7,9 @@
 // JSLAB_PhaseEpipolarReconstructor_V2_GPU.cu:352-480).  Per pair the stages
 // compute exactly what zim_reconstruct_pair computes (the same device code,
 // zim_tiles.cuh); what changes is the schedule:
-//   stage 1  decode:          item = (pair, camera, band of 8-row tile rows)
-//   stage 1b post-smooth of the decoded phase (same items), when configured
+//   stage 1  decode:          a launch per camera
+//   stage 1b post-smooth of the decoded phase, when configured:
+//            item = (pair, camera, band of 8-row tile rows)
 //   stage 2  rectify + match: item = (pair, band of rectified rows); the right
 //            row is rectified straight into shared memory and each left pixel
 //            is rectified in registers, so no rectified phase reaches HBM
@@ -36,7 +37,7 @@ namespace {
 constexpr int BT = 256;  // threads per persistent CTA (one 32 x 8 tile)
 static_assert(BT == zt::DX * zt::DY && BT == zt::RX * zt::RY, "tile shape");
 
-enum { Q_DECODE, Q_SMOOTH, Q_MATCH, Q_REPROJ, Q_PXG, Q_ROR, NQ };
+enum { Q_SMOOTH, Q_MATCH, Q_REPROJ, Q_PXG, Q_ROR, NQ };
 
 struct PairDev {
     zt::DecodeParams dp;
@@ -77,38 +78,6 @@ __device__ __forceinline__ int next_item(unsigned* counter, int* s_item) {
     if (threadIdx.x == 0) *s_item = (int)atomicAdd(counter, 1u);
     __syncthreads();
     return *s_item;
-}
-
-__global__ void __launch_bounds__(BT) batch_decode_kernel(const PairDev* __restrict__ pairs, const int4* __restrict__ items,
-                                                          int n_items, unsigned* __restrict__ counter) {
-    __shared__ zt::DecodeSmem sm;
-    __shared__ zt::DecodeParams dp;
-    __shared__ int s_item;
-    const int tid = threadIdx.x;
-    for (;;) {
-        const int it = next_item(counter, &s_item);
-        if (it >= n_items) break;
-        const int4 w = items[it];  // pair, camera, first tile row, tile rows
-        const PairDev& P = pairs[w.x];
-        {
-            const int* src = reinterpret_cast<const int*>(&P.dp);
-            int* dst = reinterpret_cast<int*>(&dp);
-            for (int k = tid; k < (int)(sizeof(zt::DecodeParams) / 4); k += BT) dst[k] = __ldg(src + k);
-        }
-        __syncthreads();
-        const int tiles_x = (P.cols + zt::DX - 1) / zt::DX;
-        const void* fr = P.frames[w.y];
-        int32_t* ord = P.order[w.y];
-        float* res = P.res[w.y];
-        for (int ty = w.z; ty < w.z + w.w; ty++)
-            for (int tx = 0; tx < tiles_x; tx++) {
-                if (P.sample_type == ZIM_SAMPLE_U8)
-                    zt::decode_tile<uint8_t>((const uint8_t*)fr, dp, tx, ty, tid, sm, ord, res, nullptr, nullptr);
-                else
-                    zt::decode_tile<uint16_t>((const uint16_t*)fr, dp, tx, ty, tid, sm, ord, res, nullptr, nullptr);
-            }
-        __syncthreads();
-    }
 }
 
 __global__ void __launch_bounds__(BT) batch_smooth_kernel(const PairDev* __restrict__ pairs,
@@ -278,13 +247,12 @@ struct zim_batch {
     int max_cols = 0, max_pha_f = 0;
     size_t match_smem = 0;
     size_t ror_smem = 0;
-    int grid[NQ] = {0, 0, 0, 0, 0, 0};
+    int grid[NQ] = {};
     cudaStream_t cap_stream = nullptr;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     // host layout of the intermediates (for resubmission with another tuning)
     std::vector<PairDev> host_pairs;
-    std::vector<char> tma;  // per pair: decoded by the bulk-copy kernel, not the queue
     size_t items_off = 0;
     // grid filters: per pair the resolved config and its buffers (x_in / m_in:
     // the pixel stages' output; x1, x2: intermediate clouds; mls_tmp: MLS
@@ -339,11 +307,9 @@ void build_items(const zim_batch* b, const zim_batch_tuning& t, std::vector<int4
         const zim_batch_pair& p = b->pairs[pi];
         const zim_rect_state& C = b->calibs[p.calib];
         const int trows = (p.rows + zt::DY - 1) / zt::DY;
-        const bool tma = (size_t)pi < b->tma.size() && b->tma[pi];
         for (int cam = 0; cam < 2; cam++)
             for (int r = 0; r < trows; r += t.decode_rows) {
                 const int4 it = make_int4(pi, cam, r, std::min(t.decode_rows, trows - r));
-                if (!tma) items[Q_DECODE].push_back(it);
                 if (p.decode.post_smooth) items[Q_SMOOTH].push_back(it);  // modes 1 and 2
             }
         for (int r = 0; r < C.rect_h; r += t.match_rows)
@@ -438,7 +404,6 @@ zim_status capture(zim_batch* b) {
     b->graph = nullptr;
     const int sms = ctx->sm_count > 0 ? ctx->sm_count : 152;
     const int want = std::max(1, b->tuning.ctas_per_sm);
-    b->grid[Q_DECODE] = sms * std::min(want, occupancy((const void*)batch_decode_kernel, 0));
     b->grid[Q_SMOOTH] = sms * std::min(want, occupancy((const void*)batch_smooth_kernel, 0));
     b->grid[Q_MATCH] = sms * std::min(want, occupancy((const void*)batch_match_kernel, b->match_smem));
     b->grid[Q_REPROJ] = sms * std::min(want, occupancy((const void*)batch_reproject_kernel, 0));
@@ -448,22 +413,12 @@ zim_status capture(zim_batch* b) {
     ZIM_CUDA_TRY(ctx, cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
     cudaMemsetAsync(b->d_counters, 0, NQ * sizeof(unsigned), s);
     const Queues& q = b->q;
-    // pairs the bulk-copy decode takes (its own launch per camera; the same
-    // arithmetic as the queue's tiles)
-    for (size_t pi = 0; pi < b->tma.size(); pi++)
-        if (b->tma[pi]) {
-            const PairDev& D = b->host_pairs[pi];
-            for (int c = 0; c < 2; c++)
-                if (!zim_decode_tma_launch(ctx, D.frames[c], D.sample_type, D.dp, D.order[c], D.res[c], s)) {
-                    cudaGraph_t g = nullptr;
-                    cudaStreamEndCapture(s, &g);
-                    if (g) cudaGraphDestroy(g);
-                    return zim_fail(ctx, ZIM_ERR_CUDA, "batch decode copy path unavailable");
-                }
-        }
-    if (q.n[Q_DECODE])
-        batch_decode_kernel<<<std::min(b->grid[Q_DECODE], q.n[Q_DECODE]), BT, 0, s>>>(
-            b->d_pairs, q.items[Q_DECODE], q.n[Q_DECODE], b->d_counters + Q_DECODE);
+    // stage 1: a launch per camera fills the GPU at every pair size
+    const unsigned long long launched = ctx->launches;
+    for (const PairDev& D : b->host_pairs)
+        for (int c = 0; c < 2; c++)
+            zim_decode_params_launch(ctx, D.frames[c], D.sample_type, D.dp, D.order[c], D.res[c], nullptr, nullptr, s);
+    ctx->launches = launched;  // captured, not run: each replay counts them
     if (q.n[Q_SMOOTH])
         batch_smooth_kernel<<<std::min(b->grid[Q_SMOOTH], q.n[Q_SMOOTH]), BT, 0, s>>>(
             b->d_pairs, q.items[Q_SMOOTH], q.n[Q_SMOOTH], b->d_counters + Q_SMOOTH);
@@ -558,10 +513,9 @@ zim_status requeue(zim_batch* b) {
 
 // Upper bound of the item space over the tunings the autotuner tries (1-row bands).
 size_t max_item_bytes(const zim_batch* b) {
-    size_t n[NQ] = {0, 0, 0, 0, 0, 0};
+    size_t n[NQ] = {};
     for (const zim_batch_pair& p : b->pairs) {
         const zim_rect_state& C = b->calibs[p.calib];
-        n[Q_DECODE] += 2 * (size_t)((p.rows + zt::DY - 1) / zt::DY);
         n[Q_SMOOTH] += 2 * (size_t)((p.rows + zt::DY - 1) / zt::DY);
         n[Q_MATCH] += (size_t)C.rect_h;
         const size_t rt = (C.rect_h + zt::RY - 1) / zt::RY;
@@ -800,12 +754,6 @@ extern "C" ZIM_API zim_status zim_batch_submit(zim_batch* b, const zim_batch_pai
         return zim_fail(ctx, ZIM_ERR_OUT_OF_MEMORY, "batch memory plan overflow");
     b->items_off = (size_t)(cur - (char*)b->d_mem);
     ZIM_CUDA_TRY(ctx, cudaMemcpy(b->d_pairs, b->host_pairs.data(), sizeof(PairDev) * n_pairs, cudaMemcpyHostToDevice));
-    b->tma.assign(n_pairs, 0);
-    for (int i = 0; i < n_pairs; i++) {
-        const PairDev& D = b->host_pairs[i];
-        b->tma[i] = zim_decode_tma_applies(D.frames[0], D.sample_type, D.dp) &&
-                    zim_decode_tma_applies(D.frames[1], D.sample_type, D.dp);
-    }
     b->n_lanes = 0;
     if (n_filtered) {
         zim_status s = setup_lanes(b, std::min(n_filtered, (int)zim_batch::MAX_LANES), lane_scratch);
@@ -819,7 +767,7 @@ extern "C" ZIM_API zim_status zim_batch_run(zim_batch* b, void* stream) {
     if (!b->exec) return zim_fail(b->ctx, ZIM_ERR_INVALID_ARG, "nothing submitted");
     ZIM_CUDA_TRY(b->ctx, cudaGraphLaunch(b->exec, zim_stream(stream)));
     for (int q = 0; q < NQ; q++) b->ctx->launches += b->q.n[q] > 0 ? 1 : 0;  // kernels in the graph
-    b->ctx->launches += b->lane_launches;
+    b->ctx->launches += 2 * b->host_pairs.size() + b->lane_launches;
     return ZIM_OK;
 }
 

@@ -7,16 +7,11 @@
 //
 // Arithmetic is FP32.  The pre-blur is linear, so the blurred sums
 // S = -sum sin_k I_k, C = sum cos_k I_k, sum I_k are the 3x3 blur of the raw
-// per-pixel sums: a CTA computes the raw sums over its tile + 1-pixel halo into
-// shared memory once per frequency and blurs 3 channels instead of N frames.
+// per-pixel sums: 3 channels per frequency are blurred instead of N frames.
 // Unwrapping keeps integer cycle counts exact and only small fractional parts
 // in FP32, so an order differs from the FP64 restatement only when a decision
 // argument sits within ~1e-6 of its threshold.
 #include <cmath>
-#include <mutex>
-
-#include <cuda.h>
-#include <cudaTypedefs.h>
 
 #include "zim_tiles.cuh"
 
@@ -24,180 +19,473 @@ namespace {
 
 using zt::DecodeParams;
 
+constexpr int MAX_PS = 4;       // phase-shift frequencies
+constexpr int DEC_WARPS = 4;    // warps per block
+constexpr int STRIP = 30;       // output columns per warp (32 read)
+constexpr int DEC_MIN_WARPS = 24;  // warps per SM a launch should have
+
+__device__ __forceinline__ float2 both(float a) { return make_float2(a, a); }
+
+// The two samples of a packed word as floats: each sample's bits under the
+// exponent of 2^23, minus 2^23 (exact, no integer-to-float conversion).
 template <typename T>
-__global__ void __launch_bounds__(zt::DX* zt::DY) decode_kernel(const T* __restrict__ frames, DecodeParams p,
-                                                                 int32_t* __restrict__ order,
-                                                                 float* __restrict__ residual,
-                                                                 float* __restrict__ mod_out,
-                                                                 uint8_t* __restrict__ valid_out) {
-    __shared__ zt::DecodeSmem sm;
-    zt::decode_tile<T>(frames, p, blockIdx.x, blockIdx.y, threadIdx.y * zt::DX + threadIdx.x, sm, order, residual,
-                       mod_out, valid_out);
+__device__ __forceinline__ float2 unpack(unsigned w) {
+    const unsigned a = sizeof(T) == 2 ? __byte_perm(w, 0x4B000000u, 0x7410) : __byte_perm(w, 0x4B000000u, 0x7440);
+    const unsigned b = sizeof(T) == 2 ? __byte_perm(w, 0x4B000000u, 0x7432) : __byte_perm(w, 0x4B000000u, 0x7441);
+    return __fadd2_rn(make_float2(__uint_as_float(a), __uint_as_float(b)), both(-8388608.f));
 }
 
-// ------------------------------------------------------------ TMA staging --
-// A decode tile's phase-shift samples (tile + 1-pixel halo, every frame) come
-// in one bulk tensor copy (cp.async.bulk.tensor) completing on an mbarrier: a
-// 3-D tensor map over (x, y, frame) of the frame stack, box BW x DHY x nfr with
-// x starting XP pixels left of the tile (a copy's x must be 16-byte aligned)
-// and y one row above.  Samples outside the image read as 0 and are never
-// used: the sums clamp to the image, as decode_stage_sums does, and add in the
-// same order, so the output is the same bit for bit.
-template <typename T>
-__host__ __device__ constexpr int tma_xpad() { return 16 / (int)sizeof(T); }
-template <typename T>
-__host__ __device__ constexpr int tma_bw() { return zt::DX + 2 * tma_xpad<T>(); }
-constexpr int TMA_MAX_FRAMES = 24;            // box depth (phase-shift frames) the path takes
-constexpr unsigned TMA_POLLS = 1u << 22;      // mbarrier polls before giving up (well over a second)
-constexpr uint32_t ERR_DECODE_COPY = 0x20u;   // device error word: a tile copy did not land
-
-__device__ __forceinline__ unsigned smem_addr(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
-
-// Phase 0 of the barrier completed; false after `polls` polls.
-__device__ __forceinline__ bool mbar_wait0(unsigned bar, unsigned polls) {
-    for (unsigned it = 0; it < polls; it++) {
-        unsigned done;
-        asm volatile(
-            "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], 0;\n selp.u32 %0, 1, 0, p;\n}\n"
-            : "=r"(done)
-            : "r"(bar)
-            : "memory");
-        if (done) return true;
-    }
-    return false;
+// A lane's pixel pair of one row as a packed word: the second sample lies d (0
+// or 1) after the first; PAIR: one aligned load of both.
+template <typename T, bool PAIR>
+__device__ __forceinline__ unsigned load_pair(const T* q, int d) {
+    if (PAIR)
+        return sizeof(T) == 2 ? __ldg(reinterpret_cast<const unsigned*>(q))
+                              : (unsigned)__ldg(reinterpret_cast<const unsigned short*>(q));
+    return (unsigned)__ldg(q) | (unsigned)__ldg(q + d) << (8 * sizeof(T));
 }
 
-// NPS / NS: frequency count and frames per frequency fixed at compile time
-// (0: from p), so the sample loops unroll with constant table offsets.
-template <typename T, int NPS, int NS>
-__global__ void __launch_bounds__(zt::DX* zt::DY) decode_tma_kernel(const __grid_constant__ CUtensorMap tmap,
-                                                                     const T* __restrict__ frames, DecodeParams p,
-                                                                     int nfr, int32_t* __restrict__ order,
-                                                                     float* __restrict__ residual,
-                                                                     float* __restrict__ mod_out,
-                                                                     uint8_t* __restrict__ valid_out,
-                                                                     uint32_t* __restrict__ err) {
-    constexpr int XP = tma_xpad<T>(), BW = tma_bw<T>();
-    __shared__ zt::DecodeSmem sm;
-    __shared__ __align__(8) unsigned long long bar;
-    extern __shared__ __align__(128) unsigned char box_raw[];  // [nfr][DHY][BW] samples
-    const T* box = reinterpret_cast<const T*>(box_raw);
-    const int tid = threadIdx.y * zt::DX + threadIdx.x;
-    const int bx = blockIdx.x, by = blockIdx.y;
-    const unsigned b = smem_addr(&bar);
-    if (tid == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(b) : "memory");
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    __syncthreads();
-    if (tid == 0) {
-        const unsigned bytes = (unsigned)(BW * zt::DHY * nfr * (int)sizeof(T));
-        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(b), "r"(bytes) : "memory");
-        asm volatile(
-            "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], "
-            "[%5];" ::"r"(smem_addr(box_raw)),
-            "l"(reinterpret_cast<unsigned long long>(&tmap)), "r"(bx * zt::DX - XP), "r"(by * zt::DY - 1), "r"(0),
-            "r"(b)
-            : "memory");
-    }
-    // bounded: a copy that never lands flags the error word; the tile waits
-    // once more (bounded) for it before leaving
-    if (!__syncthreads_and(mbar_wait0(b, TMA_POLLS))) {
-        if (tid == 0) atomicOr(err, ERR_DECODE_COPY);
-        mbar_wait0(b, TMA_POLLS);
-        return;
-    }
-    const int gx0 = bx * zt::DX - 1, gy0 = by * zt::DY - 1;
-    const int ox = bx * zt::DX - XP, oy = by * zt::DY - 1;  // box origin
-    const int plane = BW * zt::DHY;
-    for (int h = tid; h < zt::DHX * zt::DHY; h += zt::DX * zt::DY) {
-        const int hy = h / zt::DHX, hx = h - hy * zt::DHX;
-        const int gy = min(max(gy0 + hy, 0), p.rows - 1), gx = min(max(gx0 + hx, 0), p.cols - 1);
-        const T* bp = box + (gy - oy) * BW + (gx - ox);
-        const int n_ps = NPS ? NPS : p.n_ps;
+// n words of consecutive frames (npx samples apart) from q on; the choice of load
+// is the warp's (pair: every lane's pair is aligned and inside the image), so it
+// costs one branch, not two loads in the place of each.
+template <typename T, int N>
+__device__ __forceinline__ void load_pairs(const T* q, size_t npx, bool pair, int d, unsigned (&w)[N]) {
+    if (pair) {
 #pragma unroll
-        for (int i = 0; i < (NPS ? NPS : zt::DEC_MAX_PS); i++) {
+        for (int k = 0; k < N; k++) w[k] = load_pair<T, true>(q + k * npx, d);
+    } else {
+#pragma unroll
+        for (int k = 0; k < N; k++) w[k] = load_pair<T, false>(q + k * npx, d);
+    }
+}
+
+// floor(a / b) for b > 0 and |a / b| < 2^21, from the float reciprocal
+// inv_b = 1 / b: the float quotient is within one of the true one, and one
+// remainder check corrects it (an integer division costs ~40 instructions).
+__device__ __forceinline__ int floor_div(int a, int b, float inv_b) {
+    int q = __float2int_rd((float)a * inv_b);
+    const int r = a - q * b;
+    q += (r >= b) - (r < 0);
+    return q;
+}
+
+// Four-quadrant arctangent of the wrapped phase.  The octant ratio
+// t = min(|y|, |x|) / max(|y|, |x|) in [0, 1] gives atan(t) = t P(t^2) with P of
+// degree 7, fitted for this kernel by iteratively reweighted least squares on
+// Chebyshev nodes (absolute error 3.7e-8 in exact arithmetic, 1.4e-7 evaluated
+// by FP32 Horner FMAs); the octant and quadrant follow by symmetry, with atan2's
+// signed zeros (the sign bits of y and x) and 0 for (0, 0).  __fdividef is
+// exact to 2 ulp for the divisor range of these sums (far below 2^126).
+__device__ __forceinline__ float phase_atan2(float y, float x) {
+    const float ax = fabsf(x), ay = fabsf(y);
+    const float hi = fmaxf(ax, ay), lo = fminf(ax, ay);
+    const float t = hi > 0.f ? __fdividef(lo, hi) : 0.f;
+    const float s = t * t;
+    float p = -0.004054566845297813f;
+    p = fmaf(p, s, 0.021862957626581192f);
+    p = fmaf(p, s, -0.0559123270213604f);
+    p = fmaf(p, s, 0.0964219719171524f);
+    p = fmaf(p, s, -0.1390862911939621f);
+    p = fmaf(p, s, 0.19946566224098206f);
+    p = fmaf(p, s, -0.33329859375953674f);
+    p = fmaf(p, s, 0.9999993443489075f);
+    float r = t * p;
+    if (ay > ax) r = 0.5f * ZIM_PI_F - r;
+    if (signbit(x)) r = ZIM_PI_F - r;
+    return copysignf(r, y);
+}
+
+// The validity test on the normalised modulation nm = (2 |S, C| / N) / (M / N)
+// (0 when M <= 1e-3 N): nm < thr fails the pixel.  For M > 0 that is
+// 4 (S^2 + C^2) < (thr M)^2 with thr > 0, which needs neither the square root
+// nor the division; they are computed only where nm is written out
+// (want_value: frequency 0 with a modulation map).  The two forms decide
+// differently only where nm lies within float rounding of thr.
+__device__ __forceinline__ bool modulation_ok(float S, float C, float M, int N, float thr, bool want_value,
+                                              float& value) {
+    const float q = fmaf(S, S, C * C);
+    const bool has_m = M > 1e-3f * (float)N;
+    if (want_value) value = has_m ? 2.0f * sqrtf(q) / M : 0.f;
+    if (!(thr > 0.f)) return true;
+    const float tm = thr * M;
+    return has_m && !(4.0f * q < tm * tm);
+}
+
+// Absolute order k and residual r of one pixel from its wrapped phases; g1, g2:
+// its Gray codeword and, with the complementary bit, the shifted one.
+template <int NPS>
+__device__ __forceinline__ void unwrap(const DecodeParams& p, int n_ps, const float (&w)[MAX_PS], int g1, int g2,
+                                       int& k, float& r) {
+    k = 0;
+    if (p.enc == ZIM_ENC_HETERODYNE3) {
+        const float w0 = w[0], w1 = w[1], w2 = w[2];
+        float p12 = w0 > w1 ? w0 - w1 : w0 - w1 + ZIM_TWO_PI_F;
+        float p23;
+        if (p.f1_gt_f2) p23 = w1 > w2 ? w1 - w2 : w1 - w2 + ZIM_TWO_PI_F;
+        else p23 = w2 > w1 ? w2 - w1 : w2 - w1 + ZIM_TWO_PI_F;
+        float p123 = p12 > p23 ? p12 - p23 : p12 - p23 + ZIM_TWO_PI_F;
+        // uphase12 = p12 + 2 pi m12;  k = round(m12 f0 / f12 + (p12 f0 / f12 - w0) / 2 pi)
+        int m12 = (int)roundf(fmaf(p123, (float)p.f12, -p12) * ZIM_INV_TWO_PI_F);
+        int num = m12 * p.f0;
+        int q = floor_div(num, p.f12, p.inv_f12);
+        int rem = num - q * p.f12;
+        k = q + (int)roundf(fmaf((float)rem, p.inv_f12, fmaf(p12, p.f0_f12, -w0) * ZIM_INV_TWO_PI_F));
+        r = w0;
+        if (p.avg3) {
+            int m23 = (int)roundf(fmaf(p123, (float)p.f23, -p23) * ZIM_INV_TWO_PI_F);
+            int n2 = m23 * p.f1, q2 = floor_div(n2, p.f23, p.inv_f23), r2i = n2 - q2 * p.f23;
+            int k2 = q2 + (int)roundf(fmaf((float)r2i, p.inv_f23, fmaf(p23, p.f1_f23, -w1) * ZIM_INV_TWO_PI_F));
+            int n3 = m23 * p.f2, q3 = floor_div(n3, p.f23, p.inv_f23), r3i = n3 - q3 * p.f23;
+            int k3 = q3 + (int)roundf(fmaf((float)r3i, p.inv_f23, fmaf(p23, p.f2_f23, -w2) * ZIM_INV_TWO_PI_F));
+            // (uphase2 f0 / f1 - 2 pi k) = (w1 f0 + 2 pi (k2 f0 - k f1)) / f1, same for 3
+            float r2 = fmaf((float)(k2 * p.f0 - k * p.f1), ZIM_TWO_PI_F, w1 * (float)p.f0) * p.inv_f1;
+            float r3 = fmaf((float)(k3 * p.f0 - k * p.f2), ZIM_TWO_PI_F, w2 * (float)p.f0) * p.inv_f2;
+            r = (w0 + r2 + r3) * (1.0f / 3.0f);
+        }
+    } else if (p.enc == ZIM_ENC_HIERARCHICAL) {
+        r = w[0];
+#pragma unroll
+        for (int i = 1; i < NPS; i++) {
             if (i >= n_ps) break;
-            const int f0 = NS ? i * NS : p.fbase[i];  // frequencies' frames are consecutive
-            const int N = NS ? NS : p.shift[i];
-            float2 sc = make_float2(0.f, 0.f);
-            float mv = 0.f;
-#pragma unroll
-            for (int k = 0; k < (NS ? NS : 32); k++) {  // 3..32 steps
-                if (k >= N) break;
-                const float v = (float)bp[(f0 + k) * plane];
-                sc = zt::sc_add(sc, p.sinv[f0 + k], p.cosv[f0 + k], v);
-                mv += v;
-            }
-            sm.SC[i][hy][hx] = sc;
-            sm.M[i][hy][hx] = mv;
+            float a = fmaf(p.fratio[i], w[i - 1] + ZIM_PI_F, -(w[i] + ZIM_PI_F)) * ZIM_INV_TWO_PI_F;
+            k = p.iratio[i] * k + (int)roundf(a);
+            r = w[i];
+        }
+    } else {
+        k = g1;
+        r = w[0];
+        if (p.complementary) {
+            if (r <= -0.5f * ZIM_PI_F) k = g2;
+            else if (r >= 0.5f * ZIM_PI_F) k = g2 - 1;
         }
     }
-    __syncthreads();
-    zt::decode_finish<T, NPS, NS>(frames, p, bx, by, tid, sm, order, residual, mod_out, valid_out);
 }
 
-// cuTensorMapEncodeTiled from the driver, looked up once (no link to libcuda)
-PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
-    static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
-    static std::once_flag once;
-    std::call_once(once, [] {
-        void* f = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &f, 12000, cudaEnableDefault, &q) ==
-                cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            fn = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(f);
-    });
-    return fn;
+struct Outputs {
+    int32_t* order;
+    float* residual;
+    float* mod;
+    uint8_t* valid;
+};
+
+// A pixel under way: wrapped phases, modulation of frequency 0, whether nothing
+// rejected it so far.
+struct Pixel {
+    float w[MAX_PS], mod;
+    bool ok;
+};
+
+// One frequency's blurred (or fitted) sums: wrapped phase and validity.
+__device__ __forceinline__ void take_frequency(const DecodeParams& p, int i, float S, float C, float M, bool want_mod,
+                                               Pixel& px) {
+    px.w[i] = phase_atan2(S, C);
+    float v = 0.f;
+    const bool m = modulation_ok(S, C, M, p.shift[i], p.thr, want_mod && i == 0, v);
+    if (i == 0) px.mod = px.ok ? v : 0.f;
+    px.ok = px.ok && m;
 }
 
-// The frame stack's tensor map for decode_tma_kernel, or false when the path
-// does not apply (HDR, row pitch or base not 16-byte aligned, too many
-// frames, an image narrower than the box, no driver entry point).
+// Unwraps and writes a pixel.
+template <int NPS>
+__device__ __forceinline__ void finish_pixel(const DecodeParams& p, int n_ps, const Pixel& px, int g1, int g2,
+                                             size_t o, const Outputs& out) {
+    int k;
+    float r;
+    unwrap<NPS>(p, n_ps, px.w, g1, g2, k, r);
+    out.order[o] = px.ok ? k : (p.hdr ? -1 : 0);  // the HDR decoder marks invalid orders -1
+    out.residual[o] = px.ok ? r : 0.f;
+    if (out.mod) out.mod[o] = px.mod;
+    if (out.valid) out.valid[o] = px.ok;
+}
+
+// One warp decodes a strip of 30 columns (a lane per column, one more on either
+// side), marching down `band` rows: each raw row's sums are formed once,
+// exchanged with the neighbour lanes by shuffles and added to the three output
+// rows they blur into, so nothing is staged in shared memory and no warp waits
+// for another.  The next row's samples are in flight while a row is blurred and
+// unwrapped.  S and C are the lanes of the paired FP32 FMA (__ffma2_rn: each
+// rounded as fmaf).  NS: frames per frequency at compile time (0: p.shift); NPS:
+// frequencies (4: p.n_ps of them).
+//
+// Bound by instruction issue.  A tile per CTA, staged by a bulk tensor copy and
+// blurred from shared memory (nine two-word shared loads per pixel and frequency,
+// a 1.33x halo), issued 588 warp instructions per 32 pixels for three frequencies
+// of four frames; this kernel issues 434.  Two columns per lane (all sums paired,
+// half the shuffles) issued 409 but needed 120 registers and took 88 us where
+// this takes 73.  Before / now, 2448x2048: 24 8-bit frames (heterodyne) 180 / 118
+// us, 12 16-bit frames 88 / 73; 1626x1236 Gray code (rows no multiple of 16 bytes)
+// 56 / 35.
+template <typename T, int NPS, int NS>
+__global__ void __launch_bounds__(32 * DEC_WARPS) decode_strip_kernel(const T* __restrict__ frames,
+                                                                      const __grid_constant__ DecodeParams p, int band,
+                                                                      int nstrips, const __grid_constant__ Outputs out) {
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const int wid = blockIdx.x * DEC_WARPS + (threadIdx.x >> 5);
+    const int y0 = (wid / nstrips) * band;
+    if (y0 >= p.rows) return;
+    const int y1 = min(y0 + band, p.rows);
+    const int x = (wid % nstrips) * STRIP - 1 + lane;
+    const bool writes = lane > 0 && lane < 31 && x < p.cols;
+    const size_t npx = (size_t)p.rows * p.cols;
+    const int n_ps = NPS < MAX_PS ? NPS : p.n_ps;
+    // byte offset of a row's sample within any frame's plane (at most 2^31 samples):
+    // the plane's base is the same for the whole grid, so a load adds 32 bits to it
+    const int xc = min(max(x, 0), p.cols - 1);
+    auto row_off = [&](int y) {
+        return ((unsigned)min(max(y, 0), p.rows - 1) * (unsigned)p.cols + (unsigned)xc) * (unsigned)sizeof(T);
+    };
+    auto sample = [&](int f, unsigned off) {
+        return (unsigned)__ldg(reinterpret_cast<const T*>(reinterpret_cast<const char*>(frames + (size_t)f * npx) + off));
+    };
+    const bool gray = (NPS == 1 || NPS == MAX_PS) && p.gray_bits > 0;
+
+    constexpr int NW = NS ? NPS * NS : 4, GW = NPS == 1 ? 8 : 1;
+    const int nbits = p.gray_bits + p.complementary;
+    unsigned raw[NW], gw[GW];  // samples in flight (up to GW of the Gray frames)
+    auto fetch = [&](int y) {
+        const unsigned o = row_off(y);
+#pragma unroll
+        for (int f = 0; f < (NS ? NW : 0); f++) raw[f] = sample(f, o);
+        if (gray && nbits <= GW)
+#pragma unroll
+            for (int b = 0; b < GW; b++)
+                if (b < nbits) gw[b] = sample(p.gray_base + b, o);
+    };
+    // blurred sums under way: A for the row above the current raw row, B for it
+    float2 A[NPS], B[NPS];  // (S, C)
+    float AM[NPS], BM[NPS];
+#pragma unroll
+    for (int i = 0; i < NPS; i++) {
+        A[i] = B[i] = make_float2(0.f, 0.f);
+        AM[i] = BM[i] = 0.f;
+    }
+    int g1 = 0, g2 = 0, h1 = 0, h2 = 0;  // codewords of the row above, of this row
+    if (NS > 0 || gray) fetch(y0 - 1);
+    for (int y = y0 - 1; y <= y1; y++) {
+        float2 sc[NPS];
+        float m[NPS];
+#pragma unroll
+        for (int i = 0; i < NPS; i++) {
+            if (i >= n_ps) break;
+            sc[i] = make_float2(0.f, 0.f);
+            m[i] = 0.f;
+            auto add = [&](int f, unsigned w) {
+                const float v = (float)w;
+                sc[i] = make_float2(fmaf(-p.sinv[f], v, sc[i].x), fmaf(p.cosv[f], v, sc[i].y));
+                m[i] += v;
+            };
+            if constexpr (NS > 0) {
+                sc[i].y = m[i] = (float)raw[i * NS];  // step 0: sin 0 and cos 1 exactly
+#pragma unroll
+                for (int k = 1; k < NS; k++) add(i * NS + k, raw[i * NS + k]);
+            } else {
+                const int N = p.shift[i], f0 = p.fbase[i];
+                const unsigned o = row_off(y);
+                int k = 0;
+                for (; k + 4 <= N; k += 4) {  // four loads in flight
+#pragma unroll
+                    for (int u = 0; u < 4; u++) raw[u] = sample(f0 + k + u, o);
+#pragma unroll
+                    for (int u = 0; u < 4; u++) add(f0 + k + u, raw[u]);
+                }
+                for (; k < N; k++) add(f0 + k, sample(f0 + k, o));
+            }
+        }
+        if (gray) {
+            // codeword of this raw row: bit set where N g > sum of the phase frames (exact in FP32)
+            g1 = h1;
+            g2 = h2;
+            if (y >= y0 && y < y1) {
+                const float N = (float)p.shift[0];
+                auto bit = [&](unsigned w) { return N * (float)w > m[0] ? 1 : 0; };
+                int bin = 0, v = 0;
+                unsigned last;
+                if (nbits <= GW) {
+#pragma unroll
+                    for (int b = 0; b < GW; b++)
+                        if (b < p.gray_bits) {
+                            bin ^= bit(gw[b]);
+                            v = v << 1 | bin;
+                        }
+                    last = gw[0];
+#pragma unroll
+                    for (int b = 1; b < GW; b++)
+                        if (b == p.gray_bits) last = gw[b];
+                } else {
+                    const unsigned o = row_off(y);
+                    last = p.complementary ? sample(p.gray_base + p.gray_bits, o) : 0u;
+#pragma unroll 4
+                    for (int b = 0; b < p.gray_bits; b++) {
+                        bin ^= bit(sample(p.gray_base + b, o));
+                        v = v << 1 | bin;
+                    }
+                }
+                h1 = v;
+                h2 = ((v << 1 | (bin ^ bit(last))) + 1) >> 1;
+            }
+        }
+        if ((NS > 0 || gray) && y < y1) fetch(y + 1);
+        Pixel px;
+        px.ok = true;
+#pragma unroll
+        for (int i = 0; i < NPS; i++) {
+            if (i >= n_ps) break;
+            // taps in row-major order from zero, as nine sequential FMAs per output
+            auto w2 = [&](int t) { return make_float2(p.w2d[t], p.w2d[t]); };
+            const float2 c = sc[i];
+            const float2 l = make_float2(__shfl_up_sync(full, c.x, 1), __shfl_up_sync(full, c.y, 1));
+            const float2 r = make_float2(__shfl_down_sync(full, c.x, 1), __shfl_down_sync(full, c.y, 1));
+            const float2 F = __ffma2_rn(w2(8), r, __ffma2_rn(w2(7), c, __ffma2_rn(w2(6), l, A[i])));
+            A[i] = __ffma2_rn(w2(5), r, __ffma2_rn(w2(4), c, __ffma2_rn(w2(3), l, B[i])));
+            B[i] = __ffma2_rn(w2(2), r, __ffma2_rn(w2(1), c, __ffma2_rn(w2(0), l, make_float2(0.f, 0.f))));
+            const float ml = __shfl_up_sync(full, m[i], 1), mr = __shfl_down_sync(full, m[i], 1);
+            const float FM = fmaf(p.w2d[8], mr, fmaf(p.w2d[7], m[i], fmaf(p.w2d[6], ml, AM[i])));
+            AM[i] = fmaf(p.w2d[5], mr, fmaf(p.w2d[4], m[i], fmaf(p.w2d[3], ml, BM[i])));
+            BM[i] = fmaf(p.w2d[2], mr, fmaf(p.w2d[1], m[i], fmaf(p.w2d[0], ml, 0.f)));
+            if (y > y0) take_frequency(p, i, F.x, F.y, FM, out.mod != nullptr, px);
+        }
+        if (y > y0 && writes) finish_pixel<NPS>(p, n_ps, px, g1, g2, (size_t)(y - 1) * p.cols + x, out);
+    }
+}
+
+// HDR fit of one frequency at a pixel pair (JSLAB_HDRPhaseFit.h:10-61 and
+// JSLAB_PhaseShiftDecoder_V2.cpp:73-90): raw samples with 0 <= I < saturation
+// enter an equal-variance least-squares fit of I = A + C cos d - S sin d
+// (solved here from the 3x3 normal equations, the reference's cached
+// pseudo-inverse of the same subset); fewer than three samples, amplitude
+// hypot(C, S) <= min_amp or A <= 1e-3 reject the pixel.  Returns the sums the
+// phase-shift path would have formed: S N/2, C N/2, A N.  A sample's mask is the
+// factor 1 or 0 of its terms (exact), so both pixels run as one.
+template <typename T, int NS>
+__device__ __forceinline__ void hdr_fit(const T* q, size_t npx, bool pair, int d, const DecodeParams& p, int i, float2& S,
+                                        float2& C, float2& M, bool& ok0, bool& ok1) {
+    const float2 zero = both(0.f);
+    auto below = [](float v, float limit) {  // 1 or 0
+        float r;
+        asm("set.lt.f32.f32 %0, %1, %2;" : "=f"(r) : "f"(v), "f"(limit));
+        return r;
+    };
+    float2 m00 = zero, m01 = zero, m02 = zero, m11 = zero, m12 = zero, m22 = zero, r0 = zero, r1 = zero, r2 = zero;
+    const int N = NS ? NS : p.shift[i], f0 = NS ? i * NS : p.fbase[i];
+    auto add = [&](int f, unsigned w) {
+        float2 v = unpack<T>(w);
+        const float2 in = make_float2(below(v.x, p.hdr_sat), below(v.y, p.hdr_sat));
+        const float2 c = make_float2(in.x * p.cosv[f], in.y * p.cosv[f]);
+        const float2 s = make_float2(in.x * -p.sinv[f], in.y * -p.sinv[f]);
+        v = __fmul2_rn(in, v);
+        m00 = __fadd2_rn(m00, in);
+        m01 = __fadd2_rn(m01, c);
+        m02 = __fadd2_rn(m02, s);
+        m11 = __ffma2_rn(c, c, m11);
+        m12 = __ffma2_rn(c, s, m12);
+        m22 = __ffma2_rn(s, s, m22);
+        r0 = __fadd2_rn(r0, v);
+        r1 = __ffma2_rn(c, v, r1);
+        r2 = __ffma2_rn(s, v, r2);
+    };
+    if constexpr (NS > 0) {
+        unsigned w[NS];
+        load_pairs(q + (size_t)f0 * npx, npx, pair, d, w);
+#pragma unroll
+        for (int k = 0; k < NS; k++) add(f0 + k, w[k]);
+    } else {
+        for (int k = 0; k < N; k++) {
+            unsigned w[1];
+            load_pairs(q + (size_t)(f0 + k) * npx, npx, pair, d, w);
+            add(f0 + k, w[0]);
+        }
+    }
+    auto neg = [](float2 a) { return make_float2(-a.x, -a.y); };
+    // symmetric 3x3 inverse by cofactors
+    const float2 c00 = __ffma2_rn(m11, m22, __fmul2_rn(neg(m12), m12));
+    const float2 c01 = __ffma2_rn(m02, m12, __fmul2_rn(neg(m01), m22));
+    const float2 c02 = __ffma2_rn(m01, m12, __fmul2_rn(neg(m02), m11));
+    const float2 det = __ffma2_rn(m00, c00, __ffma2_rn(m01, c01, __fmul2_rn(m02, c02)));
+    const float2 c11 = __ffma2_rn(m00, m22, __fmul2_rn(neg(m02), m02));
+    const float2 c12 = __ffma2_rn(m01, m02, __fmul2_rn(neg(m00), m12));
+    const float2 c22 = __ffma2_rn(m00, m11, __fmul2_rn(neg(m01), m01));
+    const float2 id = make_float2(__frcp_rn(det.x), __frcp_rn(det.y));
+    const float2 A = __fmul2_rn(__ffma2_rn(c00, r0, __ffma2_rn(c01, r1, __fmul2_rn(c02, r2))), id);
+    C = __fmul2_rn(__ffma2_rn(c01, r0, __ffma2_rn(c11, r1, __fmul2_rn(c12, r2))), id);
+    S = __fmul2_rn(__ffma2_rn(c02, r0, __ffma2_rn(c12, r1, __fmul2_rn(c22, r2))), id);
+    auto accept = [&](float n, float det, float A, float C, float S) {
+        if (n < 3.f || !(fabsf(det) > 1e-6f * n * n * n) || !(A > 1e-3f)) return false;
+        // hypot(C, S) > min_amp, by squares where those decide beyond rounding
+        const float q = fmaf(C, C, S * S), t = p.hdr_min_amp * p.hdr_min_amp;
+        if (q > 1.00001f * t) return true;
+        if (q < 0.99999f * t) return false;
+        return hypotf(C, S) > p.hdr_min_amp;
+    };
+    ok0 = accept(m00.x, det.x, A.x, C.x, S.x);
+    ok1 = accept(m00.y, det.y, A.y, C.y, S.y);
+    const float2 n2 = both((float)N), half = both(0.5f);
+    S = __fmul2_rn(__fmul2_rn(S, n2), half);
+    C = __fmul2_rn(__fmul2_rn(C, n2), half);
+    M = __fmul2_rn(A, n2);
+}
+
+// HDR decode: raw samples, no pre-blur (saturation is classified before any
+// blur), a pixel pair per thread.  Bound by instruction issue (nine sums per
+// sample): paired over two pixels and without branches 35 us for 24 frames of
+// 1280x1024, 64 us one pixel at a time.
+template <typename T, int NPS, int NS>
+__global__ void __launch_bounds__(128) decode_hdr_kernel(const T* __restrict__ frames,
+                                                         const __grid_constant__ DecodeParams p, int aligned,
+                                                         const __grid_constant__ Outputs out) {
+    const int half = (p.cols + 1) / 2;
+    const size_t t = (size_t)blockIdx.x * 128 + threadIdx.x;
+    const int y = (int)(t / (unsigned)half);
+    if (y >= p.rows) return;
+    const int x = 2 * (int)(t - (size_t)y * half);
+    const size_t npx = (size_t)p.rows * p.cols;
+    const int n_ps = NPS < MAX_PS ? NPS : p.n_ps;
+    const T* q = frames + (size_t)y * p.cols + x;
+    const int d = x + 1 < p.cols ? 1 : 0;
+    Pixel p0, p1;
+    p0.ok = p1.ok = true;
+#pragma unroll
+    for (int i = 0; i < NPS; i++) {
+        if (i >= n_ps) break;
+        float2 S, C, M;
+        bool f0, f1;
+        hdr_fit<T, NS>(q, npx, aligned, d, p, i, S, C, M, f0, f1);
+        p0.ok = p0.ok && f0;
+        p1.ok = p1.ok && f1;
+        take_frequency(p, i, S.x, C.x, M.x, out.mod != nullptr, p0);
+        take_frequency(p, i, S.y, C.y, M.y, out.mod != nullptr, p1);
+    }
+    const size_t o = (size_t)y * p.cols + x;
+    finish_pixel<NPS>(p, n_ps, p0, 0, 0, o, out);
+    if (d) finish_pixel<NPS>(p, n_ps, p1, 0, 0, o + 1, out);
+}
+
 template <typename T>
-bool decode_tensor_map(const void* frames, const DecodeParams& p, CUtensorMap* m, int* nfr_out) {
-    if (p.hdr) return false;
-    int nfr = 0;
-    for (int i = 0; i < p.n_ps; i++) nfr += p.shift[i];
-    const size_t es = sizeof(T);
-    if (nfr < 1 || nfr > TMA_MAX_FRAMES || ((size_t)p.cols * es) % 16 != 0 || ((uintptr_t)frames & 15) != 0 ||
-        p.cols < tma_bw<T>() || p.rows < zt::DHY)
-        return false;
-    PFN_cuTensorMapEncodeTiled_v12000 enc = tensor_map_encoder();
-    if (!enc) return false;
-    const cuuint64_t dims[3] = {(cuuint64_t)p.cols, (cuuint64_t)p.rows, (cuuint64_t)nfr};
-    const cuuint64_t strides[2] = {(cuuint64_t)p.cols * es, (cuuint64_t)p.rows * p.cols * es};
-    const cuuint32_t boxd[3] = {(cuuint32_t)tma_bw<T>(), (cuuint32_t)zt::DHY, (cuuint32_t)nfr};
-    const cuuint32_t estr[3] = {1, 1, 1};
-    const CUresult r = enc(m, es == 2 ? CU_TENSOR_MAP_DATA_TYPE_UINT16 : CU_TENSOR_MAP_DATA_TYPE_UINT8, 3,
-                           const_cast<void*>(frames), dims, strides, boxd, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                           CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) return false;
-    *nfr_out = nfr;
-    return true;
-}
-
-template <typename T>
-bool launch_decode_tma(zim_ctx* ctx, const void* frames, const DecodeParams& p, dim3 grd, dim3 blk, int32_t* order,
-                       float* residual, float* mod, uint8_t* valid, cudaStream_t st) {
-    CUtensorMap m;
-    int nfr = 0;
-    if (!decode_tensor_map<T>(frames, p, &m, &nfr)) return false;
-    const size_t dsm = (size_t)tma_bw<T>() * zt::DHY * nfr * sizeof(T);
-    bool four = true;  // every frequency 4-step (the common configurations)
-    for (int i = 0; i < p.n_ps; i++) four = four && p.shift[i] == 4;
-    if (four && p.n_ps == 3)
-        decode_tma_kernel<T, 3, 4><<<grd, blk, dsm, st>>>(m, (const T*)frames, p, nfr, order, residual, mod, valid,
-                                                          ctx->d_error);
-    else if (four && p.n_ps == 1)
-        decode_tma_kernel<T, 1, 4><<<grd, blk, dsm, st>>>(m, (const T*)frames, p, nfr, order, residual, mod, valid,
-                                                          ctx->d_error);
-    else
-        decode_tma_kernel<T, 0, 0><<<grd, blk, dsm, st>>>(m, (const T*)frames, p, nfr, order, residual, mod, valid,
-                                                          ctx->d_error);
-    return true;
+void launch_decode(zim_ctx* ctx, const T* frames, const DecodeParams& p, const Outputs& out, cudaStream_t st) {
+    const int aligned = p.cols % 2 == 0 && ((uintptr_t)frames & (2 * sizeof(T) - 1)) == 0;
+    int ns = p.shift[0];
+    for (int i = 1; i < p.n_ps; i++) ns = p.shift[i] == ns ? ns : 0;
+    if (p.hdr) {
+        const unsigned blocks = (unsigned)(((size_t)p.rows * ((p.cols + 1) / 2) + 127) / 128);
+        auto k = p.n_ps == 3 && ns == 8 ? decode_hdr_kernel<T, 3, 8>
+                 : p.n_ps == 3 && ns == 4 ? decode_hdr_kernel<T, 3, 4> : decode_hdr_kernel<T, MAX_PS, 0>;
+        k<<<blocks, 128, 0, st>>>(frames, p, aligned, out);
+        return;
+    }
+    // Rows per warp: each warp reads two more than it decodes, so as many as
+    // leave DEC_MIN_WARPS warps per SM to cover the loads (1626x1236 Gray: 35 us
+    // with 24 warps, 38 with 40 and 42 with 64; larger images do not care).
+    const int nstrips = (p.cols + STRIP - 1) / STRIP;
+    const long long want = (long long)DEC_MIN_WARPS * (ctx->sm_count > 0 ? ctx->sm_count : 152);
+    int band = 32;
+    while (band > 4 && (long long)nstrips * ((p.rows + band - 1) / band) < want) band /= 2;
+    const long long warps = (long long)nstrips * ((p.rows + band - 1) / band);
+    const unsigned blocks = (unsigned)((warps + DEC_WARPS - 1) / DEC_WARPS);
+    auto k = p.n_ps == 3 && ns == 4 ? decode_strip_kernel<T, 3, 4>
+             : p.n_ps == 3 && ns == 8 ? decode_strip_kernel<T, 3, 8>
+             : p.n_ps == 1 && ns == 4 ? decode_strip_kernel<T, 1, 4>
+             : p.n_ps == 1 ? decode_strip_kernel<T, 1, 0> : decode_strip_kernel<T, MAX_PS, 0>;
+    k<<<blocks, 32 * DEC_WARPS, 0, st>>>(frames, p, band, nstrips, out);
 }
 
 // Absolute phase as f64 (startCalculate's CV_64F map; 0 where invalid), with
@@ -237,38 +525,19 @@ __global__ void phase_f64_kernel(const int32_t* __restrict__ order, const float*
 
 }  // namespace
 
-bool zim_decode_tma_applies(const void* frames, int sample_type, const zt::DecodeParams& p) {
-    CUtensorMap m;
-    int nfr = 0;
-    return sample_type == ZIM_SAMPLE_U8 ? decode_tensor_map<uint8_t>(frames, p, &m, &nfr)
-                                        : decode_tensor_map<uint16_t>(frames, p, &m, &nfr);
-}
-
-bool zim_decode_tma_launch(zim_ctx* ctx, const void* frames, int sample_type, const zt::DecodeParams& p,
-                           int32_t* order, float* residual, cudaStream_t st) {
-    dim3 blk(zt::DX, zt::DY), grd((p.cols + zt::DX - 1) / zt::DX, (p.rows + zt::DY - 1) / zt::DY);
-    const bool ok = sample_type == ZIM_SAMPLE_U8
-                        ? launch_decode_tma<uint8_t>(ctx, frames, p, grd, blk, order, residual, nullptr, nullptr, st)
-                        : launch_decode_tma<uint16_t>(ctx, frames, p, grd, blk, order, residual, nullptr, nullptr, st);
-    if (ok) ctx->launches += 1;
-    return ok;
+void zim_decode_params_launch(zim_ctx* ctx, const void* frames, int sample_type, const zt::DecodeParams& p,
+                              int32_t* order, float* residual, float* mod, uint8_t* valid, cudaStream_t st) {
+    const Outputs out{order, residual, mod, valid};
+    if (sample_type == ZIM_SAMPLE_U8) launch_decode(ctx, (const uint8_t*)frames, p, out, st);
+    else launch_decode(ctx, (const uint16_t*)frames, p, out, st);
+    ctx->launches += 1;
 }
 
 zim_status zim_decode_launch(zim_ctx* ctx, const zim_decode_config* cfg, const void* frames, int sample_type, int rows,
                              int cols, int32_t* order, float* residual, float* mod, uint8_t* valid, cudaStream_t st) {
     DecodeParams p;
     zt::decode_params(cfg, rows, cols, p);
-    dim3 blk(zt::DX, zt::DY), grd((cols + zt::DX - 1) / zt::DX, (rows + zt::DY - 1) / zt::DY);
-    // the bulk tensor copy path where it applies, else per-thread loads
-    const bool u8 = sample_type == ZIM_SAMPLE_U8;
-    const bool tma = u8 ? launch_decode_tma<uint8_t>(ctx, frames, p, grd, blk, order, residual, mod, valid, st)
-                        : launch_decode_tma<uint16_t>(ctx, frames, p, grd, blk, order, residual, mod, valid, st);
-    if (tma) {
-    } else if (u8)
-        decode_kernel<uint8_t><<<grd, blk, 0, st>>>((const uint8_t*)frames, p, order, residual, mod, valid);
-    else
-        decode_kernel<uint16_t><<<grd, blk, 0, st>>>((const uint16_t*)frames, p, order, residual, mod, valid);
-    ctx->launches += 1;
+    zim_decode_params_launch(ctx, frames, sample_type, p, order, residual, mod, valid, st);
     ZIM_LAUNCH_CHECK(ctx);
     return ZIM_OK;
 }

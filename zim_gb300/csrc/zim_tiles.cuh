@@ -18,8 +18,7 @@ namespace zt {
 
 // ---------------------------------------------------------------- decode ----
 
-constexpr int DX = 32, DY = 8;  // decode tile (threads of a block, as DX x DY)
-constexpr int DHX = DX + 2, DHY = DY + 2;
+constexpr int DX = 32, DY = 8;  // source-image tile of the batch's post-smooth queue
 
 struct DecodeParams {
     int rows, cols, enc, n_ps;
@@ -94,307 +93,6 @@ inline void decode_params(const zim_decode_config* c, int rows, int cols, Decode
     p.hdr = c->enable_hdr ? 1 : 0;
     p.hdr_sat = (float)c->hdr_saturation_gray;
     p.hdr_min_amp = (float)c->hdr_min_amplitude;
-}
-
-// HDR fit of one frequency at one pixel (JSLAB_HDRPhaseFit.h:10-61 and
-// JSLAB_PhaseShiftDecoder_V2.cpp:73-90): raw samples with 0 <= I < saturation
-// enter an equal-variance least-squares fit of I = A + C cos d - S sin d
-// (solved here from the 3x3 normal equations, the reference's cached
-// pseudo-inverse of the same subset); fewer than three samples, amplitude
-// hypot(C, S) <= min_amp or A <= 1e-3 reject the pixel.  Returns the sums the
-// phase-shift path would have formed: sin_sum = S N/2, cos_sum = C N/2,
-// sum = A N.
-template <typename T>
-__device__ __forceinline__ bool hdr_fit(const T* __restrict__ f0, size_t npx, int N, const float* sv, const float* cv,
-                                        float sat, float min_amp, float& sin_sum, float& cos_sum, float& sum) {
-    float m00 = 0.f, m01 = 0.f, m02 = 0.f, m11 = 0.f, m12 = 0.f, m22 = 0.f, r0 = 0.f, r1 = 0.f, r2 = 0.f;
-    int n = 0;
-    for (int k = 0; k < N; k++) {
-        const float v = (float)__ldg(f0 + (size_t)k * npx);
-        if (!(v >= 0.f && v < sat)) continue;
-        const float c = cv[k], s = -sv[k];
-        m00 += 1.f; m01 += c; m02 += s;
-        m11 = fmaf(c, c, m11); m12 = fmaf(c, s, m12); m22 = fmaf(s, s, m22);
-        r0 += v; r1 = fmaf(c, v, r1); r2 = fmaf(s, v, r2);
-        n++;
-    }
-    if (n < 3) return false;
-    // symmetric 3x3 inverse by cofactors
-    const float c00 = fmaf(m11, m22, -m12 * m12), c01 = fmaf(m02, m12, -m01 * m22), c02 = fmaf(m01, m12, -m02 * m11);
-    const float det = fmaf(m00, c00, fmaf(m01, c01, m02 * c02));
-    if (!(fabsf(det) > 1e-6f * m00 * m00 * m00)) return false;
-    const float c11 = fmaf(m00, m22, -m02 * m02), c12 = fmaf(m01, m02, -m00 * m12), c22 = fmaf(m00, m11, -m01 * m01);
-    const float id = 1.0f / det;
-    const float A = fmaf(c00, r0, fmaf(c01, r1, c02 * r2)) * id;
-    const float C = fmaf(c01, r0, fmaf(c11, r1, c12 * r2)) * id;
-    const float S = fmaf(c02, r0, fmaf(c12, r1, c22 * r2)) * id;
-    if (!(hypotf(C, S) > min_amp) || !(A > 1e-3f)) return false;
-    sin_sum = S * (float)N * 0.5f;
-    cos_sum = C * (float)N * 0.5f;
-    sum = A * (float)N;
-    return true;
-}
-
-// floor(a / b) for b > 0 and |a / b| < 2^21, from the float reciprocal
-// inv_b = 1 / b: the float quotient is within one of the true one, and one
-// remainder check corrects it (an integer division costs ~40 instructions).
-__device__ __forceinline__ int floor_div(int a, int b, float inv_b) {
-    int q = __float2int_rd((float)a * inv_b);
-    const int r = a - q * b;
-    q += (r >= b) - (r < 0);
-    return q;
-}
-
-// Shared memory of one decode tile: the raw per-pixel sums of the tile + halo,
-// the phase-shift pair (S, C) as one float2 so that both are staged, loaded
-// and blurred by paired FP32 instructions (__ffma2_rn: each lane rounded as
-// the scalar fmaf, so the sums are those of the scalar sequence).
-constexpr int DEC_MAX_PS = 4;  // phase-shift frequencies staged together
-struct DecodeSmem {
-    float2 SC[DEC_MAX_PS][DHY][DHX + 1];
-    float M[DEC_MAX_PS][DHY][DHX + 1];
-};
-
-// sc += (-sin_k, cos_k) v: the S and C sums of one sample in one paired FMA
-__device__ __forceinline__ float2 sc_add(float2 sc, float sn, float cs, float v) {
-    return __ffma2_rn(make_float2(-sn, cs), make_float2(v, v), sc);
-}
-
-// Four-quadrant arctangent of the wrapped phase.  The octant ratio
-// t = min(|y|, |x|) / max(|y|, |x|) in [0, 1] gives atan(t) = t P(t^2) with P of
-// degree 7, fitted for this kernel by iteratively reweighted least squares on
-// Chebyshev nodes (absolute error 3.7e-8 in exact arithmetic, 1.4e-7 evaluated
-// by FP32 Horner FMAs); the octant and quadrant follow by symmetry, with atan2's
-// signed zeros (the sign bits of y and x) and 0 for (0, 0).  __fdividef is
-// exact to 2 ulp for the divisor range of these sums (far below 2^126).
-__device__ __forceinline__ float phase_atan2(float y, float x) {
-    const float ax = fabsf(x), ay = fabsf(y);
-    const float hi = fmaxf(ax, ay), lo = fminf(ax, ay);
-    const float t = hi > 0.f ? __fdividef(lo, hi) : 0.f;
-    const float s = t * t;
-    float p = -0.004054566845297813f;
-    p = fmaf(p, s, 0.021862957626581192f);
-    p = fmaf(p, s, -0.0559123270213604f);
-    p = fmaf(p, s, 0.0964219719171524f);
-    p = fmaf(p, s, -0.1390862911939621f);
-    p = fmaf(p, s, 0.19946566224098206f);
-    p = fmaf(p, s, -0.33329859375953674f);
-    p = fmaf(p, s, 0.9999993443489075f);
-    float r = t * p;
-    if (ay > ax) r = 0.5f * ZIM_PI_F - r;
-    if (signbit(x)) r = ZIM_PI_F - r;
-    return copysignf(r, y);
-}
-
-// Raw sums of one halo pixel over the N frames of one frequency, four frames'
-// loads in flight at a time (the same accumulation order as one at a time).
-template <typename T>
-__device__ __forceinline__ void frame_sums(const T* __restrict__ src, size_t npx, int N, const float* sv,
-                                           const float* cv, float2& sc, float& m) {
-    sc = make_float2(0.f, 0.f);
-    m = 0.f;
-    int k = 0;
-    for (; k + 4 <= N; k += 4) {
-        const float v0 = (float)__ldg(src + (size_t)k * npx), v1 = (float)__ldg(src + (size_t)(k + 1) * npx);
-        const float v2 = (float)__ldg(src + (size_t)(k + 2) * npx), v3 = (float)__ldg(src + (size_t)(k + 3) * npx);
-        sc = sc_add(sc, sv[k], cv[k], v0); m += v0;
-        sc = sc_add(sc, sv[k + 1], cv[k + 1], v1); m += v1;
-        sc = sc_add(sc, sv[k + 2], cv[k + 2], v2); m += v2;
-        sc = sc_add(sc, sv[k + 3], cv[k + 3], v3); m += v3;
-    }
-    for (; k < N; k++) {
-        float v = (float)__ldg(src + (size_t)k * npx);
-        sc = sc_add(sc, sv[k], cv[k], v);
-        m += v;
-    }
-}
-
-// Raw per-pixel sums of the tile (bx, by) and its 1-pixel halo (clamped to the
-// image) into shared memory, every frequency in one pass: all of a pixel's
-// frame loads are issued before the tile waits.  Ends with a block barrier.
-template <typename T>
-__device__ __forceinline__ void decode_stage_sums(const T* __restrict__ frames, const DecodeParams& p, int bx, int by,
-                                                  int tid, DecodeSmem& sm) {
-    const int gx0 = bx * DX - 1, gy0 = by * DY - 1;
-    const size_t npx = (size_t)p.rows * p.cols;
-    for (int h = tid; h < DHX * DHY; h += DX * DY) {
-        const int hy = h / DHX, hx = h - hy * DHX;
-        const int gy = min(max(gy0 + hy, 0), p.rows - 1), gx = min(max(gx0 + hx, 0), p.cols - 1);
-        const size_t pix = (size_t)gy * p.cols + gx;
-#pragma unroll
-        for (int i = 0; i < DEC_MAX_PS; i++) {
-            if (i >= p.n_ps) break;
-            float2 sc;
-            float m;
-            frame_sums(frames + (size_t)p.fbase[i] * npx + pix, npx, p.shift[i], p.sinv + p.fbase[i],
-                       p.cosv + p.fbase[i], sc, m);
-            sm.SC[i][hy][hx] = sc;
-            sm.M[i][hy][hx] = m;
-        }
-    }
-    __syncthreads();
-}
-
-// The validity test on the normalised modulation nm = (2 |S, C| / N) / (M / N)
-// (0 when M <= 1e-3 N): nm < thr fails the pixel.  For M > 0 that is
-// 4 (S^2 + C^2) < (thr M)^2 with thr > 0, which needs neither the square root
-// nor the division; they are computed only where nm is written out
-// (want_value: frequency 0 with a modulation map).  The two forms decide
-// differently only where nm lies within float rounding of thr.
-__device__ __forceinline__ bool modulation_ok(float S, float C, float M, int N, float thr, bool want_value,
-                                              float& value) {
-    const float q = fmaf(S, S, C * C);
-    const bool has_m = M > 1e-3f * (float)N;
-    if (want_value) value = has_m ? 2.0f * sqrtf(q) / M : 0.f;
-    if (!(thr > 0.f)) return true;
-    const float tm = thr * M;
-    return has_m && !(4.0f * q < tm * tm);
-}
-
-// Decodes tile (bx, by) of DX x DY pixels with the DX * DY threads of a block
-// (tid = ty * DX + tx).  The pre-blur is linear, so the blurred sums
-// S = -sum sin_k I_k, C = sum cos_k I_k, sum I_k are the 3x3 blur of the raw
-// per-pixel sums, staged over the tile's 1-pixel halo in shared memory (by
-// decode_stage_sums or the caller, before this is called; not with HDR).
-// Ends with every thread past its last shared read, so the caller may start
-// the next tile at once.  NPS / NS: the frequency count and the frames per
-// frequency when known at compile time (0: taken from p); the arithmetic is
-// the same either way.
-template <typename T, int NPS = 0, int NS = 0>
-__device__ __forceinline__ void decode_finish(const T* __restrict__ frames, const DecodeParams& p, int bx, int by,
-                                              int tid, DecodeSmem& sm, int32_t* __restrict__ order,
-                                              float* __restrict__ residual, float* __restrict__ mod_out,
-                                              uint8_t* __restrict__ valid_out) {
-    const int tx = tid % DX, ty = tid / DX;
-    const int x = bx * DX + tx, y = by * DY + ty;
-    const size_t npx = (size_t)p.rows * p.cols;
-
-    float wrap0 = 0.f, wrap1 = 0.f, wrap2 = 0.f, wrap3 = 0.f;  // named, so they stay in registers
-    float mod0 = 0.f;
-    bool ok = true;
-    const bool inside = x < p.cols && y < p.rows;
-    const int n_ps = NPS ? NPS : p.n_ps;
-#pragma unroll
-    for (int i = 0; i < (NPS ? NPS : DEC_MAX_PS); i++) {
-        if (i >= n_ps) break;
-        const int N = NS ? NS : p.shift[i];
-        const T* fb = frames + (size_t)p.fbase[i] * npx;
-        const float* sv = p.sinv + p.fbase[i];
-        const float* cv = p.cosv + p.fbase[i];
-        if (p.hdr) {
-            // raw samples, no pre-blur: saturation is classified before any blur
-            float S = 0.f, C = 0.f, M = 0.f;
-            if (ok && inside && !hdr_fit(fb + (size_t)y * p.cols + x, npx, N, sv, cv, p.hdr_sat, p.hdr_min_amp, S, C, M))
-                ok = false;
-            if (ok) {
-                const float wr = phase_atan2(S, C);
-                if (i == 0) wrap0 = wr;
-                else if (i == 1) wrap1 = wr;
-                else if (i == 2) wrap2 = wr;
-                else wrap3 = wr;
-                if (!modulation_ok(S, C, M, N, p.thr, i == 0 && mod_out, mod0)) ok = false;
-            }
-            continue;
-        }
-        float2 SC = make_float2(0.f, 0.f);
-        float M = 0.f;
-#pragma unroll
-        for (int a = 0; a < 3; a++)
-#pragma unroll
-            for (int b = 0; b < 3; b++) {
-                float w = p.w2d[a * 3 + b];
-                SC = __ffma2_rn(make_float2(w, w), sm.SC[i][ty + a][tx + b], SC);
-                M = fmaf(w, sm.M[i][ty + a][tx + b], M);
-            }
-        const float S = SC.x, C = SC.y;
-        if (ok) {
-            const float wr = phase_atan2(S, C);
-            if (i == 0) wrap0 = wr;
-            else if (i == 1) wrap1 = wr;
-            else if (i == 2) wrap2 = wr;
-            else wrap3 = wr;
-            if (!modulation_ok(S, C, M, N, p.thr, i == 0 && mod_out, mod0)) ok = false;
-        }
-    }
-    // every thread is past its last shared read before the block's next tile
-    if (!p.hdr) __syncthreads();
-    if (x >= p.cols || y >= p.rows) return;
-    const size_t pix = (size_t)y * p.cols + x;
-    if (mod_out) mod_out[pix] = mod0;
-    int k = 0;
-    float r = 0.f;
-    if (ok) {
-        if (p.enc == ZIM_ENC_HETERODYNE3) {
-            const float w0 = wrap0, w1 = wrap1, w2 = wrap2;
-            float p12 = w0 > w1 ? w0 - w1 : w0 - w1 + ZIM_TWO_PI_F;
-            float p23;
-            if (p.f1_gt_f2) p23 = w1 > w2 ? w1 - w2 : w1 - w2 + ZIM_TWO_PI_F;
-            else p23 = w2 > w1 ? w2 - w1 : w2 - w1 + ZIM_TWO_PI_F;
-            float p123 = p12 > p23 ? p12 - p23 : p12 - p23 + ZIM_TWO_PI_F;
-            // uphase12 = p12 + 2 pi m12;  k = round(m12 f0 / f12 + (p12 f0 / f12 - w0) / 2 pi)
-            int m12 = (int)roundf(fmaf(p123, (float)p.f12, -p12) * ZIM_INV_TWO_PI_F);
-            int num = m12 * p.f0;
-            int q = floor_div(num, p.f12, p.inv_f12);
-            int rem = num - q * p.f12;
-            k = q + (int)roundf(fmaf((float)rem, p.inv_f12, fmaf(p12, p.f0_f12, -w0) * ZIM_INV_TWO_PI_F));
-            r = w0;
-            if (p.avg3) {
-                int m23 = (int)roundf(fmaf(p123, (float)p.f23, -p23) * ZIM_INV_TWO_PI_F);
-                int n2 = m23 * p.f1, q2 = floor_div(n2, p.f23, p.inv_f23), r2i = n2 - q2 * p.f23;
-                int k2 = q2 + (int)roundf(fmaf((float)r2i, p.inv_f23, fmaf(p23, p.f1_f23, -w1) * ZIM_INV_TWO_PI_F));
-                int n3 = m23 * p.f2, q3 = floor_div(n3, p.f23, p.inv_f23), r3i = n3 - q3 * p.f23;
-                int k3 = q3 + (int)roundf(fmaf((float)r3i, p.inv_f23, fmaf(p23, p.f2_f23, -w2) * ZIM_INV_TWO_PI_F));
-                // (uphase2 f0 / f1 - 2 pi k) = (w1 f0 + 2 pi (k2 f0 - k f1)) / f1, same for 3
-                float r2 = fmaf((float)(k2 * p.f0 - k * p.f1), ZIM_TWO_PI_F, w1 * (float)p.f0) * p.inv_f1;
-                float r3 = fmaf((float)(k3 * p.f0 - k * p.f2), ZIM_TWO_PI_F, w2 * (float)p.f0) * p.inv_f2;
-                r = (w0 + r2 + r3) * (1.0f / 3.0f);
-            }
-        } else if (p.enc == ZIM_ENC_HIERARCHICAL) {
-            const float wr[4] = {wrap0, wrap1, wrap2, wrap3};
-#pragma unroll
-            for (int i = 1; i < 4; i++) {
-                if (i < n_ps) {
-                    float a = fmaf(p.fratio[i], wr[i - 1] + ZIM_PI_F, -(wr[i] + ZIM_PI_F)) * ZIM_INV_TWO_PI_F;
-                    k = p.iratio[i] * k + (int)roundf(a);
-                    r = wr[i];
-                }
-            }
-            if (n_ps == 1) r = wrap0;
-        } else {
-            const int N = p.shift[0];
-            int sum_raw = 0;
-            for (int t = 0; t < N; t++) sum_raw += (int)__ldg(frames + (size_t)t * npx + pix);
-            int bin = 0, v1 = 0;
-            for (int b = 0; b < p.gray_bits; b++) {
-                int g = N * (int)__ldg(frames + (size_t)(p.gray_base + b) * npx + pix) > sum_raw ? 1 : 0;
-                bin ^= g;
-                v1 = (v1 << 1) | bin;
-            }
-            k = v1;
-            if (p.complementary) {
-                int g = N * (int)__ldg(frames + (size_t)(p.gray_base + p.gray_bits) * npx + pix) > sum_raw ? 1 : 0;
-                int v2 = (v1 << 1) | (bin ^ g);
-                int k2 = (v2 + 1) >> 1;
-                float w = wrap0;
-                if (w <= -0.5f * ZIM_PI_F) k = k2;
-                else if (w >= 0.5f * ZIM_PI_F) k = k2 - 1;
-            }
-            r = wrap0;
-        }
-    }
-    order[pix] = ok ? k : (p.hdr ? -1 : 0);  // the HDR decoder marks invalid orders -1
-    residual[pix] = r;
-    if (valid_out) valid_out[pix] = ok ? 1 : 0;
-}
-
-// One decode tile with its sums staged from global memory.
-template <typename T>
-__device__ __forceinline__ void decode_tile(const T* __restrict__ frames, const DecodeParams& p, int bx, int by,
-                                            int tid, DecodeSmem& sm, int32_t* __restrict__ order,
-                                            float* __restrict__ residual, float* __restrict__ mod_out,
-                                            uint8_t* __restrict__ valid_out) {
-    if (!p.hdr) decode_stage_sums(frames, p, bx, by, tid, sm);
-    decode_finish(frames, p, bx, by, tid, sm, order, residual, mod_out, valid_out);
 }
 
 // --------------------------------------------------------------- rectify ----
