@@ -35,7 +35,7 @@
 namespace {
 
 constexpr int BT = 256;  // threads per persistent CTA (one 32 x 8 tile)
-static_assert(BT == zt::DX * zt::DY && BT == zt::RX * zt::RY, "tile shape");
+static_assert(BT == zt::DX * zt::DY && BT == zt::RX * zt::RY && BT == 32 * zt::MED_WARPS, "tile shape");
 
 enum { Q_SMOOTH, Q_MATCH, Q_REPROJ, Q_PXG, Q_ROR, NQ };
 
@@ -177,10 +177,11 @@ __global__ void __launch_bounds__(BT) batch_reproject_kernel(const PairDev* __re
         if (it >= n_items) break;
         const int4 w = items[it];  // pair, first tile row, tile rows
         const PairDev& P = pairs[w.x];
-        const int tiles_x = (P.rw + zt::MTX - 1) / zt::MTX;
-        for (int ty = w.y; ty < w.y + w.z; ty++)
-            for (int tx = 0; tx < tiles_x; tx++)
-                zt::median_reproject_tile(P.disp_raw, P.rh, P.rw, P.rp, tx, ty, tid, sm, P.disp_out, P.x_rep, P.m_rep);
+        // the item's rows in strips, a warp each
+        const int nstrips = (P.rw + zt::MSTRIP - 1) / zt::MSTRIP;
+        for (int t = tid / 32; t < nstrips; t += zt::MED_WARPS)
+            zt::median_reproject_strip(P.disp_raw, P.rh, P.rw, P.rp, t, w.y * zt::RY,
+                                       min((w.y + w.z) * zt::RY, P.rh), tid / 32, sm, P.disp_out, P.x_rep, P.m_rep);
         __syncthreads();
     }
 }

@@ -14,12 +14,15 @@ using zt::ReprojParams;
 using zt::RX;
 using zt::RY;
 
-__global__ void __launch_bounds__(RX* RY) median_reproject_kernel(const float* __restrict__ disp, int rows, int cols,
-                                                                  ReprojParams p, float* __restrict__ disp_out,
-                                                                  float* __restrict__ xyz, uint8_t* __restrict__ mask) {
+__global__ void __launch_bounds__(32 * zt::MED_WARPS, 3) median_reproject_kernel(
+    const float* __restrict__ disp, int rows, int cols, const __grid_constant__ ReprojParams p, int band, int nstrips,
+    float* __restrict__ disp_out, float* __restrict__ xyz, uint8_t* __restrict__ mask) {
     __shared__ zt::MedianSmem sm;
-    zt::median_reproject_tile(disp, rows, cols, p, blockIdx.x, blockIdx.y, threadIdx.y * RX + threadIdx.x, sm,
-                              disp_out, xyz, mask);
+    const int w = threadIdx.x >> 5, id = blockIdx.x * zt::MED_WARPS + w;
+    const int y0 = (id / nstrips) * band;
+    if (y0 < rows)
+        zt::median_reproject_strip(disp, rows, cols, p, id % nstrips, y0, min(y0 + band, rows), w, sm, disp_out, xyz,
+                                   mask);
 }
 
 __global__ void px_gaussian_kernel(const float* __restrict__ xyz, const uint8_t* __restrict__ mask, int rows, int cols,
@@ -149,11 +152,23 @@ zim_status zim_median_reproject_launch(zim_ctx* ctx, const zim_recon_config* cfg
     ReprojParams p;
     zt::reproj_params(ctx->Q, ctx->R1, cfg, p);
     for (int k = 0; k < 3; k++) p.poly[k] = ctx->d_poly[k];
-    dim3 blk(RX, RY), grd((cols + zt::MTX - 1) / zt::MTX, (rows + RY - 1) / RY);
-    median_reproject_kernel<<<grd, blk, 0, st>>>(disp, rows, cols, p, disp_out, xyz, mask);
-    ctx->launches += 1;
+    zim_median_strips(ctx, p, disp, rows, cols, disp_out, xyz, mask, st);
     ZIM_LAUNCH_CHECK(ctx);
     return ZIM_OK;
+}
+
+// Rows per warp: a band loads four rows more than it writes, so the tallest that
+// leaves 32 warps per SM.
+void zim_median_strips(zim_ctx* ctx, const ReprojParams& p, const float* disp, int rows, int cols, float* disp_out,
+                       float* xyz, uint8_t* mask, cudaStream_t st) {
+    const int nstrips = (cols + zt::MSTRIP - 1) / zt::MSTRIP;
+    const long long want = 32ll * (ctx->sm_count > 0 ? ctx->sm_count : 152);
+    int band = 32;
+    while (band > 4 && (long long)nstrips * ((rows + band - 1) / band) < want) band /= 2;
+    const long long warps = (long long)nstrips * ((rows + band - 1) / band);
+    median_reproject_kernel<<<(unsigned)((warps + zt::MED_WARPS - 1) / zt::MED_WARPS), 32 * zt::MED_WARPS, 0, st>>>(
+        disp, rows, cols, p, band, nstrips, disp_out, xyz, mask);
+    ctx->launches += 1;
 }
 
 zim_status zim_px_gaussian_launch(zim_ctx* ctx, const float* xyz, const uint8_t* mask, int rows, int cols, float* out,

@@ -235,14 +235,6 @@ __global__ void ror_select_kernel(const unsigned long long* __restrict__ cnt, si
     m_out[i] = pre ? m_pre[i] : m_ror[i];
 }
 
-__global__ void roi_reproject_kernel(const float* __restrict__ disp, int rows, int cols, zt::ReprojParams p,
-                                     float* __restrict__ disp_out, float* __restrict__ xyz,
-                                     uint8_t* __restrict__ mask) {
-    __shared__ zt::MedianSmem sm;
-    zt::median_reproject_tile(disp, rows, cols, p, blockIdx.x, blockIdx.y, threadIdx.y * zt::RX + threadIdx.x, sm,
-                              disp_out, xyz, mask);
-}
-
 }  // namespace
 
 extern "C" ZIM_API zim_status zim_prepare_roi(zim_ctx* ctx, const zim_rotated_rect* roi, const int32_t* l_order,
@@ -387,9 +379,7 @@ extern "C" ZIM_API zim_status zim_reconstruct_roi(zim_ctx* ctx, const zim_recon_
     p.oy = L.y;
     p.gstride = RW;
     p.roi_mask = roi_mask;
-    dim3 blk(zt::RX, zt::RY), grd((W + zt::MTX - 1) / zt::MTX, (H + zt::RY - 1) / zt::RY);
-    roi_reproject_kernel<<<grd, blk, 0, st>>>(d_raw, H, W, p, d_med, xb[0], mb[0]);
-    ctx->launches += 1;
+    zim_median_strips(ctx, p, d_raw, H, W, d_med, xb[0], mb[0], st);
     ZIM_LAUNCH_CHECK(ctx);
 
     // the chain on the ROI cloud: xb[0]/mb[0] raw, then ping-pong through xb[1..2]

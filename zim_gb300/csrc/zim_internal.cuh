@@ -82,7 +82,11 @@ inline cudaStream_t zim_stream(void* s) { return reinterpret_cast<cudaStream_t>(
 // ---- internal launchers (no argument validation; callers validate) ----
 namespace zt {
 struct DecodeParams;
+struct ReprojParams;
 }
+// 5x5 median + reprojection of a disparity map with the parameters in hand.
+void zim_median_strips(zim_ctx* ctx, const zt::ReprojParams& p, const float* disp, int rows, int cols, float* disp_out,
+                       float* xyz, uint8_t* mask, cudaStream_t st);
 // One camera's decode with its parameters in hand (the batch's launches).
 void zim_decode_params_launch(zim_ctx* ctx, const void* frames, int sample_type, const zt::DecodeParams& p,
                               int32_t* order, float* residual, float* mod, uint8_t* valid, cudaStream_t st);
