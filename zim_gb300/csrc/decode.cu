@@ -69,32 +69,6 @@ __device__ __forceinline__ int floor_div(int a, int b, float inv_b) {
     return q;
 }
 
-// Four-quadrant arctangent of the wrapped phase.  The octant ratio
-// t = min(|y|, |x|) / max(|y|, |x|) in [0, 1] gives atan(t) = t P(t^2) with P of
-// degree 7, fitted for this kernel by iteratively reweighted least squares on
-// Chebyshev nodes (absolute error 3.7e-8 in exact arithmetic, 1.4e-7 evaluated
-// by FP32 Horner FMAs); the octant and quadrant follow by symmetry, with atan2's
-// signed zeros (the sign bits of y and x) and 0 for (0, 0).  __fdividef is
-// exact to 2 ulp for the divisor range of these sums (far below 2^126).
-__device__ __forceinline__ float phase_atan2(float y, float x) {
-    const float ax = fabsf(x), ay = fabsf(y);
-    const float hi = fmaxf(ax, ay), lo = fminf(ax, ay);
-    const float t = hi > 0.f ? __fdividef(lo, hi) : 0.f;
-    const float s = t * t;
-    float p = -0.004054566845297813f;
-    p = fmaf(p, s, 0.021862957626581192f);
-    p = fmaf(p, s, -0.0559123270213604f);
-    p = fmaf(p, s, 0.0964219719171524f);
-    p = fmaf(p, s, -0.1390862911939621f);
-    p = fmaf(p, s, 0.19946566224098206f);
-    p = fmaf(p, s, -0.33329859375953674f);
-    p = fmaf(p, s, 0.9999993443489075f);
-    float r = t * p;
-    if (ay > ax) r = 0.5f * ZIM_PI_F - r;
-    if (signbit(x)) r = ZIM_PI_F - r;
-    return copysignf(r, y);
-}
-
 // The validity test on the normalised modulation nm = (2 |S, C| / N) / (M / N)
 // (0 when M <= 1e-3 N): nm < thr fails the pixel.  For M > 0 that is
 // 4 (S^2 + C^2) < (thr M)^2 with thr > 0, which needs neither the square root
@@ -178,7 +152,7 @@ struct Pixel {
 // One frequency's blurred (or fitted) sums: wrapped phase and validity.
 __device__ __forceinline__ void take_frequency(const DecodeParams& p, int i, float S, float C, float M, bool want_mod,
                                                Pixel& px) {
-    px.w[i] = phase_atan2(S, C);
+    px.w[i] = zt::phase_atan2(S, C);
     float v = 0.f;
     const bool m = modulation_ok(S, C, M, p.shift[i], p.thr, want_mod && i == 0, v);
     if (i == 0) px.mod = px.ok ? v : 0.f;

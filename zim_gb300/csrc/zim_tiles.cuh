@@ -95,6 +95,32 @@ inline void decode_params(const zim_decode_config* c, int rows, int cols, Decode
     p.hdr_min_amp = (float)c->hdr_min_amplitude;
 }
 
+// Four-quadrant arctangent of the wrapped phase.  The octant ratio
+// t = min(|y|, |x|) / max(|y|, |x|) in [0, 1] gives atan(t) = t P(t^2) with P of
+// degree 7, fitted for this kernel by iteratively reweighted least squares on
+// Chebyshev nodes (absolute error 3.7e-8 in exact arithmetic, 1.4e-7 evaluated
+// by FP32 Horner FMAs); the octant and quadrant follow by symmetry, with atan2's
+// signed zeros (the sign bits of y and x) and 0 for (0, 0).  __fdividef is
+// exact to 2 ulp for the divisor range of these sums (far below 2^126).
+__device__ __forceinline__ float phase_atan2(float y, float x) {
+    const float ax = fabsf(x), ay = fabsf(y);
+    const float hi = fmaxf(ax, ay), lo = fminf(ax, ay);
+    const float t = hi > 0.f ? __fdividef(lo, hi) : 0.f;
+    const float s = t * t;
+    float p = -0.004054566845297813f;
+    p = fmaf(p, s, 0.021862957626581192f);
+    p = fmaf(p, s, -0.0559123270213604f);
+    p = fmaf(p, s, 0.0964219719171524f);
+    p = fmaf(p, s, -0.1390862911939621f);
+    p = fmaf(p, s, 0.19946566224098206f);
+    p = fmaf(p, s, -0.33329859375953674f);
+    p = fmaf(p, s, 0.9999993443489075f);
+    float r = t * p;
+    if (ay > ax) r = 0.5f * ZIM_PI_F - r;
+    if (signbit(x)) r = ZIM_PI_F - r;
+    return copysignf(r, y);
+}
+
 // --------------------------------------------------------------- rectify ----
 
 // Post-smoothed phase at a source pixel in exact integer + FP32 form:
