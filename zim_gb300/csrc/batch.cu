@@ -50,8 +50,7 @@ struct PairDev {
     float grad_threshold;
     int32_t* order[2];
     float* res[2];
-    int32_t* sk[2];  // post-smoothed taps (16 x cycles, residual), when post_smooth
-    float* sr[2];
+    int2* taps[2];  // post-smoothed taps (16 x cycles, residual), when post_smooth
     float* disp_raw;
     float* disp_out;
     float* x_rep;  // reprojection output
@@ -90,16 +89,15 @@ __global__ void __launch_bounds__(BT) batch_smooth_kernel(const PairDev* __restr
         if (it >= n_items) break;
         const int4 w = items[it];  // pair, camera, first tile row, tile rows
         const PairDev& P = pairs[w.x];
-        const int tiles_x = (P.cols + zt::DX - 1) / zt::DX;
-        for (int ty = w.z; ty < w.z + w.w; ty++)
-            for (int tx = 0; tx < tiles_x; tx++) {
-                const int x = tx * zt::DX + tid % zt::DX, y = ty * zt::DY + tid / zt::DX;
-                if (x >= P.cols || y >= P.rows) continue;
-                if (P.post_smooth == 2)
-                    zt::smooth_pixel_hdr(P.order[w.y], P.res[w.y], P.rows, P.cols, x, y, P.sk[w.y], P.sr[w.y]);
-                else
-                    zt::smooth_pixel(P.order[w.y], P.res[w.y], P.rows, P.cols, x, y, P.sk[w.y], P.sr[w.y]);
-            }
+        // the item's rows in strips, a warp each
+        const int nstrips = (P.cols + zt::SMOOTH_STRIP - 1) / zt::SMOOTH_STRIP;
+        const int y0 = w.z * zt::DY, y1 = min((w.z + w.w) * zt::DY, P.rows);
+        for (int t = tid / 32; t < nstrips; t += BT / 32) {
+            if (P.post_smooth == 2)
+                zt::smooth_strip<true>(P.order[w.y], P.res[w.y], P.rows, P.cols, t, y0, y1, P.taps[w.y]);
+            else
+                zt::smooth_strip<false>(P.order[w.y], P.res[w.y], P.rows, P.cols, t, y0, y1, P.taps[w.y]);
+        }
         __syncthreads();
     }
 }
@@ -107,10 +105,9 @@ __global__ void __launch_bounds__(BT) batch_smooth_kernel(const PairDev* __restr
 __global__ void __launch_bounds__(BT) batch_match_kernel(const PairDev* __restrict__ pairs, const int4* __restrict__ items,
                                                          int n_items, unsigned* __restrict__ counter, int max_cols) {
     extern __shared__ int4 smem_raw[];
-    int* s_ord = reinterpret_cast<int*>(smem_raw);
-    int* s_base = s_ord + max_cols;
-    float* s_res = reinterpret_cast<float*>(s_base + max_cols);
-    int* s_lo = reinterpret_cast<int*>(s_res + max_cols);
+    int2* s_ph = reinterpret_cast<int2*>(smem_raw);
+    int* s_ord = reinterpret_cast<int*>(s_ph + max_cols);
+    int* s_lo = s_ord + max_cols;
     __shared__ int s_item;
     const int tid = threadIdx.x;
     for (;;) {
@@ -132,32 +129,31 @@ __global__ void __launch_bounds__(BT) batch_match_kernel(const PairDev* __restri
                 int32_t b, o;
                 float r;
                 if (P.post_smooth == 1 || P.post_smooth == 2)
-                    zt::rectify_pixel_smoothed(P.sk[1], P.sr[1], P.order[1], P.rows, P.cols,
+                    zt::rectify_pixel_smoothed(P.taps[1], P.order[1], P.rows, P.cols,
                                                __ldg(P.map[1][0] + ro + j), __ldg(P.map[1][1] + ro + j), b, r, o);
                 else
                     zt::rectify_pixel(P.order[1], P.res[1], P.rows, P.cols, __ldg(P.map[1][0] + ro + j),
                                       __ldg(P.map[1][1] + ro + j), P.post_smooth, b, r, o);
                 s_ord[j] = o;
-                s_base[j] = b;
-                s_res[j] = r;
+                s_ph[j] = make_int2(b, __float_as_int(r));
             }
             __syncthreads();
             zt::match_spans(s_ord, cols, pha_f, s_lo, s_hi, tid, BT);
             __syncthreads();
-            zt::match_spans_check(s_ord, s_base, s_res, cols, pha_f, s_hi, s_bad, tid, BT);
+            zt::match_spans_check(s_ord, s_ph, cols, pha_f, s_hi, s_bad, tid, BT);
             __syncthreads();
             for (int j = tid; j < cols; j += BT) {
                 int32_t bL, kL;
                 float rL;
                 if (P.post_smooth == 1 || P.post_smooth == 2)
-                    zt::rectify_pixel_smoothed(P.sk[0], P.sr[0], P.order[0], P.rows, P.cols,
+                    zt::rectify_pixel_smoothed(P.taps[0], P.order[0], P.rows, P.cols,
                                                __ldg(P.map[0][0] + ro + j), __ldg(P.map[0][1] + ro + j), bL, rL, kL);
                 else
                     zt::rectify_pixel(P.order[0], P.res[0], P.rows, P.cols, __ldg(P.map[0][0] + ro + j),
                                       __ldg(P.map[0][1] + ro + j), P.post_smooth, bL, rL, kL);
                 float d;
                 int best;
-                zt::match_pixel(j, kL, bL, rL, s_ord, s_base, s_res, s_lo, s_hi, s_bad, cols, pha_f, P.grad_threshold,
+                zt::match_pixel(j, kL, bL, rL, s_ord, s_ph, s_lo, s_hi, s_bad, cols, pha_f, P.grad_threshold,
                                 d, best);
                 P.disp_raw[ro + j] = d;
             }
@@ -196,14 +192,11 @@ __global__ void __launch_bounds__(BT) batch_pxg_kernel(const PairDev* __restrict
         if (it >= n_items) break;
         const int4 w = items[it];
         const PairDev& P = pairs[w.x];
-        const int tiles_x = (P.rw + zt::RX - 1) / zt::RX;
-        for (int ty = w.y; ty < w.y + w.z; ty++)
-            for (int tx = 0; tx < tiles_x; tx++) {
-                const int x = tx * zt::RX + tid % zt::RX, y = ty * zt::RY + tid / zt::RX;
-                if (x >= P.rw || y >= P.rh) continue;
-                zt::px_gaussian_pixel(P.x_rep, P.m_rep, P.rh, P.rw, x, y, P.pxg_w00, P.pxg_w01, P.pxg_w11, P.x_pxg,
-                                      P.m_pxg);
-            }
+        // the item's rows in strips, a warp each
+        const int nstrips = (P.rw + zt::PXG_STRIP - 1) / zt::PXG_STRIP;
+        for (int t = tid / 32; t < nstrips; t += BT / 32)
+            zt::px_gaussian_strip(P.x_rep, P.m_rep, P.rh, P.rw, t, w.y * zt::RY, min((w.y + w.z) * zt::RY, P.rh),
+                                  P.pxg_w00, P.pxg_w01, P.pxg_w11, P.x_pxg, P.m_pxg);
         __syncthreads();
     }
 }
@@ -222,8 +215,8 @@ __global__ void __launch_bounds__(BT) batch_ror_kernel(const PairDev* __restrict
         const int tiles_x = (P.rw + zt::RX - 1) / zt::RX;
         for (int ty = w.y; ty < w.y + w.z; ty++)
             for (int tx = 0; tx < tiles_x; tx++)
-                zt::ror_tile(P.x_ror_in, P.m_ror_in, P.rh, P.rw, tx, ty, tid, P.ror_r2, P.ror_min_nb, P.ror_hw,
-                             ror_smem, P.x_ror, P.m_ror);
+                zt::ror_tile(P.x_ror_in, P.m_ror_in, P.rh, P.rw, tx * zt::RX, ty * zt::RY, zt::RY, tid, P.ror_r2,
+                             P.ror_min_nb, P.ror_hw, ror_smem, P.x_ror, P.m_ror);
         __syncthreads();
     }
 }
@@ -652,7 +645,7 @@ extern "C" ZIM_API zim_status zim_batch_submit(zim_batch* b, const zim_batch_pai
     b->match_smem = (size_t)max_cols * 12 + (size_t)(max_pha + 1) * 12;
     ZIM_CUDA_TRY(ctx, cudaFuncSetAttribute(batch_match_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                            (int)b->match_smem));
-    b->ror_smem = b->use_ror ? zt::ror_smem_bytes(rcfg->radius_window_size / 2) : 0;
+    b->ror_smem = b->use_ror ? zt::ror_smem_bytes(rcfg->radius_window_size / 2, zt::RY) : 0;
     if (b->use_ror)
         ZIM_CUDA_TRY(ctx, cudaFuncSetAttribute(batch_ror_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                (int)b->ror_smem));
@@ -710,8 +703,7 @@ extern "C" ZIM_API zim_status zim_batch_submit(zim_batch* b, const zim_batch_pai
             D.order[c] = (int32_t*)take(src * 4);
             D.res[c] = (float*)take(src * 4);
             if (p.decode.post_smooth) {
-                D.sk[c] = (int32_t*)take(src * 4);
-                D.sr[c] = (float*)take(src * 4);
+                D.taps[c] = (int2*)take(src * 8);
             }
         }
         D.disp_raw = (float*)take(dst * 4);

@@ -264,25 +264,25 @@ __global__ void rectify_kernel(const int32_t* __restrict__ order, const float* _
 
 // Post-smooth once per source pixel (the reference smooths the decoded phase
 // map before setData, JSLAB_PhaseShiftDecoder_V2.cpp:274-295) ...
-__global__ void smooth_kernel(const int32_t* __restrict__ order, const float* __restrict__ res, int rows, int cols,
-                              int hdr, int32_t* __restrict__ K16, float* __restrict__ R) {
-    int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y;
-    if (x >= cols || y >= rows) return;
-    if (hdr) zt::smooth_pixel_hdr(order, res, rows, cols, x, y, K16, R);
-    else zt::smooth_pixel(order, res, rows, cols, x, y, K16, R);
+constexpr int SMOOTH_WARPS = 4;
+template <bool HDR>
+__global__ void __launch_bounds__(32 * SMOOTH_WARPS) smooth_kernel(const int32_t* __restrict__ order,
+                                                                   const float* __restrict__ res, int rows, int cols,
+                                                                   int band, int nstrips, int2* __restrict__ taps) {
+    const int id = blockIdx.x * SMOOTH_WARPS + (threadIdx.x >> 5), y0 = (id / nstrips) * band;
+    if (y0 < rows) zt::smooth_strip<HDR>(order, res, rows, cols, id % nstrips, y0, min(y0 + band, rows), taps);
 }
 
 // ... then remap the smoothed taps.
-__global__ void rectify_smoothed_kernel(const int32_t* __restrict__ K16, const float* __restrict__ R,
-                                        const int32_t* __restrict__ order, int srows, int scols,
-                                        const float* __restrict__ mapx, const float* __restrict__ mapy, int drows,
-                                        int dcols, int32_t* __restrict__ rbase, float* __restrict__ rres,
+__global__ void rectify_smoothed_kernel(const int2* __restrict__ taps, const int32_t* __restrict__ order, int srows,
+                                        int scols, const float* __restrict__ mapx, const float* __restrict__ mapy,
+                                        int drows, int dcols, int32_t* __restrict__ rbase, float* __restrict__ rres,
                                         int32_t* __restrict__ rorder) {
     int j = blockIdx.x * blockDim.x + threadIdx.x;
     int i = blockIdx.y * blockDim.y + threadIdx.y;
     if (j >= dcols || i >= drows) return;
     size_t o = (size_t)i * dcols + j;
-    zt::rectify_pixel_smoothed(K16, R, order, srows, scols, mapx[o], mapy[o], rbase[o], rres[o], rorder[o]);
+    zt::rectify_pixel_smoothed(taps, order, srows, scols, mapx[o], mapy[o], rbase[o], rres[o], rorder[o]);
 }
 
 // rectifyLeftImage: cv::remap INTER_LINEAR of an 8-bit image.  OpenCV rounds
@@ -480,33 +480,35 @@ extern "C" ZIM_API zim_status zim_get_rectify_maps(zim_ctx* ctx, int cam, float*
 }
 
 zim_status zim_rectify_launch(zim_ctx* ctx, int cam, const int32_t* order, const float* residual, int rows, int cols,
-                              int post_smooth, int32_t* smooth_k16, float* smooth_r, int32_t* rbase, float* rres,
-                              int32_t* rorder, cudaStream_t st) {
+                              int post_smooth, int2* taps, int32_t* rbase, float* rres, int32_t* rorder,
+                              cudaStream_t st) {
     dim3 blk(32, 8), grd((ctx->rect_w + 31) / 32, (ctx->rect_h + 7) / 8);
     if (post_smooth == 1 || post_smooth == 2) {
-        dim3 sgrd((cols + 31) / 32, (rows + 7) / 8);
-        smooth_kernel<<<sgrd, blk, 0, st>>>(order, residual, rows, cols, post_smooth == 2 ? 1 : 0, smooth_k16,
-                                            smooth_r);
-        rectify_smoothed_kernel<<<grd, blk, 0, st>>>(smooth_k16, smooth_r, order, rows, cols, ctx->d_map[cam][0],
-                                                     ctx->d_map[cam][1], ctx->rect_h, ctx->rect_w, rbase, rres,
-                                                     rorder);
-        ctx->launches += 2;
+        zim_status s = zim_smooth_launch(ctx, order, residual, rows, cols, post_smooth, taps, st);
+        if (s) return s;
+        rectify_smoothed_kernel<<<grd, blk, 0, st>>>(taps, order, rows, cols, ctx->d_map[cam][0], ctx->d_map[cam][1],
+                                                     ctx->rect_h, ctx->rect_w, rbase, rres, rorder);
     } else {
         rectify_kernel<<<grd, blk, 0, st>>>(order, residual, rows, cols, ctx->d_map[cam][0], ctx->d_map[cam][1],
                                             ctx->rect_h, ctx->rect_w, post_smooth, rbase, rres, rorder);
-        ctx->launches += 1;
     }
+    ctx->launches += 1;
     ZIM_LAUNCH_CHECK(ctx);
     return ZIM_OK;
 }
 
-// The post-smooth alone (post_smooth 1 or 2; nothing to do otherwise), for
-// the fused rectify + match of the whole-pair path.
+// The post-smooth alone (post_smooth 1 or 2; nothing to do otherwise).
 zim_status zim_smooth_launch(zim_ctx* ctx, const int32_t* order, const float* residual, int rows, int cols,
-                             int post_smooth, int32_t* smooth_k16, float* smooth_r, cudaStream_t st) {
+                             int post_smooth, int2* taps, cudaStream_t st) {
     if (post_smooth != 1 && post_smooth != 2) return ZIM_OK;
-    dim3 blk(32, 8), sgrd((cols + 31) / 32, (rows + 7) / 8);
-    smooth_kernel<<<sgrd, blk, 0, st>>>(order, residual, rows, cols, post_smooth == 2 ? 1 : 0, smooth_k16, smooth_r);
+    const int nstrips = (cols + zt::SMOOTH_STRIP - 1) / zt::SMOOTH_STRIP;
+    const int band = strip_band(ctx, nstrips, rows, 32);
+    const long long warps = (long long)nstrips * ((rows + band - 1) / band);
+    const unsigned blocks = (unsigned)((warps + SMOOTH_WARPS - 1) / SMOOTH_WARPS);
+    if (post_smooth == 2)
+        smooth_kernel<true><<<blocks, 32 * SMOOTH_WARPS, 0, st>>>(order, residual, rows, cols, band, nstrips, taps);
+    else
+        smooth_kernel<false><<<blocks, 32 * SMOOTH_WARPS, 0, st>>>(order, residual, rows, cols, band, nstrips, taps);
     ctx->launches += 1;
     ZIM_LAUNCH_CHECK(ctx);
     return ZIM_OK;
@@ -523,17 +525,15 @@ extern "C" ZIM_API zim_status zim_rectify(zim_ctx* ctx, int cam, const int32_t* 
         return zim_fail(ctx, ZIM_ERR_INVALID_ARG, "image size differs from calibration");
     ZIM_CUDA_TRY(ctx, cudaSetDevice(ctx->device));
     if (post_smooth < 0 || post_smooth > 3) return zim_fail(ctx, ZIM_ERR_INVALID_ARG, "post_smooth must be 0..3");
-    int32_t* sk = nullptr;
-    float* sr = nullptr;
+    int2* taps = nullptr;
     if (post_smooth == 1 || post_smooth == 2) {
         const size_t src = (size_t)rows * cols;
-        zim_status s = zim_scratch_reserve(ctx, 2 * zim_align256(src * 4) + 1024);
+        zim_status s = zim_scratch_reserve(ctx, zim_align256(src * 8) + 1024);
         if (s) return s;
         zim_scratch_reset(ctx);
-        sk = (int32_t*)zim_scratch_take(ctx, src * 4);
-        sr = (float*)zim_scratch_take(ctx, src * 4);
-        if (!sk || !sr) return zim_fail(ctx, ZIM_ERR_OUT_OF_MEMORY, "rectify scratch");
+        taps = (int2*)zim_scratch_take(ctx, src * 8);
+        if (!taps) return zim_fail(ctx, ZIM_ERR_OUT_OF_MEMORY, "rectify scratch");
     }
-    return zim_rectify_launch(ctx, cam, order, residual, rows, cols, post_smooth, sk, sr, rbase, rres, rorder,
+    return zim_rectify_launch(ctx, cam, order, residual, rows, cols, post_smooth, taps, rbase, rres, rorder,
                               zim_stream(stream));
 }

@@ -231,8 +231,7 @@ namespace {
 struct PairBuffers {
     int32_t* order[2];
     float* res[2];
-    int32_t* sk[2];  // post-smoothed taps (16 x cycles, residual)
-    float* sr[2];
+    int2* taps[2];  // post-smoothed taps (16 x cycles, residual)
     float* disp_raw;
     float* disp_med;
     float* xyz[2];
@@ -244,7 +243,7 @@ size_t pair_scratch_bytes(const zim_ctx* ctx, const zim_recon_config* r, int row
                           int sample_bytes, int frames, bool host) {
     size_t src = (size_t)rows * cols, dst = (size_t)ctx->rect_h * ctx->rect_w;
     size_t b = 0;
-    b += 2 * (zim_align256(src * 4) * 4);
+    b += 2 * (zim_align256(src * 4) * 2 + zim_align256(src * 8));
     b += zim_align256(dst * 4);
     if (need_disp) b += zim_align256(dst * 4);
     b += 2 * (zim_align256(dst * 12) + zim_align256(dst));
@@ -289,7 +288,7 @@ static zim_status run_pair(zim_ctx* ctx, const zim_decode_config* d, const zim_r
         if (c == 1 && right_ready) ZIM_CUDA_TRY(ctx, cudaStreamWaitEvent(st, right_ready, 0));
         s = zim_decode_launch(ctx, d, frames[c], sample_type, rows, cols, B.order[c], B.res[c], nullptr, nullptr, st);
         if (s) return s;
-        s = zim_smooth_launch(ctx, B.order[c], B.res[c], rows, cols, post, B.sk[c], B.sr[c], st);
+        s = zim_smooth_launch(ctx, B.order[c], B.res[c], rows, cols, post, B.taps[c], st);
         if (s) return s;
     }
     const int RH = ctx->rect_h, RW = ctx->rect_w;
@@ -298,7 +297,7 @@ static zim_status run_pair(zim_ctx* ctx, const zim_decode_config* d, const zim_r
     {
         const int32_t* ord[2] = {B.order[0], B.order[1]};
         const float* res[2] = {B.res[0], B.res[1]};
-        s = zim_rectify_match_launch(ctx, ord, res, B.sk, B.sr, rows, cols, post, pha_f, r->grad_threshold,
+        s = zim_rectify_match_launch(ctx, ord, res, B.taps, rows, cols, post, pha_f, r->grad_threshold,
                                      B.disp_raw, st);
         if (s) return s;
     }
@@ -396,8 +395,7 @@ static zim_status carve_pair(zim_ctx* ctx, const zim_recon_config* r, int rows, 
     for (int c = 0; c < 2; c++) {
         B.order[c] = (int32_t*)zim_scratch_take(ctx, src * 4);
         B.res[c] = (float*)zim_scratch_take(ctx, src * 4);
-        B.sk[c] = (int32_t*)zim_scratch_take(ctx, src * 4);
-        B.sr[c] = (float*)zim_scratch_take(ctx, src * 4);
+        B.taps[c] = (int2*)zim_scratch_take(ctx, src * 8);
         B.xyz[c] = (float*)zim_scratch_take(ctx, dst * 12);
         B.mask[c] = (uint8_t*)zim_scratch_take(ctx, dst);
     }
@@ -405,7 +403,7 @@ static zim_status carve_pair(zim_ctx* ctx, const zim_recon_config* r, int rows, 
     B.disp_med = disp_out ? disp_out : (float*)zim_scratch_take(ctx, dst * 4);
     B.mls_tmp = r->use_mls ? (float*)zim_scratch_take(ctx, dst * 12) : nullptr;
     for (int c = 0; c < 2; c++)
-        if (!B.order[c] || !B.res[c] || !B.sk[c] || !B.sr[c] || !B.xyz[c] || !B.mask[c])
+        if (!B.order[c] || !B.res[c] || !B.taps[c] || !B.xyz[c] || !B.mask[c])
             return zim_fail(ctx, ZIM_ERR_OUT_OF_MEMORY, "scratch carve failed");
     if (!B.disp_raw || !B.disp_med || (r->use_mls && !B.mls_tmp))
         return zim_fail(ctx, ZIM_ERR_OUT_OF_MEMORY, "scratch carve failed");

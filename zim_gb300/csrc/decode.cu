@@ -446,13 +446,10 @@ void launch_decode(zim_ctx* ctx, const T* frames, const DecodeParams& p, const O
         k<<<blocks, 128, 0, st>>>(frames, p, aligned, out);
         return;
     }
-    // Rows per warp: each warp reads two more than it decodes, so as many as
-    // leave DEC_MIN_WARPS warps per SM to cover the loads (1626x1236 Gray: 35 us
-    // with 24 warps, 38 with 40 and 42 with 64; larger images do not care).
+    // (1626x1236 Gray: 35 us with 24 warps per SM, 38 with 40 and 42 with 64; larger
+    // images do not care)
     const int nstrips = (p.cols + STRIP - 1) / STRIP;
-    const long long want = (long long)DEC_MIN_WARPS * (ctx->sm_count > 0 ? ctx->sm_count : 152);
-    int band = 32;
-    while (band > 4 && (long long)nstrips * ((p.rows + band - 1) / band) < want) band /= 2;
+    const int band = strip_band(ctx, nstrips, p.rows, DEC_MIN_WARPS);
     const long long warps = (long long)nstrips * ((p.rows + band - 1) / band);
     const unsigned blocks = (unsigned)((warps + DEC_WARPS - 1) / DEC_WARPS);
     auto k = p.n_ps == 3 && ns == 4 ? decode_strip_kernel<T, 3, 4>

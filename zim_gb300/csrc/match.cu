@@ -10,7 +10,7 @@
 // shared-memory atomics and checked for a strictly rising phase; each left
 // pixel of order k in [1, pha_f] finds the first column of minimum
 // |phase_R - phase_L| among the right pixels of order k (strict <, so the
-// smallest column wins ties) -- by binary search on a checked span, by a scan
+// smallest column wins ties) -- by a bracketing search on a checked span, by a scan
 // of the span otherwise, the same column either way -- rejects
 // min >= grad_threshold and columns < 2 or >= cols - 1, then refines with the
 // parabola through the costs of columns best-1, best, best+1.
@@ -40,10 +40,9 @@ struct MatchWin {
 __global__ void __launch_bounds__(MATCH_THREADS) match_kernel(MatchWin w, int pha_f, float grad_threshold) {
     extern __shared__ int4 smem_raw[];
     const int cols = w.r_cols;
-    int* s_ord = reinterpret_cast<int*>(smem_raw);
-    int* s_base = s_ord + cols;
-    float* s_res = reinterpret_cast<float*>(s_base + cols);
-    int* s_lo = reinterpret_cast<int*>(s_res + cols);
+    int2* s_ph = reinterpret_cast<int2*>(smem_raw);
+    int* s_ord = reinterpret_cast<int*>(s_ph + cols);
+    int* s_lo = s_ord + cols;
     int* s_hi = s_lo + (pha_f + 1);
     int* s_bad = s_hi + (pha_f + 1);
 
@@ -56,20 +55,19 @@ __global__ void __launch_bounds__(MATCH_THREADS) match_kernel(MatchWin w, int ph
     }
     for (int j = threadIdx.x; j < cols; j += blockDim.x) {
         s_ord[j] = w.r_order[ro + j];
-        s_base[j] = w.r_base[ro + j];
-        s_res[j] = w.r_res[ro + j];
+        s_ph[j] = make_int2(w.r_base[ro + j], __float_as_int(w.r_res[ro + j]));
     }
     __syncthreads();
     zt::match_spans(s_ord, cols, pha_f, s_lo, s_hi, threadIdx.x, blockDim.x);
     __syncthreads();
-    zt::match_spans_check(s_ord, s_base, s_res, cols, pha_f, s_hi, s_bad, threadIdx.x, blockDim.x);
+    zt::match_spans_check(s_ord, s_ph, cols, pha_f, s_hi, s_bad, threadIdx.x, blockDim.x);
     __syncthreads();
     const size_t oo = (size_t)row * w.out_stride;
     for (int j = threadIdx.x; j < w.l_cols; j += blockDim.x) {
         float d = 0.f;
         int best = -1;
         if (!w.l_mask || w.l_mask[ro + j])
-            zt::match_pixel(j, w.l_order[ro + j], w.l_base[ro + j], w.l_res[ro + j], s_ord, s_base, s_res, s_lo,
+            zt::match_pixel(j, w.l_order[ro + j], w.l_base[ro + j], w.l_res[ro + j], s_ord, s_ph, s_lo,
                             s_hi, s_bad, cols, pha_f, grad_threshold, d, best, w.dx_off);
         w.disp[oo + j] = d;
         if (w.best_col) w.best_col[oo + j] = best;
@@ -91,13 +89,12 @@ zim_status launch_match(zim_ctx* ctx, const MatchWin& w, int rows, int pha_f, do
 // rectified row rectifies the right row straight into shared memory and each
 // left pixel in registers (the setData remap, zt::rectify_pixel[_smoothed], so
 // the results are those of rectify + match), and the rectified maps never
-// reach global memory.  post_smooth 1 / 2: sk / sr hold the post-smoothed taps
+// reach global memory.  post_smooth 1 / 2: taps holds the post-smoothed taps
 // of each camera (smooth_kernel); 0 / 3: the remap reads order / residual.
 struct RectMatchArgs {
     const int32_t* order[2];
     const float* res[2];
-    const int32_t* sk[2];
-    const float* sr[2];
+    const int2* taps[2];
     const float* map[2][2];
     int srows, scols, rows, cols, post_smooth;
     float* disp;
@@ -106,7 +103,7 @@ struct RectMatchArgs {
 __device__ __forceinline__ void rect_px(const RectMatchArgs& a, int cam, float mx, float my, int32_t& b, float& r,
                                         int32_t& k) {
     if (a.post_smooth == 1 || a.post_smooth == 2)
-        zt::rectify_pixel_smoothed(a.sk[cam], a.sr[cam], a.order[cam], a.srows, a.scols, mx, my, b, r, k);
+        zt::rectify_pixel_smoothed(a.taps[cam], a.order[cam], a.srows, a.scols, mx, my, b, r, k);
     else
         zt::rectify_pixel(a.order[cam], a.res[cam], a.srows, a.scols, mx, my, a.post_smooth, b, r, k);
 }
@@ -115,10 +112,9 @@ __global__ void __launch_bounds__(MATCH_THREADS) rectify_match_kernel(RectMatchA
                                                                       float grad_threshold) {
     extern __shared__ int4 smem_raw[];
     const int cols = a.cols;
-    int* s_ord = reinterpret_cast<int*>(smem_raw);
-    int* s_base = s_ord + cols;
-    float* s_res = reinterpret_cast<float*>(s_base + cols);
-    int* s_lo = reinterpret_cast<int*>(s_res + cols);
+    int2* s_ph = reinterpret_cast<int2*>(smem_raw);
+    int* s_ord = reinterpret_cast<int*>(s_ph + cols);
+    int* s_lo = s_ord + cols;
     int* s_hi = s_lo + (pha_f + 1);
     int* s_bad = s_hi + (pha_f + 1);
     const int row = blockIdx.x;
@@ -143,8 +139,7 @@ __global__ void __launch_bounds__(MATCH_THREADS) rectify_match_kernel(RectMatchA
         float r;
         rect_px(a, 1, mx, my, b, r, k);
         s_ord[j] = k;
-        s_base[j] = b;
-        s_res[j] = r;
+        s_ph[j] = make_int2(b, __float_as_int(r));
         mx = nx;
         my = ny;
     }
@@ -156,7 +151,7 @@ __global__ void __launch_bounds__(MATCH_THREADS) rectify_match_kernel(RectMatchA
     __syncthreads();
     zt::match_spans(s_ord, cols, pha_f, s_lo, s_hi, threadIdx.x, blockDim.x);
     __syncthreads();
-    zt::match_spans_check(s_ord, s_base, s_res, cols, pha_f, s_hi, s_bad, threadIdx.x, blockDim.x);
+    zt::match_spans_check(s_ord, s_ph, cols, pha_f, s_hi, s_bad, threadIdx.x, blockDim.x);
     __syncthreads();
     for (; j < cols; j += blockDim.x) {
         const int jn = j + blockDim.x;
@@ -169,7 +164,7 @@ __global__ void __launch_bounds__(MATCH_THREADS) rectify_match_kernel(RectMatchA
         my = ny;
         float d;
         int best;
-        zt::match_pixel(j, kL, bL, rL, s_ord, s_base, s_res, s_lo, s_hi, s_bad, cols, pha_f, grad_threshold, d,
+        zt::match_pixel(j, kL, bL, rL, s_ord, s_ph, s_lo, s_hi, s_bad, cols, pha_f, grad_threshold, d,
                         best);
         a.disp[ro + j] = d;
     }
@@ -178,16 +173,15 @@ __global__ void __launch_bounds__(MATCH_THREADS) rectify_match_kernel(RectMatchA
 }  // namespace
 
 // The plain path's rectify + match of both cameras (see rectify_match_kernel);
-// sk / sr: per camera the post-smoothed taps (post_smooth 1 or 2), else null.
+// taps: per camera the post-smoothed taps (post_smooth 1 or 2), else null.
 zim_status zim_rectify_match_launch(zim_ctx* ctx, const int32_t* const order[2], const float* const res[2],
-                                    int32_t* const sk[2], float* const sr[2], int srows, int scols, int post_smooth,
+                                    int2* const taps[2], int srows, int scols, int post_smooth,
                                     int pha_f, double grad_threshold, float* disp, cudaStream_t st) {
     RectMatchArgs a{};
     for (int c = 0; c < 2; c++) {
         a.order[c] = order[c];
         a.res[c] = res[c];
-        a.sk[c] = sk[c];
-        a.sr[c] = sr[c];
+        a.taps[c] = taps[c];
         a.map[c][0] = ctx->d_map[c][0];
         a.map[c][1] = ctx->d_map[c][1];
     }
@@ -256,23 +250,21 @@ extern "C" ZIM_API zim_status zim_rectify_match(zim_ctx* ctx, const int32_t* l_o
     if (post_smooth < 0 || post_smooth > 3) return zim_fail(ctx, ZIM_ERR_INVALID_ARG, "post_smooth must be 0..3");
     if (pha_f < 0 || pha_f > ZIM_MAX_ORDER) return zim_fail(ctx, ZIM_ERR_INVALID_ARG, "pha_f out of range");
     ZIM_CUDA_TRY(ctx, cudaSetDevice(ctx->device));
-    int32_t* sk[2] = {nullptr, nullptr};
-    float* sr[2] = {nullptr, nullptr};
+    int2* taps[2] = {nullptr, nullptr};
     cudaStream_t st = zim_stream(stream);
     const int32_t* ord[2] = {l_order, r_order};
     const float* res[2] = {l_res, r_res};
     if (post_smooth == 1 || post_smooth == 2) {
         const size_t src = (size_t)rows * cols;
-        zim_status s = zim_scratch_reserve(ctx, 4 * zim_align256(src * 4) + 1024);
+        zim_status s = zim_scratch_reserve(ctx, 2 * zim_align256(src * 8) + 1024);
         if (s) return s;
         zim_scratch_reset(ctx);
         for (int c = 0; c < 2; c++) {
-            sk[c] = (int32_t*)zim_scratch_take(ctx, src * 4);
-            sr[c] = (float*)zim_scratch_take(ctx, src * 4);
-            if (!sk[c] || !sr[c]) return zim_fail(ctx, ZIM_ERR_OUT_OF_MEMORY, "rectify scratch");
-            s = zim_smooth_launch(ctx, ord[c], res[c], rows, cols, post_smooth, sk[c], sr[c], st);
+            taps[c] = (int2*)zim_scratch_take(ctx, src * 8);
+            if (!taps[c]) return zim_fail(ctx, ZIM_ERR_OUT_OF_MEMORY, "rectify scratch");
+            s = zim_smooth_launch(ctx, ord[c], res[c], rows, cols, post_smooth, taps[c], st);
             if (s) return s;
         }
     }
-    return zim_rectify_match_launch(ctx, ord, res, sk, sr, rows, cols, post_smooth, pha_f, grad_threshold, disp, st);
+    return zim_rectify_match_launch(ctx, ord, res, taps, rows, cols, post_smooth, pha_f, grad_threshold, disp, st);
 }

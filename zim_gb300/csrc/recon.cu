@@ -25,20 +25,25 @@ __global__ void __launch_bounds__(32 * zt::MED_WARPS, 3) median_reproject_kernel
                                    mask);
 }
 
-__global__ void px_gaussian_kernel(const float* __restrict__ xyz, const uint8_t* __restrict__ mask, int rows, int cols,
-                                   float w00, float w01, float w11, float* __restrict__ out,
-                                   uint8_t* __restrict__ mask_out) {
-    int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y;
-    if (x >= cols || y >= rows) return;
-    zt::px_gaussian_pixel(xyz, mask, rows, cols, x, y, w00, w01, w11, out, mask_out);
+constexpr int PXG_WARPS = 4;
+constexpr size_t ROR_SMEM = 52 * 1024;  // shared memory of a radius-filter tile taller than RY rows
+__global__ void __launch_bounds__(32 * PXG_WARPS) px_gaussian_kernel(const float* __restrict__ xyz,
+                                                                     const uint8_t* __restrict__ mask, int rows,
+                                                                     int cols, int band, int nstrips, float w00,
+                                                                     float w01, float w11, float* __restrict__ out,
+                                                                     uint8_t* __restrict__ mask_out) {
+    const int id = blockIdx.x * PXG_WARPS + (threadIdx.x >> 5), y0 = (id / nstrips) * band;
+    if (y0 < rows)
+        zt::px_gaussian_strip(xyz, mask, rows, cols, id % nstrips, y0, min(y0 + band, rows), w00, w01, w11, out,
+                              mask_out);
 }
 
 __global__ void __launch_bounds__(RX* RY) ror_kernel(const float* __restrict__ xyz, const uint8_t* __restrict__ mask,
-                                                     int rows, int cols, float r2, int min_nb, int hw,
+                                                     int rows, int cols, int th, float r2, int min_nb, int hw,
                                                      float* __restrict__ out, uint8_t* __restrict__ mask_out) {
     extern __shared__ float4 ror_smem[];
-    zt::ror_tile(xyz, mask, rows, cols, blockIdx.x, blockIdx.y, threadIdx.y * RX + threadIdx.x, r2, min_nb, hw,
-                 ror_smem, out, mask_out);
+    zt::ror_tile(xyz, mask, rows, cols, blockIdx.x * RX, blockIdx.y * th, th, threadIdx.x, r2, min_nb, hw, ror_smem, out,
+                 mask_out);
 }
 
 constexpr int CB = 1024;  // compaction block
@@ -157,14 +162,10 @@ zim_status zim_median_reproject_launch(zim_ctx* ctx, const zim_recon_config* cfg
     return ZIM_OK;
 }
 
-// Rows per warp: a band loads four rows more than it writes, so the tallest that
-// leaves 32 warps per SM.
 void zim_median_strips(zim_ctx* ctx, const ReprojParams& p, const float* disp, int rows, int cols, float* disp_out,
                        float* xyz, uint8_t* mask, cudaStream_t st) {
     const int nstrips = (cols + zt::MSTRIP - 1) / zt::MSTRIP;
-    const long long want = 32ll * (ctx->sm_count > 0 ? ctx->sm_count : 152);
-    int band = 32;
-    while (band > 4 && (long long)nstrips * ((rows + band - 1) / band) < want) band /= 2;
+    const int band = strip_band(ctx, nstrips, rows, 32);
     const long long warps = (long long)nstrips * ((rows + band - 1) / band);
     median_reproject_kernel<<<(unsigned)((warps + zt::MED_WARPS - 1) / zt::MED_WARPS), 32 * zt::MED_WARPS, 0, st>>>(
         disp, rows, cols, p, band, nstrips, disp_out, xyz, mask);
@@ -175,8 +176,10 @@ zim_status zim_px_gaussian_launch(zim_ctx* ctx, const float* xyz, const uint8_t*
                                   uint8_t* mask_out, cudaStream_t st) {
     float w00, w01, w11;
     zt::px_gaussian_weights(w00, w01, w11);
-    dim3 blk(32, 8), grd((cols + 31) / 32, (rows + 7) / 8);
-    px_gaussian_kernel<<<grd, blk, 0, st>>>(xyz, mask, rows, cols, w00, w01, w11, out, mask_out);
+    const int nstrips = (cols + zt::PXG_STRIP - 1) / zt::PXG_STRIP, band = strip_band(ctx, nstrips, rows, 32);
+    const long long warps = (long long)nstrips * ((rows + band - 1) / band);
+    px_gaussian_kernel<<<(unsigned)((warps + PXG_WARPS - 1) / PXG_WARPS), 32 * PXG_WARPS, 0, st>>>(
+        xyz, mask, rows, cols, band, nstrips, w00, w01, w11, out, mask_out);
     ctx->launches += 1;
     ZIM_LAUNCH_CHECK(ctx);
     return ZIM_OK;
@@ -185,10 +188,17 @@ zim_status zim_px_gaussian_launch(zim_ctx* ctx, const float* xyz, const uint8_t*
 zim_status zim_ror_launch(zim_ctx* ctx, const float* xyz, const uint8_t* mask, int rows, int cols, float radius,
                           int min_neighbors, int window_size, float* out, uint8_t* mask_out, cudaStream_t st) {
     const int hw = window_size / 2;
-    const size_t smem = zt::ror_smem_bytes(hw);
+    // Rows per tile: tall tiles stage less halo per point, as long as four CTAs
+    // share an SM and the launch fills it
+    int th = 32;
+    const long long want = 4ll * (ctx->sm_count > 0 ? ctx->sm_count : 152);
+    while (th > RY && (zt::ror_smem_bytes(hw, th) > ROR_SMEM ||
+                       (long long)((cols + RX - 1) / RX) * ((rows + th - 1) / th) < want))
+        th /= 2;
+    const size_t smem = zt::ror_smem_bytes(hw, th);
     ZIM_CUDA_TRY(ctx, cudaFuncSetAttribute(ror_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    dim3 blk(RX, RY), grd((cols + RX - 1) / RX, (rows + RY - 1) / RY);
-    ror_kernel<<<grd, blk, smem, st>>>(xyz, mask, rows, cols, radius * radius, min_neighbors, hw, out, mask_out);
+    dim3 grd((cols + RX - 1) / RX, (rows + th - 1) / th);
+    ror_kernel<<<grd, RX * RY, smem, st>>>(xyz, mask, rows, cols, th, radius * radius, min_neighbors, hw, out, mask_out);
     ctx->launches += 1;
     ZIM_LAUNCH_CHECK(ctx);
     return ZIM_OK;

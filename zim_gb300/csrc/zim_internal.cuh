@@ -79,6 +79,16 @@ inline size_t zim_align256(size_t b) { return (b + 255) & ~(size_t)255; }
 
 inline cudaStream_t zim_stream(void* s) { return reinterpret_cast<cudaStream_t>(s); }
 
+// Rows per warp of the kernels that march a warp down a strip of columns: a band
+// reads a few rows more than it writes, so the tallest of 32, 16, 8 and 4 rows
+// that still gives warps_per_sm warps to every SM.
+inline int strip_band(const zim_ctx* ctx, int nstrips, int rows, int warps_per_sm) {
+    const long long want = (long long)warps_per_sm * (ctx->sm_count > 0 ? ctx->sm_count : 152);
+    int band = 32;
+    while (band > 4 && (long long)nstrips * ((rows + band - 1) / band) < want) band /= 2;
+    return band;
+}
+
 // ---- internal launchers (no argument validation; callers validate) ----
 namespace zt {
 struct DecodeParams;
@@ -93,10 +103,9 @@ void zim_decode_params_launch(zim_ctx* ctx, const void* frames, int sample_type,
 zim_status zim_decode_launch(zim_ctx* ctx, const zim_decode_config* cfg, const void* frames,
                              int sample_type, int rows, int cols, int32_t* order, float* residual,
                              float* mod, uint8_t* valid, cudaStream_t st);
-// post_smooth: smooth_k16 / smooth_r are rows*cols scratch for the smoothed taps.
+// post_smooth: taps is rows*cols scratch for the smoothed taps.
 zim_status zim_rectify_launch(zim_ctx* ctx, int cam, const int32_t* order, const float* residual,
-                              int rows, int cols, int post_smooth, int32_t* smooth_k16, float* smooth_r,
-                              int32_t* rect_base, float* rect_res, int32_t* rect_order, cudaStream_t st);
+                              int rows, int cols, int post_smooth, int2* taps, int32_t* rect_base, float* rect_res, int32_t* rect_order, cudaStream_t st);
 zim_status zim_match_launch(zim_ctx* ctx, const int32_t* l_base, const float* l_res,
                             const int32_t* l_order, const int32_t* r_base, const float* r_res,
                             const int32_t* r_order, int rows, int cols, int pha_f,
@@ -129,10 +138,10 @@ zim_status zim_ror_launch(zim_ctx* ctx, const float* xyz, const uint8_t* mask, i
                           float radius, int min_neighbors, int window_size, float* out,
                           uint8_t* mask_out, cudaStream_t st);
 zim_status zim_smooth_launch(zim_ctx* ctx, const int32_t* order, const float* residual, int rows, int cols,
-                             int post_smooth, int32_t* smooth_k16, float* smooth_r, cudaStream_t st);
+                             int post_smooth, int2* taps, cudaStream_t st);
 zim_status zim_rectify_match_launch(zim_ctx* ctx, const int32_t* const order[2], const float* const res[2],
-                                    int32_t* const sk[2], float* const sr[2], int srows, int scols, int post_smooth,
-                                    int pha_f, double grad_threshold, float* disp, cudaStream_t st);
+                                    int2* const taps[2], int srows, int scols, int post_smooth, int pha_f,
+                                    double grad_threshold, float* disp, cudaStream_t st);
 zim_status zim_mls_launch(zim_ctx* ctx, const float* xyz, const uint8_t* mask, int rows, int cols,
                           int window, float sigma, int order, float max_radius, int iterations,
                           float* out, float* tmp, const zim_ray_model& rays, cudaStream_t st);
