@@ -17,8 +17,9 @@
 // position Jacobians and the phase slopes, then
 //   dLoss/dtheta += -(g . P)/w * dw/dtheta   (g = upstream dLoss/dP)
 //   J_r = -(n . P)/w * dw/dtheta             (plane distance, for J^T J).
-// Reductions are FP64: per thread, per warp, per block in a fixed order, then
-// a fixed-order sum of the block partials.
+// The loss is summed in FP64 per thread, the gradient as two-float sums, J^T J in
+// FP32 over 22 points and then as two-float sums; warps, blocks and their partials
+// add in FP64 in a fixed order.
 #include <cmath>
 #include <cstring>
 #include <vector>
@@ -27,12 +28,14 @@
 
 namespace {
 
-constexpr int DIFF_T = 256;   // threads per block
+constexpr int DIFF_T = 128;   // threads per block
 constexpr int DIFF_W = DIFF_T / 32;
 constexpr int NP = ZIM_DIFF_NPARAMS;
 constexpr int NJ = NP * (NP + 1) / 2;  // 136 upper-triangle entries of J^T J
 constexpr int NACC = 2 + NP + NJ;       // loss, count, grad, jtj
 constexpr int MAX_VIEWS = 4096;
+// blocks per SM
+constexpr int DIFF_FWD = 6, DIFF_BWD = 4, DIFF_UP = 3;
 
 struct DiffCam {
     float ir[9];  // rectified pixel -> camera ray
@@ -59,28 +62,21 @@ struct ViewDev {
     float* gphase[2];
 };
 
-// (a, b), a <= b, of upper-triangle entry e of J^T J in row-major order
-__device__ __forceinline__ void jtj_pair(int e, int& a, int& b) {
-    a = 0;
-    while (e >= NP - a) {
-        e -= NP - a;
-        a++;
-    }
-    b = a + e;
-}
-
-// One phase sample of camera cam at rectified (col, row): position (u, v) in
-// the source image, bilinear phase base + frac (phase = 2 pi base + frac), the
-// phase slopes, and optionally d(u, v)/d(params of this camera): fx fy cx cy
-// k1 k2 and, for the right camera, the three rotation components.
+// One phase sample of camera cam at rectified (col, row): normalised ray (x, y),
+// source pixel (x0, y0) + (a, b), bilinear phase base + frac (phase = 2 pi base +
+// frac) and its slopes.  In three steps, so that a point's samples can be located
+// first and all their taps loaded together.
 struct Sample {
     int base, x0, y0;
-    float frac, a, b, gu, gv;
+    float frac, a, b, gu, gv, x, y;
+};
+struct Taps {
+    int k[4];
+    float r[4];
 };
 
-__device__ __forceinline__ bool take_sample(const DiffCam& c, float col, float row, const int32_t* __restrict__ ord,
-                                            const float* __restrict__ res, int sw, int sh, Sample& s, float* ju,
-                                            float* jv, bool rot) {
+// False when a tap lies outside the image (also for NaN).
+__device__ __forceinline__ bool locate(const DiffCam& c, float col, float row, int sw, int sh, Sample& s) {
     const float X0 = fmaf(c.ir[0], col, fmaf(c.ir[1], row, c.ir[2]));
     const float X1 = fmaf(c.ir[3], col, fmaf(c.ir[4], row, c.ir[5]));
     const float X2 = fmaf(c.ir[6], col, fmaf(c.ir[7], row, c.ir[8]));
@@ -90,48 +86,79 @@ __device__ __forceinline__ bool take_sample(const DiffCam& c, float col, float r
     const float xd = fmaf(x, sd, fmaf(2.0f * c.p1, x * y, c.p2 * fmaf(2.0f * x, x, r2)));
     const float yd = fmaf(y, sd, fmaf(c.p1, fmaf(2.0f * y, y, r2), 2.0f * c.p2 * x * y));
     const float u = fmaf(c.fx, xd, c.cx), v = fmaf(c.fy, yd, c.cy);
-    // all four taps inside the image (also rejects NaN)
-    if (!(u >= 0.f && v >= 0.f && u < (float)(sw - 1) && v < (float)(sh - 1))) return false;
-    const int x0 = (int)u, y0 = (int)v;
-    if (x0 + 1 >= sw || y0 + 1 >= sh) return false;
-    const size_t o = (size_t)y0 * sw + x0;
-    const int k00 = __ldg(ord + o), k10 = __ldg(ord + o + 1), k01 = __ldg(ord + o + sw), k11 = __ldg(ord + o + sw + 1);
-    if (k00 < 1 || k10 < 1 || k01 < 1 || k11 < 1) return false;
-    const float r00 = __ldg(res + o), r10 = __ldg(res + o + 1), r01 = __ldg(res + o + sw), r11 = __ldg(res + o + sw + 1);
+    const bool in = u >= 0.f && v >= 0.f && u < (float)(sw - 1) && v < (float)(sh - 1);
+    s.x0 = (int)u;
+    s.y0 = (int)v;
+    s.a = u - (float)s.x0;
+    s.b = v - (float)s.y0;
+    s.x = x;
+    s.y = y;
+    return in && s.x0 + 1 < sw && s.y0 + 1 < sh;
+}
+
+__device__ __forceinline__ void load_taps(const int32_t* __restrict__ ord, const float* __restrict__ res, int sw,
+                                          const Sample& s, bool in, Taps& t) {
+    const size_t o = in ? (size_t)s.y0 * sw + s.x0 : 0;
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        const size_t e = o + (q >> 1) * (size_t)sw + (q & 1);
+        t.k[q] = in ? __ldg(ord + e) : 0;
+        t.r[q] = in ? __ldg(res + e) : 0.f;
+    }
+}
+
+// False when a tap is invalid (order < 1).
+__device__ __forceinline__ bool interpolate(const Taps& t, Sample& s) {
+    if (t.k[0] < 1 || t.k[1] < 1 || t.k[2] < 1 || t.k[3] < 1) return false;
     // phases relative to tap 00, integer cycles subtracted exactly
-    const float p10 = fmaf((float)(k10 - k00), ZIM_TWO_PI_F, r10 - r00);
-    const float p01 = fmaf((float)(k01 - k00), ZIM_TWO_PI_F, r01 - r00);
-    const float p11 = fmaf((float)(k11 - k00), ZIM_TWO_PI_F, r11 - r00);
-    const float a = u - (float)x0, b = v - (float)y0;
-    s.base = k00;
-    s.frac = r00 + fmaf(a * (1.0f - b), p10, fmaf((1.0f - a) * b, p01, a * b * p11));
+    const float p10 = fmaf((float)(t.k[1] - t.k[0]), ZIM_TWO_PI_F, t.r[1] - t.r[0]);
+    const float p01 = fmaf((float)(t.k[2] - t.k[0]), ZIM_TWO_PI_F, t.r[2] - t.r[0]);
+    const float p11 = fmaf((float)(t.k[3] - t.k[0]), ZIM_TWO_PI_F, t.r[3] - t.r[0]);
+    const float a = s.a, b = s.b;
+    s.base = t.k[0];
+    s.frac = t.r[0] + fmaf(a * (1.0f - b), p10, fmaf((1.0f - a) * b, p01, a * b * p11));
     s.gu = fmaf(1.0f - b, p10, b * (p11 - p01));
     s.gv = fmaf(1.0f - a, p01, a * (p11 - p10));
-    s.x0 = x0;
-    s.y0 = y0;
-    s.a = a;
-    s.b = b;
-    if (ju) {
-        const float r4 = r2 * r2;
-        ju[0] = xd; ju[1] = 0.f; ju[2] = 1.f; ju[3] = 0.f; ju[4] = c.fx * x * r2; ju[5] = c.fx * x * r4;
-        jv[0] = 0.f; jv[1] = yd; jv[2] = 0.f; jv[3] = 1.f; jv[4] = c.fy * y * r2; jv[5] = c.fy * y * r4;
-        if (rot) {
-            // ray X -> X + X x eps: d(x, y)/d eps_k for k = 0, 1, 2
-            const float dx[3] = {x * y, -1.0f - x * x, y};
-            const float dy[3] = {1.0f + y * y, -x * y, -x};
-            const float s1 = fmaf(r2, fmaf(3.0f * c.k3, r2, 2.0f * c.k2), c.k1);  // d sd / d r2
-            const float dxd_dx = sd + 2.0f * x * x * s1 + 2.0f * c.p1 * y + 6.0f * c.p2 * x;
-            const float dxd_dy = 2.0f * x * y * s1 + 2.0f * c.p1 * x + 2.0f * c.p2 * y;
-            const float dyd_dx = dxd_dy;
-            const float dyd_dy = sd + 2.0f * y * y * s1 + 6.0f * c.p1 * y + 2.0f * c.p2 * x;
-#pragma unroll
-            for (int k = 0; k < 3; k++) {
-                ju[6 + k] = c.fx * fmaf(dxd_dx, dx[k], dxd_dy * dy[k]);
-                jv[6 + k] = c.fy * fmaf(dyd_dx, dx[k], dyd_dy * dy[k]);
-            }
-        }
-    }
     return true;
+}
+
+__device__ __forceinline__ bool take_sample(const DiffCam& c, float col, float row, const int32_t* __restrict__ ord,
+                                            const float* __restrict__ res, int sw, int sh, Sample& s) {
+    if (!locate(c, col, row, sw, sh, s)) return false;
+    Taps t;
+    load_taps(ord, res, sw, s, true, t);
+    return interpolate(t, s);
+}
+
+// Adds to Jc (fx fy cx cy k1 k2) and, for the right camera, to Jrot what a sample
+// of weight W = dw/dphi contributes to dw/dtheta: W (gu du/dtheta + gv dv/dtheta).
+template <bool ROT>
+__device__ __forceinline__ void add_jacobian(const DiffCam& c, const Sample& s, float W, float* Jc, float* Jrot) {
+    const float x = s.x, y = s.y, P = W * s.gu, Q = W * s.gv;
+    const float r2 = fmaf(x, x, y * y);
+    const float sd = fmaf(r2, fmaf(r2, fmaf(r2, c.k3, c.k2), c.k1), 1.0f);
+    const float xd = fmaf(x, sd, fmaf(2.0f * c.p1, x * y, c.p2 * fmaf(2.0f * x, x, r2)));
+    const float yd = fmaf(y, sd, fmaf(c.p1, fmaf(2.0f * y, y, r2), 2.0f * c.p2 * x * y));
+    const float Pf = P * c.fx, Qf = Q * c.fy;
+    const float t = r2 * fmaf(Pf, x, Qf * y);
+    Jc[0] = fmaf(P, xd, Jc[0]);
+    Jc[1] = fmaf(Q, yd, Jc[1]);
+    Jc[2] += P;
+    Jc[3] += Q;
+    Jc[4] += t;
+    Jc[5] = fmaf(t, r2, Jc[5]);
+    if (ROT) {
+        // ray X -> X + X x eps: d(x, y)/d eps = (x y, -1 - x^2, y), (1 + y^2, -x y, -x)
+        const float s1 = fmaf(r2, fmaf(3.0f * c.k3, r2, 2.0f * c.k2), c.k1);  // d sd / d r2
+        const float dxd_dx = sd + 2.0f * x * x * s1 + 2.0f * c.p1 * y + 6.0f * c.p2 * x;
+        const float dxd_dy = 2.0f * x * y * s1 + 2.0f * c.p1 * x + 2.0f * c.p2 * y;
+        const float dyd_dy = sd + 2.0f * y * y * s1 + 6.0f * c.p1 * y + 2.0f * c.p2 * x;
+        const float A = fmaf(Pf, dxd_dx, Qf * dxd_dy), B = fmaf(Pf, dxd_dy, Qf * dyd_dy);  // dyd_dx = dxd_dy
+        const float xy = x * y;
+        Jrot[0] += fmaf(A, xy, B * fmaf(y, y, 1.0f));
+        Jrot[1] -= fmaf(A, fmaf(x, x, 1.0f), B * xy);
+        Jrot[2] += fmaf(A, y, -(B * x));
+    }
 }
 
 __global__ void diff_rectify_kernel(DiffDev P, int cam, const int32_t* __restrict__ ord, const float* __restrict__ res,
@@ -141,7 +168,7 @@ __global__ void diff_rectify_kernel(DiffDev P, int cam, const int32_t* __restric
     if (j >= P.rw || i >= P.rh) return;
     Sample s;
     const size_t o = (size_t)i * P.rw + j;
-    if (take_sample(P.cam[cam], (float)j, (float)i, ord, res, P.sw, P.sh, s, nullptr, nullptr, false)) {
+    if (take_sample(P.cam[cam], (float)j, (float)i, ord, res, P.sw, P.sh, s)) {
         const int nx = s.a >= 0.5f ? s.x0 + 1 : s.x0, ny = s.b >= 0.5f ? s.y0 + 1 : s.y0;
         rbase[o] = s.base;
         rres[o] = s.frac;
@@ -162,47 +189,110 @@ __device__ __forceinline__ void scatter_phase(float* g, int sw, const Sample& s,
     atomicAdd(g + o + sw + 1, v * s.a * s.b);
 }
 
-template <bool BWD>
-__global__ void __launch_bounds__(DIFF_T) diff_kernel(DiffDev P, const ViewDev* __restrict__ views, int n_views,
-                                                       float loss_weight, double* __restrict__ part) {
-    __shared__ float Js[DIFF_W][32][NP + 1];
+// Sum of many FP32 values as an unevaluated pair of floats (Knuth's two-sum: the
+// rounding error of each addition is added to lo).  The values are added as they
+// are rounded: a product fused into the addition would not match its error term.
+// An infinite sum has no error term (its lo is NaN).  Over 704 values the error to
+// the exact sum is that of FP64 sums of the same values (1.2e-10 of the sum of
+// magnitudes, from the values' own rounding); J^T J's, with 22 instead of 32 rows
+// in FP32, is 1.0e-9 (1.4e-9).
+struct Sum2 {
+    float hi, lo;
+    __device__ __forceinline__ void add(float v) {
+        const float t = __fadd_rn(hi, v), z = __fsub_rn(t, hi);
+        lo = __fadd_rn(lo, __fadd_rn(__fsub_rn(hi, __fsub_rn(t, z)), __fsub_rn(v, z)));
+        hi = t;
+    }
+    __device__ __forceinline__ double value() const {
+        return isfinite(hi) ? (double)hi + (double)lo : (double)hi;
+    }
+};
+
+// The blocks of J^T J that are kept, 4 x 4 each: the ten on and above the diagonal.
+constexpr int NBLK = 10;
+constexpr int ROW = 20;  // floats per staged row of J (16 used): 16-byte loads without bank conflicts
+__device__ __forceinline__ int block_row(int q) { return q < 4 ? 0 : q < 7 ? 1 : q < 9 ? 2 : 3; }
+__device__ __forceinline__ int block_col(int q) { return q < 4 ? q : q < 7 ? q - 3 : q < 9 ? q - 5 : 3; }
+// upper-triangle entry (a, b), a <= b, in row-major order
+__device__ __forceinline__ int jtj_entry(int a, int b) { return a * NP - a * (a - 1) / 2 + b - a; }
+
+// A thread per rectified left pixel of a view.  BWD: also J^T J and the gradient.
+// UP: an upstream gradient of the points or a phase gradient is asked for.
+//
+// The gradient's FP32 terms add up as two-float sums (with an upstream gradient per
+// thread, else lane k of a half-warp component k of the warp's staged rows: two
+// registers instead of 32).  J^T J: a warp's 32 rows go through shared memory, and
+// three groups of ten lanes each add up the
+// ten blocks of the outer products of a third of the rows, 16 products per two
+// 16-byte loads, in FP32 over 22 rows and then as two-float sums.  (One product per
+// two 4-byte loads, and 37 FP64 conversions and additions per 32 points, held the
+// kernel at the FP64 and shared-memory pipes.)  A point's four samples are located
+// before any of their 32 loads, so that these are in flight together.  Four
+// 2448x2048 views: 4.23 -> 1.21 ms; bound by issue and latency, with 16 warps
+// per SM, and the FP64 pipe half busy with the points' distances.
+template <bool BWD, bool UP>
+__global__ void __launch_bounds__(DIFF_T, BWD ? (UP ? DIFF_UP : DIFF_BWD) : DIFF_FWD)
+    diff_kernel(const __grid_constant__ DiffDev P,
+                                                         const ViewDev* __restrict__ views, int n_views,
+                                                         float loss_weight, double* __restrict__ part) {
+    __shared__ __align__(16) float rows[BWD ? DIFF_W : 1][32][ROW];
     __shared__ double red[DIFF_W][NACC];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    const size_t npx = (size_t)P.rw * P.rh, total = npx * (size_t)n_views;
+    const size_t npx = (size_t)P.rw * P.rh;
     const size_t nwarps = (size_t)gridDim.x * DIFF_W;
-    double loss = 0.0, cnt = 0.0;
-    double g[NP];
-    double jacc[(NJ + 31) / 32];
+    double loss = 0.0;
+    unsigned cnt = 0u;
+    Sum2 g[UP ? NP : 1];
+    float acc[16];
+    Sum2 sum[16];
 #pragma unroll
-    for (int k = 0; k < NP; k++) g[k] = 0.0;
-    int pa[(NJ + 31) / 32], pb[(NJ + 31) / 32];
+    for (int k = 0; k < (UP ? NP : 1); k++) g[k] = Sum2{0.f, 0.f};
 #pragma unroll
-    for (int q = 0; q < (NJ + 31) / 32; q++) {
-        jacc[q] = 0.0;
-        jtj_pair(min(lane + 32 * q, NJ - 1), pa[q], pb[q]);
+    for (int k = 0; k < 16; k++) {
+        acc[k] = 0.f;
+        sum[k] = Sum2{0.f, 0.f};
     }
+    const int grp = lane / NBLK, blk = lane - grp * NBLK;  // lanes 30 and 31 repeat others' work
+    const int br = 4 * block_row(blk), bc = 4 * block_col(blk);
+    auto flush = [&]() {
+#pragma unroll
+        for (int k = 0; k < 16; k++) {
+            sum[k].add(acc[k]);
+            acc[k] = 0.f;
+        }
+    };
 
-    // the loop bound depends on the warp only, so the lanes stay together for
-    // the J^T J staging
-    for (size_t base = ((size_t)blockIdx.x * DIFF_W + wib) * 32; base < total; base += nwarps * 32) {
-        const size_t t = base + lane;
-        float Jr[NP];
+    // a warp strides over each view's pixels: the loop bound depends on the warp
+    // only, so the lanes stay together, and (i, j) follow without divisions
+    bool odd = false;
+    const int stride = (int)nwarps * 32, di = stride / P.rw, dj = stride - di * P.rw;
+    const size_t base0 = ((size_t)blockIdx.x * DIFF_W + wib) * 32;
+    for (int vi = 0; vi < n_views; vi++) {
+        const ViewDev& V = views[vi];
+        size_t pix = base0 + lane;
+        int i = (int)(pix / P.rw), j = (int)(pix - (size_t)i * P.rw);
+        int bnext = pix < npx ? __ldg(V.best + pix) : -1;
+        for (size_t base = base0; base < npx; base += stride, pix += stride) {
+            float J[NP], r = 0.f;
 #pragma unroll
-        for (int k = 0; k < NP; k++) Jr[k] = 0.f;
-        if (t < total) {
-            const int vi = (int)(t / npx);
-            const size_t pix = t - (size_t)vi * npx;
-            const ViewDev& V = views[vi];
-            const int i = (int)(pix / P.rw), j = (int)(pix - (size_t)i * P.rw);
-            const int b = V.best[pix];
-            bool ok = b >= 1 && b + 1 < P.rw;
+            for (int k = 0; k < NP; k++) J[k] = 0.f;
+            const int b = bnext;
+            bnext = pix + stride < npx ? __ldg(V.best + pix + stride) : -1;
+            bool ok = pix < npx && b >= 1 && b + 1 < P.rw;
             Sample sL, sR[3];
-            if (ok) ok = take_sample(P.cam[0], (float)j, (float)i, V.order[0], V.res[0], P.sw, P.sh, sL, nullptr,
-                                     nullptr, false);
+            {
+                Taps tL, tR[3];
+                const bool l = ok && locate(P.cam[0], (float)j, (float)i, P.sw, P.sh, sL);
+                bool in[3];
 #pragma unroll
-            for (int m = 0; m < 3; m++)
-                if (ok) ok = take_sample(P.cam[1], (float)(b - 1 + m), (float)i, V.order[1], V.res[1], P.sw, P.sh,
-                                         sR[m], nullptr, nullptr, false);
+                for (int m = 0; m < 3; m++) in[m] = ok && locate(P.cam[1], (float)(b - 1 + m), (float)i, P.sw, P.sh, sR[m]);
+                load_taps(V.order[0], V.res[0], P.sw, sL, l, tL);
+#pragma unroll
+                for (int m = 0; m < 3; m++) load_taps(V.order[1], V.res[1], P.sw, sR[m], in[m], tR[m]);
+                ok = l && in[0] && in[1] && in[2] && interpolate(tL, sL);
+#pragma unroll
+                for (int m = 0; m < 3; m++) ok = ok && interpolate(tR[m], sR[m]);
+            }
             float c[3] = {0.f, 0.f, 0.f};
             float delta = 0.f, dd[3] = {0.f, 0.f, 0.f};  // d delta / d c_m
             float X = 0.f, Y = 0.f, Z = 0.f, w = 0.f, d = 0.f;
@@ -240,7 +330,7 @@ __global__ void __launch_bounds__(DIFF_T) diff_kernel(DiffDev P, const ViewDev* 
                 }
                 ok = Z > P.zmin && Z < P.zmax && isfinite(X) && isfinite(Y);
             }
-            if (!BWD) {
+            if (!BWD && pix < npx) {
                 if (V.xyz) {
                     V.xyz[3 * pix] = ok ? X : 0.f;
                     V.xyz[3 * pix + 1] = ok ? Y : 0.f;
@@ -254,100 +344,119 @@ __global__ void __launch_bounds__(DIFF_T) diff_kernel(DiffDev P, const ViewDev* 
                 const double Nd = fma(V.nd[0], (double)j + P.q03d,
                                       fma(V.nd[1], (double)i + P.q13d, fma(V.nd[2], P.q23d, V.pdd * wd)));
                 const float iw = 1.0f / w;
-                const float r = (float)Nd * iw;
+                r = (float)Nd * iw;
                 loss += (double)r * (double)r;
-                cnt += 1.0;
+                cnt++;
                 if (BWD) {
-                    // dLoss/dw = -(g . P)/w with g = lw 2 r n + grad_xyz, and n . P = r - d
+                    // n . P = r - d, and dr/dw = -(n . P)/w
                     const float nP = r - (float)V.pdd;
-                    float gP = loss_weight * 2.0f * r * nP;
-                    if (V.gxyz)
-                        gP += fmaf(V.gxyz[3 * pix], X, fmaf(V.gxyz[3 * pix + 1], Y, V.gxyz[3 * pix + 2] * Z));
-                    const float s_up = -gP * iw;
-                    const float s_r = -nP * iw;  // dr/dw
+                    const float s_r = -nP * iw;
                     // dw/dphi: d = j - b - delta, w = q32 d + q33
                     const float wR[3] = {-P.q32 * dd[0], -P.q32 * dd[1], -P.q32 * dd[2]};
                     const float wL = -(wR[0] + wR[1] + wR[2]);
-                    float Jw[NP];
+                    J[12] = fmaf(d, P.dq32, P.dq33);
+                    add_jacobian<false>(P.cam[0], sL, wL, J, nullptr);
 #pragma unroll
-                    for (int k = 0; k < NP; k++) Jw[k] = 0.f;
-                    Jw[12] = fmaf(d, P.dq32, P.dq33);
-                    float ju[9], jv[9];
-                    take_sample(P.cam[0], (float)j, (float)i, V.order[0], V.res[0], P.sw, P.sh, sL, ju, jv, false);
+                    for (int m = 0; m < 3; m++) add_jacobian<true>(P.cam[1], sR[m], wR[m], J + 6, J + 13);
+                    // dLoss/dw = -(g . P)/w with g = lw 2 r n + grad_xyz
+                    float gP = loss_weight * 2.0f * r * nP;
+                    if (UP && V.gxyz)
+                        gP += fmaf(V.gxyz[3 * pix], X, fmaf(V.gxyz[3 * pix + 1], Y, V.gxyz[3 * pix + 2] * Z));
+                    const float s_up = -gP * iw;
+                    if (UP) {
+                        scatter_phase(V.gphase[0], P.sw, sL, s_up * wL);
 #pragma unroll
-                    for (int k = 0; k < 6; k++) Jw[k] = wL * fmaf(sL.gu, ju[k], sL.gv * jv[k]);
-                    scatter_phase(V.gphase[0], P.sw, sL, s_up * wL);
-#pragma unroll
-                    for (int m = 0; m < 3; m++) {
-                        take_sample(P.cam[1], (float)(b - 1 + m), (float)i, V.order[1], V.res[1], P.sw, P.sh, sR[m], ju,
-                                    jv, true);
-#pragma unroll
-                        for (int k = 0; k < 6; k++) Jw[6 + k] = fmaf(wR[m], fmaf(sR[m].gu, ju[k], sR[m].gv * jv[k]), Jw[6 + k]);
-#pragma unroll
-                        for (int k = 0; k < 3; k++)
-                            Jw[13 + k] = fmaf(wR[m], fmaf(sR[m].gu, ju[6 + k], sR[m].gv * jv[6 + k]), Jw[13 + k]);
-                        scatter_phase(V.gphase[1], P.sw, sR[m], s_up * wR[m]);
+                        for (int m = 0; m < 3; m++) scatter_phase(V.gphase[1], P.sw, sR[m], s_up * wR[m]);
                     }
 #pragma unroll
                     for (int k = 0; k < NP; k++) {
-                        g[k] += (double)(s_up * Jw[k]);
-                        Jr[k] = s_r * Jw[k];
+                        if (UP) g[k].add(__fmul_rn(s_up, J[k]));
+                        J[k] *= s_r;
                     }
                 }
             }
-        }
-        if (BWD) {
+            if (BWD) {
+                float4* row = reinterpret_cast<float4*>(rows[wib][lane]);
 #pragma unroll
-            for (int k = 0; k < NP; k++) Js[wib][lane][k] = Jr[k];
-            __syncwarp();
-#pragma unroll
-            for (int q = 0; q < (NJ + 31) / 32; q++) {
-                const int e = lane + 32 * q;
-                if (e < NJ) {
-                    float acc = 0.f;
-                    for (int rr = 0; rr < 32; rr++) acc = fmaf(Js[wib][rr][pa[q]], Js[wib][rr][pb[q]], acc);
-                    jacc[q] += (double)acc;
+                for (int k = 0; k < 4; k++) row[k] = make_float4(J[4 * k], J[4 * k + 1], J[4 * k + 2], J[4 * k + 3]);
+                if (!UP) rows[wib][lane][NP] = loss_weight * 2.0f * r;
+                __syncwarp();
+                if (!UP) {
+                    // lane k of each half-warp: component k over half of the rows (those
+                    // apart by four, whose words lie in other banks)
+#pragma unroll 4
+                    for (int p = 0; p < 16; p++) {
+                        const float* row = rows[wib][(p & 3) | (p & 12) << 1 | (lane & 16) >> 2];
+                        g[0].add(__fmul_rn(row[NP], row[lane & 15]));
+                    }
                 }
+#pragma unroll 4
+                for (int p = grp; p < 32; p += 3) {
+                    const float4 u4 = *reinterpret_cast<const float4*>(&rows[wib][p][br]);
+                    const float4 v4 = *reinterpret_cast<const float4*>(&rows[wib][p][bc]);
+                    const float u[4] = {u4.x, u4.y, u4.z, u4.w}, v[4] = {v4.x, v4.y, v4.z, v4.w};
+#pragma unroll
+                    for (int a = 0; a < 4; a++)
+#pragma unroll
+                        for (int e = 0; e < 4; e++) acc[4 * a + e] = fmaf(u[a], v[e], acc[4 * a + e]);
+                }
+                if (odd) flush();
+                odd = !odd;
+                __syncwarp();
             }
-            __syncwarp();
+            i += di;
+            j += dj;
+            if (j >= P.rw) {
+                j -= P.rw;
+                i++;
+            }
         }
     }
     // warp sums (fixed shuffle tree), then per-warp rows summed in warp order
+    double dcnt = (double)cnt;
     for (int off = 16; off; off >>= 1) {
         loss += __shfl_xor_sync(0xffffffffu, loss, off);
-        cnt += __shfl_xor_sync(0xffffffffu, cnt, off);
-    }
-    if (BWD) {
-#pragma unroll
-        for (int k = 0; k < NP; k++)
-            for (int off = 16; off; off >>= 1) g[k] += __shfl_xor_sync(0xffffffffu, g[k], off);
+        dcnt += __shfl_xor_sync(0xffffffffu, dcnt, off);
     }
     if (lane == 0) {
         red[wib][0] = loss;
-        red[wib][1] = cnt;
-#pragma unroll
-        for (int k = 0; k < NP; k++) red[wib][2 + k] = BWD ? g[k] : 0.0;
+        red[wib][1] = dcnt;
     }
+    if (BWD) {
 #pragma unroll
-    for (int q = 0; q < (NJ + 31) / 32; q++) {
-        const int e = lane + 32 * q;
-        if (e < NJ) red[wib][2 + NP + e] = BWD ? jacc[q] : 0.0;
+        for (int k = 0; k < (UP ? NP : 1); k++) {
+            double v = g[k].value();
+            for (int off = 16; off >= (UP ? 1 : 16); off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+            if (UP && lane == 0) red[wib][2 + k] = v;
+            if (!UP && lane < NP) red[wib][2 + lane] = v;
+        }
+        flush();
+#pragma unroll
+        for (int k = 0; k < 16; k++) {
+            double v = sum[k].value();
+            // the three groups' shares of the rows
+            const double v1 = __shfl_down_sync(0xffffffffu, v, NBLK), v2 = __shfl_down_sync(0xffffffffu, v, 2 * NBLK);
+            v = (v + v1) + v2;
+            const int a = br + k / 4, e = bc + k % 4;
+            if (lane < NBLK && a <= e) red[wib][2 + NP + jtj_entry(a, e)] = v;
+        }
     }
     __syncthreads();
-    for (int e = threadIdx.x; e < NACC; e += DIFF_T) {
+    for (int e = threadIdx.x; e < (BWD ? NACC : 2); e += DIFF_T) {
         double s = 0.0;
         for (int ww = 0; ww < DIFF_W; ww++) s += red[ww][e];
         part[(size_t)blockIdx.x * NACC + e] = s;
     }
 }
 
-// Fixed-order sum of the block partials: one thread per accumulator.
-__global__ void diff_total_kernel(const double* __restrict__ part, int nblk, double* __restrict__ out) {
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= NACC) return;
+// Fixed-order sum of the block partials: a warp per accumulator.
+__global__ void diff_total_kernel(const double* __restrict__ part, int nblk, int n, double* __restrict__ out) {
+    const int e = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (e >= n) return;
     double s = 0.0;
-    for (int b = 0; b < nblk; b++) s += part[(size_t)b * NACC + e];
-    out[e] = s;
+    for (int b = lane; b < nblk; b += 32) s += part[(size_t)b * NACC + e];
+    for (int off = 16; off; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
+    if (lane == 0) out[e] = s;
 }
 
 // Rotation matrix of a rotation vector (Rodrigues' formula), row-major.
@@ -438,7 +547,10 @@ zim_status run(zim_ctx* ctx, const zim_diff_params* params, const zim_diff_view*
         H.mask = bwd ? nullptr : V.mask;
         H.gxyz = bwd ? V.grad_xyz : nullptr;
     }
-    const int nblk = 4 * (ctx->sm_count > 0 ? ctx->sm_count : 152);
+    bool up = false;  // an upstream gradient, or phase gradients
+    for (const ViewDev& H : hv) up = up || H.gxyz || H.gphase[0] || H.gphase[1];
+    // all blocks resident at once
+    const int nblk = (!bwd ? DIFF_FWD : up ? DIFF_UP : DIFF_BWD) * (ctx->sm_count > 0 ? ctx->sm_count : 152);
     zim_scratch_reset(ctx);
     s = zim_scratch_reserve(ctx, zim_align256(hv.size() * sizeof(ViewDev)) + zim_align256((size_t)nblk * NACC * 8) +
                                      zim_align256(NACC * 8) + 4096);
@@ -449,11 +561,10 @@ zim_status run(zim_ctx* ctx, const zim_diff_params* params, const zim_diff_view*
     cudaStream_t st = zim_stream(stream);
     static_assert(NACC * 8 <= 4096, "totals fit the pinned staging");
     ZIM_CUDA_TRY(ctx, cudaMemcpyAsync(dv, hv.data(), hv.size() * sizeof(ViewDev), cudaMemcpyHostToDevice, st));
-    if (bwd)
-        diff_kernel<true><<<nblk, DIFF_T, 0, st>>>(D, dv, n_views, (float)loss_weight, part);
-    else
-        diff_kernel<false><<<nblk, DIFF_T, 0, st>>>(D, dv, n_views, (float)loss_weight, part);
-    diff_total_kernel<<<1, 160, 0, st>>>(part, nblk, tot);
+    auto kern = !bwd ? diff_kernel<false, false> : up ? diff_kernel<true, true> : diff_kernel<true, false>;
+    kern<<<nblk, DIFF_T, 0, st>>>(D, dv, n_views, (float)loss_weight, part);
+    const int n = bwd ? NACC : 2;
+    diff_total_kernel<<<(n + 7) / 8, 256, 0, st>>>(part, nblk, n, tot);
     ctx->launches += 2;
     ZIM_LAUNCH_CHECK(ctx);
     double* h = (double*)ctx->h_pinned;
