@@ -12,7 +12,7 @@
 //
 // SOR on a cloud with pixel rays (the organised cloud of the calibrated size):
 //   window pass: one thread per pixel walks its 15x15 window in a spiral with
-//            a max-heap of the k + 1 nearest, certified exact by a bound on
+//            the k + 1 nearest in groups of five, certified exact by a bound on
 //            the distance to every point seen along another pixel's ray;
 //   tree search: one warp per remaining point reads the leaves whose box lies
 //            within the (k + 1)-th distance held.
@@ -747,38 +747,48 @@ __device__ __forceinline__ int win_len2(int o) { return c_win.ent[o] >> 16; }
 // offsets whose squared length is at most r2 (r2 >= 0 or +inf)
 __device__ __forceinline__ int win_upto(float r2) { return r2 < (float)WR2MAX ? c_win.upto[(int)r2] : WN; }
 
-// Per-thread max-heap of the K1 smallest squared distances seen so far, in
-// column tid of a [K1][WT_T] shared array (conflict-free): the root is the
-// current K1-th smallest, and a nearer point replaces it with one sift-down.
-template <int KC>  // the heap size at compile time (0: K1)
-struct WinHeap {
-    float* L;
-    int K1_;
-    __device__ __forceinline__ int size() const { return KC ? KC : K1_; }
-    __device__ __forceinline__ float& at(int j) { return L[j * WT_T]; }
-    // places v at j, moving larger children up
-    __device__ __forceinline__ void sift(int j, float v) {
-        const int K1 = size();
-#pragma unroll
-        for (int lev = 0; lev < 6; lev++) {  // a heap of at most 64 entries is 6 levels deep
-            int c = 2 * j + 1;
-            if (c >= K1) break;
-            float cv = at(c);
-            if (c + 1 < K1) {
-                const float c2 = at(c + 1);
-                if (c2 > cv) {
-                    cv = c2;
-                    c++;
-                }
-            }
-            if (!(cv > v)) break;
-            at(j) = cv;
-            j = c;
-        }
-        at(j) = v;
+// The k + 1 smallest squared distances a thread has seen, in G groups of five: a
+// group's largest in a register, the other four as one float4 in column tid of a
+// [G][WT_T] shared array (conflict-free).  The largest of all is the largest of
+// the registers; a nearer point takes its place, and one pass over its group finds
+// the group's next largest.  Unused places hold 0, the query's own distance: never
+// the largest unless all are 0, and no part of a sum of roots.
+//
+// A binary heap in shared memory took its place, five or six dependent loads deep
+// per replacement and with a build besides.  Window pass, k = 50, 1280 x 1024: 234
+// -> 150 us; k = 20: 127 -> 79 us.  Groups of nine take two loads and fewer
+// registers, but hold fewer CTAs at k = 50 (688 against 660 us for the whole filter
+// of a 2448 x 2048 cloud); at the other k they are even.
+constexpr int NS_N = 5;  // values per group
+template <int G>
+struct NearSet {
+    float4* S;
+    float top[G];
+    // the larger of t and e stays in t
+    static __device__ __forceinline__ void order(float& e, float& t) {
+        const float lo = fminf(e, t);
+        t = fmaxf(e, t);
+        e = lo;
     }
-    __device__ __forceinline__ void build() {
-        for (int j = size() / 2 - 1; j >= 0; j--) sift(j, at(j));
+    __device__ __forceinline__ float largest() const {
+        float m = top[0];
+#pragma unroll
+        for (int g = 1; g < G; g++) m = fmaxf(m, top[g]);
+        return m;
+    }
+    // v in the place of the largest (m = largest())
+    __device__ __forceinline__ void replace(float v, float m) {
+        int g = 0;
+#pragma unroll
+        for (int j = 1; j < G; j++) g = top[j] == m ? j : g;
+        float4 a = S[g * WT_T];
+        order(a.x, v);
+        order(a.y, v);
+        order(a.z, v);
+        order(a.w, v);
+        S[g * WT_T] = a;
+#pragma unroll
+        for (int j = 0; j < G; j++) top[j] = j == g ? v : top[j];
     }
 };
 
@@ -798,54 +808,82 @@ __device__ __forceinline__ void defer_query_bound(zl::Head* h, unsigned* deferre
     deferred[atomicAdd(&h->n_deferred, 1u)] = (unsigned)i;
 }
 
-// The heap's first K1T - 1 distances (heap slots K1T - 2 down to 0) from the
-// first K1T - 1 spiral offsets, invalid pixels as +inf.
-template <int K1T, int... O>
-__device__ __forceinline__ void fill_first(WinHeap<K1T>& heap, const float4* W, int wc, float4 q,
-                                           std::integer_sequence<int, O...>) {
-    auto d2 = [&](const float4 p) { return p.w == 0.f ? INFINITY : sqdist(p.x - q.x, p.y - q.y, p.z - q.z); };
-    ((heap.at(K1T - 2 - O) = d2(W[wc + win_off_c<O>()])), ...);
+// The window pass's staged points: coordinates in two arrays (12 bytes a point
+// hold one CTA more per SM than 16), +inf for an invalid pixel's.
+constexpr size_t WIN_BYTES = (size_t)WW * WH * 12;
+static_assert(WIN_BYTES % 16 == 0, "the sets behind the window are float4");
+struct WinPoints {
+    float2* xy;
+    float* z;
+    __device__ __forceinline__ float d2(int e, float x, float y, float zq) const {
+        const float2 p = xy[e];
+        return sqdist(p.x - x, p.y - y, z[e] - zq);
+    }
+};
+
+// Group g of the set: spiral offsets 5 g to 5 g + 4, in the last group those below k.
+template <int G, int g, int... J>
+__device__ __forceinline__ void fill_group(NearSet<G>& set, const WinPoints& W, int wc, float qx, float qy, float qz,
+                                           int k, std::integer_sequence<int, J...>) {
+    float v[NS_N] = {(g + 1 < G || NS_N * g + J < k ? W.d2(wc + win_off_c<NS_N * g + J>(), qx, qy, qz) : 0.f)...};
+    float t = v[NS_N - 1];
+#pragma unroll
+    for (int j = 0; j < NS_N - 1; j++) NearSet<G>::order(v[j], t);
+    set.S[g * WT_T] = make_float4(v[0], v[1], v[2], v[3]);
+    set.top[g] = t;
+}
+template <int G, int... g>
+__device__ __forceinline__ void fill_groups(NearSet<G>& set, const WinPoints& W, int wc, float qx, float qy, float qz,
+                                            int k, std::integer_sequence<int, g...>) {
+    (fill_group<G, g>(set, W, wc, qx, qy, qz, k, std::make_integer_sequence<int, NS_N>{}), ...);
 }
 
-// K1T: k + 1 at compile time (0: from k)
-template <int K1T>
+// G: groups of the set, (k + 1) / NS_N rounded up
+template <int G>
 __global__ void __launch_bounds__(WT_T) sor_window_kernel(const float* __restrict__ xyz,
                                                             const uint8_t* __restrict__ mask, int rows, int cols,
-                                                            int k, RayParams rp, zl::Head* __restrict__ h,
+                                                            int k, RayParams rp, zl::Tree t,
                                                             float* __restrict__ md_out,
                                                             unsigned* __restrict__ deferred,
                                                             float* __restrict__ bound) {
     extern __shared__ float4 win_smem[];
-    float4* W = win_smem;                                      // WW x WH window, w = 1 valid
-    float* Ls = reinterpret_cast<float*>(win_smem + WW * WH);  // (k + 1) x WT_T heaps
+    const WinPoints W{reinterpret_cast<float2*>(win_smem),
+                      reinterpret_cast<float*>(reinterpret_cast<float2*>(win_smem) + WW * WH)};
     const int tid = threadIdx.x;
     const int x0 = blockIdx.x * WT_X, y0 = blockIdx.y * WT_Y;
-    __shared__ unsigned warp_dev[WT_T / 32];
-    unsigned tdev = 0u;  // largest dev of this thread's staged points (float bits, >= 0)
+    zl::Head* h = t.head;
+    // largest ray distance of the leaves that the window touches (float bits, >= 0)
+    __shared__ unsigned win_dev;
+    if (tid < 32) {
+        const int lx0 = max(x0 - WR, 0) / zl::LEAF, lx1 = min((x0 + WT_X - 1 + WR) / zl::LEAF, t.lw - 1);
+        const int ly0 = max(y0 - WR, 0) / zl::LEAF, ly1 = min((y0 + WT_Y - 1 + WR) / zl::LEAF, t.lh - 1);
+        const int nx = lx1 - lx0 + 1;
+        unsigned d = 0u;
+        for (int e = tid; e < nx * (ly1 - ly0 + 1); e += 32)
+            d = max(d, __float_as_uint(__ldg(t.leaf + 2 * ((size_t)(ly0 + e / nx) * t.lw + lx0 + e % nx) + 1).w));
+        d = __reduce_max_sync(0xffffffffu, d);
+        if (tid == 0) win_dev = d;
+    }
 #pragma unroll
-    for (int t = tid; t < WW * WH; t += WT_T) {
-        const int wx = x0 - WR + t % WW, wy = y0 - WR + t / WW;
-        // invalid and off-image pixels: NaN coordinates (their squared distance
-        // never passes a comparison), w = 0
-        const float nan = __int_as_float(0x7fc00000);
-        float4 v = make_float4(nan, nan, nan, 0.f);
+    for (int e = tid; e < WW * WH; e += WT_T) {
+        const int wx = x0 - WR + e % WW, wy = y0 - WR + e / WW;
+        // invalid and off-image pixels and points without finite coordinates at
+        // +inf: nearer than no point
+        float2 vxy = make_float2(INFINITY, INFINITY);
+        float vz = INFINITY;
         if (wx >= 0 && wx < cols && wy >= 0 && wy < rows) {
             const size_t j = (size_t)wy * cols + wx;
-            if (mask[j]) {
-                v = make_float4(xyz[3 * j], xyz[3 * j + 1], xyz[3 * j + 2], 1.f);
-                float ax, ay, az;
-                ray_dir(rp, wx, wy, ax, ay, az);
-                const float d = ray_dev(v.x, v.y, v.z, ax, ay, az);
-                tdev = max(tdev, __float_as_uint(d == d ? d : INFINITY));  // NaN counts as unbounded
+            const float px = xyz[3 * j], py = xyz[3 * j + 1], pz = xyz[3 * j + 2];
+            if (mask[j] && fabsf(px) + fabsf(py) + fabsf(pz) < INFINITY) {
+                vxy = make_float2(px, py);
+                vz = pz;
             }
         }
-        W[t] = v;
+        W.xy[e] = vxy;
+        W.z[e] = vz;
     }
-    tdev = __reduce_max_sync(0xffffffffu, tdev);
-    if ((tid & 31) == 0) warp_dev[tid >> 5] = tdev;
     __syncthreads();
-#pragma unroll
-    for (int j = 0; j < WT_T / 32; j++) tdev = max(tdev, warp_dev[j]);
+    const unsigned tdev = win_dev;
     const int tx = tid % WT_X, ty = tid / WT_X;
     const int x = x0 + tx, y = y0 + ty;
     if (x >= cols || y >= rows) return;  // no block-wide synchronisation below
@@ -855,47 +893,27 @@ __global__ void __launch_bounds__(WT_T) sor_window_kernel(const float* __restric
         return;
     }
     const int wc = (ty + WR) * WW + tx + WR;
-    const float4 q = W[wc];
-    const int K1 = K1T ? K1T : k + 1;
-    // the query and its first k valid window pixels in spiral order fill the
-    // heap; its root (their largest distance) is the first bound.  They fill
-    // it from the last slot backwards: the spiral meets pixels roughly by
-    // increasing distance, so the array is close to descending -- close to a
-    // max-heap already -- and the build sifts little.  (Only the multiset of
-    // the heap's values matters: the root is its maximum, a replacement drops
-    // the maximum, and the mean distance is an order-free fixed-point sum.)
-    WinHeap<K1T> heap{Ls + tid, K1};
-    heap.at(K1 - 1) = 0.f;
-    int o = 0;
-    if constexpr (K1T > 0) {
-        // k known at compile time: the first k spiral offsets fill the heap
-        // straight from constant tile offsets, an invalid pixel as +inf (the
-        // largest value: the first valid distance to come replaces it, and a
-        // heap still holding one at the end means fewer than k + 1 points)
-        fill_first<K1T>(heap, W, wc, q, std::make_integer_sequence<int, K1T - 1>{});
-        o = K1T - 1;
-    } else {
-        int cnt = 1;
-        for (; o < WN && cnt < K1; o++) {
-            const float4 p = W[wc + win_off(o)];
-            if (p.w == 0.f) continue;
-            heap.at(K1 - 1 - cnt++) = sqdist(p.x - q.x, p.y - q.y, p.z - q.z);
-        }
-        if (cnt < K1) {
-            defer_query(h, deferred, md_out, i);
-            return;
-        }
+    const float qx = W.xy[wc].x, qy = W.xy[wc].y, qz = W.z[wc];
+    if (!(qx < INFINITY)) {
+        defer_query(h, deferred, md_out, i);
+        return;
     }
-    heap.build();
-    float thr = heap.at(0);
+    // the query and its first k window pixels in spiral order fill the set, an
+    // invalid pixel at +inf (the first valid distance to come replaces it; a set
+    // still holding one at the end means fewer than k + 1 points)
+    NearSet<G> set;
+    set.S = win_smem + WIN_BYTES / 16 + tid;
+    fill_groups<G>(set, W, wc, qx, qy, qz, k, std::make_integer_sequence<int, G>{});
+    int o = k;
+    float thr = set.largest();
     // bound(r) = C r / (an + r): no point of a pixel at distance >= r from the
     // query's lies nearer than bound(r) - dev (slack: float rounding, 1e-5 |q|)
     float ax, ay, az;
     ray_dir(rp, x, y, ax, ay, az);
     const float an = sqrtf(fmaf(ax, ax, fmaf(ay, ay, az * az)));
-    const float qn = sqrtf(fmaf(q.x, q.x, fmaf(q.y, q.y, q.z * q.z)));
+    const float qn = sqrtf(fmaf(qx, qx, fmaf(qy, qy, qz * qz)));
     const float C = qn * rp.f / an;
-    const float dev_q = ray_dev(q.x, q.y, q.z, ax, ay, az) + 1e-5f * qn;
+    const float dev_q = ray_dev(qx, qy, qz, ax, ay, az) + 1e-5f * qn;
     const float dev = dev_q + __uint_as_float(tdev);                    // window pixels
     const float dev_out = dev_q + __uint_as_float(h->ray_dev_bits);     // pixels outside it
     // squared pixel distance beyond which every window point is farther than
@@ -911,14 +929,23 @@ __global__ void __launch_bounds__(WT_T) sor_window_kernel(const float* __restric
     // the spiral runs by increasing length: once past the stop distance, the
     // rest of the window (and everything outside it) is provably farther
     int lim = win_upto(stop_r2(thr));
-    for (; o < lim; o++) {
-        const float4 p = W[wc + win_off(o)];
-        const float d2 = sqdist(p.x - q.x, p.y - q.y, p.z - q.z);
-        if (d2 < thr) {  // false for an invalid pixel (NaN)
-            heap.sift(0, d2);
-            thr = heap.at(0);
-            lim = win_upto(stop_r2(thr));
+    auto at = [&](int o) { return o < WN ? W.d2(wc + win_off(o), qx, qy, qz) : INFINITY; };
+    for (; o < lim; o += 4) {
+        float d0 = at(o), d1 = at(o + 1), d2 = at(o + 2), d3 = at(o + 3);
+        if (!(fminf(fminf(d0, d1), fminf(d2, d3)) < thr)) continue;
+        // one replacement of every lane that has any, until none has
+        for (;;) {
+            const bool c0 = d0 < thr, c1 = d1 < thr, c2 = d2 < thr, c3 = d3 < thr;
+            if (!(c0 || c1 || c2 || c3)) break;
+            const float v = c0 ? d0 : c1 ? d1 : c2 ? d2 : d3;
+            if (c0) d0 = INFINITY;
+            else if (c1) d1 = INFINITY;
+            else if (c2) d2 = INFINITY;
+            else d3 = INFINITY;
+            set.replace(v, thr);
+            thr = set.largest();
         }
+        lim = win_upto(stop_r2(thr));
     }
     if (!(thr < INFINITY)) {  // fewer than k + 1 points in the whole window
         defer_query(h, deferred, md_out, i);
@@ -932,8 +959,8 @@ __global__ void __launch_bounds__(WT_T) sor_window_kernel(const float* __restric
     const float rk = sqrtf(kth), ro = (float)(WR + 1);
     const bool ok = C * rbreak / (an + rbreak) - dev > rk && C * ro / (an + ro) - dev_out > rk;
     if (!ok) {
-        // the heap holds k + 1 distances of cloud points (the query's own 0
-        // among them): its root bounds the (k + 1)-th smallest from above
+        // the set holds k + 1 distances of cloud points (the query's own 0
+        // among them): its largest bounds the (k + 1)-th smallest from above
         defer_query_bound(h, deferred, md_out, bound, i, kth);
         return;
     }
@@ -941,11 +968,19 @@ __global__ void __launch_bounds__(WT_T) sor_window_kernel(const float* __restric
     const float sc = root_scale(e);
     unsigned sum = 0;
 #pragma unroll
-    for (int j = 0; j < (K1T ? K1T : 64); j++) {
-        if (j >= K1) break;
-        sum += root_fixed(heap.at(j), sc);
+    for (int g = 0; g < G; g++) {
+        sum += root_fixed(set.top[g], sc);
+        const float4 v = set.S[g * WT_T];
+        sum += root_fixed(v.x, sc) + root_fixed(v.y, sc) + root_fixed(v.z, sc) + root_fixed(v.w, sc);
     }
     md_out[i] = fixed_mean(sum, e, k);
+}
+
+// the window pass's kernel by number of groups, 1 to 13
+template <int... g>
+auto sor_window_of(int groups, std::integer_sequence<int, g...>) {
+    static constexpr decltype(&sor_window_kernel<1>) k[] = {sor_window_kernel<g + 1>...};
+    return k[groups - 1];
 }
 
 constexpr int FW_CAP = 384;  // tree search: list entries per warp (12 per lane)
@@ -978,7 +1013,7 @@ __device__ __forceinline__ unsigned warp_kth_key(const unsigned (&keys)[FW_CAP /
 
 // Tree search: one warp per deferred query.  The warp keeps the squared
 // distances below its bound in a list; the bound starts at the window pass's
-// (the root of its heap) or, without one, at the farthest corner of the
+// (the largest it holds) or, without one, at the farthest corner of the
 // nearest-cornered node and then leaf that holds k + 1 points, and tightens to
 // the (k + 1)-th smallest held whenever the list fills.  With pixel rays the
 // bound also limits the search to a rectangle of pixels (the window pass's ray
@@ -1676,11 +1711,11 @@ zim_status zim_sor_launch(zim_ctx* ctx, const float* xyz, const uint8_t* mask, i
     if (s) return s;
     if (rays.valid) {
         const dim3 wgrid((cols + WT_X - 1) / WT_X, (rows + WT_Y - 1) / WT_Y);
-        const size_t wsm = (size_t)WW * WH * sizeof(float4) + (size_t)(mean_k + 1) * WT_T * 4;
-        // k = 30 and 50 (the configurations') with a compile-time heap size
-        auto kern = mean_k == 30 ? sor_window_kernel<31> : mean_k == 50 ? sor_window_kernel<51> : sor_window_kernel<0>;
+        const int groups = (mean_k + NS_N) / NS_N;  // (k + 1) / NS_N rounded up
+        const size_t wsm = WIN_BYTES + sizeof(float4) * groups * WT_T;
+        auto kern = sor_window_of(groups, std::make_integer_sequence<int, (KNN_MAX_K1 + NS_N - 1) / NS_N>{});
         ZIM_CUDA_TRY(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)wsm));
-        kern<<<wgrid, WT_T, wsm, st>>>(xyz, mask, rows, cols, mean_k, rp, t.head, md, deferred, bound);
+        kern<<<wgrid, WT_T, wsm, st>>>(xyz, mask, rows, cols, mean_k, rp, t, md, deferred, bound);
     } else {
         // cell ~ 3.5 x spacing: the (k+1)-th neighbour of a surface point
         // lies within one ring for ~98% of points at k = 30
