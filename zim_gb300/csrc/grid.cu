@@ -983,9 +983,10 @@ auto sor_window_of(int groups, std::integer_sequence<int, g...>) {
     return k[groups - 1];
 }
 
-constexpr int FW_CAP = 384;  // tree search: list entries per warp (12 per lane)
+constexpr int FW_CAP = 256;  // tree search: list entries per warp (8 per lane)
 constexpr int TS_QUEUE = 256;  // tree search: queued leaves per warp
-constexpr int TS_LEAVES = 4;  // tree search: leaves read together (at most 256 new entries)
+constexpr int TS_NODES = 2;  // tree search: nodes whose leaves are tested together
+constexpr int TS_LEAVES = 2;  // tree search: leaves read together (at most 128 new entries)
 
 // Smallest list value v with at least K entries <= v (entries: lane j holds
 // keys[r], 0xffffffff = empty; keys are non-negative float bits).  Bisection on
@@ -1022,11 +1023,14 @@ __device__ __forceinline__ unsigned warp_kth_key(const unsigned (&keys)[FW_CAP /
 // handed out through an atomic counter.
 //
 // Bound by the latency of its dependent loads (one box or pixel access takes
-// ~1000 cycles with eight CTAs per SM) and of its own instructions, so the leaves
-// in question are queued first and read four at a time, those within a third of
-// the bound before the others (they tighten it), and no index is divided.  It took the place of a
-// counting-sorted coarse grid with a ring search and an occupied-cell search,
-// whose build alone was eleven launches.
+// ~1000 cycles with eight CTAs per SM) and, at the end, by its longest queries
+// (5 MP: 47 thousand cycles on average, 230 thousand the longest).  So the leaves
+// of two nodes are tested together, a leaf of k + 1 points bounds the search
+// before any pixel is read, leaves are queued and read two at a time, and no index
+// is divided.  5 MP, k = 30: 105 -> 83 us; 640 x 480, k = 50: 63 -> 22.  Reading four or eight leaves at a time
+// or testing four nodes is no faster (a longer list costs each selection more).
+// The search took the place of a counting-sorted coarse grid with a ring search
+// and an occupied-cell search, whose build alone was eleven launches.
 __global__ void __launch_bounds__(TS_WARPS * 32) sor_tree_kernel(const float* __restrict__ xyz,
                                                                  const uint8_t* __restrict__ mask, int rows, int cols,
                                                                  int k, int rays, RayParams rp, zl::Tree t,
@@ -1042,20 +1046,19 @@ __global__ void __launch_bounds__(TS_WARPS * 32) sor_tree_kernel(const float* __
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int K1 = k + 1;
     float* lw = lst[w];
-    const unsigned nd = t.head->n_deferred;
-    for (;;) {
-        unsigned item = 0;
-        if (lane == 0) item = atomicAdd(&t.head->next, 1u);
-        item = __shfl_sync(full, item, 0);
-        if (item >= nd) break;
+    const unsigned nd = t.head->n_deferred, nwarps = gridDim.x * TS_WARPS;
+    // the first query of each warp by its index: thousands of warps asking one
+    // counter at once took 4 us
+    for (unsigned item = blockIdx.x * TS_WARPS + w; item < nd;) {
         const unsigned i = deferred[item];
         const float q[3] = {xyz[3 * (size_t)i], xyz[3 * (size_t)i + 1], xyz[3 * (size_t)i + 2]};
         // entries lie strictly below thr; bounds are met by equality, so they
         // start one float above (finite non-negative floats order as their bits)
         auto above = [](float b) { return b < INFINITY ? __uint_as_float(__float_as_uint(b) + 1u) : INFINITY; };
+        const float b0 = bound[i];  // set where md says so
         float thr = INFINITY;
         if (md_out[i] == MD_BOUND) {
-            thr = above(bound[i]);
+            thr = above(b0);
         } else {
             unsigned long long best = ~0ull;  // (distance bits, node)
             for (int n0 = lane; n0 < t.nw * t.nh; n0 += 32) {
@@ -1121,13 +1124,13 @@ __global__ void __launch_bounds__(TS_WARPS * 32) sor_tree_kernel(const float* __
             thr = __uint_as_float(kk);
             __syncwarp();
         };
-        // reads the queued leaves with a box distance in [from, to) and below thr
+        // reads the queued leaves with a box distance below thr
         int nq = 0;
-        auto scan = [&](float from, float to) {
+        auto flush = [&]() {
+            __syncwarp();
             for (int q0 = 0; q0 < nq; q0 += 32) {
                 const float d = q0 + lane < nq ? qd2[w][q0 + lane] : INFINITY;
-                const bool mine = d >= from && d < to;
-                for (unsigned m = __ballot_sync(full, mine && d < thr); m; m &= __ballot_sync(full, d < thr)) {
+                for (unsigned m = __ballot_sync(full, d < thr); m; m &= __ballot_sync(full, d < thr)) {
                     float d2[TS_LEAVES][2];
 #pragma unroll
                     for (int g = 0; g < TS_LEAVES; g++) {
@@ -1160,13 +1163,6 @@ __global__ void __launch_bounds__(TS_WARPS * 32) sor_tree_kernel(const float* __
                     }
                 }
             }
-        };
-        auto flush = [&]() {
-            __syncwarp();
-            const float near = thr < INFINITY ? 0.1f * thr : 0.f;
-            scan(0.f, near);
-            if (n >= K1 && n > 2 * K1 && K1 <= FW_CAP - NEW) tighten();
-            scan(near, INFINITY);
             __syncwarp();
             nq = 0;
         };
@@ -1180,38 +1176,48 @@ __global__ void __launch_bounds__(TS_WARPS * 32) sor_tree_kernel(const float* __
                 const zl::Box b = zl::load_box(t.node, ny * t.nw + nx);
                 if (b.n) nd2 = zl::gap_d2(b, q, q);
             }
-            unsigned nm = __ballot_sync(full, nd2 < thr);
-            while (nm) {
-                const int nb = __ffs(nm) - 1;
-                nm &= nm - 1;
-                if (!(__shfl_sync(full, nd2, nb) < thr)) continue;  // the bound may have moved
-                const int lx0 = __shfl_sync(full, nx, nb) * zl::FAN, ly0 = __shfl_sync(full, ny, nb) * zl::FAN;
-                const int lx = lx0 + (lane & 7), ly = ly0 + (lane >> 3);
-                float ld2[2];
+            for (unsigned nm = __ballot_sync(full, nd2 < thr); nm; nm &= __ballot_sync(full, nd2 < thr)) {
+                float ld2[TS_NODES][2];
+                int lx[TS_NODES], ly[TS_NODES];
+                unsigned fb = 0xffffffffu;
 #pragma unroll
-                for (int h = 0; h < 2; h++) {
-                    ld2[h] = INFINITY;
-                    if (lx < t.lw && ly + 4 * h < t.lh) {
-                        const zl::Box b = zl::load_box(t.leaf, (ly + 4 * h) * t.lw + lx);
-                        if (b.n) ld2[h] = zl::gap_d2(b, q, q);
+                for (int g = 0; g < TS_NODES; g++) {
+                    const int nb = nm ? __ffs(nm) - 1 : 0;
+                    const bool any = nm != 0u;
+                    nm &= nm - 1;
+                    lx[g] = __shfl_sync(full, nx, nb) * zl::FAN + (lane & 7);
+                    ly[g] = __shfl_sync(full, ny, nb) * zl::FAN + (lane >> 3);
+#pragma unroll
+                    for (int h = 0; h < 2; h++) {
+                        const bool in = any && lx[g] < t.lw && ly[g] + 4 * h < t.lh;
+                        const zl::Box b = zl::load_box(t.leaf, in ? (ly[g] + 4 * h) * t.lw + lx[g] : 0);
+                        ld2[g][h] = in && b.n ? zl::gap_d2(b, q, q) : INFINITY;
+                        if (in && b.n >= (unsigned)K1) fb = min(fb, __float_as_uint(zl::far_d2(b, q)));
                     }
                 }
+                // a leaf of k + 1 points bounds the search by its farthest corner
+                fb = __reduce_min_sync(full, fb);
+                if (fb < __float_as_uint(thr)) thr = fminf(thr, above(__uint_as_float(fb)));
 #pragma unroll
-                for (int h = 0; h < 2; h++) {
-                    const bool hit = ld2[h] < thr;
-                    const unsigned bb = __ballot_sync(full, hit);
-                    if (hit) {
-                        const int at = nq + __popc(bb & ((1u << lane) - 1u));
-                        qpos[w][at] = make_int2(lx * zl::LEAF, (ly + 4 * h) * zl::LEAF);
-                        qd2[w][at] = ld2[h];
+                for (int g = 0; g < TS_NODES; g++)
+#pragma unroll
+                    for (int h = 0; h < 2; h++) {
+                        const bool hit = ld2[g][h] < thr;
+                        const unsigned bb = __ballot_sync(full, hit);
+                        if (hit) {
+                            const int at = nq + __popc(bb & ((1u << lane) - 1u));
+                            qpos[w][at] = make_int2(lx[g] * zl::LEAF, (ly[g] + 4 * h) * zl::LEAF);
+                            qd2[w][at] = ld2[g][h];
+                        }
+                        nq += __popc(bb);
                     }
-                    nq += __popc(bb);
-                }
-                if (nq > TS_QUEUE - 64) flush();
+                if (nq > TS_QUEUE - 64 * TS_NODES) flush();
             }
         }
         flush();
         __syncwarp();
+        if (lane == 0) item = nwarps + atomicAdd(&t.head->next, 1u);
+        item = __shfl_sync(full, item, 0);
         if (n < K1 || K1 > FW_CAP - NEW) {  // fewer than k + 1 finite points (or a k beyond the list)
             if (lane == 0) {
                 atomicOr(err, 0x10u);
