@@ -11,6 +11,7 @@
 // Order selection follows the CPU reference: order drops to 0 when fewer than
 // {3, 5, 8}[order] neighbours.  Coordinates are accumulated relative to the
 // query point, which keeps FP32 sums at millimetre scale.
+#include <algorithm>
 #include <cmath>
 
 #include "zim_leaf.cuh"
@@ -333,10 +334,13 @@ __device__ __forceinline__ void mls_solve_project(const MlsFrame& F, int cur, co
 // MLS of one valid point.  visit(fn) calls fn((dx, dy), dz) with the offset from
 // the query point of every valid neighbour of its window (in a fixed order);
 // the distance test against the cut-off is made here.  ORDER2 false: orders 0 and
-// 1 only, without the second sweep's code and registers.
-template <bool ORDER2 = true, typename Visit>
+// 1 only, without the second sweep's code and registers.  BLOCK: visit is a
+// collective of the block's threads (valid point or not), which calls fn where
+// `on` holds.
+template <bool ORDER2 = true, bool BLOCK = false, typename Visit>
 __device__ __forceinline__ void mls_point(float inv_2s2, int order, float r2c, Visit visit, float& ox, float& oy,
-                                          float& oz, bool& moved) {
+                                          float& oz, bool& moved, bool& on) {
+    static_assert(ORDER2 || !BLOCK, "the collective form has the second sweep");
     moved = false;
     const float kw = -1.44269504088896341f * inv_2s2;  // -log2(e) / (2 s^2)
     // 1. weighted centroid and covariance in one sweep, from the moments about
@@ -365,12 +369,23 @@ __device__ __forceinline__ void mls_point(float inv_2s2, int order, float r2c, V
     });
     MlsFrame F;
     float C[3][3];
-    if (!mls_frame(ws, nv, cxy.x, cxy.y, cz, m00_11.x, m01, m02, m00_11.y, m12, m22, order, F, C)) return;
+    const bool go = mls_frame(ws, nv, cxy.x, cxy.y, cz, m00_11.x, m01, m02, m00_11.y, m12, m22, order, F, C);
     // Polynomial basis in tangent coordinates scaled by 1/h (h = cut-off
     // radius): the fitted surface is the same, the normal equations are O(1).
     const float is = rsqrtf(r2c);
+    if constexpr (BLOCK) {
+        // the second sweep with every thread of the block if any needs it
+        on = go && F.cur == 2;
+        if (__syncthreads_or(on)) {
+            if (!go) F = MlsFrame{};
+            float A[6][6], bv[6];
+            fit_normal_equations<6>(visit, kw, r2c, is, ws, C, F, A, bv);
+            if (on) mls_solve_project<6>(F, 2, A, bv, is, ox, oy, oz);
+        }
+    }
+    if (!go) return;
     if (ORDER2 && F.cur == 2) {
-        if constexpr (ORDER2) {
+        if constexpr (ORDER2 && !BLOCK) {
             float A[6][6], bv[6];
             fit_normal_equations<6>(visit, kw, r2c, is, ws, C, F, A, bv);
             mls_solve_project<6>(F, 2, A, bv, is, ox, oy, oz);
@@ -392,7 +407,7 @@ __global__ void __launch_bounds__(MX* MY) mls_kernel(const float* __restrict__ s
     const size_t o = (size_t)y * cols + x;
     const float px = src[3 * o], py = src[3 * o + 1], pz = src[3 * o + 2];
     float ox = 0.f, oy = 0.f, oz = 0.f;
-    bool moved = false;
+    bool moved = false, on = true;
     if (mask[o]) {
         const int r0 = max(0, y - hw), r1 = min(rows, y + hw + 1), c0 = max(0, x - hw), c1 = min(cols, x + hw + 1);
         auto visit = [&](auto&& fn) {
@@ -403,7 +418,7 @@ __global__ void __launch_bounds__(MX* MY) mls_kernel(const float* __restrict__ s
                     fn(make_float2(__ldg(src + 3 * q) - px, __ldg(src + 3 * q + 1) - py), __ldg(src + 3 * q + 2) - pz);
                 }
         };
-        mls_point(inv_2s2, order, r2c, visit, ox, oy, oz, moved);
+        mls_point(inv_2s2, order, r2c, visit, ox, oy, oz, moved, on);
     }
     dst[3 * o] = moved ? px + ox : px;
     dst[3 * o + 1] = moved ? py + oy : py;
@@ -417,7 +432,9 @@ inline size_t mls_smem_bytes(int hw) { return (size_t)(MX + 2 * hw) * (MY + 2 * 
 
 // Without pixel rays: the whole window.  HW: the half-window at compile time (0:
 // the hw argument), which makes the tile width and every neighbour offset
-// constants.
+// constants.  Five neighbours per step of a row's loop: 15 x 15, order 2,
+// 2448 x 2048: 1713 -> 1504 us; 61 x 61, order 1: 10.4 -> 9.3 ms (three per step
+// 1590 and 9.4).
 template <int HW>
 __global__ void __launch_bounds__(MX* MY) mls_smem_kernel(const float* __restrict__ src,
                                                           const uint8_t* __restrict__ mask, int rows, int cols, int hw_arg,
@@ -444,160 +461,288 @@ __global__ void __launch_bounds__(MX* MY) mls_smem_kernel(const float* __restric
     const float px = src[3 * o], py = src[3 * o + 1], pz = src[3 * o + 2];
     const float2 npxy = make_float2(-px, -py);  // q - p as q + (-p): the same rounding
     float ox = 0.f, oy = 0.f, oz = 0.f;
-    bool moved = false;
+    bool moved = false, on = true;
     if (mls_sp[cc].w != 0.f) {
         // invalid and off-image neighbours are NaN and fail the distance test
         auto visit = [&](auto&& fn) {
 #pragma unroll 1
             for (int i = -hw; i <= hw; i++)
+#pragma unroll 5
                 for (int j = -hw; j <= hw; j++) {
                     const float4 q = mls_sp[cc + i * TW + j];
                     fn(__fadd2_rn(make_float2(q.x, q.y), npxy), q.z - pz);
                 }
         };
-        mls_point(inv_2s2, order, r2c, visit, ox, oy, oz, moved);
+        mls_point(inv_2s2, order, r2c, visit, ox, oy, oz, moved, on);
     }
     dst[3 * o] = moved ? px + ox : px;
     dst[3 * o + 1] = moved ? py + oy : py;
     dst[3 * o + 2] = moved ? pz + oz : pz;
 }
 
-// With pixel rays: what the cut-off needs is usually a few pixels, whatever the
+// With pixel rays, what the cut-off needs is usually a few pixels, whatever the
 // window (the reference's default of 61 x 61 pixels with a 1.8 mm cut-off needs
-// 11 x 11 at 0.38 mm a pixel), so the tile stages only that. The ray bound with the largest ray distance of the window's leaves
-// (zim_leaf.cuh) gives each query a pixel radius; once more with the leaves
-// within the tile's largest radius, and the tile and a halo of that radius go to
-// shared memory.  Beyond MLS_LEAF_R pixels the neighbours are read from global
-// memory instead.  The neighbours and their order are those of the full window.
-// The default parameters (three passes) on a 2448 x 2048 cloud: 4975 us with the
-// whole window staged (two CTAs per SM, 22 staged points per query), 1733 us so;
-// a 15 x 15 window (order 2, 2 mm) takes the same time either way.
-constexpr int MLS_LEAF_R = 12;
-template <bool ORDER2>
-__global__ void __launch_bounds__(MX* MY) mls_leaf_kernel(const float* __restrict__ src,
-                                                          const uint8_t* __restrict__ mask, int rows, int cols, int hw,
-                                                          float inv_2s2, int order, float r2c, zt::RayParams rp,
-                                                          zl::Tree t, float* __restrict__ dst) {
-    constexpr int TMAX = MX + 2 * MLS_LEAF_R, WARPS = MX * MY / 32;
-    __shared__ float4 sp[TMAX * TMAX];
-    __shared__ unsigned s_red[2][WARPS];
-    __shared__ signed char s_w[WARPS][MLS_LEAF_R + 1];
-    const unsigned full = 0xffffffffu;
-    const int tid = threadIdx.y * MX + threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    const int x0 = blockIdx.x * MX, y0 = blockIdx.y * MY;
-    const int x = x0 + threadIdx.x, y = y0 + threadIdx.y;
-    const bool inside = x < cols && y < rows;
-    const size_t o = inside ? (size_t)y * cols + x : 0;
-    const bool act = inside && __ldg(mask + o) != 0;
-    const float px = __ldg(src + 3 * o), py = __ldg(src + 3 * o + 1), pz = __ldg(src + 3 * o + 2);
-    // largest value over the block (float bits, >= 0); each use has its own slots
-    auto block_max = [&](unsigned v, unsigned* slots) {
-        v = __reduce_max_sync(full, v);
-        if (lane == 0) slots[wid] = v;
-        __syncthreads();
-#pragma unroll
-        for (int j = 0; j < WARPS; j++) v = max(v, slots[j]);
-        return v;
-    };
-    // largest ray distance of the leaves that the tile dilated by R touches
-    auto leaf_dev = [&](int R) {
-        const int lx0 = max(x0 - R, 0) / zl::LEAF, lx1 = min((x0 + MX - 1 + R) / zl::LEAF, t.lw - 1);
-        const int ly0 = max(y0 - R, 0) / zl::LEAF, ly1 = min((y0 + MY - 1 + R) / zl::LEAF, t.lh - 1);
-        const int nx = lx1 - lx0 + 1, n = nx * (ly1 - ly0 + 1);
-        unsigned d = 0u;
-        for (int e = tid; e < n; e += MX * MY)
-            d = max(d, __float_as_uint(__ldg(t.leaf + 2 * ((size_t)(ly0 + e / nx) * t.lw + lx0 + e % nx) + 1).w));
-        return __uint_as_float(block_max(d, s_red[0]));
-    };
-    float ax, ay, az;
-    zt::ray_dir(rp, x, y, ax, ay, az);
-    const float an = sqrtf(fmaf(ax, ax, fmaf(ay, ay, az * az)));
-    const float qn = sqrtf(fmaf(px, px, fmaf(py, py, pz * pz)));
-    const float C = qn * rp.f / an;
-    const float sd0 = sqrtf(r2c) + zt::ray_dev(px, py, pz, ax, ay, az) + 1e-5f * qn;
-    // squared pixel radius beyond which no window point lies within the cut-off
-    auto radius2 = [&](float dev) {
+// 11 x 11 at 0.38 mm a pixel).  A query's ray bound with the largest ray distance
+// of the points around gives it a pixel radius, and a warp walks the disk of its
+// largest.  The neighbours and their order are those of the full window.
+//
+// Half-windows up to MLS_R: the window's tile is staged whole, and its ray
+// distances are taken on the way.  Above, they come from the leaves (zim_leaf.cuh):
+// with those of the whole window, then with those within the tile's largest radius,
+// and only that radius is staged; tiles that need more than MLS_R pixels are left
+// to mls_wide_kernel.  The default parameters (30 pixels, three passes) on a
+// 2448 x 2048 cloud: 4975 us with the whole window staged (two CTAs per SM, 22
+// staged points per query), 1620 us so.  At 10 pixels (order 2, 2 mm) the tree's
+// build is 5 us of 33 at 640 x 480, and the two are even at 2448 x 2048 (1.35 ms);
+// at 12 all of them, 6.79 against 6.53 ms.  Bound by issue and the FP32 pipe: a
+// neighbour is 50 instructions of both sweeps.
+constexpr int MLS_R = 12;
+
+// One tile of queries: its place, this thread's query and its bound.
+struct MlsTile {
+    const float* src;
+    const uint8_t* mask;
+    int rows, cols, x0, y0;
+    int tid, lane, wid, x, y;
+    bool inside, act;
+    size_t o;
+    float px, py, pz;
+    float an, C, sd0;  // of the ray bound
+
+    __device__ __forceinline__ MlsTile(const float* s, const uint8_t* m, int r, int c, int bx, int by)
+        : src(s), mask(m), rows(r), cols(c), x0(bx * MX), y0(by * MY), tid(threadIdx.y * MX + threadIdx.x),
+          lane(tid & 31), wid(tid >> 5), x(x0 + threadIdx.x), y(y0 + threadIdx.y), inside(x < c && y < r),
+          o(inside ? (size_t)y * c + x : 0) {
+        act = inside && __ldg(mask + o) != 0;
+        px = __ldg(src + 3 * o);
+        py = __ldg(src + 3 * o + 1);
+        pz = __ldg(src + 3 * o + 2);
+    }
+    __device__ __forceinline__ void ray_bound(float r2c, const zt::RayParams& rp) {
+        float ax, ay, az;
+        zt::ray_dir(rp, x, y, ax, ay, az);
+        an = sqrtf(fmaf(ax, ax, fmaf(ay, ay, az * az)));
+        const float qn = sqrtf(fmaf(px, px, fmaf(py, py, pz * pz)));
+        C = qn * rp.f / an;
+        sd0 = sqrtf(r2c) + zt::ray_dev(px, py, pz, ax, ay, az) + 1e-5f * qn;
+    }
+    // squared pixel radius beyond which no point within dev of its ray lies within
+    // the cut-off
+    __device__ __forceinline__ float radius2(float dev) const {
         if (!act) return 0.f;
         const float sd = sd0 + dev;
         if (!(C > sd)) return INFINITY;
         const float r = sd * an / (C - sd);
         return r * r;
-    };
-    int R = hw;
-    float rs2 = 0.f;
-    for (int pass = 0; pass < 2; pass++) {
-        rs2 = radius2(leaf_dev(R));
-        const float br2 = __uint_as_float(block_max(__float_as_uint(rs2), s_red[1]));
-        const int Rn = br2 < (float)(hw * hw) ? (int)sqrtf(br2) : hw;
-        if (Rn >= R) break;
-        R = Rn;
     }
-    const float wr2 = __uint_as_float(__reduce_max_sync(full, __float_as_uint(rs2)));
-    const bool staged = R <= MLS_LEAF_R;  // uniform over the block
-    const int TW = MX + 2 * R;
-    if (staged) {
-        if (lane <= R) {  // half-width of window rows +-lane, -1: row skipped
-            const float rem = wr2 - (float)(lane * lane);
-            s_w[wid][lane] = rem < 0.f ? -1 : (rem < (float)(hw * hw) ? min((int)sqrtf(rem), R) : R);
+    // largest value over the block (float bits, >= 0); each use has its own slots
+    __device__ __forceinline__ unsigned block_max(unsigned v, unsigned* slots) const {
+        v = __reduce_max_sync(0xffffffffu, v);
+        if (lane == 0) slots[wid] = v;
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < MX * MY / 32; j++) v = max(v, slots[j]);
+        return v;
+    }
+    static __device__ __forceinline__ float warp_max(float v) {  // v >= 0
+        return __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(v)));
+    }
+    // Pixel radius R of the window that the tile needs, and the squared radius of
+    // this warp's queries: a collective of the block.  red: two sets of slots.
+    __device__ __forceinline__ int radius(int hw, const zl::Tree& t, unsigned (*red)[MX * MY / 32], float& wr2) const {
+        // largest ray distance of the leaves that the tile dilated by R touches
+        auto leaf_dev = [&](int R) {
+            const int lx0 = max(x0 - R, 0) / zl::LEAF, lx1 = min((x0 + MX - 1 + R) / zl::LEAF, t.lw - 1);
+            const int ly0 = max(y0 - R, 0) / zl::LEAF, ly1 = min((y0 + MY - 1 + R) / zl::LEAF, t.lh - 1);
+            const int nx = lx1 - lx0 + 1, n = nx * (ly1 - ly0 + 1);
+            unsigned d = 0u;
+            for (int e = tid; e < n; e += MX * MY)
+                d = max(d, __float_as_uint(__ldg(t.leaf + 2 * ((size_t)(ly0 + e / nx) * t.lw + lx0 + e % nx) + 1).w));
+            return __uint_as_float(block_max(d, red[0]));
+        };
+        int R = hw;
+        float rs2 = 0.f;
+        for (int pass = 0; pass < 2; pass++) {
+            rs2 = radius2(leaf_dev(R));
+            const float br2 = __uint_as_float(block_max(__float_as_uint(rs2), red[1]));
+            const int Rn = br2 < (float)(hw * hw) ? (int)sqrtf(br2) : hw;
+            if (Rn >= R) break;
+            R = Rn;
         }
-        for (int e = tid; e < TW * (MY + 2 * R); e += MX * MY) {
-            const int ey = e / TW, gx = x0 - R + (e - ey * TW), gy = y0 - R + ey;
+        wr2 = warp_max(rs2);
+        return R;
+    }
+    // n rows of the tile and its halo of R pixels, from image row r0.  With rp:
+    // returns the largest ray distance of this thread's points (float bits).
+    __device__ __forceinline__ unsigned stage(float4* sp, int R, int r0, int n,
+                                              const zt::RayParams* rp = nullptr) const {
+        const int TW = MX + 2 * R;
+        unsigned dev = 0u;
+        for (int e = tid; e < TW * n; e += MX * MY) {
+            const int ey = e / TW, gx = x0 - R + (e - ey * TW), gy = r0 + ey;
             const float nan = __int_as_float(0x7fc00000);  // invalid and off-image: the distance test fails
             float4 v = make_float4(nan, nan, nan, 0.f);
             if (gx >= 0 && gy >= 0 && gx < cols && gy < rows) {
                 const size_t q = (size_t)gy * cols + gx;
                 const float vx = __ldg(src + 3 * q), vy = __ldg(src + 3 * q + 1), vz = __ldg(src + 3 * q + 2);
-                if (__ldg(mask + q)) v = make_float4(vx, vy, vz, 1.f);
+                if (__ldg(mask + q)) {
+                    v = make_float4(vx, vy, vz, 1.f);
+                    if (rp) {
+                        float ax, ay, az;
+                        zt::ray_dir(*rp, gx, gy, ax, ay, az);
+                        const float d = zt::ray_dev(vx, vy, vz, ax, ay, az);
+                        dev = max(dev, __float_as_uint(d == d ? d : INFINITY));  // NaN counts as unbounded
+                    }
+                }
             }
             sp[e] = v;
         }
-        __syncthreads();
+        return dev;
     }
-    if (!inside) return;
+    // half-width of the window's row at distance i that holds points within
+    // squared pixel radius wr2, -1: none
+    static __device__ __forceinline__ int row_width(float wr2, int i, int hw, int R) {
+        const float rem = wr2 - (float)(i * i);
+        return rem < 0.f ? -1 : (rem < (float)(hw * hw) ? min((int)sqrtf(rem), R) : R);
+    }
+    __device__ __forceinline__ void store(float* __restrict__ dst, bool moved, float ox, float oy, float oz) const {
+        if (!inside) return;
+        dst[3 * o] = moved ? px + ox : px;
+        dst[3 * o + 1] = moved ? py + oy : py;
+        dst[3 * o + 2] = moved ? pz + oz : pz;
+    }
+};
+
+// NEAR: half-windows up to MLS_R.  HW: the half-window at compile time (0: hw_arg),
+// which makes the tile's width constant.  With four CTAs per SM asked for, the
+// second order keeps to 64 registers.
+template <bool ORDER2, bool NEAR, int HW>
+__global__ void __launch_bounds__(MX* MY, ORDER2 && NEAR ? 4 : 1) mls_ray_kernel(const float* __restrict__ src,
+                                                          const uint8_t* __restrict__ mask, int rows, int cols,
+                                                          int hw_arg, float inv_2s2, int order, float r2c,
+                                                          zt::RayParams rp, zl::Tree t, unsigned* __restrict__ wide,
+                                                          float* __restrict__ dst) {
+    const int hw = HW ? HW : hw_arg;
+    constexpr int RMAX = HW ? HW : MLS_R, TMAX = MX + 2 * RMAX, WARPS = MX * MY / 32;
+    __shared__ float4 sp[TMAX * TMAX];
+    __shared__ unsigned s_red[2][WARPS];
+    __shared__ signed char s_w[WARPS][RMAX + 1];
+    MlsTile T(src, mask, rows, cols, blockIdx.x, blockIdx.y);
+    int R = hw;
+    float wr2;
+    if constexpr (NEAR) {
+        const unsigned dev = T.stage(sp, hw, T.y0 - hw, MY + 2 * hw, &rp);
+        T.ray_bound(r2c, rp);
+        wr2 = T.warp_max(T.radius2(__uint_as_float(T.block_max(dev, s_red[0]))));  // the tile is staged
+    } else {
+        T.ray_bound(r2c, rp);
+        R = T.radius(hw, t, s_red, wr2);
+        if (R > MLS_R) {  // uniform over the block
+            if (T.tid == 0) wide[atomicAdd(&t.head->n_deferred, 1u)] = blockIdx.y * gridDim.x + blockIdx.x;
+            return;
+        }
+        T.stage(sp, R, T.y0 - R, MY + 2 * R);
+    }
+    const int lane = T.lane, wid = T.wid;
+    if (lane <= R) s_w[wid][lane] = MlsTile::row_width(wr2, lane, hw, R);
+    if (NEAR) __syncwarp();
+    else __syncthreads();
     float ox = 0.f, oy = 0.f, oz = 0.f;
-    bool moved = false;
-    if (act) {
-        const float2 npxy = make_float2(-px, -py);  // q - p as q + (-p): the same rounding
-        if (staged) {
-            const float4* c = sp + (threadIdx.y + R) * TW + threadIdx.x + R;
-            auto visit = [&](auto&& fn) {
+    bool moved = false, on = true;
+    if (T.act) {
+        const int TW = MX + 2 * R;
+        const int Rw = wr2 < (float)(R * R) ? (int)sqrtf(wr2) : R;  // rows that hold any
+        const float pz = T.pz;
+        const float2 npxy = make_float2(-T.px, -T.py);  // q - p as q + (-p): the same rounding
+        const float4* c = sp + (threadIdx.y + R) * TW + threadIdx.x + R;
+        auto visit = [&](auto&& fn) {
 #pragma unroll 1
-                for (int i = -R; i <= R; i++) {
-                    const int w = s_w[wid][i < 0 ? -i : i];
-                    const float4* row = c + i * TW;
-                    for (int j = -w; j <= w; j++) {
+            for (int i = -Rw; i <= Rw; i++) {
+                const int w = s_w[wid][i < 0 ? -i : i];
+                const float4* row = c + i * TW;
+                for (int j = -w; j <= w; j++) {
+                    const float4 q = row[j];
+                    fn(__fadd2_rn(make_float2(q.x, q.y), npxy), q.z - pz);
+                }
+            }
+        };
+        mls_point<ORDER2>(inv_2s2, order, r2c, visit, ox, oy, oz, moved, on);
+    }
+    T.store(dst, moved, ox, oy, oz);
+}
+
+// The tiles that need more than MLS_R pixels (points far off their rays, wide
+// cut-offs).  Where the tile and its halo exceed the shared memory (cap points), a
+// few rows of the window at a time, the whole block together.  Four neighbours are
+// tested before any adds: where the radius comes from a point far off its ray, few
+// pass (a 640 x 480 cloud with three such tiles: 646 us with neighbours read from
+// global memory, 125 us so; with the whole window staged for every tile, 176).
+__global__ void __launch_bounds__(MX* MY, 2) mls_wide_kernel(const float* __restrict__ src,
+                                                             const uint8_t* __restrict__ mask, int rows, int cols,
+                                                             int hw, float inv_2s2, int order, float r2c,
+                                                             zt::RayParams rp, zl::Tree t,
+                                                             const unsigned* __restrict__ wide, int cap,
+                                                             float* __restrict__ dst) {
+    extern __shared__ float4 sp[];
+    __shared__ unsigned s_red[2][MX * MY / 32];
+    const unsigned n = t.head->n_deferred, nx = (cols + MX - 1) / MX;
+    for (unsigned item = blockIdx.x; item < n; item += gridDim.x) {
+        const unsigned tile = wide[item];
+        MlsTile T(src, mask, rows, cols, tile % nx, tile / nx);
+        T.ray_bound(r2c, rp);
+        __syncthreads();  // the slots of the tile before
+        float wr2;
+        const int R = T.radius(hw, t, s_red, wr2);
+        const int TW = MX + 2 * R, CH = cap / TW;
+        const float2 npxy = make_float2(-T.px, -T.py);
+        const float pz = T.pz;
+        float ox = 0.f, oy = 0.f, oz = 0.f;
+        bool moved = false, on = T.act;
+        auto visit = [&](auto&& fn) {
+            for (int r0 = T.y0 - R; r0 < T.y0 + MY + R; r0 += CH) {
+                __syncthreads();
+                T.stage(sp, R, r0, min(CH, T.y0 + MY + R - r0));
+                __syncthreads();
+                if (!on) continue;
+#pragma unroll 1
+                for (int i = max(r0, T.y - R); i <= min(r0 + CH - 1, T.y + R); i++) {
+                    const int w = MlsTile::row_width(wr2, i - T.y, hw, R);
+                    const float4* row = sp + (i - r0) * TW + threadIdx.x + R;
+                    int j = -w;
+                    for (; j + 3 <= w; j += 4) {
+                        float2 d[4];
+                        float dz[4], m = INFINITY;
+#pragma unroll
+                        for (int u = 0; u < 4; u++) {
+                            const float4 q = row[j + u];
+                            d[u] = __fadd2_rn(make_float2(q.x, q.y), npxy);
+                            dz[u] = q.z - pz;
+                            m = fminf(m, fmaf(dz[u], dz[u], fmaf(d[u].y, d[u].y, d[u].x * d[u].x)));
+                        }
+                        if (!(m <= r2c)) continue;
+#pragma unroll
+                        for (int u = 0; u < 4; u++) fn(d[u], dz[u]);
+                    }
+                    for (; j <= w; j++) {
                         const float4 q = row[j];
                         fn(__fadd2_rn(make_float2(q.x, q.y), npxy), q.z - pz);
                     }
                 }
-            };
-            mls_point<ORDER2>(inv_2s2, order, r2c, visit, ox, oy, oz, moved);
-        } else {
-            auto visit = [&](auto&& fn) {
-#pragma unroll 1
-                for (int i = max(-R, -y); i <= min(R, rows - 1 - y); i++) {
-                    const float rem = wr2 - (float)(i * i);
-                    if (rem < 0.f) continue;
-                    const int w = rem < (float)(hw * hw) ? (int)sqrtf(rem) : hw;
-                    for (int j = max(-w, -x); j <= min(w, cols - 1 - x); j++) {
-                        const size_t q = o + (ptrdiff_t)i * cols + j;
-                        if (!__ldg(mask + q)) continue;
-                        fn(__fadd2_rn(make_float2(__ldg(src + 3 * q), __ldg(src + 3 * q + 1)), npxy),
-                           __ldg(src + 3 * q + 2) - pz);
-                    }
-                }
-            };
-            mls_point<ORDER2>(inv_2s2, order, r2c, visit, ox, oy, oz, moved);
-        }
+            }
+        };
+        mls_point<true, true>(inv_2s2, order, r2c, visit, ox, oy, oz, moved, on);
+        T.store(dst, moved, ox, oy, oz);
     }
-    dst[3 * o] = moved ? px + ox : px;
-    dst[3 * o + 1] = moved ? py + oy : py;
-    dst[3 * o + 2] = moved ? pz + oz : pz;
 }
 
 }  // namespace
 
-size_t zim_mls_scratch_bytes(int rows, int cols) { return zim_leaf_bytes(rows, cols); }
+constexpr size_t MLS_SMEM = 96 * 1024;  // shared memory of a tile: two CTAs per SM
+static size_t mls_tiles(int rows, int cols) { return (size_t)((cols + MX - 1) / MX) * ((rows + MY - 1) / MY); }
+
+size_t zim_mls_scratch_bytes(int rows, int cols) {
+    return zim_leaf_bytes(rows, cols) + zim_align256(mls_tiles(rows, cols) * 4);
+}
 
 zim_status zim_mls_launch(zim_ctx* ctx, const float* xyz, const uint8_t* mask, int rows, int cols, int window,
                           float sigma, int order, float max_radius, int iterations, float* out, float* tmp,
@@ -608,15 +753,22 @@ zim_status zim_mls_launch(zim_ctx* ctx, const float* xyz, const uint8_t* mask, i
     const int n_iter = iterations < 1 ? 1 : iterations;
     dim3 blk(MX, MY), grd((cols + MX - 1) / MX, (rows + MY - 1) / MY);
     const size_t smem = mls_smem_bytes(window);
-    const bool use_smem = smem <= 96 * 1024;
+    const bool use_smem = smem <= MLS_SMEM;
     auto kern = window == 7 ? mls_smem_kernel<7> : mls_smem_kernel<0>;
-    if (use_smem) ZIM_CUDA_TRY(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (use_smem)
+        ZIM_CUDA_TRY(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const zt::RayParams rp = zt::ray_params(rays);
-    const bool leaf = rays.valid != 0;
+    const bool near = rays.valid != 0 && window <= MLS_R, leaf = rays.valid != 0 && !near;
     zl::Tree t{};
+    unsigned* wide = nullptr;  // tiles left to mls_wide_kernel
+    const size_t wide_smem = std::min(smem, MLS_SMEM);
     if (leaf) {
         zim_status s = zim_leaf_carve(ctx, rows, cols, t);
         if (s) return s;
+        wide = (unsigned*)zim_scratch_take(ctx, mls_tiles(rows, cols) * 4);
+        if (!wide) return zim_fail(ctx, ZIM_ERR_OUT_OF_MEMORY, "MLS scratch carve");
+        ZIM_CUDA_TRY(ctx, cudaFuncSetAttribute(mls_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (int)wide_smem));
     }
     // ping-pong so that the last pass lands in `out`
     const float* in = xyz;
@@ -626,8 +778,17 @@ zim_status zim_mls_launch(zim_ctx* ctx, const float* xyz, const uint8_t* mask, i
         if (leaf) {
             zim_status s = zim_leaf_build(ctx, in, mask, rows, cols, &rp, t, st);
             if (s) return s;
-            auto lk = ord == 2 ? mls_leaf_kernel<true> : mls_leaf_kernel<false>;
-            lk<<<grd, blk, 0, st>>>(in, mask, rows, cols, window, inv_2s2, ord, r2c, rp, t, dst);
+            auto lk = ord == 2 ? mls_ray_kernel<true, false, 0> : mls_ray_kernel<false, false, 0>;
+            lk<<<grd, blk, 0, st>>>(in, mask, rows, cols, window, inv_2s2, ord, r2c, rp, t, wide, dst);
+            ZIM_LAUNCH_CHECK(ctx);
+            const unsigned sms = ctx->sm_count > 0 ? ctx->sm_count : 152;
+            mls_wide_kernel<<<(unsigned)std::min<size_t>(mls_tiles(rows, cols), 2 * sms), blk, wide_smem, st>>>(
+                in, mask, rows, cols, window, inv_2s2, ord, r2c, rp, t, wide, (int)(wide_smem / sizeof(float4)), dst);
+            ctx->launches += 1;
+        } else if (near) {
+            auto nk = window == 7 ? (ord == 2 ? mls_ray_kernel<true, true, 7> : mls_ray_kernel<false, true, 7>)
+                                  : (ord == 2 ? mls_ray_kernel<true, true, 0> : mls_ray_kernel<false, true, 0>);
+            nk<<<grd, blk, 0, st>>>(in, mask, rows, cols, window, inv_2s2, ord, r2c, rp, t, wide, dst);
         } else if (use_smem)
             kern<<<grd, blk, smem, st>>>(in, mask, rows, cols, window, inv_2s2, ord, r2c, dst);
         else
