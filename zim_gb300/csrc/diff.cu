@@ -18,7 +18,7 @@
 //   dLoss/dtheta += -(g . P)/w * dw/dtheta   (g = upstream dLoss/dP)
 //   J_r = -(n . P)/w * dw/dtheta             (plane distance, for J^T J).
 // The loss is summed in FP64 per thread, the gradient as two-float sums, J^T J in
-// FP32 over 22 points and then as two-float sums; warps, blocks and their partials
+// FP32 over 32 points and then as two-float sums; warps, blocks and their partials
 // add in FP64 in a fixed order.
 #include <cmath>
 #include <cstring>
@@ -134,30 +134,33 @@ __device__ __forceinline__ bool take_sample(const DiffCam& c, float col, float r
 // of weight W = dw/dphi contributes to dw/dtheta: W (gu du/dtheta + gv dv/dtheta).
 template <bool ROT>
 __device__ __forceinline__ void add_jacobian(const DiffCam& c, const Sample& s, float W, float* Jc, float* Jrot) {
-    const float x = s.x, y = s.y, P = W * s.gu, Q = W * s.gv;
+    const float x = s.x, y = s.y, gu = s.gu, gv = s.gv;
     const float r2 = fmaf(x, x, y * y);
     const float sd = fmaf(r2, fmaf(r2, fmaf(r2, c.k3, c.k2), c.k1), 1.0f);
     const float xd = fmaf(x, sd, fmaf(2.0f * c.p1, x * y, c.p2 * fmaf(2.0f * x, x, r2)));
     const float yd = fmaf(y, sd, fmaf(c.p1, fmaf(2.0f * y, y, r2), 2.0f * c.p2 * x * y));
-    const float Pf = P * c.fx, Qf = Q * c.fy;
-    const float t = r2 * fmaf(Pf, x, Qf * y);
-    Jc[0] = fmaf(P, xd, Jc[0]);
-    Jc[1] = fmaf(Q, yd, Jc[1]);
-    Jc[2] += P;
-    Jc[3] += Q;
-    Jc[4] += t;
-    Jc[5] = fmaf(t, r2, Jc[5]);
+    const float r4 = r2 * r2, fx = c.fx * x, fy = c.fy * y;
+    Jc[0] = fmaf(W, __fmul_rn(gu, xd), Jc[0]);
+    Jc[1] = fmaf(W, __fmul_rn(gv, yd), Jc[1]);
+    Jc[2] = fmaf(W, gu, Jc[2]);
+    Jc[3] = fmaf(W, gv, Jc[3]);
+    Jc[4] = fmaf(W, fmaf(gu, fx * r2, __fmul_rn(gv, fy * r2)), Jc[4]);
+    Jc[5] = fmaf(W, fmaf(gu, fx * r4, __fmul_rn(gv, fy * r4)), Jc[5]);
     if (ROT) {
-        // ray X -> X + X x eps: d(x, y)/d eps = (x y, -1 - x^2, y), (1 + y^2, -x y, -x)
+        // ray X -> X + X x eps: d(x, y)/d eps_k for k = 0, 1, 2
+        const float dx[3] = {x * y, -1.0f - x * x, y};
+        const float dy[3] = {1.0f + y * y, -x * y, -x};
         const float s1 = fmaf(r2, fmaf(3.0f * c.k3, r2, 2.0f * c.k2), c.k1);  // d sd / d r2
         const float dxd_dx = sd + 2.0f * x * x * s1 + 2.0f * c.p1 * y + 6.0f * c.p2 * x;
         const float dxd_dy = 2.0f * x * y * s1 + 2.0f * c.p1 * x + 2.0f * c.p2 * y;
+        const float dyd_dx = dxd_dy;
         const float dyd_dy = sd + 2.0f * y * y * s1 + 6.0f * c.p1 * y + 2.0f * c.p2 * x;
-        const float A = fmaf(Pf, dxd_dx, Qf * dxd_dy), B = fmaf(Pf, dxd_dy, Qf * dyd_dy);  // dyd_dx = dxd_dy
-        const float xy = x * y;
-        Jrot[0] += fmaf(A, xy, B * fmaf(y, y, 1.0f));
-        Jrot[1] -= fmaf(A, fmaf(x, x, 1.0f), B * xy);
-        Jrot[2] += fmaf(A, y, -(B * x));
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            const float ju = c.fx * fmaf(dxd_dx, dx[k], dxd_dy * dy[k]);
+            const float jv = c.fy * fmaf(dyd_dx, dx[k], dyd_dy * dy[k]);
+            Jrot[k] = fmaf(W, fmaf(gu, ju, __fmul_rn(gv, jv)), Jrot[k]);
+        }
     }
 }
 
@@ -194,8 +197,7 @@ __device__ __forceinline__ void scatter_phase(float* g, int sw, const Sample& s,
 // are rounded: a product fused into the addition would not match its error term.
 // An infinite sum has no error term (its lo is NaN).  Over 704 values the error to
 // the exact sum is that of FP64 sums of the same values (1.2e-10 of the sum of
-// magnitudes, from the values' own rounding); J^T J's, with 22 instead of 32 rows
-// in FP32, is 1.0e-9 (1.4e-9).
+// magnitudes, from the values' own rounding).
 struct Sum2 {
     float hi, lo;
     __device__ __forceinline__ void add(float v) {
@@ -220,22 +222,23 @@ __device__ __forceinline__ int jtj_entry(int a, int b) { return a * NP - a * (a 
 // UP: an upstream gradient of the points or a phase gradient is asked for.
 //
 // The gradient's FP32 terms add up as two-float sums (with an upstream gradient per
-// thread, else lane k of a half-warp component k of the warp's staged rows: two
-// registers instead of 32).  J^T J: a warp's 32 rows go through shared memory, and
-// three groups of ten lanes each add up the
-// ten blocks of the outer products of a third of the rows, 16 products per two
-// 16-byte loads, in FP32 over 22 rows and then as two-float sums.  (One product per
-// two 4-byte loads, and 37 FP64 conversions and additions per 32 points, held the
-// kernel at the FP64 and shared-memory pipes.)  A point's four samples are located
-// before any of their 32 loads, so that these are in flight together.  Four
-// 2448x2048 views: 4.23 -> 1.21 ms; bound by issue and latency, with 16 warps
-// per SM, and the FP64 pipe half busy with the points' distances.
+// thread, else through shared memory, lane k of a half-warp component k of the
+// warp's points: two registers instead of 32).  J^T J: the rows of 3 x 32 points go
+// through shared memory, and three groups of ten lanes each add up the ten blocks of
+// 32 rows' outer products, 16 products per two 16-byte loads, in FP32 over the 32 and
+// then as two-float sums.  (One product per two 4-byte loads, and 37 FP64 conversions
+// and additions per 32 points, held the kernel at the FP64 and shared-memory pipes.)
+// A point's four samples are located before any of their 32 loads, so that these are
+// in flight together.  Four 2448x2048 views: 4.23 -> 1.18 ms; bound by issue and
+// latency, with 16 warps per SM (12: 1.27), and the FP64 pipe half busy with the
+// points' distances.
 template <bool BWD, bool UP>
 __global__ void __launch_bounds__(DIFF_T, BWD ? (UP ? DIFF_UP : DIFF_BWD) : DIFF_FWD)
     diff_kernel(const __grid_constant__ DiffDev P,
                                                          const ViewDev* __restrict__ views, int n_views,
                                                          float loss_weight, double* __restrict__ part) {
-    __shared__ __align__(16) float rows[BWD ? DIFF_W : 1][32][ROW];
+    __shared__ __align__(16) float rows[BWD ? DIFF_W : 1][3][32][ROW];
+    __shared__ __align__(16) float terms[BWD && !UP ? DIFF_W : 1][32][ROW];
     __shared__ double red[DIFF_W][NACC];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const size_t npx = (size_t)P.rw * P.rh;
@@ -243,37 +246,51 @@ __global__ void __launch_bounds__(DIFF_T, BWD ? (UP ? DIFF_UP : DIFF_BWD) : DIFF
     double loss = 0.0;
     unsigned cnt = 0u;
     Sum2 g[UP ? NP : 1];
-    float acc[16];
     Sum2 sum[16];
 #pragma unroll
     for (int k = 0; k < (UP ? NP : 1); k++) g[k] = Sum2{0.f, 0.f};
 #pragma unroll
-    for (int k = 0; k < 16; k++) {
-        acc[k] = 0.f;
-        sum[k] = Sum2{0.f, 0.f};
-    }
+    for (int k = 0; k < 16; k++) sum[k] = Sum2{0.f, 0.f};
     const int grp = lane / NBLK, blk = lane - grp * NBLK;  // lanes 30 and 31 repeat others' work
     const int br = 4 * block_row(blk), bc = 4 * block_col(blk);
-    auto flush = [&]() {
+    // adds the n staged sets of 32 rows, one per group of lanes
+    int n_sets = 0;
+    auto add_sets = [&]() {
+        if (grp < n_sets) {
+            float acc[16];
 #pragma unroll
-        for (int k = 0; k < 16; k++) {
-            sum[k].add(acc[k]);
-            acc[k] = 0.f;
+            for (int k = 0; k < 16; k++) acc[k] = 0.f;
+#pragma unroll 4
+            for (int p = 0; p < 32; p++) {
+                const float4 u4 = *reinterpret_cast<const float4*>(&rows[wib][grp][p][br]);
+                const float4 v4 = *reinterpret_cast<const float4*>(&rows[wib][grp][p][bc]);
+                const float u[4] = {u4.x, u4.y, u4.z, u4.w}, v[4] = {v4.x, v4.y, v4.z, v4.w};
+#pragma unroll
+                for (int a = 0; a < 4; a++)
+#pragma unroll
+                    for (int e = 0; e < 4; e++) acc[4 * a + e] = fmaf(u[a], v[e], acc[4 * a + e]);
+            }
+#pragma unroll
+            for (int k = 0; k < 16; k++) sum[k].add(acc[k]);
         }
+        n_sets = 0;
     };
 
-    // a warp strides over each view's pixels: the loop bound depends on the warp
-    // only, so the lanes stay together, and (i, j) follow without divisions
-    bool odd = false;
+    // A warp strides over each view's pixels: the loop bound depends on the warp only,
+    // so the lanes stay together, and (i, j) follow without divisions.  The sets of 32
+    // pixels are those of all views' pixels in one row, whose first and last in a view
+    // may be incomplete.
     const int stride = (int)nwarps * 32, di = stride / P.rw, dj = stride - di * P.rw;
     const size_t base0 = ((size_t)blockIdx.x * DIFF_W + wib) * 32;
     for (int vi = 0; vi < n_views; vi++) {
         const ViewDev& V = views[vi];
-        size_t pix = base0 + lane;
-        int i = (int)(pix / P.rw), j = (int)(pix - (size_t)i * P.rw);
+        const int shift = (int)(vi * npx & 31);
+        size_t pix = base0 + lane - shift;  // wraps above npx for the shift's first lanes
+        int i = (int)((base0 + lane - shift + 32 * (size_t)P.rw) / P.rw) - 32;
+        int j = (int)(pix - (size_t)i * P.rw);
         int bnext = pix < npx ? __ldg(V.best + pix) : -1;
-        for (size_t base = base0; base < npx; base += stride, pix += stride) {
-            float J[NP], r = 0.f;
+        for (size_t base = base0; base < npx + shift; base += stride, pix += stride) {
+            float J[NP], s_r = 0.f, s_up = 0.f;
 #pragma unroll
             for (int k = 0; k < NP; k++) J[k] = 0.f;
             const int b = bnext;
@@ -344,13 +361,13 @@ __global__ void __launch_bounds__(DIFF_T, BWD ? (UP ? DIFF_UP : DIFF_BWD) : DIFF
                 const double Nd = fma(V.nd[0], (double)j + P.q03d,
                                       fma(V.nd[1], (double)i + P.q13d, fma(V.nd[2], P.q23d, V.pdd * wd)));
                 const float iw = 1.0f / w;
-                r = (float)Nd * iw;
+                const float r = (float)Nd * iw;
                 loss += (double)r * (double)r;
                 cnt++;
                 if (BWD) {
                     // n . P = r - d, and dr/dw = -(n . P)/w
                     const float nP = r - (float)V.pdd;
-                    const float s_r = -nP * iw;
+                    s_r = -nP * iw;
                     // dw/dphi: d = j - b - delta, w = q32 d + q33
                     const float wR[3] = {-P.q32 * dd[0], -P.q32 * dd[1], -P.q32 * dd[2]};
                     const float wL = -(wR[0] + wR[1] + wR[2]);
@@ -362,46 +379,37 @@ __global__ void __launch_bounds__(DIFF_T, BWD ? (UP ? DIFF_UP : DIFF_BWD) : DIFF
                     float gP = loss_weight * 2.0f * r * nP;
                     if (UP && V.gxyz)
                         gP += fmaf(V.gxyz[3 * pix], X, fmaf(V.gxyz[3 * pix + 1], Y, V.gxyz[3 * pix + 2] * Z));
-                    const float s_up = -gP * iw;
+                    s_up = -gP * iw;
                     if (UP) {
                         scatter_phase(V.gphase[0], P.sw, sL, s_up * wL);
 #pragma unroll
                         for (int m = 0; m < 3; m++) scatter_phase(V.gphase[1], P.sw, sR[m], s_up * wR[m]);
                     }
 #pragma unroll
-                    for (int k = 0; k < NP; k++) {
+                    for (int k = 0; k < NP; k++)
                         if (UP) g[k].add(__fmul_rn(s_up, J[k]));
-                        J[k] *= s_r;
-                    }
                 }
             }
             if (BWD) {
-                float4* row = reinterpret_cast<float4*>(rows[wib][lane]);
+                // dLoss/dw J_w and the row of J_r = dr/dw J_w (0 where there is no point)
+                float4* row = reinterpret_cast<float4*>(rows[wib][n_sets][lane]);
 #pragma unroll
-                for (int k = 0; k < 4; k++) row[k] = make_float4(J[4 * k], J[4 * k + 1], J[4 * k + 2], J[4 * k + 3]);
-                if (!UP) rows[wib][lane][NP] = loss_weight * 2.0f * r;
+                for (int k = 0; k < NP; k += 4) {
+                    if (!UP)
+                        reinterpret_cast<float4*>(terms[wib][lane])[k / 4] =
+                            make_float4(s_up * J[k], s_up * J[k + 1], s_up * J[k + 2], s_up * J[k + 3]);
+                    row[k / 4] = make_float4(s_r * J[k], s_r * J[k + 1], s_r * J[k + 2], s_r * J[k + 3]);
+                }
+                n_sets++;
                 __syncwarp();
                 if (!UP) {
                     // lane k of each half-warp: component k over half of the rows (those
                     // apart by four, whose words lie in other banks)
 #pragma unroll 4
-                    for (int p = 0; p < 16; p++) {
-                        const float* row = rows[wib][(p & 3) | (p & 12) << 1 | (lane & 16) >> 2];
-                        g[0].add(__fmul_rn(row[NP], row[lane & 15]));
-                    }
+                    for (int p = 0; p < 16; p++)
+                        g[0].add(terms[wib][(p & 3) | (p & 12) << 1 | (lane & 16) >> 2][lane & 15]);
                 }
-#pragma unroll 4
-                for (int p = grp; p < 32; p += 3) {
-                    const float4 u4 = *reinterpret_cast<const float4*>(&rows[wib][p][br]);
-                    const float4 v4 = *reinterpret_cast<const float4*>(&rows[wib][p][bc]);
-                    const float u[4] = {u4.x, u4.y, u4.z, u4.w}, v[4] = {v4.x, v4.y, v4.z, v4.w};
-#pragma unroll
-                    for (int a = 0; a < 4; a++)
-#pragma unroll
-                        for (int e = 0; e < 4; e++) acc[4 * a + e] = fmaf(u[a], v[e], acc[4 * a + e]);
-                }
-                if (odd) flush();
-                odd = !odd;
+                if (n_sets == 3) add_sets();
                 __syncwarp();
             }
             i += di;
@@ -430,7 +438,7 @@ __global__ void __launch_bounds__(DIFF_T, BWD ? (UP ? DIFF_UP : DIFF_BWD) : DIFF
             if (UP && lane == 0) red[wib][2 + k] = v;
             if (!UP && lane < NP) red[wib][2 + lane] = v;
         }
-        flush();
+        add_sets();
 #pragma unroll
         for (int k = 0; k < 16; k++) {
             double v = sum[k].value();
