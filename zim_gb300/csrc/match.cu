@@ -20,7 +20,14 @@
 
 namespace {
 
-constexpr int MATCH_THREADS = 256;
+// A row's staged columns hold four CTAs per SM at 4185 columns: 16 warps each hide
+// the latency that 8 do not (whole-frame match, 4185 x 3064: 227 -> 165 us; 653 to
+// 2500 columns: even).  The fused kernel holds more registers and gathers for
+// longer, and 8 warps are enough (2500 x 2092: 94 us, 16 warps 113), except where
+// one wave of larger CTAs takes all rows (RM_SMALL_THREADS; 653 x 488: 21 -> 19 us;
+// 1300 x 1041, more than a wave: 46 us against 50).
+constexpr int MATCH_THREADS = 512;
+constexpr int RM_THREADS = 256, RM_SMALL_THREADS = 384, RM_SMALL_CTAS = 3;  // per SM
 
 // Left and right windows of one launch.  The whole-frame match uses the full
 // rows of both images; the ROI match a left rectangle and a right column
@@ -53,22 +60,35 @@ __global__ void __launch_bounds__(MATCH_THREADS) match_kernel(MatchWin w, int ph
         s_hi[k] = -1;
         s_bad[k] = 0;
     }
+#pragma unroll 4
     for (int j = threadIdx.x; j < cols; j += blockDim.x) {
-        s_ord[j] = w.r_order[ro + j];
-        s_ph[j] = make_int2(w.r_base[ro + j], __float_as_int(w.r_res[ro + j]));
+        s_ord[j] = __ldg(w.r_order + ro + j);
+        s_ph[j] = make_int2(__ldg(w.r_base + ro + j), __float_as_int(__ldg(w.r_res + ro + j)));
     }
+    // the left row's values are loaded one step ahead, the first across the barriers
+    int nk = 0, nb = 0, j = threadIdx.x;
+    float nr = 0.f;
+    auto left = [&](int j) {
+        nk = __ldg(w.l_order + ro + j);
+        nb = __ldg(w.l_base + ro + j);
+        nr = __ldg(w.l_res + ro + j);
+    };
+    if (j < w.l_cols) left(j);
     __syncthreads();
     zt::match_spans(s_ord, cols, pha_f, s_lo, s_hi, threadIdx.x, blockDim.x);
     __syncthreads();
     zt::match_spans_check(s_ord, s_ph, cols, pha_f, s_hi, s_bad, threadIdx.x, blockDim.x);
     __syncthreads();
     const size_t oo = (size_t)row * w.out_stride;
-    for (int j = threadIdx.x; j < w.l_cols; j += blockDim.x) {
+    for (; j < w.l_cols; j += blockDim.x) {
+        const int k = nk, b = nb;
+        const float r = nr;
+        const int jn = j + blockDim.x;
+        if (jn < w.l_cols) left(jn);
         float d = 0.f;
         int best = -1;
         if (!w.l_mask || w.l_mask[ro + j])
-            zt::match_pixel(j, w.l_order[ro + j], w.l_base[ro + j], w.l_res[ro + j], s_ord, s_ph, s_lo,
-                            s_hi, s_bad, cols, pha_f, grad_threshold, d, best, w.dx_off);
+            zt::match_pixel(j, k, b, r, s_ord, s_ph, s_lo, s_hi, s_bad, cols, pha_f, grad_threshold, d, best, w.dx_off);
         w.disp[oo + j] = d;
         if (w.best_col) w.best_col[oo + j] = best;
     }
@@ -108,7 +128,8 @@ __device__ __forceinline__ void rect_px(const RectMatchArgs& a, int cam, float m
         zt::rectify_pixel(a.order[cam], a.res[cam], a.srows, a.scols, mx, my, a.post_smooth, b, r, k);
 }
 
-__global__ void __launch_bounds__(MATCH_THREADS) rectify_match_kernel(RectMatchArgs a, int pha_f,
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS) rectify_match_kernel(RectMatchArgs a, int pha_f,
                                                                       float grad_threshold) {
     extern __shared__ int4 smem_raw[];
     const int cols = a.cols;
@@ -194,9 +215,11 @@ zim_status zim_rectify_match_launch(zim_ctx* ctx, const int32_t* const order[2],
     if (a.cols > ZIM_MAX_MATCH_COLS)
         return zim_fail(ctx, ZIM_ERR_INVALID_ARG, "rectified width %d above %d", a.cols, ZIM_MAX_MATCH_COLS);
     const size_t smem = (size_t)a.cols * 12 + (size_t)(pha_f + 1) * 12;
-    ZIM_CUDA_TRY(ctx, cudaFuncSetAttribute(rectify_match_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)smem));
-    rectify_match_kernel<<<a.rows, MATCH_THREADS, smem, st>>>(a, pha_f, (float)grad_threshold);
+    const int sms = ctx->sm_count > 0 ? ctx->sm_count : 152;
+    const bool small = a.rows <= RM_SMALL_CTAS * sms + sms / 4;
+    auto kern = small ? rectify_match_kernel<RM_SMALL_THREADS> : rectify_match_kernel<RM_THREADS>;
+    ZIM_CUDA_TRY(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    kern<<<a.rows, small ? RM_SMALL_THREADS : RM_THREADS, smem, st>>>(a, pha_f, (float)grad_threshold);
     ctx->launches += 1;
     ZIM_LAUNCH_CHECK(ctx);
     return ZIM_OK;
