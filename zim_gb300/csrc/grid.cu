@@ -1611,7 +1611,9 @@ __global__ void __launch_bounds__(MT_WARPS * 32) metric_gaussian_tree_kernel(
             }
         }
         if (act) {
-            const double kd = (double)r / (double)sw;  // (S / 2^40 * r) / (W / 2^40)
+            // (S / 2^40 * r) / (W / 2^40); W = 0 for a point without finite coordinates,
+            // which is nobody's neighbour, not its own either: it stays
+            const double kd = sw ? (double)r / (double)sw : 0.0;
             out[3 * i] = (float)((double)q[0] + (double)sx * kd);
             out[3 * i + 1] = (float)((double)q[1] + (double)sy * kd);
             out[3 * i + 2] = (float)((double)q[2] + (double)sz * kd);
