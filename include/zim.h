@@ -299,7 +299,7 @@ ZIM_API zim_status zim_filter_sor(zim_ctx* ctx, const float* xyz, const uint8_t*
 /* Statistics of the last SOR run on this context (zim_filter_sor or the SOR
  * stage of zim_reconstruct_pair): valid points, mean and standard deviation of
  * the per-point mean k-NN distance, the threshold mean + std_mul * stddev, and
- * how many points needed the second (outlier) search phase.  Synchronises. */
+ * how many points the window pass left to the tree search.  Synchronises. */
 typedef struct zim_sor_stats {
     double n_valid, mean, stddev, threshold;
     uint32_t n_far_search;
@@ -408,9 +408,10 @@ ZIM_API zim_status zim_reconstruct_pair_host_async(zim_ctx* ctx, const zim_decod
  * median, reprojection, 3x3 Gaussian and radius outlier filter, then the grid
  * filters (SOR -> MLS -> metric Gaussian) that the pair's filter config turns
  * on (zim_batch_pair.filters, or the submission's config).
- * Execution: one persistent kernel per pixel-domain stage drains a device work
- * queue of (pair, row band) items over all pairs (decode; rectify fused into
- * match; median + reprojection; each pixel filter); then the pairs' grid
+ * Execution: a decode launch per camera, then one persistent kernel per
+ * pixel-domain stage drains a device work queue of (pair, row band) items over
+ * all pairs (post-smooth; rectify fused into match; median + reprojection; each
+ * pixel filter); then the pairs' grid
  * filters run on up to six lanes (streams, each with its own scratch) side by
  * side, the largest pairs first, each to the least-loaded lane, so one pair's
  * latency-bound searches overlap another's kernels.  The whole sequence is captured once as a CUDA
@@ -437,7 +438,7 @@ typedef struct zim_batch_pair {
 } zim_batch_pair;
 
 typedef struct zim_batch_tuning {
-    int decode_rows;   /* 8-pixel tile rows per decode work item */
+    int decode_rows;   /* 8-pixel tile rows per post-smooth work item */
     int match_rows;    /* rectified rows per rectify+match work item */
     int filter_rows;   /* 8-pixel tile rows per median/filter work item */
     int ctas_per_sm;   /* persistent CTAs per SM (capped by occupancy) */

@@ -353,7 +353,7 @@ static zim_status run_pair(zim_ctx* ctx, const zim_decode_config* d, const zim_r
         if (s) return s;
         cx = ox; cm = om;
     }
-    // the grid filters carve their hash tables from the same region in turn
+    // the cloud filters carve their trees and tables from the same region in turn
     const size_t grid_mark = ctx->scratch_used;
     if (on[ST_SOR]) {
         uint8_t* om = next_m(ST_SOR);
