@@ -408,7 +408,7 @@ ZIM_API zim_status zim_reconstruct_pair_host_async(zim_ctx* ctx, const zim_decod
  * median, reprojection, 3x3 Gaussian and radius outlier filter, then the grid
  * filters (SOR -> MLS -> metric Gaussian) that the pair's filter config turns
  * on (zim_batch_pair.filters, or the submission's config).
- * Execution: a decode launch per camera, then one persistent kernel per
+ * Execution: a decode launch per pair, then one persistent kernel per
  * pixel-domain stage drains a device work queue of (pair, row band) items over
  * all pairs (post-smooth; rectify fused into match; median + reprojection; each
  * pixel filter); then the pairs' grid

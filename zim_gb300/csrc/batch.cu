@@ -7,7 +7,7 @@
 // JSLAB_PhaseEpipolarReconstructor_V2_GPU.cu:352-480).  Per pair the stages
 // compute exactly what zim_reconstruct_pair computes (the same device code,
 // zim_tiles.cuh); what changes is the schedule:
-//   stage 1  decode:          a launch per camera
+//   stage 1  decode:          a launch per pair
 //   stage 1b post-smooth of the decoded phase, when configured:
 //            item = (pair, camera, band of 8-row tile rows)
 //   stage 2  rectify + match: item = (pair, band of rectified rows); the right
@@ -407,11 +407,10 @@ zim_status capture(zim_batch* b) {
     ZIM_CUDA_TRY(ctx, cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
     cudaMemsetAsync(b->d_counters, 0, NQ * sizeof(unsigned), s);
     const Queues& q = b->q;
-    // stage 1: a launch per camera fills the GPU at every pair size
+    // stage 1: a launch per pair fills the GPU at every pair size
     const unsigned long long launched = ctx->launches;
     for (const PairDev& D : b->host_pairs)
-        for (int c = 0; c < 2; c++)
-            zim_decode_params_launch(ctx, D.frames[c], D.sample_type, D.dp, D.order[c], D.res[c], nullptr, nullptr, s);
+        zim_decode_params_launch(ctx, 2, D.frames, D.sample_type, D.dp, D.order, D.res, nullptr, nullptr, s);
     ctx->launches = launched;  // captured, not run: each replay counts them
     if (q.n[Q_SMOOTH])
         batch_smooth_kernel<<<std::min(b->grid[Q_SMOOTH], q.n[Q_SMOOTH]), BT, 0, s>>>(

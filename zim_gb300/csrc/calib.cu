@@ -265,10 +265,17 @@ __global__ void rectify_kernel(const int32_t* __restrict__ order, const float* _
 // Post-smooth once per source pixel (the reference smooths the decoded phase
 // map before setData, JSLAB_PhaseShiftDecoder_V2.cpp:274-295) ...
 constexpr int SMOOTH_WARPS = 4;
+struct SmoothCams {  // one or two cameras, one per blockIdx.y
+    const int32_t* order[2];
+    const float* res[2];
+    int2* taps[2];
+};
 template <bool HDR>
-__global__ void __launch_bounds__(32 * SMOOTH_WARPS) smooth_kernel(const int32_t* __restrict__ order,
-                                                                   const float* __restrict__ res, int rows, int cols,
-                                                                   int band, int nstrips, int2* __restrict__ taps) {
+__global__ void __launch_bounds__(32 * SMOOTH_WARPS) smooth_kernel(const __grid_constant__ SmoothCams cams, int rows,
+                                                                   int cols, int band, int nstrips) {
+    const int32_t* __restrict__ order = cams.order[blockIdx.y];
+    const float* __restrict__ res = cams.res[blockIdx.y];
+    int2* __restrict__ taps = cams.taps[blockIdx.y];
     const int id = blockIdx.x * SMOOTH_WARPS + (threadIdx.x >> 5), y0 = (id / nstrips) * band;
     if (y0 < rows) zt::smooth_strip<HDR>(order, res, rows, cols, id % nstrips, y0, min(y0 + band, rows), taps);
 }
@@ -484,7 +491,7 @@ zim_status zim_rectify_launch(zim_ctx* ctx, int cam, const int32_t* order, const
                               cudaStream_t st) {
     dim3 blk(32, 8), grd((ctx->rect_w + 31) / 32, (ctx->rect_h + 7) / 8);
     if (post_smooth == 1 || post_smooth == 2) {
-        zim_status s = zim_smooth_launch(ctx, order, residual, rows, cols, post_smooth, taps, st);
+        zim_status s = zim_smooth_launch(ctx, 1, &order, &residual, rows, cols, post_smooth, &taps, st);
         if (s) return s;
         rectify_smoothed_kernel<<<grd, blk, 0, st>>>(taps, order, rows, cols, ctx->d_map[cam][0], ctx->d_map[cam][1],
                                                      ctx->rect_h, ctx->rect_w, rbase, rres, rorder);
@@ -497,18 +504,24 @@ zim_status zim_rectify_launch(zim_ctx* ctx, int cam, const int32_t* order, const
     return ZIM_OK;
 }
 
-// The post-smooth alone (post_smooth 1 or 2; nothing to do otherwise).
-zim_status zim_smooth_launch(zim_ctx* ctx, const int32_t* order, const float* residual, int rows, int cols,
-                             int post_smooth, int2* taps, cudaStream_t st) {
+// The post-smooth of n cameras (post_smooth 1 or 2; nothing to do otherwise).
+zim_status zim_smooth_launch(zim_ctx* ctx, int n, const int32_t* const* order, const float* const* residual, int rows,
+                             int cols, int post_smooth, int2* const* taps, cudaStream_t st) {
     if (post_smooth != 1 && post_smooth != 2) return ZIM_OK;
     const int nstrips = (cols + zt::SMOOTH_STRIP - 1) / zt::SMOOTH_STRIP;
-    const int band = strip_band(ctx, nstrips, rows, 32);
+    const int band = strip_band(ctx, nstrips * n, rows, 32);
     const long long warps = (long long)nstrips * ((rows + band - 1) / band);
-    const unsigned blocks = (unsigned)((warps + SMOOTH_WARPS - 1) / SMOOTH_WARPS);
+    const dim3 blocks((unsigned)((warps + SMOOTH_WARPS - 1) / SMOOTH_WARPS), n);
+    SmoothCams cams{};
+    for (int c = 0; c < n; c++) {
+        cams.order[c] = order[c];
+        cams.res[c] = residual[c];
+        cams.taps[c] = taps[c];
+    }
     if (post_smooth == 2)
-        smooth_kernel<true><<<blocks, 32 * SMOOTH_WARPS, 0, st>>>(order, residual, rows, cols, band, nstrips, taps);
+        smooth_kernel<true><<<blocks, 32 * SMOOTH_WARPS, 0, st>>>(cams, rows, cols, band, nstrips);
     else
-        smooth_kernel<false><<<blocks, 32 * SMOOTH_WARPS, 0, st>>>(order, residual, rows, cols, band, nstrips, taps);
+        smooth_kernel<false><<<blocks, 32 * SMOOTH_WARPS, 0, st>>>(cams, rows, cols, band, nstrips);
     ctx->launches += 1;
     ZIM_LAUNCH_CHECK(ctx);
     return ZIM_OK;

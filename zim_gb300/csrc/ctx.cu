@@ -284,11 +284,14 @@ static zim_status run_pair(zim_ctx* ctx, const zim_decode_config* d, const zim_r
     zim_status s;
     const void* frames[2] = {lf, rf};
     const int post = d->enable_hdr ? (d->post_smooth ? 2 : 3) : (d->post_smooth ? 1 : 0);
-    for (int c = 0; c < 2; c++) {
-        if (c == 1 && right_ready) ZIM_CUDA_TRY(ctx, cudaStreamWaitEvent(st, right_ready, 0));
-        s = zim_decode_launch(ctx, d, frames[c], sample_type, rows, cols, B.order[c], B.res[c], nullptr, nullptr, st);
+    // both cameras per launch, or one after the other where the right one's frames are on their way
+    const int step = right_ready ? 1 : 2;
+    for (int c = 0; c < 2; c += step) {
+        if (c == 1) ZIM_CUDA_TRY(ctx, cudaStreamWaitEvent(st, right_ready, 0));
+        s = zim_decode_launch(ctx, d, step, frames + c, sample_type, rows, cols, B.order + c, B.res + c, nullptr, nullptr,
+                              st);
         if (s) return s;
-        s = zim_smooth_launch(ctx, B.order[c], B.res[c], rows, cols, post, B.taps[c], st);
+        s = zim_smooth_launch(ctx, step, B.order + c, B.res + c, rows, cols, post, B.taps + c, st);
         if (s) return s;
     }
     const int RH = ctx->rect_h, RW = ctx->rect_w;

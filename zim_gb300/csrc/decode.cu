@@ -12,6 +12,7 @@
 // in FP32, so an order differs from the FP64 restatement only when a decision
 // argument sits within ~1e-6 of its threshold.
 #include <cmath>
+#include <type_traits>
 
 #include "zim_tiles.cuh"
 
@@ -141,6 +142,15 @@ struct Outputs {
     float* mod;
     uint8_t* valid;
 };
+// The one or two cameras of a launch, one per blockIdx.y: the cameras of a small
+// pair together fill the GPU, and a large pair has one last wave less (a whole pair
+// with SOR, hierarchical: 99 -> 93 us at 640 x 480, 188 -> 181 at 1280 x 1024, 507 ->
+// 500 at 2448 x 2048).  A single camera has a kernel of its own: its frames' base is
+// then a constant of the launch (24 frames: 117 us; 127 without).
+struct Cameras {
+    const void* frames[2];
+    Outputs out[2];
+};
 
 // A pixel under way: wrapped phases, modulation of frequency 0, whether nothing
 // rejected it so far.
@@ -190,9 +200,8 @@ __device__ __forceinline__ void finish_pixel(const DecodeParams& p, int n_ps, co
 // us, 12 16-bit frames 88 / 73; 1626x1236 Gray code (rows no multiple of 16 bytes)
 // 56 / 35.
 template <typename T, int NPS, int NS>
-__global__ void __launch_bounds__(32 * DEC_WARPS) decode_strip_kernel(const T* __restrict__ frames,
-                                                                      const __grid_constant__ DecodeParams p, int band,
-                                                                      int nstrips, const __grid_constant__ Outputs out) {
+__device__ __forceinline__ void decode_strip(const T* __restrict__ frames, const DecodeParams& p, int band, int nstrips,
+                                             const Outputs& out) {
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     const int wid = blockIdx.x * DEC_WARPS + (threadIdx.x >> 5);
@@ -322,6 +331,18 @@ __global__ void __launch_bounds__(32 * DEC_WARPS) decode_strip_kernel(const T* _
         if (y > y0 && writes) finish_pixel<NPS>(p, n_ps, px, g1, g2, (size_t)(y - 1) * p.cols + x, out);
     }
 }
+template <typename T, int NPS, int NS>
+__global__ void __launch_bounds__(32 * DEC_WARPS) decode_strip_kernel(const T* __restrict__ frames,
+                                                                      const __grid_constant__ DecodeParams p, int band,
+                                                                      int nstrips, const __grid_constant__ Outputs out) {
+    decode_strip<T, NPS, NS>(frames, p, band, nstrips, out);
+}
+template <typename T, int NPS, int NS>
+__global__ void __launch_bounds__(32 * DEC_WARPS) decode_strips_kernel(const __grid_constant__ Cameras cams,
+                                                                       const __grid_constant__ DecodeParams p, int band,
+                                                                       int nstrips) {
+    decode_strip<T, NPS, NS>(static_cast<const T*>(cams.frames[blockIdx.y]), p, band, nstrips, cams.out[blockIdx.y]);
+}
 
 // HDR fit of one frequency at a pixel pair (JSLAB_HDRPhaseFit.h:10-61 and
 // JSLAB_PhaseShiftDecoder_V2.cpp:73-90): raw samples with 0 <= I < saturation
@@ -404,9 +425,11 @@ __device__ __forceinline__ void hdr_fit(const T* q, size_t npx, bool pair, int d
 // sample): paired over two pixels and without branches 35 us for 24 frames of
 // 1280x1024, 64 us one pixel at a time.
 template <typename T, int NPS, int NS>
-__global__ void __launch_bounds__(128) decode_hdr_kernel(const T* __restrict__ frames,
-                                                         const __grid_constant__ DecodeParams p, int aligned,
-                                                         const __grid_constant__ Outputs out) {
+__global__ void __launch_bounds__(128) decode_hdr_kernel(const __grid_constant__ Cameras cams,
+                                                         const __grid_constant__ DecodeParams p, int aligned_cams) {
+    const T* __restrict__ frames = static_cast<const T*>(cams.frames[blockIdx.y]);
+    const Outputs& out = cams.out[blockIdx.y];
+    const int aligned = aligned_cams >> blockIdx.y & 1;
     const int half = (p.cols + 1) / 2;
     const size_t t = (size_t)blockIdx.x * 128 + threadIdx.x;
     const int y = (int)(t / (unsigned)half);
@@ -435,28 +458,46 @@ __global__ void __launch_bounds__(128) decode_hdr_kernel(const T* __restrict__ f
 }
 
 template <typename T>
-void launch_decode(zim_ctx* ctx, const T* frames, const DecodeParams& p, const Outputs& out, cudaStream_t st) {
-    const int aligned = p.cols % 2 == 0 && ((uintptr_t)frames & (2 * sizeof(T) - 1)) == 0;
+void launch_decode(zim_ctx* ctx, const Cameras& cams, int n, const DecodeParams& p, cudaStream_t st) {
+    int aligned = 0;  // bit per camera
+    for (int c = 0; c < n; c++)
+        aligned |= (p.cols % 2 == 0 && ((uintptr_t)cams.frames[c] & (2 * sizeof(T) - 1)) == 0) << c;
     int ns = p.shift[0];
     for (int i = 1; i < p.n_ps; i++) ns = p.shift[i] == ns ? ns : 0;
     if (p.hdr) {
         const unsigned blocks = (unsigned)(((size_t)p.rows * ((p.cols + 1) / 2) + 127) / 128);
         auto k = p.n_ps == 3 && ns == 8 ? decode_hdr_kernel<T, 3, 8>
                  : p.n_ps == 3 && ns == 4 ? decode_hdr_kernel<T, 3, 4> : decode_hdr_kernel<T, MAX_PS, 0>;
-        k<<<blocks, 128, 0, st>>>(frames, p, aligned, out);
+        k<<<dim3(blocks, n), 128, 0, st>>>(cams, p, aligned);
+        ctx->launches += 1;
         return;
     }
-    // (1626x1236 Gray: 35 us with 24 warps per SM, 38 with 40 and 42 with 64; larger
-    // images do not care)
     const int nstrips = (p.cols + STRIP - 1) / STRIP;
-    const int band = strip_band(ctx, nstrips, p.rows, DEC_MIN_WARPS);
+    // (1626x1236 Gray: 33 us with 24 warps per SM, 38 with 40 and 42 with 64; larger
+    // images do not care)
+    const int band = strip_band(ctx, nstrips * n, p.rows, DEC_MIN_WARPS);
     const long long warps = (long long)nstrips * ((p.rows + band - 1) / band);
-    const unsigned blocks = (unsigned)((warps + DEC_WARPS - 1) / DEC_WARPS);
-    auto k = p.n_ps == 3 && ns == 4 ? decode_strip_kernel<T, 3, 4>
-             : p.n_ps == 3 && ns == 8 ? decode_strip_kernel<T, 3, 8>
-             : p.n_ps == 1 && ns == 4 ? decode_strip_kernel<T, 1, 4>
-             : p.n_ps == 1 ? decode_strip_kernel<T, 1, 0> : decode_strip_kernel<T, MAX_PS, 0>;
-    k<<<blocks, 32 * DEC_WARPS, 0, st>>>(frames, p, band, nstrips, out);
+    const dim3 blocks((unsigned)((warps + DEC_WARPS - 1) / DEC_WARPS), n);
+    auto run = [&](auto nps, auto nsteps) {
+        constexpr int NPS = decltype(nps)::value, NS = decltype(nsteps)::value;
+        if (n == 2)
+            decode_strips_kernel<T, NPS, NS><<<blocks, 32 * DEC_WARPS, 0, st>>>(cams, p, band, nstrips);
+        else
+            decode_strip_kernel<T, NPS, NS><<<blocks, 32 * DEC_WARPS, 0, st>>>(static_cast<const T*>(cams.frames[0]), p,
+                                                                               band, nstrips, cams.out[0]);
+    };
+    constexpr std::integral_constant<int, 0> c0;
+    constexpr std::integral_constant<int, 1> c1;
+    constexpr std::integral_constant<int, 3> c3;
+    constexpr std::integral_constant<int, 4> c4;
+    constexpr std::integral_constant<int, 8> c8;
+    constexpr std::integral_constant<int, MAX_PS> cm;
+    if (p.n_ps == 3 && ns == 4) run(c3, c4);
+    else if (p.n_ps == 3 && ns == 8) run(c3, c8);
+    else if (p.n_ps == 1 && ns == 4) run(c1, c4);
+    else if (p.n_ps == 1) run(c1, c0);
+    else run(cm, c0);
+    ctx->launches += 1;
 }
 
 // Absolute phase as f64 (startCalculate's CV_64F map; 0 where invalid), with
@@ -496,19 +537,24 @@ __global__ void phase_f64_kernel(const int32_t* __restrict__ order, const float*
 
 }  // namespace
 
-void zim_decode_params_launch(zim_ctx* ctx, const void* frames, int sample_type, const zt::DecodeParams& p,
-                              int32_t* order, float* residual, float* mod, uint8_t* valid, cudaStream_t st) {
-    const Outputs out{order, residual, mod, valid};
-    if (sample_type == ZIM_SAMPLE_U8) launch_decode(ctx, (const uint8_t*)frames, p, out, st);
-    else launch_decode(ctx, (const uint16_t*)frames, p, out, st);
-    ctx->launches += 1;
+void zim_decode_params_launch(zim_ctx* ctx, int n, const void* const* frames, int sample_type,
+                              const zt::DecodeParams& p, int32_t* const* order, float* const* residual, float* mod,
+                              uint8_t* valid, cudaStream_t st) {
+    Cameras cams{};
+    for (int c = 0; c < n; c++) {
+        cams.frames[c] = frames[c];
+        cams.out[c] = Outputs{order[c], residual[c], mod, valid};
+    }
+    if (sample_type == ZIM_SAMPLE_U8) launch_decode<uint8_t>(ctx, cams, n, p, st);
+    else launch_decode<uint16_t>(ctx, cams, n, p, st);
 }
 
-zim_status zim_decode_launch(zim_ctx* ctx, const zim_decode_config* cfg, const void* frames, int sample_type, int rows,
-                             int cols, int32_t* order, float* residual, float* mod, uint8_t* valid, cudaStream_t st) {
+zim_status zim_decode_launch(zim_ctx* ctx, const zim_decode_config* cfg, int n, const void* const* frames,
+                             int sample_type, int rows, int cols, int32_t* const* order, float* const* residual,
+                             float* mod, uint8_t* valid, cudaStream_t st) {
     DecodeParams p;
     zt::decode_params(cfg, rows, cols, p);
-    zim_decode_params_launch(ctx, frames, sample_type, p, order, residual, mod, valid, st);
+    zim_decode_params_launch(ctx, n, frames, sample_type, p, order, residual, mod, valid, st);
     ZIM_LAUNCH_CHECK(ctx);
     return ZIM_OK;
 }
@@ -525,7 +571,8 @@ extern "C" ZIM_API zim_status zim_decode(zim_ctx* ctx, const zim_decode_config* 
     if (sample_type != ZIM_SAMPLE_U8 && sample_type != ZIM_SAMPLE_U16)
         return zim_fail(ctx, ZIM_ERR_INVALID_ARG, "bad sample type");
     ZIM_CUDA_TRY(ctx, cudaSetDevice(ctx->device));
-    return zim_decode_launch(ctx, cfg, frames, sample_type, rows, cols, order, residual, mod, valid, zim_stream(stream));
+    return zim_decode_launch(ctx, cfg, 1, &frames, sample_type, rows, cols, &order, &residual, mod, valid,
+                             zim_stream(stream));
 }
 
 extern "C" ZIM_API zim_status zim_decode_phase_f64(zim_ctx* ctx, const int32_t* order, const float* residual, int rows,

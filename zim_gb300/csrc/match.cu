@@ -285,9 +285,9 @@ extern "C" ZIM_API zim_status zim_rectify_match(zim_ctx* ctx, const int32_t* l_o
         for (int c = 0; c < 2; c++) {
             taps[c] = (int2*)zim_scratch_take(ctx, src * 8);
             if (!taps[c]) return zim_fail(ctx, ZIM_ERR_OUT_OF_MEMORY, "rectify scratch");
-            s = zim_smooth_launch(ctx, ord[c], res[c], rows, cols, post_smooth, taps[c], st);
-            if (s) return s;
         }
+        s = zim_smooth_launch(ctx, 2, ord, res, rows, cols, post_smooth, taps, st);
+        if (s) return s;
     }
     return zim_rectify_match_launch(ctx, ord, res, taps, rows, cols, post_smooth, pha_f, grad_threshold, disp, st);
 }

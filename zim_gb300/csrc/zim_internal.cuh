@@ -97,11 +97,13 @@ struct ReprojParams;
 // 5x5 median + reprojection of a disparity map with the parameters in hand.
 void zim_median_strips(zim_ctx* ctx, const zt::ReprojParams& p, const float* disp, int rows, int cols, float* disp_out,
                        float* xyz, uint8_t* mask, cudaStream_t st);
-// One camera's decode with its parameters in hand (the batch's launches).
-void zim_decode_params_launch(zim_ctx* ctx, const void* frames, int sample_type, const zt::DecodeParams& p,
-                              int32_t* order, float* residual, float* mod, uint8_t* valid, cudaStream_t st);
-zim_status zim_decode_launch(zim_ctx* ctx, const zim_decode_config* cfg, const void* frames,
-                             int sample_type, int rows, int cols, int32_t* order, float* residual,
+// The decode of n cameras (1 or 2; mod and valid with one only) with its parameters
+// in hand (the batch's launches).
+void zim_decode_params_launch(zim_ctx* ctx, int n, const void* const* frames, int sample_type,
+                              const zt::DecodeParams& p, int32_t* const* order, float* const* residual, float* mod,
+                              uint8_t* valid, cudaStream_t st);
+zim_status zim_decode_launch(zim_ctx* ctx, const zim_decode_config* cfg, int n, const void* const* frames,
+                             int sample_type, int rows, int cols, int32_t* const* order, float* const* residual,
                              float* mod, uint8_t* valid, cudaStream_t st);
 // post_smooth: taps is rows*cols scratch for the smoothed taps.
 zim_status zim_rectify_launch(zim_ctx* ctx, int cam, const int32_t* order, const float* residual,
@@ -137,8 +139,8 @@ zim_status zim_px_gaussian_launch(zim_ctx* ctx, const float* xyz, const uint8_t*
 zim_status zim_ror_launch(zim_ctx* ctx, const float* xyz, const uint8_t* mask, int rows, int cols,
                           float radius, int min_neighbors, int window_size, float* out,
                           uint8_t* mask_out, cudaStream_t st);
-zim_status zim_smooth_launch(zim_ctx* ctx, const int32_t* order, const float* residual, int rows, int cols,
-                             int post_smooth, int2* taps, cudaStream_t st);
+zim_status zim_smooth_launch(zim_ctx* ctx, int n, const int32_t* const* order, const float* const* residual, int rows,
+                             int cols, int post_smooth, int2* const* taps, cudaStream_t st);
 zim_status zim_rectify_match_launch(zim_ctx* ctx, const int32_t* const order[2], const float* const res[2],
                                     int2* const taps[2], int srows, int scols, int post_smooth, int pha_f,
                                     double grad_threshold, float* disp, cudaStream_t st);
