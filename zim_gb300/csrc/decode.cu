@@ -12,7 +12,11 @@
 // in FP32, so an order differs from the FP64 restatement only when a decision
 // argument sits within ~1e-6 of its threshold.
 #include <cmath>
+#include <mutex>
 #include <type_traits>
+
+#include <cuda.h>
+#include <cudaTypedefs.h>
 
 #include "zim_tiles.cuh"
 
@@ -188,17 +192,13 @@ __device__ __forceinline__ void finish_pixel(const DecodeParams& p, int n_ps, co
 // rows they blur into, so nothing is staged in shared memory and no warp waits
 // for another.  The next row's samples are in flight while a row is blurred and
 // unwrapped.  S and C are the lanes of the paired FP32 FMA (__ffma2_rn: each
-// rounded as fmaf).  NS: frames per frequency at compile time (0: p.shift); NPS:
-// frequencies (4: p.n_ps of them).
+// rounded as fmaf).  NS: frames per frequency; NPS: frequencies (no Gray code).
 //
-// Bound by instruction issue.  A tile per CTA, staged by a bulk tensor copy and
-// blurred from shared memory (nine two-word shared loads per pixel and frequency,
-// a 1.33x halo), issued 588 warp instructions per 32 pixels for three frequencies
-// of four frames; this kernel issues 434.  Two columns per lane (all sums paired,
-// half the shuffles) issued 409 but needed 120 registers and took 88 us where
-// this takes 73.  Before / now, 2448x2048: 24 8-bit frames (heterodyne) 180 / 118
-// us, 12 16-bit frames 88 / 73; 1626x1236 Gray code (rows no multiple of 16 bytes)
-// 56 / 35.
+// Bound by instruction issue.  A tile (decode_tile_kernel: nine two-word shared loads
+// per pixel and frequency, a 1.33x halo) issues 588 warp instructions per 32 pixels
+// for three frequencies of four frames; this kernel issues 434.  Two columns per lane
+// (all sums paired, half the shuffles) issued 409 but needed 120 registers and took 88
+// us where this takes 73 (2448x2048, 12 16-bit frames; tiles 83).
 template <typename T, int NPS, int NS>
 __device__ __forceinline__ void decode_strip(const T* __restrict__ frames, const DecodeParams& p, int band, int nstrips,
                                              const Outputs& out) {
@@ -211,7 +211,6 @@ __device__ __forceinline__ void decode_strip(const T* __restrict__ frames, const
     const int x = (wid % nstrips) * STRIP - 1 + lane;
     const bool writes = lane > 0 && lane < 31 && x < p.cols;
     const size_t npx = (size_t)p.rows * p.cols;
-    const int n_ps = NPS < MAX_PS ? NPS : p.n_ps;
     // byte offset of a row's sample within any frame's plane (at most 2^31 samples):
     // the plane's base is the same for the whole grid, so a load adds 32 bits to it
     const int xc = min(max(x, 0), p.cols - 1);
@@ -221,19 +220,12 @@ __device__ __forceinline__ void decode_strip(const T* __restrict__ frames, const
     auto sample = [&](int f, unsigned off) {
         return (unsigned)__ldg(reinterpret_cast<const T*>(reinterpret_cast<const char*>(frames + (size_t)f * npx) + off));
     };
-    const bool gray = (NPS == 1 || NPS == MAX_PS) && p.gray_bits > 0;
-
-    constexpr int NW = NS ? NPS * NS : 4, GW = NPS == 1 ? 8 : 1;
-    const int nbits = p.gray_bits + p.complementary;
-    unsigned raw[NW], gw[GW];  // samples in flight (up to GW of the Gray frames)
+    constexpr int NW = NPS * NS;
+    unsigned raw[NW];  // samples in flight
     auto fetch = [&](int y) {
         const unsigned o = row_off(y);
 #pragma unroll
-        for (int f = 0; f < (NS ? NW : 0); f++) raw[f] = sample(f, o);
-        if (gray && nbits <= GW)
-#pragma unroll
-            for (int b = 0; b < GW; b++)
-                if (b < nbits) gw[b] = sample(p.gray_base + b, o);
+        for (int f = 0; f < NW; f++) raw[f] = sample(f, o);
     };
     // blurred sums under way: A for the row above the current raw row, B for it
     float2 A[NPS], B[NPS];  // (S, C)
@@ -243,77 +235,27 @@ __device__ __forceinline__ void decode_strip(const T* __restrict__ frames, const
         A[i] = B[i] = make_float2(0.f, 0.f);
         AM[i] = BM[i] = 0.f;
     }
-    int g1 = 0, g2 = 0, h1 = 0, h2 = 0;  // codewords of the row above, of this row
-    if (NS > 0 || gray) fetch(y0 - 1);
+    fetch(y0 - 1);
     for (int y = y0 - 1; y <= y1; y++) {
         float2 sc[NPS];
         float m[NPS];
 #pragma unroll
         for (int i = 0; i < NPS; i++) {
-            if (i >= n_ps) break;
             sc[i] = make_float2(0.f, 0.f);
-            m[i] = 0.f;
             auto add = [&](int f, unsigned w) {
                 const float v = (float)w;
                 sc[i] = make_float2(fmaf(-p.sinv[f], v, sc[i].x), fmaf(p.cosv[f], v, sc[i].y));
                 m[i] += v;
             };
-            if constexpr (NS > 0) {
-                sc[i].y = m[i] = (float)raw[i * NS];  // step 0: sin 0 and cos 1 exactly
+            sc[i].y = m[i] = (float)raw[i * NS];  // step 0: sin 0 and cos 1 exactly
 #pragma unroll
-                for (int k = 1; k < NS; k++) add(i * NS + k, raw[i * NS + k]);
-            } else {
-                const int N = p.shift[i], f0 = p.fbase[i];
-                const unsigned o = row_off(y);
-                int k = 0;
-                for (; k + 4 <= N; k += 4) {  // four loads in flight
-#pragma unroll
-                    for (int u = 0; u < 4; u++) raw[u] = sample(f0 + k + u, o);
-#pragma unroll
-                    for (int u = 0; u < 4; u++) add(f0 + k + u, raw[u]);
-                }
-                for (; k < N; k++) add(f0 + k, sample(f0 + k, o));
-            }
+            for (int k = 1; k < NS; k++) add(i * NS + k, raw[i * NS + k]);
         }
-        if (gray) {
-            // codeword of this raw row: bit set where N g > sum of the phase frames (exact in FP32)
-            g1 = h1;
-            g2 = h2;
-            if (y >= y0 && y < y1) {
-                const float N = (float)p.shift[0];
-                auto bit = [&](unsigned w) { return N * (float)w > m[0] ? 1 : 0; };
-                int bin = 0, v = 0;
-                unsigned last;
-                if (nbits <= GW) {
-#pragma unroll
-                    for (int b = 0; b < GW; b++)
-                        if (b < p.gray_bits) {
-                            bin ^= bit(gw[b]);
-                            v = v << 1 | bin;
-                        }
-                    last = gw[0];
-#pragma unroll
-                    for (int b = 1; b < GW; b++)
-                        if (b == p.gray_bits) last = gw[b];
-                } else {
-                    const unsigned o = row_off(y);
-                    last = p.complementary ? sample(p.gray_base + p.gray_bits, o) : 0u;
-#pragma unroll 4
-                    for (int b = 0; b < p.gray_bits; b++) {
-                        bin ^= bit(sample(p.gray_base + b, o));
-                        v = v << 1 | bin;
-                    }
-                }
-                h1 = v;
-                h2 = ((v << 1 | (bin ^ bit(last))) + 1) >> 1;
-            }
-        }
-        if ((NS > 0 || gray) && y < y1) fetch(y + 1);
+        if (y < y1) fetch(y + 1);
         Pixel px;
         px.ok = true;
 #pragma unroll
         for (int i = 0; i < NPS; i++) {
-            if (i >= n_ps) break;
             // taps in row-major order from zero, as nine sequential FMAs per output
             auto w2 = [&](int t) { return make_float2(p.w2d[t], p.w2d[t]); };
             const float2 c = sc[i];
@@ -328,7 +270,7 @@ __device__ __forceinline__ void decode_strip(const T* __restrict__ frames, const
             BM[i] = fmaf(p.w2d[2], mr, fmaf(p.w2d[1], m[i], fmaf(p.w2d[0], ml, 0.f)));
             if (y > y0) take_frequency(p, i, F.x, F.y, FM, out.mod != nullptr, px);
         }
-        if (y > y0 && writes) finish_pixel<NPS>(p, n_ps, px, g1, g2, (size_t)(y - 1) * p.cols + x, out);
+        if (y > y0 && writes) finish_pixel<NPS>(p, NPS, px, 0, 0, (size_t)(y - 1) * p.cols + x, out);
     }
 }
 template <typename T, int NPS, int NS>
@@ -342,6 +284,207 @@ __global__ void __launch_bounds__(32 * DEC_WARPS) decode_strips_kernel(const __g
                                                                        const __grid_constant__ DecodeParams p, int band,
                                                                        int nstrips) {
     decode_strip<T, NPS, NS>(static_cast<const T*>(cams.frames[blockIdx.y]), p, band, nstrips, cams.out[blockIdx.y]);
+}
+
+// ------------------------------------------------------------------ tiles --
+// A block decodes 32 x 8 pixels: the raw sums of the tile and its 1-pixel halo go
+// to shared memory, each frequency's three channels are blurred from there.  NPS /
+// NS: frequencies and frames per frequency at compile time (0: from p).  TMA: the
+// phase-shift samples come in one bulk tensor copy (cp.async.bulk.tensor) completing
+// on an mbarrier, from a 3-D map over (x, y, frame) of the frame stack; box BW x HY x
+// nfr, its x XPAD pixels left of the tile (a copy's x must be 16-byte aligned), its y
+// one row above.  Samples outside the image read as 0 and are never used: the sums
+// clamp to the image.  All forms add in the strips' order, so the bits are the same.
+//
+// The loads of a tile are all in flight at once whatever the step count, where a
+// strip keeps one row ahead and only a step count known at compile time can be held
+// in registers, and a small image has its latency once instead of once a row.  Times
+// of tiles / strips are at the rule (use_strips).
+constexpr int TX = 32, TY = 8, HX = TX + 2, HY = TY + 2;
+template <typename T>
+__host__ __device__ constexpr int tma_xpad() { return 16 / (int)sizeof(T); }
+template <typename T>
+__host__ __device__ constexpr int tma_bw() { return TX + 2 * tma_xpad<T>(); }
+constexpr int TMA_MAX_FRAMES = 24;           // box depth (phase-shift frames) the copy takes
+constexpr unsigned TMA_POLLS = 1u << 22;     // mbarrier polls before giving up (well over a second)
+constexpr uint32_t ERR_DECODE_COPY = 0x20u;  // device error word: a tile's copy did not land
+
+struct TileMaps {
+    CUtensorMap m[2];  // per camera
+};
+
+__device__ __forceinline__ unsigned smem_addr(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
+
+// Phase 0 of the barrier completed; false after `polls` polls.
+__device__ __forceinline__ bool mbar_wait0(unsigned bar, unsigned polls) {
+    for (unsigned it = 0; it < polls; it++) {
+        unsigned done;
+        asm volatile(
+            "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], 0;\n selp.u32 %0, 1, 0, p;\n}\n"
+            : "=r"(done)
+            : "r"(bar)
+            : "memory");
+        if (done) return true;
+    }
+    return false;
+}
+
+template <typename T, int NPS, int NS, bool TMA>
+__global__ void __launch_bounds__(TX* TY) decode_tile_kernel(const __grid_constant__ TileMaps maps,
+                                                             const __grid_constant__ Cameras cams,
+                                                             const __grid_constant__ DecodeParams p, int nfr,
+                                                             unsigned tiles_x, uint32_t* __restrict__ err) {
+    constexpr int MPS = NPS ? NPS : MAX_PS;
+    __shared__ float2 s_sc[MPS][HY][HX + 1];
+    __shared__ float s_m[MPS][HY][HX + 1];
+    const T* __restrict__ frames = static_cast<const T*>(cams.frames[blockIdx.y]);
+    const int tid = threadIdx.x, n_ps = NPS ? NPS : p.n_ps;
+    const int x0 = (int)(blockIdx.x % tiles_x) * TX, y0 = (int)(blockIdx.x / tiles_x) * TY;
+    const size_t npx = (size_t)p.rows * p.cols;
+    constexpr int XPAD = tma_xpad<T>(), BW = tma_bw<T>();
+    extern __shared__ __align__(128) unsigned char box_raw[];  // [nfr][HY][BW] samples
+    if constexpr (TMA) {
+        __shared__ __align__(8) unsigned long long bar;
+        const unsigned b = smem_addr(&bar);
+        if (tid == 0) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(b) : "memory");
+            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        }
+        __syncthreads();
+        if (tid == 0) {
+            const unsigned bytes = (unsigned)(BW * HY * nfr * (int)sizeof(T));
+            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(b), "r"(bytes) : "memory");
+            asm volatile(
+                "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], "
+                "[%5];" ::"r"(smem_addr(box_raw)),
+                "l"(reinterpret_cast<unsigned long long>(&maps.m[blockIdx.y])), "r"(x0 - XPAD), "r"(y0 - 1), "r"(0), "r"(b)
+                : "memory");
+        }
+        // bounded: a copy that never lands flags the error word; the tile waits
+        // once more (bounded) for it before leaving
+        if (!__syncthreads_and(mbar_wait0(b, TMA_POLLS))) {
+            if (tid == 0) atomicOr(err, ERR_DECODE_COPY);
+            mbar_wait0(b, TMA_POLLS);
+            return;
+        }
+    }
+    for (int h = tid; h < HX * HY; h += TX * TY) {
+        const int hy = h / HX, hx = h - hy * HX;
+        const int gy = min(max(y0 - 1 + hy, 0), p.rows - 1), gx = min(max(x0 - 1 + hx, 0), p.cols - 1);
+        const T* box = reinterpret_cast<const T*>(box_raw) + (gy - (y0 - 1)) * BW + (gx - (x0 - XPAD));
+        const T* pix = frames + (size_t)gy * p.cols + gx;
+#pragma unroll
+        for (int i = 0; i < MPS; i++) {
+            if (i >= n_ps) break;
+            const int f0 = NS ? i * NS : p.fbase[i];  // frequencies' frames are consecutive
+            const int N = NS ? NS : p.shift[i];
+            float2 sc = make_float2(0.f, 0.f);
+            float m = 0.f;
+            auto add = [&](int f, T v) {  // the S and C sums of one sample in one paired FMA
+                sc = __ffma2_rn(make_float2(-p.sinv[f], p.cosv[f]), both((float)v), sc);
+                m += (float)v;
+            };
+            if (TMA) {
+#pragma unroll
+                for (int k = 0; k < (NS ? NS : 32); k++) {  // 3..32 steps
+                    if (k >= N) break;
+                    add(f0 + k, box[(f0 + k) * (BW * HY)]);
+                }
+            } else if constexpr (NS > 0) {
+                T v[NS];
+#pragma unroll
+                for (int k = 0; k < NS; k++) v[k] = __ldg(pix + (size_t)(f0 + k) * npx);
+#pragma unroll
+                for (int k = 0; k < NS; k++) add(f0 + k, v[k]);
+            } else {
+                int k = 0;
+                for (; k + 4 <= N; k += 4) {  // four loads in flight
+                    T v[4];
+#pragma unroll
+                    for (int u = 0; u < 4; u++) v[u] = __ldg(pix + (size_t)(f0 + k + u) * npx);
+#pragma unroll
+                    for (int u = 0; u < 4; u++) add(f0 + k + u, v[u]);
+                }
+                for (; k < N; k++) add(f0 + k, __ldg(pix + (size_t)(f0 + k) * npx));
+            }
+            s_sc[i][hy][hx] = sc;
+            s_m[i][hy][hx] = m;
+        }
+    }
+    __syncthreads();
+    const int tx = tid % TX, ty = tid / TX, x = x0 + tx, y = y0 + ty;
+    if (x >= p.cols || y >= p.rows) return;
+    const Outputs& out = cams.out[blockIdx.y];
+    Pixel px;
+    px.ok = true;
+    px.mod = 0.f;
+#pragma unroll
+    for (int i = 0; i < MPS; i++) {
+        if (i >= n_ps) break;
+        float2 sc = make_float2(0.f, 0.f);
+        float m = 0.f;
+#pragma unroll
+        for (int a = 0; a < 3; a++)
+#pragma unroll
+            for (int b = 0; b < 3; b++) {
+                const float w = p.w2d[a * 3 + b];
+                sc = __ffma2_rn(both(w), s_sc[i][ty + a][tx + b], sc);
+                m = fmaf(w, s_m[i][ty + a][tx + b], m);
+            }
+        take_frequency(p, i, sc.x, sc.y, m, out.mod != nullptr, px);
+    }
+    const size_t o = (size_t)y * p.cols + x;
+    int g1 = 0, g2 = 0;
+    if ((NPS == 1 || !NPS) && p.gray_bits > 0 && px.ok) {
+        // codeword: bit set where N g > sum of the phase frames (exact in FP32)
+        const float N = (float)p.shift[0], sum = s_m[0][ty + 1][tx + 1];
+        auto bit = [&](int f) { return N * (float)__ldg(frames + (size_t)(p.gray_base + f) * npx + o) > sum ? 1 : 0; };
+        int bin = 0;
+        for (int f = 0; f < p.gray_bits; f++) {
+            bin ^= bit(f);
+            g1 = g1 << 1 | bin;
+        }
+        if (p.complementary) g2 = ((g1 << 1 | (bin ^ bit(p.gray_bits))) + 1) >> 1;
+    }
+    finish_pixel<MPS>(p, n_ps, px, g1, g2, o, out);
+}
+
+// cuTensorMapEncodeTiled from the driver, looked up once (no link to libcuda)
+PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
+    static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
+    static std::once_flag once;
+    std::call_once(once, [] {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &f, 12000, cudaEnableDefault, &q) ==
+                cudaSuccess &&
+            q == cudaDriverEntryPointSuccess)
+            fn = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(f);
+    });
+    return fn;
+}
+
+// The cameras' tensor maps, or false where the copy does not apply (row pitch or base
+// not 16-byte aligned, too many frames, an image smaller than the box).
+template <typename T>
+bool tile_maps(const Cameras& cams, int n, const DecodeParams& p, int nfr, TileMaps& maps) {
+    const size_t pitch = (size_t)p.cols * sizeof(T);
+    if (nfr > TMA_MAX_FRAMES || pitch % 16 != 0 || p.cols < tma_bw<T>() || p.rows < HY) return false;
+    for (int c = 0; c < n; c++)
+        if (((uintptr_t)cams.frames[c] & 15) != 0) return false;
+    PFN_cuTensorMapEncodeTiled_v12000 enc = tensor_map_encoder();
+    if (!enc) return false;
+    const cuuint64_t dims[3] = {(cuuint64_t)p.cols, (cuuint64_t)p.rows, (cuuint64_t)nfr};
+    const cuuint64_t strides[2] = {(cuuint64_t)pitch, (cuuint64_t)pitch * p.rows};
+    const cuuint32_t box[3] = {(cuuint32_t)tma_bw<T>(), (cuuint32_t)HY, (cuuint32_t)nfr};
+    const cuuint32_t one[3] = {1, 1, 1};
+    for (int c = 0; c < n; c++)
+        if (enc(&maps.m[c], sizeof(T) == 2 ? CU_TENSOR_MAP_DATA_TYPE_UINT16 : CU_TENSOR_MAP_DATA_TYPE_UINT8, 3,
+                const_cast<void*>(cams.frames[c]), dims, strides, box, one, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+            return false;
+    return true;
 }
 
 // HDR fit of one frequency at a pixel pair (JSLAB_HDRPhaseFit.h:10-61 and
@@ -457,6 +600,25 @@ __global__ void __launch_bounds__(128) decode_hdr_kernel(const __grid_constant__
     if (d) finish_pixel<NPS>(p, n_ps, p1, 0, 0, o + 1, out);
 }
 
+// Strips or tiles, where both have the step count (tma: the tiles come by bulk copy;
+// n cameras).  Strips issue least, but a row at a time: they win once the launch is
+// many waves deep.  us, tiles / strips: three frequencies of four steps, 8-bit,
+// hierarchical, 1280x1024 23 / 24, 1626x1236 36 / 34, 2448x2048 83 / 74; heterodyne 26 /
+// 28, 40 / 41, 92 / 91; both cameras of 1280x1024 even, of 2448x2048 20 less in strips.
+// Eight steps, bulk copy, 8-bit 2448x2048: 108 / 115 (4096x3000: 258 / 261), 16-bit 112 /
+// 111 (267 / 252); without it (2501x2092) 139 / 118 and 168 / 114, 16-bit from 487x365
+// (8.2 / 8.2) on.  Other step counts hold too few samples ahead in a strip (five steps,
+// 8-bit, 2448x2048: 127 / 304), Gray codes read their frames late (four steps, five
+// bits: 2448x2048 76 / 91, 1626x1236 28 / 29), and small images wait a strip's rows
+// out (three by eight steps, 64x64: 3.5 / 6).
+template <typename T>
+bool use_strips(const DecodeParams& p, int n, int ns, bool tma) {
+    if (p.n_ps != 3 || (ns != 4 && ns != 8)) return false;
+    const double px = (double)n * p.rows * p.cols;
+    if (ns == 8 && tma && sizeof(T) == 1) return false;
+    return px >= (ns == 8 && !tma && sizeof(T) == 2 ? 0.18e6 : 1.5e6);
+}
+
 template <typename T>
 void launch_decode(zim_ctx* ctx, const Cameras& cams, int n, const DecodeParams& p, cudaStream_t st) {
     int aligned = 0;  // bit per camera
@@ -472,31 +634,46 @@ void launch_decode(zim_ctx* ctx, const Cameras& cams, int n, const DecodeParams&
         ctx->launches += 1;
         return;
     }
-    const int nstrips = (p.cols + STRIP - 1) / STRIP;
-    // (1626x1236 Gray: 33 us with 24 warps per SM, 38 with 40 and 42 with 64; larger
-    // images do not care)
-    const int band = strip_band(ctx, nstrips * n, p.rows, DEC_MIN_WARPS);
-    const long long warps = (long long)nstrips * ((p.rows + band - 1) / band);
-    const dim3 blocks((unsigned)((warps + DEC_WARPS - 1) / DEC_WARPS), n);
-    auto run = [&](auto nps, auto nsteps) {
-        constexpr int NPS = decltype(nps)::value, NS = decltype(nsteps)::value;
-        if (n == 2)
-            decode_strips_kernel<T, NPS, NS><<<blocks, 32 * DEC_WARPS, 0, st>>>(cams, p, band, nstrips);
-        else
-            decode_strip_kernel<T, NPS, NS><<<blocks, 32 * DEC_WARPS, 0, st>>>(static_cast<const T*>(cams.frames[0]), p,
-                                                                               band, nstrips, cams.out[0]);
+    int nfr = 0;
+    for (int i = 0; i < p.n_ps; i++) nfr += p.shift[i];
+    TileMaps maps{};
+    const bool tma = tile_maps<T>(cams, n, p, nfr, maps);
+    auto by_steps = [&](auto run) {  // the step counts with code of their own
+        constexpr std::integral_constant<int, 0> c0;
+        constexpr std::integral_constant<int, 1> c1;
+        constexpr std::integral_constant<int, 3> c3;
+        constexpr std::integral_constant<int, 4> c4;
+        constexpr std::integral_constant<int, 8> c8;
+        if (p.n_ps == 3 && ns == 4) run(c3, c4);
+        else if (p.n_ps == 3 && ns == 8) run(c3, c8);
+        else if (p.n_ps == 1 && ns == 4) run(c1, c4);
+        else run(c0, c0);
     };
-    constexpr std::integral_constant<int, 0> c0;
-    constexpr std::integral_constant<int, 1> c1;
-    constexpr std::integral_constant<int, 3> c3;
-    constexpr std::integral_constant<int, 4> c4;
-    constexpr std::integral_constant<int, 8> c8;
-    constexpr std::integral_constant<int, MAX_PS> cm;
-    if (p.n_ps == 3 && ns == 4) run(c3, c4);
-    else if (p.n_ps == 3 && ns == 8) run(c3, c8);
-    else if (p.n_ps == 1 && ns == 4) run(c1, c4);
-    else if (p.n_ps == 1) run(c1, c0);
-    else run(cm, c0);
+    const bool strips = use_strips<T>(p, n, ns, tma);
+    by_steps([&](auto nps, auto nsteps) {
+        constexpr int NPS = decltype(nps)::value, NS = decltype(nsteps)::value;
+        if constexpr (NPS == 3) {
+            if (strips) {
+                const int nstrips = (p.cols + STRIP - 1) / STRIP;
+                const int band = strip_band(ctx, nstrips * n, p.rows, DEC_MIN_WARPS);
+                const long long warps = (long long)nstrips * ((p.rows + band - 1) / band);
+                const dim3 blocks((unsigned)((warps + DEC_WARPS - 1) / DEC_WARPS), n);
+                if (n == 2)
+                    decode_strips_kernel<T, NPS, NS><<<blocks, 32 * DEC_WARPS, 0, st>>>(cams, p, band, nstrips);
+                else
+                    decode_strip_kernel<T, NPS, NS><<<blocks, 32 * DEC_WARPS, 0, st>>>(
+                        static_cast<const T*>(cams.frames[0]), p, band, nstrips, cams.out[0]);
+                return;
+            }
+        }
+        const unsigned tiles_x = (p.cols + TX - 1) / TX;
+        const dim3 grid(tiles_x * (unsigned)((p.rows + TY - 1) / TY), n);
+        if (tma)
+            decode_tile_kernel<T, NPS, NS, true><<<grid, TX * TY, sizeof(T) * tma_bw<T>() * HY * nfr, st>>>(
+                maps, cams, p, nfr, tiles_x, ctx->d_error);
+        else
+            decode_tile_kernel<T, NPS, NS, false><<<grid, TX * TY, 0, st>>>(maps, cams, p, nfr, tiles_x, ctx->d_error);
+    });
     ctx->launches += 1;
 }
 
