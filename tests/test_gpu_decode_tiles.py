@@ -99,3 +99,17 @@ def test_other_step_counts_keep_up(native, few, many, dtype, factor):
         fr = _frames(CONFIGS[c], 2048, 2448, dtype, c)
         t.append(_microseconds(lambda: _decode(ctx, CONFIGS[c], fr)))
     assert t[0] <= factor * t[1], t
+
+
+@pytest.mark.parametrize("dtype", [torch.uint8, torch.uint16])
+def test_hdr_step_counts_keep_up(native, dtype):
+    """36 HDR frames (twelve steps, no code of their own) against 24 (eight) at 2448 x
+    2048: the frames' ratio and half as much again at most."""
+    from zim_gb300 import api
+    ctx = api.Context(0)
+    t = []
+    for c in (4, 0):
+        cfg = dict(CONFIGS[c], enable_hdr=True, hdr_saturation_gray=200.0 if dtype == torch.uint8 else 3200.0)
+        fr = _frames(cfg, 2048, 2448, dtype, c)
+        t.append(_microseconds(lambda: _decode(ctx, cfg, fr)))
+    assert t[0] <= 1.5 * 36 / 24 * t[1], t
