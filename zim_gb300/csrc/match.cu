@@ -14,19 +14,28 @@
 // of the span otherwise, the same column either way -- rejects
 // min >= grad_threshold and columns < 2 or >= cols - 1, then refines with the
 // parabola through the costs of columns best-1, best, best+1.
+#include <algorithm>
 #include <climits>
 
 #include "zim_tiles.cuh"
 
 namespace {
 
-// A row's staged columns hold four CTAs per SM at 4185 columns: 16 warps each hide
-// the latency that 8 do not (whole-frame match, 4185 x 3064: 227 -> 165 us; 653 to
-// 2500 columns: even).  The fused kernel holds more registers and gathers for
+// Threads of a match CTA, by the wider window's columns.  While one wave of 512-thread
+// CTAs (four per SM) takes all rows, those: 700 x 64 4.5 us (128 threads 8.8), 64 x 64
+// 2.7.  With more rows, narrow windows leave such a CTA mostly idle: 64 columns x 3000
+// rows 11.9 us with 512 threads, 4.7 with 64; 200 x 1000 5.9 and 5.1 with 128; 400 x
+// 3000 19.9 and 17.0 with 256 (1280 x 1024: 17.4 and 16.8); wide rows need the warps:
+// 2448 x 2048 58 with 256, 55 with 512; 4185 x 3064 176 and 134.
+constexpr int MATCH_THREADS = 512, MATCH_CTAS = 4;  // per SM
+inline int match_threads(int sms, int rows, int cols) {
+    if (rows <= MATCH_CTAS * sms || cols > 2048) return MATCH_THREADS;
+    return cols <= 64 ? 64 : cols <= 256 ? 128 : 256;
+}
+// The fused kernel holds more registers and gathers for
 // longer, and 8 warps are enough (2500 x 2092: 94 us, 16 warps 113), except where
 // one wave of larger CTAs takes all rows (RM_SMALL_THREADS; 653 x 488: 21 -> 19 us;
 // 1300 x 1041, more than a wave: 46 us against 50).
-constexpr int MATCH_THREADS = 512;
 constexpr int RM_THREADS = 256, RM_SMALL_THREADS = 384, RM_SMALL_CTAS = 3;  // per SM
 
 // Left and right windows of one launch.  The whole-frame match uses the full
@@ -99,7 +108,8 @@ zim_status launch_match(zim_ctx* ctx, const MatchWin& w, int rows, int pha_f, do
     size_t smem = (size_t)w.r_cols * 12 + (size_t)(pha_f + 1) * 12;
     // the attribute is per device and per function: set it on every call
     ZIM_CUDA_TRY(ctx, cudaFuncSetAttribute(match_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    match_kernel<<<rows, MATCH_THREADS, smem, st>>>(w, pha_f, (float)grad_threshold);
+    const int threads = match_threads(ctx->sm_count > 0 ? ctx->sm_count : 152, rows, std::max(w.l_cols, w.r_cols));
+    match_kernel<<<rows, threads, smem, st>>>(w, pha_f, (float)grad_threshold);
     ctx->launches += 1;
     ZIM_LAUNCH_CHECK(ctx);
     return ZIM_OK;
