@@ -1,7 +1,8 @@
 """The whole-row match at widths around the rule that chooses its block size (64, 256
 and 2048 columns, and all rows in one wave of the largest blocks), against itself on
 a few rows at a time (the largest blocks), bit for bit; narrow windows cost less than
-wide ones."""
+wide ones; and the fused rectification and match against the two apart at row counts
+around one wave of its larger blocks."""
 import pytest
 import torch
 
@@ -68,3 +69,22 @@ def test_narrow_windows_cost_less(native):
         (l, r), pha_f = _row_pair(3000, cols, 1)
         t.append(_microseconds(lambda: api.match(ctx, l, r, pha_f, want_best=False)))
     assert t[0] <= 0.6 * t[1], t
+
+
+@pytest.mark.parametrize("cols", [37, 383, 384, 385, 700])
+@pytest.mark.parametrize("more", [0, 1])
+def test_fused_rows_of_a_wave(native, cols, more):
+    from zim_gb300 import api, synth
+    rows = 4 * torch.cuda.get_device_properties(0).multi_processor_count + more
+    ctx = api.Context(0)
+    ctx.set_calibration(synth.make_rig(cols, rows, 1000.0, 100.0).as_dict(), False)
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(cols)
+    left, right = _side(rows, cols, 8.0, gen), _side(rows, cols, 0.0, gen)
+    pha_f = int(max(left[0].max(), right[0].max()))
+    for smooth in (False, True):
+        disp = api.rectify_match(ctx, left, right, pha_f, smooth)
+        l, r = api.rectify(ctx, 0, *left, smooth), api.rectify(ctx, 1, *right, smooth)
+        apart, _ = api.match(ctx, l, r, pha_f)
+        assert torch.equal(disp.view(torch.int32), apart.view(torch.int32))
+    assert int((disp != 0).sum()) > 0 or cols < 64

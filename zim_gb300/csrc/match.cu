@@ -32,11 +32,13 @@ inline int match_threads(int sms, int rows, int cols) {
     if (rows <= MATCH_CTAS * sms || cols > 2048) return MATCH_THREADS;
     return cols <= 64 ? 64 : cols <= 256 ? 128 : 256;
 }
-// The fused kernel holds more registers and gathers for
-// longer, and 8 warps are enough (2500 x 2092: 94 us, 16 warps 113), except where
-// one wave of larger CTAs takes all rows (RM_SMALL_THREADS; 653 x 488: 21 -> 19 us;
-// 1300 x 1041, more than a wave: 46 us against 50).
-constexpr int RM_THREADS = 256, RM_SMALL_THREADS = 384, RM_SMALL_CTAS = 3;  // per SM
+// The fused kernel gathers for longer and is held at 40 registers, 1536 threads per SM:
+// at 48 (1280 threads) noisy fringes, whose spans are scanned in full, took 137 us at
+// 1024 x 768 and 237 at 2448 x 2048 (121 fringes), against 122 and 216.  CTAs of 384
+// threads, four per SM, while one wave of them takes all rows: 488 x 653 10.0 us against
+// 10.5 with 256 threads, six per SM (noisy fringes 36 against 45), 600 x 800 12.5
+// against 13.1; one row count on, 700 x 930, 17.6 against 16.4.
+constexpr int RM_THREADS = 256, RM_CTAS = 6, RM_SMALL_THREADS = 384, RM_SMALL_CTAS = 4;  // per SM
 
 // Left and right windows of one launch.  The whole-frame match uses the full
 // rows of both images; the ROI match a left rectangle and a right column
@@ -138,8 +140,8 @@ __device__ __forceinline__ void rect_px(const RectMatchArgs& a, int cam, float m
         zt::rectify_pixel(a.order[cam], a.res[cam], a.srows, a.scols, mx, my, a.post_smooth, b, r, k);
 }
 
-template <int THREADS>
-__global__ void __launch_bounds__(THREADS) rectify_match_kernel(RectMatchArgs a, int pha_f,
+template <int THREADS, int CTAS>
+__global__ void __launch_bounds__(THREADS, CTAS) rectify_match_kernel(RectMatchArgs a, int pha_f,
                                                                       float grad_threshold) {
     extern __shared__ int4 smem_raw[];
     const int cols = a.cols;
@@ -226,8 +228,8 @@ zim_status zim_rectify_match_launch(zim_ctx* ctx, const int32_t* const order[2],
         return zim_fail(ctx, ZIM_ERR_INVALID_ARG, "rectified width %d above %d", a.cols, ZIM_MAX_MATCH_COLS);
     const size_t smem = (size_t)a.cols * 12 + (size_t)(pha_f + 1) * 12;
     const int sms = ctx->sm_count > 0 ? ctx->sm_count : 152;
-    const bool small = a.rows <= RM_SMALL_CTAS * sms + sms / 4;
-    auto kern = small ? rectify_match_kernel<RM_SMALL_THREADS> : rectify_match_kernel<RM_THREADS>;
+    const bool small = a.rows <= RM_SMALL_CTAS * sms;
+    auto kern = small ? rectify_match_kernel<RM_SMALL_THREADS, RM_SMALL_CTAS> : rectify_match_kernel<RM_THREADS, RM_CTAS>;
     ZIM_CUDA_TRY(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     kern<<<a.rows, small ? RM_SMALL_THREADS : RM_THREADS, smem, st>>>(a, pha_f, (float)grad_threshold);
     ctx->launches += 1;
