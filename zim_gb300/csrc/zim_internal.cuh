@@ -81,11 +81,14 @@ inline cudaStream_t zim_stream(void* s) { return reinterpret_cast<cudaStream_t>(
 
 // Rows per warp of the kernels that march a warp down a strip of columns: a band
 // reads a few rows more than it writes, so the tallest of 32, 16, 8 and 4 rows
-// that still gives warps_per_sm warps to every SM.
+// that still gives warps_per_sm warps to every SM.  Where even 4 rows give less than
+// two fifths of that, the launch is as long as one warp and a band is 2 rows or 1.
 inline int strip_band(const zim_ctx* ctx, int nstrips, int rows, int warps_per_sm) {
     const long long want = (long long)warps_per_sm * (ctx->sm_count > 0 ? ctx->sm_count : 152);
+    auto warps = [&](int band) { return (long long)nstrips * ((rows + band - 1) / band); };
     int band = 32;
-    while (band > 4 && (long long)nstrips * ((rows + band - 1) / band) < want) band /= 2;
+    while (band > 4 && warps(band) < want) band /= 2;
+    while (band > 1 && 5 * warps(band) < 2 * want) band /= 2;
     return band;
 }
 
