@@ -201,6 +201,7 @@ __global__ void __launch_bounds__(BT) batch_pxg_kernel(const PairDev* __restrict
     }
 }
 
+template <bool WIDE>
 __global__ void __launch_bounds__(BT) batch_ror_kernel(const PairDev* __restrict__ pairs,
                                                        const int4* __restrict__ items, int n_items,
                                                        unsigned* __restrict__ counter) {
@@ -215,7 +216,7 @@ __global__ void __launch_bounds__(BT) batch_ror_kernel(const PairDev* __restrict
         const int tiles_x = (P.rw + zt::RX - 1) / zt::RX;
         for (int ty = w.y; ty < w.y + w.z; ty++)
             for (int tx = 0; tx < tiles_x; tx++)
-                zt::ror_tile(P.x_ror_in, P.m_ror_in, P.rh, P.rw, tx * zt::RX, ty * zt::RY, zt::RY, tid, P.ror_r2,
+                zt::ror_tile<WIDE>(P.x_ror_in, P.m_ror_in, P.rh, P.rw, tx * zt::RX, ty * zt::RY, zt::RY, tid, P.ror_r2,
                              P.ror_min_nb, P.ror_hw, ror_smem, P.x_ror, P.m_ror);
         __syncthreads();
     }
@@ -241,6 +242,7 @@ struct zim_batch {
     int max_cols = 0, max_pha_f = 0;
     size_t match_smem = 0;
     size_t ror_smem = 0;
+    void (*ror_kernel)(const PairDev*, const int4*, int, unsigned*) = nullptr;
     int grid[NQ] = {};
     cudaStream_t cap_stream = nullptr;
     cudaGraph_t graph = nullptr;
@@ -402,7 +404,7 @@ zim_status capture(zim_batch* b) {
     b->grid[Q_MATCH] = sms * std::min(want, occupancy((const void*)batch_match_kernel, b->match_smem));
     b->grid[Q_REPROJ] = sms * std::min(want, occupancy((const void*)batch_reproject_kernel, 0));
     b->grid[Q_PXG] = sms * std::min(want, occupancy((const void*)batch_pxg_kernel, 0));
-    b->grid[Q_ROR] = sms * std::min(want, occupancy((const void*)batch_ror_kernel, b->ror_smem));
+    b->grid[Q_ROR] = sms * std::min(want, occupancy((const void*)b->ror_kernel, b->ror_smem));
     cudaStream_t s = b->cap_stream;
     ZIM_CUDA_TRY(ctx, cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
     cudaMemsetAsync(b->d_counters, 0, NQ * sizeof(unsigned), s);
@@ -425,7 +427,7 @@ zim_status capture(zim_batch* b) {
         batch_pxg_kernel<<<std::min(b->grid[Q_PXG], q.n[Q_PXG]), BT, 0, s>>>(b->d_pairs, q.items[Q_PXG], q.n[Q_PXG],
                                                                             b->d_counters + Q_PXG);
     if (q.n[Q_ROR])
-        batch_ror_kernel<<<std::min(b->grid[Q_ROR], q.n[Q_ROR]), BT, b->ror_smem, s>>>(
+        b->ror_kernel<<<std::min(b->grid[Q_ROR], q.n[Q_ROR]), BT, b->ror_smem, s>>>(
             b->d_pairs, q.items[Q_ROR], q.n[Q_ROR], b->d_counters + Q_ROR);
     cudaError_t le = cudaGetLastError();
     // the grid filters: the lanes fork from the capture after the pixel stages
@@ -644,9 +646,10 @@ extern "C" ZIM_API zim_status zim_batch_submit(zim_batch* b, const zim_batch_pai
     b->match_smem = (size_t)max_cols * 12 + (size_t)(max_pha + 1) * 12;
     ZIM_CUDA_TRY(ctx, cudaFuncSetAttribute(batch_match_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                            (int)b->match_smem));
+    b->ror_kernel = rcfg->radius_window_size / 2 > zt::ROR_WIDE ? batch_ror_kernel<true> : batch_ror_kernel<false>;
     b->ror_smem = b->use_ror ? zt::ror_smem_bytes(rcfg->radius_window_size / 2, zt::RY) : 0;
     if (b->use_ror)
-        ZIM_CUDA_TRY(ctx, cudaFuncSetAttribute(batch_ror_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        ZIM_CUDA_TRY(ctx, cudaFuncSetAttribute(b->ror_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                (int)b->ror_smem));
 
     // memory plan: descriptors, counters, per-pair intermediates, items

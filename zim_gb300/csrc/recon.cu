@@ -27,6 +27,14 @@ __global__ void __launch_bounds__(32 * zt::MED_WARPS, 3) median_reproject_kernel
 
 constexpr int PXG_WARPS = 4;
 constexpr size_t ROR_SMEM = 52 * 1024;  // shared memory of a radius-filter tile taller than RY rows
+// Rows of a radius-filter tile: tall tiles stage less halo per point, but few of them
+// end in a nearly empty wave.
+inline int ror_rows(int sms, int rows, int cols, int hw) {
+    int th = 32;
+    auto blocks = [&](int th) { return (long long)((cols + RX - 1) / RX) * ((rows + th - 1) / th); };
+    while (th > RY && (zt::ror_smem_bytes(hw, th) > ROR_SMEM || blocks(th) < (th == 32 ? 64ll : 12ll) * sms)) th /= 2;
+    return th;
+}
 __global__ void __launch_bounds__(32 * PXG_WARPS) px_gaussian_kernel(const float* __restrict__ xyz,
                                                                      const uint8_t* __restrict__ mask, int rows,
                                                                      int cols, int band, int nstrips, float w00,
@@ -38,11 +46,12 @@ __global__ void __launch_bounds__(32 * PXG_WARPS) px_gaussian_kernel(const float
                               mask_out);
 }
 
+template <bool WIDE>
 __global__ void __launch_bounds__(RX* RY) ror_kernel(const float* __restrict__ xyz, const uint8_t* __restrict__ mask,
                                                      int rows, int cols, int th, float r2, int min_nb, int hw,
                                                      float* __restrict__ out, uint8_t* __restrict__ mask_out) {
     extern __shared__ float4 ror_smem[];
-    zt::ror_tile(xyz, mask, rows, cols, blockIdx.x * RX, blockIdx.y * th, th, threadIdx.x, r2, min_nb, hw, ror_smem, out,
+    zt::ror_tile<WIDE>(xyz, mask, rows, cols, blockIdx.x * RX, blockIdx.y * th, th, threadIdx.x, r2, min_nb, hw, ror_smem, out,
                  mask_out);
 }
 
@@ -188,17 +197,12 @@ zim_status zim_px_gaussian_launch(zim_ctx* ctx, const float* xyz, const uint8_t*
 zim_status zim_ror_launch(zim_ctx* ctx, const float* xyz, const uint8_t* mask, int rows, int cols, float radius,
                           int min_neighbors, int window_size, float* out, uint8_t* mask_out, cudaStream_t st) {
     const int hw = window_size / 2;
-    // Rows per tile: tall tiles stage less halo per point, as long as four CTAs
-    // share an SM and the launch fills it
-    int th = 32;
-    const long long want = 4ll * (ctx->sm_count > 0 ? ctx->sm_count : 152);
-    while (th > RY && (zt::ror_smem_bytes(hw, th) > ROR_SMEM ||
-                       (long long)((cols + RX - 1) / RX) * ((rows + th - 1) / th) < want))
-        th /= 2;
+    const int th = ror_rows(ctx->sm_count > 0 ? ctx->sm_count : 152, rows, cols, hw);
     const size_t smem = zt::ror_smem_bytes(hw, th);
-    ZIM_CUDA_TRY(ctx, cudaFuncSetAttribute(ror_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    auto kern = hw > zt::ROR_WIDE ? ror_kernel<true> : ror_kernel<false>;
+    ZIM_CUDA_TRY(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     dim3 grd((cols + RX - 1) / RX, (rows + th - 1) / th);
-    ror_kernel<<<grd, RX * RY, smem, st>>>(xyz, mask, rows, cols, th, radius * radius, min_neighbors, hw, out, mask_out);
+    kern<<<grd, RX * RY, smem, st>>>(xyz, mask, rows, cols, th, radius * radius, min_neighbors, hw, out, mask_out);
     ctx->launches += 1;
     ZIM_LAUNCH_CHECK(ctx);
     return ZIM_OK;

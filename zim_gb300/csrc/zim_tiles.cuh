@@ -920,10 +920,19 @@ __device__ __forceinline__ void px_gaussian_strip(const float* __restrict__ xyz,
 // at 4185x3064: 372 us with tiles of 8 rows scanned row by row, 302 with rings, 200
 // with rings and tiles of 32 rows, 147 with the count checked every four neighbours
 // and no division in the staging (every eight: 177).
+//
+// WIDE (half-windows above ROR_WIDE): ROR_RINGS rings, then the rest of the window row
+// by row.  A long ring has four bases to step and its count to test every four
+// neighbours; where nobody has enough, a window of 91 took 33.0 ms in rings at
+// 2448x2048, 21.8 row by row and 21.5 so (41: 3.60, 3.49, 3.49), and where the first
+// rings settle it all are the rings' (91, 5 mm: 1.57).  Narrow windows in rings alone:
+// the second loop's registers cost the 11 x 11 filter 15 %.
+constexpr int ROR_WIDE = 10, ROR_RINGS = 6;
 __host__ __device__ inline size_t ror_smem_bytes(int hw, int th) {
     return (size_t)(RX + 2 * hw) * (th + 2 * hw) * sizeof(float4);
 }
 
+template <bool WIDE>
 __device__ __forceinline__ void ror_tile(const float* __restrict__ xyz, const uint8_t* __restrict__ mask, int rows,
                                          int cols, int x0, int y0, int TH, int tid, float r2, int min_nb, int hw,
                                          float4* sp, float* __restrict__ out, uint8_t* __restrict__ mask_out) {
@@ -962,7 +971,8 @@ __device__ __forceinline__ void ror_tile(const float* __restrict__ xyz, const ui
                 const float dx = c.x - p.x, dy = c.y - p.y, dz = c.z - p.z;
                 cnt += fmaf(dz, dz, fmaf(dy, dy, dx * dx)) <= r2 ? 1 : 0;
             };
-            for (int r = 1; r <= hw && cnt <= min_nb; r++) {
+            const int nr = WIDE ? ROR_RINGS : hw;
+            for (int r = 1; r <= nr && cnt <= min_nb; r++) {
                 const float4* a = centre - r * TW - r;  // the four sides, one step each
                 const float4* b = centre + r * TW + r;
                 const float4* l = centre + r * TW - r;
@@ -974,6 +984,14 @@ __device__ __forceinline__ void ror_tile(const float* __restrict__ xyz, const ui
                     test(*l);
                     test(*g);
                 }
+            }
+            for (int i = -hw; WIDE && i <= hw && cnt <= min_nb; i++) {
+                const float4* row = centre + i * TW;
+                const bool split = i >= -nr && i <= nr;
+                const int e = split ? -nr - 1 : hw;
+                for (int j = -hw; j <= e; j++) test(row[j]);
+                if (split)
+                    for (int j = nr + 1; j <= hw; j++) test(row[j]);
             }
             keep = cnt > min_nb;
         }
