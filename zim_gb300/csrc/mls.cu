@@ -497,6 +497,7 @@ __global__ void __launch_bounds__(MX* MY) mls_smem_kernel(const float* __restric
 // at 12 all of them, 6.79 against 6.53 ms.  Bound by issue and the FP32 pipe: a
 // neighbour is 50 instructions of both sweeps.
 constexpr int MLS_R = 12;
+constexpr int MLS_MAX_HW = 64;  // largest half-window
 
 // One tile of queries: its place, this thread's query and its bound.
 struct MlsTile {
@@ -613,18 +614,23 @@ struct MlsTile {
     }
 };
 
-// NEAR: half-windows up to MLS_R.  HW: the half-window at compile time (0: hw_arg),
-// which makes the tile's width constant.  With four CTAs per SM asked for, the
-// second order keeps to 64 registers.
+// NEAR: the window staged whole.  HW: the half-window at compile time, which makes the
+// tile's width constant (0: hw_arg, up to MLS_R; MLS_DYN: hw_arg beyond it, the tile in
+// dynamic shared memory, which costs the others 1 to 2 %).  With four CTAs per SM asked
+// for, the second order keeps to 64 registers.
+constexpr int MLS_DYN = -1;
 template <bool ORDER2, bool NEAR, int HW>
 __global__ void __launch_bounds__(MX* MY, ORDER2 && NEAR ? 4 : 1) mls_ray_kernel(const float* __restrict__ src,
                                                           const uint8_t* __restrict__ mask, int rows, int cols,
                                                           int hw_arg, float inv_2s2, int order, float r2c,
                                                           zt::RayParams rp, zl::Tree t, unsigned* __restrict__ wide,
                                                           float* __restrict__ dst) {
-    const int hw = HW ? HW : hw_arg;
-    constexpr int RMAX = HW ? HW : MLS_R, TMAX = MX + 2 * RMAX, WARPS = MX * MY / 32;
-    __shared__ float4 sp[TMAX * TMAX];
+    const int hw = HW > 0 ? HW : hw_arg;
+    constexpr bool DYN = HW == MLS_DYN;
+    constexpr int RMAX = DYN ? MLS_MAX_HW : HW ? HW : MLS_R, TMAX = DYN ? 1 : MX + 2 * RMAX, WARPS = MX * MY / 32;
+    __shared__ float4 s_tile[TMAX * TMAX];
+    extern __shared__ float4 d_tile[];
+    float4* sp = DYN ? d_tile : s_tile;
     __shared__ unsigned s_red[2][WARPS];
     __shared__ signed char s_w[WARPS][RMAX + 1];
     MlsTile T(src, mask, rows, cols, blockIdx.x, blockIdx.y);
@@ -645,6 +651,7 @@ __global__ void __launch_bounds__(MX* MY, ORDER2 && NEAR ? 4 : 1) mls_ray_kernel
     }
     const int lane = T.lane, wid = T.wid;
     if (lane <= R) s_w[wid][lane] = MlsTile::row_width(wr2, lane, hw, R);
+    if (DYN && lane + 32 <= R) s_w[wid][lane + 32] = MlsTile::row_width(wr2, lane + 32, hw, R);
     if (NEAR) __syncwarp();
     else __syncthreads();
     float ox = 0.f, oy = 0.f, oz = 0.f;
@@ -738,7 +745,22 @@ __global__ void __launch_bounds__(MX* MY, 2) mls_wide_kernel(const float* __rest
 }  // namespace
 
 constexpr size_t MLS_SMEM = 96 * 1024;  // shared memory of a tile: two CTAs per SM
+constexpr size_t MLS_SM = 228 * 1024;   // and of an SM
 static size_t mls_tiles(int rows, int cols) { return (size_t)((cols + MX - 1) / MX) * ((rows + MY - 1) / MY); }
+
+// Whether a cloud with pixel rays has its window staged whole: up to MLS_R, and beyond it
+// where the tree's build and the list's kernel (6 us) are more than the staging, while
+// one wave of the tiles' CTAs takes the cloud (order 1, us, staged / tree: half-window 13,
+// 640x480 34.9 / 39.2, 1024x768 83.3 / 83.5; 16, 320x240 14.3 / 20.5; 20, 400x300 21.3 /
+// 25.5, 500x360 32.6 / 29.5; 24, 320x240 18.0 / 20.5, 400x300 28.7 / 25.5; 30, 16x16 10.7 /
+// 16.4, 160x120 19.5 / 18.5).
+static bool mls_near(int sms, int rows, int cols, int hw) {
+    if (hw <= MLS_R) return true;
+    const size_t smem = mls_smem_bytes(hw), tiles = mls_tiles(rows, cols);
+    if (smem > MLS_SMEM) return false;
+    if (hw > 24) return tiles <= (size_t)sms / 12;
+    return tiles <= (size_t)sms * std::min<size_t>(8, MLS_SM / (smem + 2048));
+}
 
 size_t zim_mls_scratch_bytes(int rows, int cols) {
     return zim_leaf_bytes(rows, cols) + zim_align256(mls_tiles(rows, cols) * 4);
@@ -758,7 +780,8 @@ zim_status zim_mls_launch(zim_ctx* ctx, const float* xyz, const uint8_t* mask, i
     if (use_smem)
         ZIM_CUDA_TRY(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const zt::RayParams rp = zt::ray_params(rays);
-    const bool near = rays.valid != 0 && window <= MLS_R, leaf = rays.valid != 0 && !near;
+    const bool near = rays.valid != 0 && mls_near(ctx->sm_count > 0 ? ctx->sm_count : 152, rows, cols, window);
+    const bool leaf = rays.valid != 0 && !near;
     zl::Tree t{};
     unsigned* wide = nullptr;  // tiles left to mls_wide_kernel
     const size_t wide_smem = std::min(smem, MLS_SMEM);
@@ -787,8 +810,13 @@ zim_status zim_mls_launch(zim_ctx* ctx, const float* xyz, const uint8_t* mask, i
             ctx->launches += 1;
         } else if (near) {
             auto nk = window == 7 ? (ord == 2 ? mls_ray_kernel<true, true, 7> : mls_ray_kernel<false, true, 7>)
-                                  : (ord == 2 ? mls_ray_kernel<true, true, 0> : mls_ray_kernel<false, true, 0>);
-            nk<<<grd, blk, 0, st>>>(in, mask, rows, cols, window, inv_2s2, ord, r2c, rp, t, wide, dst);
+                      : window <= MLS_R
+                          ? (ord == 2 ? mls_ray_kernel<true, true, 0> : mls_ray_kernel<false, true, 0>)
+                          : (ord == 2 ? mls_ray_kernel<true, true, MLS_DYN> : mls_ray_kernel<false, true, MLS_DYN>);
+            const size_t dyn = window > MLS_R ? smem : 0;
+            if (dyn)
+                ZIM_CUDA_TRY(ctx, cudaFuncSetAttribute(nk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
+            nk<<<grd, blk, dyn, st>>>(in, mask, rows, cols, window, inv_2s2, ord, r2c, rp, t, wide, dst);
         } else if (use_smem)
             kern<<<grd, blk, smem, st>>>(in, mask, rows, cols, window, inv_2s2, ord, r2c, dst);
         else
@@ -805,7 +833,7 @@ extern "C" ZIM_API zim_status zim_filter_mls(zim_ctx* ctx, const float* xyz, con
                                              float* out, void* stream) {
     if (!ctx) return ZIM_ERR_INVALID_ARG;
     if (!xyz || !mask || !out || rows <= 0 || cols <= 0) return zim_fail(ctx, ZIM_ERR_INVALID_ARG, "bad argument");
-    if (window < 0 || window > 64 || !(sigma > 0)) return zim_fail(ctx, ZIM_ERR_INVALID_ARG, "bad MLS parameter");
+    if (window < 0 || window > MLS_MAX_HW || !(sigma > 0)) return zim_fail(ctx, ZIM_ERR_INVALID_ARG, "bad MLS parameter");
     if (out == xyz) return zim_fail(ctx, ZIM_ERR_INVALID_ARG, "MLS in-place not supported");
     ZIM_CUDA_TRY(ctx, cudaSetDevice(ctx->device));
     float* tmp = nullptr;
