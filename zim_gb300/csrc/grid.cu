@@ -1279,7 +1279,9 @@ __device__ __forceinline__ double warp_sum2(double a, double b) {
 }
 
 // Three blocks per SM, four pixels per thread and step and four steps' loads in
-// flight (md 16-byte, mask 4-byte aligned: vec).  The
+// flight; vec: md 16-byte and mask 4-byte aligned, one load each for the four (else
+// one per pixel: the same pixels in the same order, so the sums do not depend on
+// where the buffers lie).  The
 // threshold mean + std_mul * stddev; the classifier compares the float mean
 // distances with thr_f, the largest float <= thr, which decides exactly as
 // (double)md > thr.
@@ -1293,7 +1295,7 @@ __global__ void __launch_bounds__(GB) sor_stats_kernel(const uint8_t* __restrict
         comp_add(as, ac, v);
         comp_add(bs, bc, v * v);  // PCL: float square, double sum
     };
-    const size_t step = (size_t)gridDim.x * GB, full4 = vec ? n / 4 : 0;
+    const size_t step = (size_t)gridDim.x * GB, full4 = n / 4;
     size_t g = (size_t)blockIdx.x * GB + threadIdx.x;
     for (; g < full4; g += SOR_STAT_STEPS * step) {
         uchar4 m[SOR_STAT_STEPS];
@@ -1302,9 +1304,14 @@ __global__ void __launch_bounds__(GB) sor_stats_kernel(const uint8_t* __restrict
         for (int u = 0; u < SOR_STAT_STEPS; u++) {
             m[u] = make_uchar4(0, 0, 0, 0);
             v[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (g + u * step < full4) {
-                m[u] = __ldg(reinterpret_cast<const uchar4*>(mask) + g + u * step);
-                v[u] = __ldg(reinterpret_cast<const float4*>(md) + g + u * step);
+            const size_t e = g + u * step;
+            if (e >= full4) continue;
+            if (vec) {
+                m[u] = __ldg(reinterpret_cast<const uchar4*>(mask) + e);
+                v[u] = __ldg(reinterpret_cast<const float4*>(md) + e);
+            } else {
+                m[u] = make_uchar4(mask[4 * e], mask[4 * e + 1], mask[4 * e + 2], mask[4 * e + 3]);
+                v[u] = make_float4(md[4 * e], md[4 * e + 1], md[4 * e + 2], md[4 * e + 3]);
             }
         }
 #pragma unroll
