@@ -143,13 +143,12 @@ __global__ void spacing1_kernel(const float* __restrict__ xyz, const uint8_t* __
             }
 #pragma unroll
             for (int u = 0; u < U; u++) {
-                if (!m[u]) continue;
-                const int x = xb + u * (int)blockDim.x;
+                if (!m[u] || !zl::finite_point(p[u][0], p[u][1], p[u][2])) continue;
                 for (int a = 0; a < 3; a++) {
                     mn[a] = min(mn[a], fbits(p[u][a]));
                     mx[a] = max(mx[a], fbits(p[u][a]));
                 }
-                if (mr[u]) {
+                if (mr[u] && zl::finite_point(q[u][0], q[u][1], q[u][2])) {
                     float dx = q[u][0] - p[u][0], dy = q[u][1] - p[u][1], dz = q[u][2] - p[u][2];
                     df += sqrtf(dx * dx + dy * dy + dz * dz);
                     ci++;
@@ -279,7 +278,7 @@ __global__ void hash_count_kernel(const float* __restrict__ xyz, const uint8_t* 
                                   unsigned* __restrict__ counts) {
     for (size_t b = (size_t)blockIdx.x * blockDim.x; b < n; b += (size_t)gridDim.x * blockDim.x) {
         const size_t i = b + threadIdx.x;
-        const bool v = i < n && mask[i];
+        const bool v = i < n && mask[i] && zl::finite_point(xyz[3 * i], xyz[3 * i + 1], xyz[3 * i + 2]);
         const unsigned h = v ? grid_slot(s, tmask, xyz[3 * i], xyz[3 * i + 1], xyz[3 * i + 2]) : 0xffffffffu;
         const unsigned grp = __match_any_sync(0xffffffffu, h);
         if (v && (threadIdx.x & 31) == __ffs(grp) - 1) atomicAdd(&counts[h], (unsigned)__popc(grp));
@@ -358,7 +357,7 @@ __global__ void hash_scatter_kernel(const float* __restrict__ xyz, const uint8_t
                                     float4* __restrict__ pts) {
     for (size_t b = (size_t)blockIdx.x * blockDim.x; b < n; b += (size_t)gridDim.x * blockDim.x) {
         const size_t i = b + threadIdx.x;
-        const bool v = i < n && mask[i];
+        const bool v = i < n && mask[i] && zl::finite_point(xyz[3 * i], xyz[3 * i + 1], xyz[3 * i + 2]);
         float x = 0.f, y = 0.f, z = 0.f;
         unsigned h = 0xffffffffu;
         if (v) {
@@ -441,23 +440,27 @@ __global__ void __launch_bounds__(TILE_T) sor_knn_tile_kernel(const float* __res
     const int x = x0 + (tid % TILE_X), y = y0 + (tid / TILE_X);
     const bool in = x < cols && y < rows;
     const size_t i = in ? (size_t)y * cols + x : 0;
-    const bool active = in && mask[i] && h->n_valid > (unsigned)k;
-    if (in && !active) md_out[i] = 0.f;
-    if (!__syncthreads_or(active)) return;  // the whole CTA leaves together
+    const bool valid = in && mask[i] && h->n_valid > (unsigned)k;
+    if (in && !valid) md_out[i] = 0.f;
+    if (!__syncthreads_or(valid)) return;  // the whole CTA leaves together
     const float ic = s->inv_cell, cell = s->cell;
     float qx = 0.f, qy = 0.f, qz = 0.f;
     int c[3] = {0, 0, 0};
-    if (active) {
+    bool active = false;  // a query without finite coordinates is not searched here
+    if (valid) {
         qx = xyz[3 * i]; qy = xyz[3 * i + 1]; qz = xyz[3 * i + 2];
-        cell_of(qx, qy, qz, ic, c[0], c[1], c[2]);
+        active = zl::finite_point(qx, qy, qz);
     }
-    // window bound tau0 from the pixel neighbourhood (staged in cand; w = 0 marks invalid)
+    if (active) cell_of(qx, qy, qz, ic, c[0], c[1], c[2]);
+    // window bound tau0 from the pixel neighbourhood (staged in cand; w = 0 marks
+    // pixels without a finite point)
     for (int t = tid; t < WIN_W * WIN_H; t += TILE_T) {
         const int wx = x0 - WIN_R + t % WIN_W, wy = y0 - WIN_R + t / WIN_W;
         float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
         if (wx >= 0 && wx < cols && wy >= 0 && wy < rows) {
             const size_t j = (size_t)wy * cols + wx;
-            if (mask[j]) v = make_float4(xyz[3 * j], xyz[3 * j + 1], xyz[3 * j + 2], 1.f);
+            const float px = xyz[3 * j], py = xyz[3 * j + 1], pz = xyz[3 * j + 2];
+            if (mask[j] && zl::finite_point(px, py, pz)) v = make_float4(px, py, pz, 1.f);
         }
         cand[t] = v;
     }
@@ -681,7 +684,7 @@ __global__ void __launch_bounds__(TILE_T) sor_knn_tile_kernel(const float* __res
             }
         }
     }
-    if (active && !done) {
+    if (valid && !done) {
         md_out[i] = -1.f;
         const unsigned slot = atomicAdd(&h->n_deferred, 1u);
         deferred[slot] = (unsigned)i;
@@ -1049,9 +1052,22 @@ __global__ void __launch_bounds__(TS_WARPS * 32) sor_tree_kernel(const float* __
     const unsigned nd = t.head->n_deferred, nwarps = gridDim.x * TS_WARPS;
     // the first query of each warp by its index: thousands of warps asking one
     // counter at once took 4 us
+    auto next_item = [&]() {
+        unsigned n = 0;
+        if (lane == 0) n = nwarps + atomicAdd(&t.head->next, 1u);
+        return __shfl_sync(full, n, 0);
+    };
     for (unsigned item = blockIdx.x * TS_WARPS + w; item < nd;) {
         const unsigned i = deferred[item];
         const float q[3] = {xyz[3 * (size_t)i], xyz[3 * (size_t)i + 1], xyz[3 * (size_t)i + 2]};
+        if (!zl::finite_point(q[0], q[1], q[2])) {  // no neighbours, not even itself
+            if (lane == 0) {
+                atomicOr(err, 0x10u);
+                md_out[i] = 0.f;
+            }
+            item = next_item();
+            continue;
+        }
         // entries lie strictly below thr; bounds are met by equality, so they
         // start one float above (finite non-negative floats order as their bits)
         auto above = [](float b) { return b < INFINITY ? __uint_as_float(__float_as_uint(b) + 1u) : INFINITY; };
@@ -1216,8 +1232,7 @@ __global__ void __launch_bounds__(TS_WARPS * 32) sor_tree_kernel(const float* __
         }
         flush();
         __syncwarp();
-        if (lane == 0) item = nwarps + atomicAdd(&t.head->next, 1u);
-        item = __shfl_sync(full, item, 0);
+        item = next_item();
         if (n < K1 || K1 > FW_CAP - NEW) {  // fewer than k + 1 finite points (or a k beyond the list)
             if (lane == 0) {
                 atomicOr(err, 0x10u);

@@ -57,8 +57,7 @@ __global__ void __launch_bounds__(LB) leaf_kernel(const float* __restrict__ xyz,
         for (int u = 0; u < 4; u++) {
             if (!v[u]) continue;
             nv++;
-            // points with a NaN or infinite coordinate are nobody's neighbour: outside every box
-            if (fmaf(p[u][0], 0.f, fmaf(p[u][1], 0.f, p[u][2] * 0.f)) == 0.f) {
+            if (zl::finite_point(p[u][0], p[u][1], p[u][2])) {
                 a.n++;
 #pragma unroll
                 for (int c = 0; c < 3; c++) {

@@ -53,6 +53,12 @@ __device__ __forceinline__ Box load_box(const float4* boxes, int i) {
     return Box{{a.x, a.y, a.z}, {b.x, b.y, b.z}, __float_as_uint(a.w)};
 }
 
+// Points with a NaN or infinite coordinate are nobody's neighbour: outside every box,
+// window and grid.
+__device__ __forceinline__ bool finite_point(float x, float y, float z) {
+    return fmaf(x, 0.f, fmaf(y, 0.f, z * 0.f)) == 0.f;
+}
+
 __device__ __forceinline__ float sq3(float dx, float dy, float dz) { return fmaf(dz, dz, fmaf(dy, dy, dx * dx)); }
 
 // Squared distance between the box and the box [lo, hi] (a point: lo = hi).
