@@ -267,7 +267,7 @@ struct zim_batch {
     cudaStream_t lane_stream[MAX_LANES] = {};
     cudaEvent_t fork_ev = nullptr;
     cudaEvent_t join_ev[MAX_LANES] = {};
-    unsigned long long lane_launches = 0;  // grid-filter kernels per graph replay
+    unsigned long long decode_launches = 0, lane_launches = 0;  // decode and grid-filter kernels per graph replay
 };
 
 namespace {
@@ -413,6 +413,7 @@ zim_status capture(zim_batch* b) {
     const unsigned long long launched = ctx->launches;
     for (const PairDev& D : b->host_pairs)
         zim_decode_params_launch(ctx, 2, D.frames, D.sample_type, D.dp, D.order, D.res, nullptr, nullptr, s);
+    b->decode_launches = ctx->launches - launched;
     ctx->launches = launched;  // captured, not run: each replay counts them
     if (q.n[Q_SMOOTH])
         batch_smooth_kernel<<<std::min(b->grid[Q_SMOOTH], q.n[Q_SMOOTH]), BT, 0, s>>>(
@@ -762,7 +763,7 @@ extern "C" ZIM_API zim_status zim_batch_run(zim_batch* b, void* stream) {
     if (!b->exec) return zim_fail(b->ctx, ZIM_ERR_INVALID_ARG, "nothing submitted");
     ZIM_CUDA_TRY(b->ctx, cudaGraphLaunch(b->exec, zim_stream(stream)));
     for (int q = 0; q < NQ; q++) b->ctx->launches += b->q.n[q] > 0 ? 1 : 0;  // kernels in the graph
-    b->ctx->launches += 2 * b->host_pairs.size() + b->lane_launches;
+    b->ctx->launches += b->decode_launches + b->lane_launches;
     return ZIM_OK;
 }
 
