@@ -64,3 +64,25 @@ def test_wide_windows_without_neighbours(native):
     xyz, mask = _cloud(768, 1024, 5)
     t = [_microseconds(lambda: api.filter_ror(ctx, xyz, mask, 0.1, 10, w)) for w in (40, 90)]
     assert t[1] <= 7.2 * t[0], t
+
+
+@pytest.mark.parametrize("window", [4, 30])
+@pytest.mark.parametrize("radius", [7.5, 1e20])
+def test_points_without_finite_coordinates(native, window, radius):
+    """The definition as the reference counts: float distances over the window, the point's
+    own among them, at least min_nb + 1 (any with min_nb 0).  A point without finite
+    coordinates does not count itself, and with a radius whose square is infinite one at
+    infinity has the finite ones near."""
+    from zim_gb300 import api
+    ctx = api.Context(0)
+    xyz = torch.arange(3 * 25, device="cuda", dtype=torch.float32).view(5, 5, 3)
+    mask = torch.ones((5, 5), dtype=torch.uint8, device="cuda")
+    xyz[2, 2, 0], xyz[0, 0] = float("inf"), float("nan")
+    p, r = xyz.view(25, 3), torch.tensor(radius, dtype=torch.float32, device="cuda")
+    y, x = torch.arange(25, device="cuda") // 5, torch.arange(25, device="cuda") % 5
+    near = ((y[:, None] - y).abs() <= window // 2) & ((x[:, None] - x).abs() <= window // 2)
+    count = ((((p[:, None] - p) ** 2).sum(-1) <= r * r) & near).sum(1).view(5, 5)
+    for min_nb in (0, 1, 2, 8, 14, 22, 23, 24):
+        _, mo = api.filter_ror(ctx, xyz, mask, radius, min_nb, window)
+        want = (count >= min_nb + 1) | (min_nb == 0)
+        assert torch.equal(mo, want.to(torch.uint8)), min_nb

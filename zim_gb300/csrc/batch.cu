@@ -647,7 +647,7 @@ extern "C" ZIM_API zim_status zim_batch_submit(zim_batch* b, const zim_batch_pai
     b->match_smem = (size_t)max_cols * 12 + (size_t)(max_pha + 1) * 12;
     ZIM_CUDA_TRY(ctx, cudaFuncSetAttribute(batch_match_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                            (int)b->match_smem));
-    b->ror_kernel = rcfg->radius_window_size / 2 > zt::ROR_WIDE ? batch_ror_kernel<true> : batch_ror_kernel<false>;
+    b->ror_kernel = zt::ror_wide(rcfg->radius_window_size / 2, rcfg->radius_search) ? batch_ror_kernel<true> : batch_ror_kernel<false>;
     b->ror_smem = b->use_ror ? zt::ror_smem_bytes(rcfg->radius_window_size / 2, zt::RY) : 0;
     if (b->use_ror)
         ZIM_CUDA_TRY(ctx, cudaFuncSetAttribute(b->ror_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,

@@ -199,7 +199,7 @@ zim_status zim_ror_launch(zim_ctx* ctx, const float* xyz, const uint8_t* mask, i
     const int hw = window_size / 2;
     const int th = ror_rows(ctx->sm_count > 0 ? ctx->sm_count : 152, rows, cols, hw);
     const size_t smem = zt::ror_smem_bytes(hw, th);
-    auto kern = hw > zt::ROR_WIDE ? ror_kernel<true> : ror_kernel<false>;
+    auto kern = zt::ror_wide(hw, radius) ? ror_kernel<true> : ror_kernel<false>;
     ZIM_CUDA_TRY(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     dim3 grd((cols + RX - 1) / RX, (rows + th - 1) / th);
     kern<<<grd, RX * RY, smem, st>>>(xyz, mask, rows, cols, th, radius * radius, min_neighbors, hw, out, mask_out);

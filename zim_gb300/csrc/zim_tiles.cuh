@@ -913,8 +913,8 @@ __device__ __forceinline__ void px_gaussian_strip(const float* __restrict__ xyz,
 // sqrt(r2).  The tile and its hw halo are staged in shared memory (ror_smem_bytes)
 // as float4 with invalid and off-image pixels NaN, so a neighbour test is one
 // shared load and an FP32 distance that compares false for NaN.  The point itself
-// counts (distance 0), so the count including it must reach min_nb + 1.  Ends past
-// the last shared read.
+// counts (distance 0), so the count including it must reach min_nb + 1 (with min_nb <= 0
+// every valid point stays).  Ends past the last shared read.
 //
 // Bound by issue, staging first.  The default filter (11 x 11 window, 10 neighbours)
 // at 4185x3064: 372 us with tiles of 8 rows scanned row by row, 302 with rings, 200
@@ -928,6 +928,8 @@ __device__ __forceinline__ void px_gaussian_strip(const float* __restrict__ xyz,
 // rings settle it all are the rings' (91, 5 mm: 1.57).  Narrow windows in rings alone:
 // the second loop's registers cost the 11 x 11 filter 15 %.
 constexpr int ROR_WIDE = 10, ROR_RINGS = 6;
+// (The wide form also takes a radius whose square is infinite.)
+inline bool ror_wide(int hw, float radius) { return hw > ROR_WIDE || !(radius * radius < INFINITY); }
 __host__ __device__ inline size_t ror_smem_bytes(int hw, int th) {
     return (size_t)(RX + 2 * hw) * (th + 2 * hw) * sizeof(float4);
 }
@@ -971,7 +973,11 @@ __device__ __forceinline__ void ror_tile(const float* __restrict__ xyz, const ui
                 const float dx = c.x - p.x, dy = c.y - p.y, dz = c.z - p.z;
                 cnt += fmaf(dz, dz, fmaf(dy, dy, dx * dx)) <= r2 ? 1 : 0;
             };
-            const int nr = WIDE ? ROR_RINGS : hw;
+            if (WIDE && !(r2 < INFINITY)) {  // by its own distance, which is no number at infinity
+                cnt = 0;
+                test(c);
+            }
+            const int nr = WIDE ? min(hw, ROR_RINGS) : hw;
             for (int r = 1; r <= nr && cnt <= min_nb; r++) {
                 const float4* a = centre - r * TW - r;  // the four sides, one step each
                 const float4* b = centre + r * TW + r;
@@ -985,7 +991,7 @@ __device__ __forceinline__ void ror_tile(const float* __restrict__ xyz, const ui
                     test(*g);
                 }
             }
-            for (int i = -hw; WIDE && i <= hw && cnt <= min_nb; i++) {
+            for (int i = -hw; WIDE && nr < hw && i <= hw && cnt <= min_nb; i++) {
                 const float4* row = centre + i * TW;
                 const bool split = i >= -nr && i <= nr;
                 const int e = split ? -nr - 1 : hw;
@@ -993,7 +999,7 @@ __device__ __forceinline__ void ror_tile(const float* __restrict__ xyz, const ui
                 if (split)
                     for (int j = nr + 1; j <= hw; j++) test(row[j]);
             }
-            keep = cnt > min_nb;
+            keep = cnt > min_nb || (WIDE && min_nb <= 0);
         }
         const size_t o = (size_t)y * cols + x;
         out[3 * o] = keep ? c.x : 0.f;
