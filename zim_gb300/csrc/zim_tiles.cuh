@@ -123,40 +123,18 @@ __device__ __forceinline__ float phase_atan2(float y, float x) {
 
 // --------------------------------------------------------------- rectify ----
 
-// Post-smoothed phase at a source pixel in exact integer + FP32 form:
-// phase_s = 2*pi*K16/16 + R, K16 = sum (1 2 1)x(1 2 1) * order (BORDER_REPLICATE).
-__device__ __forceinline__ void smoothed_tap(const int32_t* __restrict__ order, const float* __restrict__ res, int x,
-                                             int y, int rows, int cols, int post_smooth, int& K16, float& R) {
-    // post_smooth 0: the tap as decoded; 3: the same for HDR decodes, whose
-    // invalid pixels (order -1) have phase 0
-    if (post_smooth == 0 || post_smooth == 3) {
-        size_t o = (size_t)y * cols + x;
-        const int k = __ldg(order + o);
-        const bool zero = post_smooth == 3 && k < 0;
-        K16 = zero ? 0 : 16 * k;
-        R = zero ? 0.f : __ldg(res + o);
-        return;
-    }
-    int k = 0;
-    float r = 0.f;
-#pragma unroll
-    for (int a = -1; a <= 1; a++) {
-        int yy = min(max(y + a, 0), rows - 1);
-        int ca = a == 0 ? 2 : 1;
-#pragma unroll
-        for (int b = -1; b <= 1; b++) {
-            int xx = min(max(x + b, 0), cols - 1);
-            int cw = ca * (b == 0 ? 2 : 1);
-            size_t o = (size_t)yy * cols + xx;
-            k += cw * __ldg(order + o);
-            r = fmaf((float)cw * 0.0625f, __ldg(res + o), r);
-        }
-    }
-    K16 = k;
-    R = r;
+// Decoded phase at source pixel o in exact integer + FP32 form: phase = 2 pi K16 / 16 +
+// R.  post_smooth 0: as decoded; 3: the same for HDR decodes, whose invalid pixels
+// (order -1) have phase 0.
+__device__ __forceinline__ void decoded_tap(const int32_t* __restrict__ order, const float* __restrict__ res, size_t o,
+                                            int post_smooth, int& K16, float& R) {
+    const int k = __ldg(order + o);
+    const bool zero = post_smooth == 3 && k < 0;
+    K16 = zero ? 0 : 16 * k;
+    R = zero ? 0.f : __ldg(res + o);
 }
 
-// setData remap of one rectified pixel: INTER_LINEAR of the (post-smoothed)
+// setData remap of one rectified pixel without post-smooth: INTER_LINEAR of the
 // phase with OpenCV's 1/32-pixel quantised weights and BORDER_CONSTANT 0,
 // INTER_NEAREST of the order.  The phase is kept as an integer cycle count
 // (exact: every weight is a multiple of 1/16384) plus an FP32 residual.
@@ -179,7 +157,7 @@ __device__ __forceinline__ void rectify_pixel(const int32_t* __restrict__ order,
         if (wq == 0) continue;
         int K16;
         float R;
-        smoothed_tap(order, res, xx, yy, srows, scols, post_smooth, K16, R);
+        decoded_tap(order, res, (size_t)yy * scols + xx, post_smooth, K16, R);
         I += (long long)wq * K16;
         Rs = fmaf((float)wq * (1.0f / 1024.0f), R, Rs);
     }
@@ -193,8 +171,8 @@ __device__ __forceinline__ void rectify_pixel(const int32_t* __restrict__ order,
 
 // Post-smooth of the decoded phase once per source pixel, so that a rectified
 // pixel reads 4 taps instead of 4 x 9: a tap is (K16, bits of R) with smoothed
-// phase = 2 pi K16 / 16 + R, exactly what smoothed_tap computes, the two words
-// together so that a tap is one load.
+// phase = 2 pi K16 / 16 + R, K16 = sum (1 2 1)x(1 2 1) * order (BORDER_REPLICATE), the
+// two words together so that a tap is one load.
 //
 // HDR (JSLAB_PhaseShiftDecoder_V2.cpp:280-291): the blurred phase divided by the
 // blurred validity (invalid pixels, order < 0, count as phase 0 with weight 0), 0
