@@ -1042,6 +1042,7 @@ __global__ void __launch_bounds__(TS_WARPS * 32) sor_tree_kernel(const float* __
                                                                  const float* __restrict__ bound,
                                                                  uint32_t* __restrict__ err) {
     constexpr int NEW = TS_LEAVES * zl::LEAF * zl::LEAF;  // entries a step may add
+    static_assert(KNN_MAX_K1 <= FW_CAP - NEW, "a tightened list has room for a step");
     __shared__ float lst[TS_WARPS][FW_CAP];
     __shared__ int2 qpos[TS_WARPS][TS_QUEUE];   // queued leaves: first pixel
     __shared__ float qd2[TS_WARPS][TS_QUEUE];   // and squared box distance
@@ -1173,10 +1174,7 @@ __global__ void __launch_bounds__(TS_WARPS * 32) sor_tree_kernel(const float* __
                             if (kp) lw[n + __popc(bb & ((1u << lane) - 1u))] = d2[g][u];
                             n += __popc(bb);
                         }
-                    if (n > FW_CAP - NEW) {
-                        if (K1 <= FW_CAP - NEW) tighten();
-                        else n = 0;
-                    }
+                    if (n > FW_CAP - NEW) tighten();
                 }
             }
             __syncwarp();
@@ -1233,7 +1231,7 @@ __global__ void __launch_bounds__(TS_WARPS * 32) sor_tree_kernel(const float* __
         flush();
         __syncwarp();
         item = next_item();
-        if (n < K1 || K1 > FW_CAP - NEW) {  // fewer than k + 1 finite points (or a k beyond the list)
+        if (n < K1) {  // fewer than k + 1 finite points
             if (lane == 0) {
                 atomicOr(err, 0x10u);
                 md_out[i] = 0.f;
