@@ -39,11 +39,17 @@ static_assert(BT == zt::DX * zt::DY && BT == zt::RX * zt::RY && BT == 32 * zt::M
 
 enum { Q_SMOOTH, Q_MATCH, Q_REPROJ, Q_PXG, Q_ROR, NQ };
 
-struct PairDev {
-    zt::DecodeParams dp;
-    zt::ReprojParams rp;
+// What a pair's decode launch takes (on the host: captured, not queued).
+struct PairDecode {
+    zt::DecodeParams p;
     int sample_type;
     const void* frames[2];
+    int32_t* order[2];
+    float* res[2];
+};
+
+struct PairDev {
+    zt::ReprojParams rp;
     const float* map[2][2];
     int rows, cols, rw, rh;
     int post_smooth, pha_f;
@@ -249,6 +255,7 @@ struct zim_batch {
     cudaGraphExec_t exec = nullptr;
     // host layout of the intermediates (for resubmission with another tuning)
     std::vector<PairDev> host_pairs;
+    std::vector<PairDecode> decodes;
     size_t items_off = 0;
     // grid filters: per pair the resolved config and its buffers (x_in / m_in:
     // the pixel stages' output; x1, x2: intermediate clouds; mls_tmp: MLS
@@ -411,8 +418,8 @@ zim_status capture(zim_batch* b) {
     const Queues& q = b->q;
     // stage 1: a launch per pair fills the GPU at every pair size
     const unsigned long long launched = ctx->launches;
-    for (const PairDev& D : b->host_pairs)
-        zim_decode_params_launch(ctx, 2, D.frames, D.sample_type, D.dp, D.order, D.res, nullptr, nullptr, s);
+    for (const PairDecode& d : b->decodes)
+        zim_decode_params_launch(ctx, 2, d.frames, d.sample_type, d.p, d.order, d.res, nullptr, nullptr, s);
     b->decode_launches = ctx->launches - launched;
     ctx->launches = launched;  // captured, not run: each replay counts them
     if (q.n[Q_SMOOTH])
@@ -686,25 +693,27 @@ extern "C" ZIM_API zim_status zim_batch_submit(zim_batch* b, const zim_batch_pai
     float w00, w01, w11;
     zt::px_gaussian_weights(w00, w01, w11);
     b->host_pairs.assign(n_pairs, PairDev{});
+    b->decodes.assign(n_pairs, PairDecode{});
     for (int i = 0; i < n_pairs; i++) {
         const zim_batch_pair& p = b->pairs[i];
         const zim_rect_state& C = b->calibs[p.calib];
         PairDev& D = b->host_pairs[i];
         std::memset(&D, 0, sizeof D);
-        zt::decode_params(&p.decode, p.rows, p.cols, D.dp);
+        PairDecode& E = b->decodes[i];
+        zt::decode_params(&p.decode, p.rows, p.cols, E.p);
+        E.sample_type = p.sample_type;
         zt::reproj_params(C.Q, C.R1, rcfg, D.rp);
-        D.sample_type = p.sample_type;
         D.rows = p.rows; D.cols = p.cols; D.rw = C.rect_w; D.rh = C.rect_h;
         D.post_smooth = p.decode.enable_hdr ? (p.decode.post_smooth ? 2 : 3) : (p.decode.post_smooth ? 1 : 0);
         D.pha_f = p.pha_f > 0 ? p.pha_f : zim_decode_max_order(&p.decode);
         D.grad_threshold = (float)rcfg->grad_threshold;
         const size_t src = (size_t)p.rows * p.cols, dst = (size_t)C.rect_w * C.rect_h;
         for (int c = 0; c < 2; c++) {
-            D.frames[c] = p.frames[c];
             D.map[c][0] = C.d_map[c][0];
             D.map[c][1] = C.d_map[c][1];
-            D.order[c] = (int32_t*)take(src * 4);
-            D.res[c] = (float*)take(src * 4);
+            E.frames[c] = p.frames[c];
+            E.order[c] = D.order[c] = (int32_t*)take(src * 4);
+            E.res[c] = D.res[c] = (float*)take(src * 4);
             if (p.decode.post_smooth) {
                 D.taps[c] = (int2*)take(src * 8);
             }
