@@ -990,6 +990,8 @@ constexpr int FW_CAP = 256;  // tree search: list entries per warp (8 per lane)
 constexpr int TS_QUEUE = 256;  // tree search: queued leaves per warp
 constexpr int TS_NODES = 2;  // tree search: nodes whose leaves are tested together
 constexpr int TS_LEAVES = 2;  // tree search: leaves read together (at most 128 new entries)
+constexpr int TS_AROUND = 7;  // tree search: leaves on either side of the query's own that bound it
+static_assert((2 * TS_AROUND + 1) * (2 * TS_AROUND + 1) <= FW_CAP && FW_CAP <= TS_QUEUE, "lists of the leaves around");
 
 // Smallest list value v with at least K entries <= v (entries: lane j holds
 // keys[r], 0xffffffff = empty; keys are non-negative float bits).  Bisection on
@@ -1017,9 +1019,10 @@ __device__ __forceinline__ unsigned warp_kth_key(const unsigned (&keys)[FW_CAP /
 
 // Tree search: one warp per deferred query.  The warp keeps the squared
 // distances below its bound in a list; the bound starts at the window pass's
-// (the largest it holds) or, without one, at the farthest corner of the
-// nearest-cornered node and then leaf that holds k + 1 points, and tightens to
-// the (k + 1)-th smallest held whenever the list fills.  With pixel rays the
+// (the largest it holds) or, without one, at the nearest farthest corners of
+// leaves around the query's own that hold k + 1 points together (7 x 7, then 15 x
+// 15; else of the nearest-cornered node and then leaf that holds k + 1), and tightens
+// to the (k + 1)-th smallest held whenever the list fills.  With pixel rays the
 // bound also limits the search to a rectangle of pixels (the window pass's ray
 // bound with the cloud's largest ray distance).  Nodes, then their leaves, then
 // the leaves' pixels are read only where the box lies below the bound.  Work is
@@ -1030,8 +1033,11 @@ __device__ __forceinline__ unsigned warp_kth_key(const unsigned (&keys)[FW_CAP /
 // (5 MP: 47 thousand cycles on average, 230 thousand the longest).  So the leaves
 // of two nodes are tested together, a leaf of k + 1 points bounds the search
 // before any pixel is read, leaves are queued and read two at a time, and no index
-// is divided.  5 MP, k = 30: 105 -> 83 us; 640 x 480, k = 50: 63 -> 22.  Reading four or eight leaves at a time
-// or testing four nodes is no faster (a longer list costs each selection more).
+// is divided.  5 MP, k = 30: 105 -> 83 us; 640 x 480, k = 50: 63 -> 22.  Reading four
+// or eight leaves at a time or testing four nodes is no faster (a longer list costs
+// each selection more).  Where one pixel in ten holds a point no leaf has k + 1, and a
+// node's far corner admits a hundred leaves: 1626 x 1236, k = 30, 2.89 ms with the
+// nodes' bound alone (the coarse grid 1.57), 1.24 with that of the leaves around.
 // The search took the place of a counting-sorted coarse grid with a ring search
 // and an occupied-cell search, whose build alone was eleven launches.
 __global__ void __launch_bounds__(TS_WARPS * 32) sor_tree_kernel(const float* __restrict__ xyz,
@@ -1077,23 +1083,57 @@ __global__ void __launch_bounds__(TS_WARPS * 32) sor_tree_kernel(const float* __
         if (md_out[i] == MD_BOUND) {
             thr = above(b0);
         } else {
-            unsigned long long best = ~0ull;  // (distance bits, node)
-            for (int n0 = lane; n0 < t.nw * t.nh; n0 += 32) {
-                const zl::Box b = zl::load_box(t.node, n0);
-                if (b.n < (unsigned)K1) continue;
-                const float f = zl::far_d2(b, q);
-                if (f < INFINITY) best = min(best, (unsigned long long)__float_as_uint(f) << 32 | (unsigned)n0);
-            }
-            for (int off = 16; off; off >>= 1) best = min(best, __shfl_xor_sync(full, best, off));
-            if (best != ~0ull) {
-                unsigned fb = (unsigned)(best >> 32);
-                for (int c = lane; c < zl::FAN * zl::FAN; c += 32) {
-                    const int l = zl::child_leaf(t, (int)(unsigned)best, c);
-                    if (l < 0) continue;
-                    const zl::Box b = zl::load_box(t.leaf, l);
-                    if (b.n >= (unsigned)K1) fb = min(fb, __float_as_uint(zl::far_d2(b, q)));
+            // the farthest corners of the leaves around the query's own that hold k + 1
+            // points: the nearest such set, to 2^-7 of its squared distance
+            bool bounded = false;
+            const int qlx = (int)(i % (unsigned)cols) / zl::LEAF, qly = (int)(i / (unsigned)cols) / zl::LEAF;
+            for (int R = 3; R <= TS_AROUND && !bounded; R += TS_AROUND - 3) {
+                const int lx0 = max(qlx - R, 0), lx1 = min(qlx + R, t.lw - 1);
+                const int ly0 = max(qly - R, 0), ly1 = min(qly + R, t.lh - 1), lnx = lx1 - lx0 + 1;
+                const int m = lnx * (ly1 - ly0 + 1);  // at most (2 TS_AROUND + 1)^2
+                unsigned held = 0u, hi = 0u, lo = 0u;
+                for (int e = lane; e < m; e += 32) {
+                    const zl::Box b = zl::load_box(t.leaf, (ly0 + e / lnx) * t.lw + lx0 + e % lnx);
+                    const unsigned f = b.n ? __float_as_uint(zl::far_d2(b, q)) : 0x7f800000u;
+                    const unsigned c = f < 0x7f800000u ? b.n : 0u;
+                    lw[e] = __uint_as_float(f);
+                    qpos[w][e].x = (int)c;
+                    held += c;
+                    hi = max(hi, c ? f : 0u);
                 }
-                thr = above(__uint_as_float(__reduce_min_sync(full, fb)));
+                bounded = __reduce_add_sync(full, held) >= (unsigned)K1;
+                if (bounded) {
+                    hi = __reduce_max_sync(full, hi);
+                    while (hi - lo > 0x10000u) {
+                        const unsigned mid = lo + ((hi - lo) >> 1);
+                        unsigned c = 0u;
+                        for (int e = lane; e < m; e += 32) c += __float_as_uint(lw[e]) <= mid ? (unsigned)qpos[w][e].x : 0u;
+                        if (__reduce_add_sync(full, c) >= (unsigned)K1) hi = mid;
+                        else lo = mid + 1;
+                    }
+                    thr = above(__uint_as_float(hi));
+                }
+                __syncwarp();
+            }
+            if (!bounded) {
+                unsigned long long best = ~0ull;  // (distance bits, node)
+                for (int n0 = lane; n0 < t.nw * t.nh; n0 += 32) {
+                    const zl::Box b = zl::load_box(t.node, n0);
+                    if (b.n < (unsigned)K1) continue;
+                    const float f = zl::far_d2(b, q);
+                    if (f < INFINITY) best = min(best, (unsigned long long)__float_as_uint(f) << 32 | (unsigned)n0);
+                }
+                for (int off = 16; off; off >>= 1) best = min(best, __shfl_xor_sync(full, best, off));
+                if (best != ~0ull) {
+                    unsigned fb = (unsigned)(best >> 32);
+                    for (int c = lane; c < zl::FAN * zl::FAN; c += 32) {
+                        const int l = zl::child_leaf(t, (int)(unsigned)best, c);
+                        if (l < 0) continue;
+                        const zl::Box b = zl::load_box(t.leaf, l);
+                        if (b.n >= (unsigned)K1) fb = min(fb, __float_as_uint(zl::far_d2(b, q)));
+                    }
+                    thr = above(__uint_as_float(__reduce_min_sync(full, fb)));
+                }
             }
         }
         // the nodes of the rectangle of pixels that can hold a point below thr
