@@ -1466,15 +1466,35 @@ __global__ void __launch_bounds__(GB) sor_classify_kernel(const float* __restric
 // The window fast path: the points within r of a query, summed row by row over
 // the disk of its window out to the pixel distance beyond which the ray bound
 // puts every point farther than r (see sor_window_kernel).  The queries it
-// cannot certify are left as set bits of `pending` (one word per warp: 16 x 2
-// pixels) for metric_gaussian_tree_kernel.
+// cannot certify are left to metric_gaussian_tree_kernel: a list of (word, its set
+// bits), a word being a warp's 16 x 2 pixels.
 constexpr int WRG = WR;
 constexpr int GW = WT_X + 2 * WRG, GH = WT_Y + 2 * WRG;
+
+// Appends this warp's word of the tile to the list if any bit is set.
+__device__ __forceinline__ void list_word(uint2* __restrict__ list, zl::Head* h, unsigned tile, int tid, unsigned word) {
+    if ((tid & 31) == 0 && word)
+        list[atomicAdd(&h->n_deferred, 1u)] = make_uint2(tile * (WT_T / 32) + (tid >> 5), word);
+}
+
+// Without pixel rays every valid point is listed; the others pass through.
+__global__ void __launch_bounds__(WT_T) mg_list_kernel(const float* __restrict__ xyz, const uint8_t* __restrict__ mask,
+                                                       int rows, int cols, unsigned tiles_x, zl::Tree t,
+                                                       uint2* __restrict__ list, float* __restrict__ out) {
+    const int tid = threadIdx.x;
+    const int x = (int)(blockIdx.x % tiles_x) * WT_X + tid % WT_X, y = (int)(blockIdx.x / tiles_x) * WT_Y + tid / WT_X;
+    const bool in = x < cols && y < rows;
+    const size_t i = in ? (size_t)y * cols + x : 0;
+    const bool left = in && mask[i];
+    list_word(list, t.head, blockIdx.x, tid, __ballot_sync(0xffffffffu, left));
+    if (in && !left)
+        for (int a = 0; a < 3; a++) out[3 * i + a] = xyz[3 * i + a];
+}
 
 __global__ void __launch_bounds__(WT_T) mg_window_kernel(const float* __restrict__ xyz,
                                                            const uint8_t* __restrict__ mask, int rows, int cols,
                                                            float r, float inv2s2, RayParams rp,
-                                                           zl::Tree t, unsigned* __restrict__ pending,
+                                                           zl::Tree t, uint2* __restrict__ list,
                                                            float* __restrict__ out) {
     __shared__ float4 W[GW * GH];
     const int tid = threadIdx.x;
@@ -1524,10 +1544,7 @@ __global__ void __launch_bounds__(WT_T) mg_window_kernel(const float* __restrict
     const float ro = (float)(WRG + 1);
     const bool left = q.w != 0.f && (!(rs < ro) || !(C * ro / (an + ro) - dev_out > r));
     const unsigned word = __ballot_sync(0xffffffffu, left);
-    if ((tid & 31) == 0) {
-        pending[((size_t)blockIdx.y * gridDim.x + blockIdx.x) * (WT_T / 32) + (tid >> 5)] = word;
-        if (word) atomicAdd(&t.head->n_deferred, (unsigned)__popc(word));
-    }
+    list_word(list, t.head, blockIdx.y * gridDim.x + blockIdx.x, tid, word);
     if (!in || left) return;
     if (q.w == 0.f) {  // invalid points pass through
         out[3 * i] = xyz[3 * i];
@@ -1567,46 +1584,40 @@ __global__ void __launch_bounds__(WT_T) mg_window_kernel(const float* __restrict
     out[3 * i + 2] = q.z + sz * iw;
 }
 
-// Queries over the tree's leaves, a warp per word of 16 x 2 pixels (pending null:
-// every pixel is a query, invalid ones pass through): the boxes within r of the
-// warp's queries pick the leaves, whose 64 points go through shared memory, each
-// lane summing those within r of its own query.  64-bit fixed-point sums (each
-// term rounded on its own): the result does not depend on the visiting order.
-// When the window pass left nothing, the launch costs one wave of blocks that
-// return at once (the hash grid it replaced took ten gated launches: 102 -> 63 us
-// for a 1280 x 1024 cloud).  With every query left to it (no pixel rays) a
-// 2448 x 2048 cloud takes 7.3 ms at sigma 0.5 and 29 ms at 1.5, against 8.4 and
-// 46 ms with the grid.
+// Queries over the tree's leaves, a warp per listed word of 16 x 2 pixels: the box of
+// the warp's queries picks the leaves and their points within r of it, which go through
+// shared memory, each lane summing those within r of its own query.  64-bit fixed-point
+// sums (each term rounded on its own): the result depends neither on the visiting order
+// nor on the list's.  When nothing is listed, the launch costs one wave of blocks that
+// return at once (the hash grid it replaced took ten gated launches: 102 -> 63 us for
+// a 1280 x 1024 cloud).  With every query left to it (no pixel rays) a 2448 x 2048
+// cloud takes 6.1 ms at sigma 0.5 and 14 ms at 1, against 10 and 29 ms with the grid.
+//
+// A cloud after the pixel Gaussian has its rejected pixels valid at the origin, all
+// within r of each other, and most of them on the image's border: a few lanes of some
+// words with thousands of neighbours.  So the words are listed, which spreads them over
+// the SMs (strided, the border tiles of a 1024-pixel image fall to one block in 64), and
+// only the points near the queries' box are summed over, not a leaf's 64 pixels: such a
+// 1024 x 768 cloud 9.2 -> 2.7 ms (the grid: 5.7).
 constexpr int MT_WARPS = 8;
 __global__ void __launch_bounds__(MT_WARPS * 32) metric_gaussian_tree_kernel(
     const float* __restrict__ xyz, const uint8_t* __restrict__ mask, int rows, int cols, float r2, float inv2s2,
-    zl::Tree t, const unsigned* __restrict__ pending, float* __restrict__ out) {
-    if (pending && t.head->n_deferred == 0u) return;
+    zl::Tree t, const uint2* __restrict__ list, float* __restrict__ out) {
+    const unsigned words = t.head->n_deferred;
     __shared__ float4 pts[MT_WARPS][zl::LEAF * zl::LEAF];
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     float4* pw = pts[w];
-    const int tiles_x = (cols + WT_X - 1) / WT_X, tiles_y = (rows + WT_Y - 1) / WT_Y;
-    const long long words = (long long)tiles_x * tiles_y * (WT_T / 32);
+    const unsigned tiles_x = (cols + WT_X - 1) / WT_X;
     const int nn = t.nw * t.nh;
     const float r = sqrtf(r2), sc = 1099511627776.0f / r;  // 2^40 / r
-    for (long long wd = (long long)blockIdx.x * MT_WARPS + w; wd < words; wd += (long long)gridDim.x * MT_WARPS) {
-        const long long tile = wd / (WT_T / 32);
+    for (unsigned item = blockIdx.x * MT_WARPS + w; item < words; item += gridDim.x * MT_WARPS) {
+        const uint2 e = list[item];
+        const unsigned tile = e.x / (WT_T / 32);
         const int x = (int)(tile % tiles_x) * WT_X + (lane & 15);
-        const int y = (int)(tile / tiles_x) * WT_Y + (int)(wd % (WT_T / 32)) * 2 + (lane >> 4);
-        const bool in = x < cols && y < rows;
-        const size_t i = in ? (size_t)y * cols + x : 0;
-        bool act;
-        if (pending) {
-            const unsigned word = pending[wd];
-            if (!word) continue;
-            act = word >> lane & 1u;
-        } else {
-            act = in && mask[i];
-            if (in && !act)
-                for (int a = 0; a < 3; a++) out[3 * i + a] = xyz[3 * i + a];
-            if (!__any_sync(full, act)) continue;
-        }
+        const int y = (int)(tile / tiles_x) * WT_Y + (int)(e.x % (WT_T / 32)) * 2 + (lane >> 4);
+        const bool act = e.y >> lane & 1u;
+        const size_t i = act ? (size_t)y * cols + x : 0;
         float q[3] = {0.f, 0.f, 0.f}, lo[3], hi[3];
 #pragma unroll
         for (int a = 0; a < 3; a++) {
@@ -1622,10 +1633,8 @@ __global__ void __launch_bounds__(MT_WARPS * 32) metric_gaussian_tree_kernel(
                 const zl::Box b = zl::load_box(t.node, n0 + lane);
                 hit = b.n && zl::gap_d2(b, lo, hi) <= r2;
             }
-            unsigned nm = __ballot_sync(full, hit);
-            while (nm) {
+            for (unsigned nm = __ballot_sync(full, hit); nm; nm &= nm - 1) {
                 const int nb = n0 + __ffs(nm) - 1;
-                nm &= nm - 1;
 #pragma unroll 1
                 for (int h = 0; h < 2; h++) {
                     const int ll = zl::child_leaf(t, nb, lane + 32 * h);
@@ -1634,29 +1643,28 @@ __global__ void __launch_bounds__(MT_WARPS * 32) metric_gaussian_tree_kernel(
                         const zl::Box b = zl::load_box(t.leaf, ll);
                         lhit = b.n && zl::gap_d2(b, lo, hi) <= r2;
                     }
-                    unsigned lm = __ballot_sync(full, lhit);
-                    while (lm) {
+                    for (unsigned lm = __ballot_sync(full, lhit); lm; lm &= lm - 1) {
                         const int l = __shfl_sync(full, ll, __ffs(lm) - 1);
-                        lm &= lm - 1;
                         const int px = (l % t.lw) * zl::LEAF + (lane & 7), py = (l / t.lw) * zl::LEAF + (lane >> 3);
+                        // the leaf's points within r of the queries' box
+                        int np = 0;
                         __syncwarp();
 #pragma unroll
                         for (int u = 0; u < 2; u++) {
-                            const float nan = __int_as_float(0x7fc00000);  // invalid: its distance test fails
-                            float4 v = make_float4(nan, nan, nan, 0.f);
-                            const int yy = py + 4 * u;
-                            if (px < cols && yy < rows) {
-                                const size_t j = (size_t)yy * cols + px;
-                                if (__ldg(mask + j))
-                                    v = make_float4(__ldg(xyz + 3 * j), __ldg(xyz + 3 * j + 1), __ldg(xyz + 3 * j + 2), 0.f);
-                            }
-                            pw[lane + 32 * u] = v;
+                            const bool in = px < cols && py + 4 * u < rows;
+                            const size_t j = in ? (size_t)(py + 4 * u) * cols + px : 0;
+                            const float vx = __ldg(xyz + 3 * j), vy = __ldg(xyz + 3 * j + 1), vz = __ldg(xyz + 3 * j + 2);
+                            const bool v = in && __ldg(mask + j) != 0 &&
+                                           zl::gap_d2(zl::Box{{vx, vy, vz}, {vx, vy, vz}, 1u}, lo, hi) <= r2;
+                            const unsigned bb = __ballot_sync(full, v);
+                            if (v) pw[np + __popc(bb & ((1u << lane) - 1u))] = make_float4(vx, vy, vz, 0.f);
+                            np += __popc(bb);
                         }
                         __syncwarp();
                         if (act)
 #pragma unroll 4
-                            for (int e = 0; e < zl::LEAF * zl::LEAF; e++) {
-                                const float4 p = pw[e];
+                            for (int k = 0; k < np; k++) {
+                                const float4 p = pw[k];
                                 const float dx = p.x - q[0], dy = p.y - q[1], dz = p.z - q[2];
                                 const float d2 = sqdist(dx, dy, dz);
                                 if (!(d2 <= r2)) continue;
@@ -1744,8 +1752,8 @@ zim_status build_grid(zim_ctx* ctx, const float* xyz, const uint8_t* mask, int r
     return ZIM_OK;
 }
 
-// Words of the metric Gaussian's pending bits.
-size_t pending_words(int rows, int cols) {
+// Words of the metric Gaussian's list.
+size_t mg_words(int rows, int cols) {
     return (size_t)((cols + WT_X - 1) / WT_X) * ((rows + WT_Y - 1) / WT_Y) * (WT_T / 32);
 }
 
@@ -1753,12 +1761,12 @@ size_t pending_words(int rows, int cols) {
 
 // Scratch of the filters of one cloud (they carve it in turn): SOR's statistics,
 // mean distances, deferred queries and bounds, the tree, and without pixel rays
-// the grid; the metric Gaussian needs less (the tree and its pending bits).
+// the grid; the metric Gaussian needs less (the tree and its list).
 size_t zim_grid_scratch_bytes(int rows, int cols, bool rays) {
     const size_t n = (size_t)rows * cols;
     return zim_leaf_bytes(rows, cols) + zim_align256(sizeof(GridStats)) + 3 * zim_align256(n * 4) +
            zim_align256((size_t)SOR_STAT_BLOCKS * 2 * sizeof(double)) + (rays ? 0 : grid_bytes(n)) +
-           zim_align256(pending_words(rows, cols) * 4);
+           zim_align256(mg_words(rows, cols) * sizeof(uint2));
 }
 
 zim_status zim_sor_launch(zim_ctx* ctx, const float* xyz, const uint8_t* mask, int rows, int cols, int mean_k,
@@ -1829,19 +1837,18 @@ zim_status zim_metric_gaussian_launch(zim_ctx* ctx, const float* xyz, const uint
     s = zim_leaf_build(ctx, xyz, mask, rows, cols, rays.valid ? &rp : nullptr, t, st);
     if (s) return s;
     const float inv2s2 = (float)(1.0 / (2.0 * sigma * sigma));
-    unsigned* pending = nullptr;
-    if (rays.valid) {
-        pending = (unsigned*)zim_scratch_take(ctx, pending_words(rows, cols) * 4);
-        if (!pending) return zim_fail(ctx, ZIM_ERR_OUT_OF_MEMORY, "metric Gaussian scratch carve");
-        const dim3 tgrid((cols + WT_X - 1) / WT_X, (rows + WT_Y - 1) / WT_Y);
-        mg_window_kernel<<<tgrid, WT_T, 0, st>>>(xyz, mask, rows, cols, rad, inv2s2, rp, t, pending, out);
-        ctx->launches += 1;
-    }
-    const size_t blocks = (pending_words(rows, cols) + MT_WARPS - 1) / MT_WARPS;
-    const unsigned mblk = (unsigned)std::min<size_t>(blocks, 8 * (ctx->sm_count > 0 ? ctx->sm_count : 152));
-    metric_gaussian_tree_kernel<<<mblk, MT_WARPS * 32, 0, st>>>(xyz, mask, rows, cols, rad * rad, inv2s2, t, pending,
-                                                                out);
-    ctx->launches += 1;
+    const size_t words = mg_words(rows, cols);
+    uint2* list = (uint2*)zim_scratch_take(ctx, words * sizeof(uint2));
+    if (!list) return zim_fail(ctx, ZIM_ERR_OUT_OF_MEMORY, "metric Gaussian scratch carve");
+    const dim3 tgrid((cols + WT_X - 1) / WT_X, (rows + WT_Y - 1) / WT_Y);
+    if (rays.valid)
+        mg_window_kernel<<<tgrid, WT_T, 0, st>>>(xyz, mask, rows, cols, rad, inv2s2, rp, t, list, out);
+    else
+        mg_list_kernel<<<tgrid.x * tgrid.y, WT_T, 0, st>>>(xyz, mask, rows, cols, tgrid.x, t, list, out);
+    const unsigned mblk = (unsigned)std::min<size_t>((words + MT_WARPS - 1) / MT_WARPS,
+                                                     8 * (ctx->sm_count > 0 ? ctx->sm_count : 152));
+    metric_gaussian_tree_kernel<<<mblk, MT_WARPS * 32, 0, st>>>(xyz, mask, rows, cols, rad * rad, inv2s2, t, list, out);
+    ctx->launches += 2;
     ZIM_LAUNCH_CHECK(ctx);
     return ZIM_OK;
 }
