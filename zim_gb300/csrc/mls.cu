@@ -486,8 +486,9 @@ __global__ void __launch_bounds__(MX* MY) mls_smem_kernel(const float* __restric
 // of the points around gives it a pixel radius, and a warp walks the disk of its
 // largest.  The neighbours and their order are those of the full window.
 //
-// Half-windows up to MLS_R: the window's tile is staged whole, and its ray
-// distances are taken on the way.  Above, they come from the leaves (zim_leaf.cuh):
+// Half-windows up to MLS_R (and wider ones of small clouds, mls_near): the window's
+// tile is staged whole, and its ray distances are taken on the way.  Above, they come
+// from the leaves (zim_leaf.cuh):
 // with those of the whole window, then with those within the tile's largest radius,
 // and only that radius is staged; tiles that need more than MLS_R pixels are left
 // to mls_wide_kernel.  The default parameters (30 pixels, three passes) on a
@@ -758,7 +759,7 @@ static bool mls_near(int sms, int rows, int cols, int hw) {
     if (hw <= MLS_R) return true;
     const size_t smem = mls_smem_bytes(hw), tiles = mls_tiles(rows, cols);
     if (smem > MLS_SMEM) return false;
-    if (hw > 24) return tiles <= (size_t)sms / 12;
+    if (hw > 24) return tiles <= (size_t)sms / 4;
     return tiles <= (size_t)sms * std::min<size_t>(8, MLS_SM / (smem + 2048));
 }
 
