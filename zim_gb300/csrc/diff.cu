@@ -418,9 +418,11 @@ __global__ void __launch_bounds__(DIFF_T, BWD ? (UP ? DIFF_UP : DIFF_BWD) : DIFF
 #pragma unroll 4
                     for (int p = 0; p < 16; p++)
                         g[0].add(terms[wib][(p & 3) | (p & 12) << 1 | (lane & 16) >> 2][lane & 15]);
-                    g[0].normalise();
                 }
-                if (n_sets == 3) add_sets();
+                if (n_sets == 3) {
+                    add_sets();
+                    if (!UP) g[0].normalise();
+                }
                 __syncwarp();
             }
             i += di;
