@@ -522,7 +522,7 @@ def run_diff(api, local, steps, warmup, want_cpu=True):
            "forward_ms": round(fwd_ms, 3), "forward_adjoint_ms": round(bwd_ms, 3),
            "rematch_ms": round(match_ms, 3),
            "forward_adjoint_mpoints_s": round(r["n_points"] / (bwd_ms * 1e-3) / 1e6, 2),
-           "reductions": "FP64, fixed order (bit-reproducible)"}
+           "reductions": "float pairs per thread, FP64 across threads, fixed order (bit-reproducible)"}
     if want_cpu:
         one = diff.backward(ctx, th, views[:1])
         o, dt = cpu_diff_baseline(specs[0], ctx, poses[0], th)

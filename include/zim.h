@@ -23,7 +23,9 @@
  * which keeps 1e-6 rad resolution at hundreds of fringe periods in FP32.
  * Errors: every call returns a zim_status; nothing throws across the ABI;
  * zim_last_error() describes the last failure on that context.
- * Threading: one context per host thread; a context is not re-entrant.
+ * Threading: one context per host thread; a context is not re-entrant.  Calls on
+ * one context share its scratch (a single MLS pass, too, keeps its tree there with
+ * half-windows above 12): give them one stream, or order them yourself.
  */
 #ifndef ZIM_H
 #define ZIM_H
@@ -408,7 +410,7 @@ ZIM_API zim_status zim_reconstruct_pair_host_async(zim_ctx* ctx, const zim_decod
  * median, reprojection, 3x3 Gaussian and radius outlier filter, then the grid
  * filters (SOR -> MLS -> metric Gaussian) that the pair's filter config turns
  * on (zim_batch_pair.filters, or the submission's config).
- * Execution: a decode launch per pair, then one persistent kernel per
+ * Execution: a decode launch per pair (both cameras), then one persistent kernel per
  * pixel-domain stage drains a device work queue of (pair, row band) items over
  * all pairs (post-smooth; rectify fused into match; median + reprojection; each
  * pixel filter); then the pairs' grid
@@ -521,9 +523,10 @@ typedef struct zim_diff_view {
     float* grad_phase[2];
 } zim_diff_view;
 
-/* Sums over all views, reduced in FP64 in a fixed order (bit-reproducible):
- * loss, points used, the gradient of loss_weight * loss (+ the grad_xyz
- * terms) and J^T J of the point-to-plane distances (Gauss-Newton). */
+/* Sums over all views in a fixed order (bit-reproducible): loss, points used, the
+ * gradient of loss_weight * loss (+ the grad_xyz terms) and J^T J of the
+ * point-to-plane distances (Gauss-Newton).  The loss is summed in FP64; a thread sums
+ * its FP32 terms of the others in pairs of floats, and the threads' sums add in FP64. */
 typedef struct zim_diff_result {
     double loss;
     double n_points;

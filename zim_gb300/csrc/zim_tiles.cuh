@@ -327,7 +327,7 @@ __device__ __forceinline__ void match_pixel(int j, int k, int bL, float rL, cons
     if (s_bad && !s_bad[k] && abs(s_ph[lo].x - bL) < 1024 && abs(s_ph[hi].x - bL) < 1024) {
         // d rises strictly: the sign change between adjacent columns a and b.  The
         // phase is close to linear over a span, so the first probe interpolates
-        // and the next tries its neighbour; from the third on the bracket halves.
+        // and the next two try the neighbour; from the fourth on the bracket halves.
         int a = lo, b = hi;
         float da = diff(a), db = diff(b);
         if (!(da < 0.f) || db < 0.f) {

@@ -145,7 +145,7 @@ class Reconstruct(torch.autograd.Function):
     theta: (16,) float64 CPU tensor; residuals: device float32 phase residuals
     (phase = 2 pi order + residual).  points: (rect_h, rect_w, 3) float32 on the
     device, 0 where excluded.  The backward takes dLoss/dpoints and returns the
-    gradient for theta (FP64 reduction) and for both residual maps."""
+    gradient for theta (FP64 across threads) and for both residual maps."""
 
     @staticmethod
     def forward(fctx, theta, residual_l, residual_r, ctx, order_l, order_r, best_col, z_min=0.0, z_max=1e4):
