@@ -62,7 +62,7 @@ def env_rank():
 # DRAM bytes per launch (read + write) of a stage's kernel on the 5 MP
 # workload, from one ncu capture (profiles/pair_5mp_kernels.md): the
 # roofline's `traffic` for that kernel when it dominates the step.
-MEASURED_TRAFFIC = {("mls", 2448, 2048): (68081664 + 25512704, "profiles/pair_5mp_kernels.md")}
+MEASURED_TRAFFIC = {("mls", 2448, 2048): (68378624 + 25504000, "profiles/pair_5mp_kernels.md")}
 # Warp instructions per launch and the FMA pipe's busy fraction of a stage's
 # kernel on the 5 MP workload, from the same capture: the
 # issue-slot side of the roofline for kernels bound by instruction issue.

@@ -28,7 +28,9 @@ __global__ void __launch_bounds__(32 * zt::MED_WARPS, 3) median_reproject_kernel
 constexpr int PXG_WARPS = 4;
 constexpr size_t ROR_SMEM = 52 * 1024;  // shared memory of a radius-filter tile taller than RY rows
 // Rows of a radius-filter tile: tall tiles stage less halo per point, but few of them
-// end in a nearly empty wave.
+// end in a nearly empty wave.  us, with this rule / with 32 rows throughout: 11 x 11,
+// nobody with enough neighbours, 1024 x 768 46.5 / 51.7; 21 x 21 155 / 197; the
+// default filter 1280 x 1024 30.2 / 35.8.
 inline int ror_rows(int sms, int rows, int cols, int hw) {
     int th = 32;
     auto blocks = [&](int th) { return (long long)((cols + RX - 1) / RX) * ((rows + th - 1) / th); };
